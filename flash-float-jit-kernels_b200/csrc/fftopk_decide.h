@@ -53,8 +53,50 @@ FFTOPK_DECIDE_HD uint32_t sample_upper_rank(uint32_t k, uint32_t n_s, float len)
 // factor * k row elements (estimated from the bin's share of the sample).
 FFTOPK_DECIDE_HD bool sample_bin_too_coarse(uint32_t bin_count, uint32_t sample_total, float len, uint32_t k,
                                             float factor) {
-  const float in_bin = (float)bin_count * len / (float)(sample_total ? sample_total : 1u);
-  return in_bin > factor * (float)k;
+  // (no division: one thread of a CTA decides this while the others wait)
+  return (float)bin_count * len > factor * (float)k * (float)(sample_total ? sample_total : 1u);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Sample digit: a monotone map of the float's bits onto 4096 bins that is fine where logits live, and
+// costs six integer instructions. Magnitudes in [2^-16, 2^16) get 64 bins per octave (bits [30:17]),
+// for either sign; smaller ones share the two bins around zero, larger ones (and NaN) the outermost
+// two. A bin then holds about 1/64 octave of values: the guess made on it admits few elements beyond
+// the sampling margin (a plain 12-bit digit has 8 bins per octave, which on crowded rows - sums over
+// heads, all of one sign and magnitude - costs thousands of extra candidates or a second look).
+// The sample only makes a guess that is checked afterwards: where NaN and -0 fall is of no concern.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSampleBins = 4096;
+constexpr int kSampleShift = 17;
+constexpr int32_t kSampleBase = 111 << 23;              // 2^-16
+constexpr int32_t kSampleSpan = (32 << 23) - 1;         // 32 octaves
+FFTOPK_DECIDE_HD uint32_t sample_digit(uint32_t bits) {
+  const int32_t sign = (int32_t)bits >> 31;
+  int32_t d = (int32_t)(bits & 0x7fffffffu) - kSampleBase;
+#if defined(__CUDA_ARCH__)
+  d = __vimin_s32_relu(d, kSampleSpan);
+#else
+  d = d < 0 ? 0 : (d < kSampleSpan ? d : kSampleSpan);
+#endif
+  return (uint32_t)(((d >> kSampleShift) ^ sign) + kSampleBins / 2);
+}
+// the smallest key of a bin (a bin ends where the next one starts; the last one holds every key above)
+FFTOPK_DECIDE_HD uint32_t sample_digit_low(uint32_t bin) {
+  if (bin >= (uint32_t)kSampleBins / 2) {
+    const uint32_t e = bin - kSampleBins / 2;
+    return 0x80000000u | (e == 0u ? 0u : (uint32_t)kSampleBase + (e << kSampleShift));
+  }
+  const uint32_t e = kSampleBins / 2 - 1 - bin;  // magnitudes [e, e + 1) of the negative side
+  return e == (uint32_t)kSampleBins / 2 - 1 ? 0u : ~(0x80000000u | ((uint32_t)kSampleBase + ((e + 1u) << kSampleShift))) + 1u;
+}
+FFTOPK_DECIDE_HD uint32_t sample_digit_high(uint32_t bin) {
+  return bin == (uint32_t)kSampleBins - 1 ? 0xffffffffu : sample_digit_low(bin + 1u) - 1u;
+}
+
+// A guess whose share of the sample stands for a quarter more row elements than there is room for is
+// given up before the row is read for it (rows with thousands of copies of one value).
+FFTOPK_DECIDE_HD bool sample_admits_too_much(uint32_t admitted, uint32_t sample_total, float len, uint32_t room) {
+  return (float)admitted * len > 1.25f * (float)room * (float)(sample_total ? sample_total : 1u);
 }
 
 // The finer sample histogram (key bits [27:16]) may replace the coarse one (bits [31:20]) only if

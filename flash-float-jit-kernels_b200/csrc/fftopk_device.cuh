@@ -26,6 +26,7 @@ constexpr int kMaxCluster = 16;        // CTAs per row (non-portable cluster siz
 #endif
 constexpr int kSmall = FFTOPK_KSMALL;            // undecided candidates that are ranked directly instead of another radix round
 constexpr unsigned kFull = 0xffffffffu;
+static_assert(kSampleBins <= kMaxBins, "a sample histogram fits the bins of a distributed round");
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
@@ -67,6 +68,77 @@ __device__ __forceinline__ uint32_t atom_shared_add(uint32_t* p, uint32_t v) {
   uint32_t old;
   asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
   return old;
+}
+
+// The same for plain accesses, and with the address as the 32-bit shared-memory address it is: a
+// pointer whose address space the compiler has lost costs 64-bit address arithmetic and a generic
+// load or store. In passes that every warp of an SM makes at once (8 issue cycles per instruction with
+// 32 warps) that is most of the time.
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint64_t lds64(uint32_t a) {
+  uint64_t v;
+  asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64x2(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t lo, uint32_t hi) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(lo), "r"(hi) : "memory");
+}
+__device__ __forceinline__ void sts_zero16(uint32_t a) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(a), "r"(0) : "memory");
+}
+// A peer CTA's shared memory: the address of what lies at `a` here in the CTA of rank `r`, and stores to it.
+__device__ __forceinline__ uint32_t peer_smem(uint32_t a, int r) {
+  uint32_t v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(r));
+  return v;
+}
+__device__ __forceinline__ void st_peer32(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void st_peer64(uint32_t a, uint64_t v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
+__device__ __forceinline__ void red_shared_inc(uint32_t a) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(a) : "memory"); }
+
+// Predicated steps of the passes over candidates, spelled out. Left to the compiler, `if (c > t) ... else
+// if ...` over four candidates became a tree of branches whose lanes came together only behind the
+// last of them: up to 81 paths, one after the other (2,300 cycles for counting four candidates per
+// lane; 300 like this).
+__device__ __forceinline__ void count_if_above(uint32_t& n, uint64_t c, uint64_t thr, uint32_t add) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.u64 p, %1, %2;\n\t@p add.u32 %0, %0, %3;\n\t}" : "+r"(n) : "l"(c), "l"(thr), "r"(add));
+}
+__device__ __forceinline__ void red_shared_inc_if(uint32_t a, uint32_t nonzero, uint32_t off, uint32_t span) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tsetp.le.and.u32 p, %2, %3, p;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(a),
+      "r"(nonzero), "r"(off), "r"(span)
+      : "memory");
+}
+__device__ __forceinline__ void st_global_if(bool on, void* a, uint32_t v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(a), "r"(v), "r"((uint32_t)on)
+               : "memory");
+}
+__device__ __forceinline__ void sts64_if(bool on, uint32_t a, uint64_t v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u64 [%0], %1;\n\t}" ::"r"(a), "l"(v), "r"((uint32_t)on)
+               : "memory");
+}
+__device__ __forceinline__ uint64_t lds64_if(bool on, uint32_t a) {
+  uint64_t v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u64 %0, 0;\n\t@p ld.shared.u64 %0, [%1];\n\t}"
+               : "=&l"(v)
+               : "r"(a), "r"((uint32_t)on)
+               : "memory");
+  return v;
 }
 
 // Histogram update: a plain shared-memory reduction (no result). Measured on B200 (64K updates
@@ -132,17 +204,19 @@ struct Ctrl {
   // cluster-wide allocation counters, meaningful in rank 0 only (targets of remote atomics)
   uint32_t win_count;
   uint32_t cand_count;
-  uint32_t over_flag;  // rank 0 only: some CTA's candidate list overflowed (remote OR)
-  uint32_t max_key;    // rank 0 only: largest key among the gathered candidates (remote max)
+  uint32_t extra_count;  // rank 0 only: candidates beyond their CTAs' regions (remote atomics)
   // published to the peers before a cluster barrier
   uint32_t pub_flag;
   // per-pass local slot counters
   uint32_t wslot;
   uint32_t cslot;
   uint32_t fslot;
-  uint32_t small_n;
   uint32_t lcount;  // entries pushed to this CTA's spill area (may exceed its capacity)
-  uint32_t spill_kmax;  // largest key among the spilled entries
+  // what the sample search leaves: the guess and the bound for the finish (keys), what to do about them
+  uint32_t guess;
+  uint32_t focus;
+  uint32_t guess_flags;
+  uint32_t need_hi;
   // result of the most recent threshold search
   int32_t t;
   uint32_t above;
@@ -164,9 +238,9 @@ struct Ctrl {
   uint32_t totb[kSup];  // first sample round: super-bin totals of the second (finer) histogram
   uint32_t dual_b;      // ... whether the finer histogram was usable, and for which top nibble
   uint32_t dual_g;
-  int32_t focus_bin;    // first sample round of a lone CTA: bin the threshold will not lie above (-1: none)
   uint32_t wtot[32];
   uint32_t wmax[32];
+  uint32_t cnt_of[kMaxCluster];  // candidates of every CTA of the cluster (each writes its own entry everywhere)
   // merge of candidate lists: this CTA's record about its shard, read by the cluster's other CTAs
   uint32_t thr_key;      // warm start: smallest key among the winners of the finish
   uint32_t merge_count;  // valid candidates
@@ -406,128 +480,97 @@ __device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked&
 
 // ---------------------------------------------------------------------------------------------
 // Candidate sources of the finish. A source tells a thread which candidates are its share:
-//   for_each_key(f)     f(key) for every slot of the share (any order, any trip count)
-//   for_each_uniform(f) f(composite) with the same trip count in all lanes of a warp (f may vote);
-//                       lanes without a candidate get 0, which is also what an empty slot holds
-//   for_each_uniform4(f4)  the same, four composites per call
-// Loads are issued four at a time (a plain loop waits out the full shared-memory latency once per
-// element: measured 190 cycles per element with 16 warps on the SM).
+// for_each4(f4) calls f4 with an array of four composites at a time - loads in flight together, same trip count in
+// all lanes of a warp - and 0 where there is none. Which candidates a thread sees, and in which order,
+// is the same in every call.
 // ---------------------------------------------------------------------------------------------
+
+// A dense array in shared memory walked by a group of warps (`first`: this lane's first index, `step`: lanes in
+// the group; first - lane is the same in all lanes of a warp)
+template <class F4>
+__device__ __forceinline__ void walk4(uint32_t a /* shared address */, int n, int first, int step, F4&& f4) {
+  const int lane = lane_id();
+  for (int i = first; i - lane < n; i += 4 * step) {
+    const uint32_t at = a + (uint32_t)i * 8u;
+    uint64_t c[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) c[u] = lds64_if(i + u * step < n, at + (uint32_t)(u * step) * 8u);
+    f4(c);
+  }
+}
 
 // One dense array cand[0..n); slots equal to 0 are empty.
 template <int NT>
 struct DenseCands {
-  static constexpr bool kEmpties = true;
-  const uint64_t* cand;
+  uint32_t cand;  // shared address
   int n;
-  template <class F>
-  __device__ __forceinline__ void for_each_key(F&& f) const {
-    const uint32_t* hi32 = reinterpret_cast<const uint32_t*>(cand) + 1;  // little endian: word 1 = key
-    int i = threadIdx.x;
-    for (; i + 3 * NT < n; i += 4 * NT) {
-      const uint32_t k0 = hi32[2 * i], k1 = hi32[2 * (i + NT)], k2 = hi32[2 * (i + 2 * NT)], k3 = hi32[2 * (i + 3 * NT)];
-      f(k0);
-      f(k1);
-      f(k2);
-      f(k3);
-    }
-    for (; i < n; i += NT) f(hi32[2 * i]);
-  }
+  __device__ __forceinline__ DenseCands(const uint64_t* c, int n_) : cand(smem_u32(c)), n(n_) {}
   template <class F4>
-  __device__ __forceinline__ void for_each_uniform4(F4&& f4) const {
-    const int tid = threadIdx.x;
-    for (int i0 = 0; i0 < n; i0 += 4 * NT) {
-      const int i = i0 + tid;
-      const uint64_t c0 = (i < n) ? cand[i] : 0ull;
-      const uint64_t c1 = (i + NT < n) ? cand[i + NT] : 0ull;
-      const uint64_t c2 = (i + 2 * NT < n) ? cand[i + 2 * NT] : 0ull;
-      const uint64_t c3 = (i + 3 * NT < n) ? cand[i + 3 * NT] : 0ull;
-      f4(c0, c1, c2, c3);
-    }
-  }
-  template <class F>
-  __device__ __forceinline__ void for_each_uniform(F&& f) const {
-    for_each_uniform4([&](uint64_t c0, uint64_t c1, uint64_t c2, uint64_t c3) {
-      f(c0);
-      f(c1);
-      f(c2);
-      f(c3);
-    });
+  __device__ __forceinline__ void for_each4(F4&& f4) const {
+    walk4(cand, n, (int)threadIdx.x, NT, f4);
   }
 };
 
 // What the filter of a lone CTA leaves behind: one dense segment per warp (each warp walks its own;
-// `wn`, its length, is the same in all lanes) plus the shared spill area of `sn` entries. No slot
-// is empty.
+// `wn`, its length, is the same in all lanes) plus the shared spill area of `sn` entries.
 template <int NT>
 struct WarpSegCands {
-  static constexpr bool kEmpties = false;
-  const uint64_t* seg;
+  uint32_t seg;  // shared address of this warp's segment
   int wn;
-  const uint64_t* spill;
+  uint32_t spill;
   int sn;
-  template <class F>
-  __device__ __forceinline__ void for_each_key(F&& f) const {
-    const uint32_t* hi32 = reinterpret_cast<const uint32_t*>(seg) + 1;
-    int i = lane_id();
-    for (; i + 96 < wn; i += 128) {
-      const uint32_t k0 = hi32[2 * i], k1 = hi32[2 * (i + 32)], k2 = hi32[2 * (i + 64)], k3 = hi32[2 * (i + 96)];
-      f(k0);
-      f(k1);
-      f(k2);
-      f(k3);
-    }
-    for (; i < wn; i += 32) f(hi32[2 * i]);
-    const uint32_t* sp32 = reinterpret_cast<const uint32_t*>(spill) + 1;
-    for (int j = threadIdx.x; j < sn; j += NT) f(sp32[2 * j]);
-  }
   template <class F4>
-  __device__ __forceinline__ void for_each_uniform4(F4&& f4) const {
-    const int lane = lane_id();
-    for (int i0 = 0; i0 < wn; i0 += 128) {
-      const int i = i0 + lane;
-      const uint64_t c0 = (i < wn) ? seg[i] : 0ull;
-      const uint64_t c1 = (i + 32 < wn) ? seg[i + 32] : 0ull;
-      const uint64_t c2 = (i + 64 < wn) ? seg[i + 64] : 0ull;
-      const uint64_t c3 = (i + 96 < wn) ? seg[i + 96] : 0ull;
-      f4(c0, c1, c2, c3);
-    }
-    const int tid = threadIdx.x;
-    for (int j0 = 0; j0 < sn; j0 += 4 * NT) {
-      const int j = j0 + tid;
-      const uint64_t c0 = (j < sn) ? spill[j] : 0ull;
-      const uint64_t c1 = (j + NT < sn) ? spill[j + NT] : 0ull;
-      const uint64_t c2 = (j + 2 * NT < sn) ? spill[j + 2 * NT] : 0ull;
-      const uint64_t c3 = (j + 3 * NT < sn) ? spill[j + 3 * NT] : 0ull;
-      f4(c0, c1, c2, c3);
-    }
+  __device__ __forceinline__ void for_each4(F4&& f4) const {
+    walk4(seg, wn, lane_id(), 32, f4);
+    if (sn > 0) walk4(spill, sn, (int)threadIdx.x, NT, f4);
   }
-  template <class F>
-  __device__ __forceinline__ void for_each_uniform(F&& f) const {
-    for_each_uniform4([&](uint64_t c0, uint64_t c1, uint64_t c2, uint64_t c3) {
-      f(c0);
-      f(c1);
-      f(c2);
-      f(c3);
-    });
+};
+
+// What a cluster leaves in its first CTA: one region of `region` slots per CTA, filled densely with
+// count_of[r] candidates, and `extra` candidates that did not fit in front of those behind the last
+// region. A region belongs to 2^lper warps (or, lper = 0, a warp to several regions).
+template <int NT>
+struct RegionCands {
+  uint32_t cand;      // shared addresses
+  uint32_t count_of;
+  int region, C, extra;
+  template <class F4>
+  __device__ __forceinline__ void for_each4(F4&& f4) const {
+    constexpr int kLogNW = NT == 1024 ? 5 : (NT == 512 ? 4 : 3);
+    const int warp = threadIdx.x >> 5;
+    const int lper = max(kLogNW - (31 - __clz(C)), 0);  // (NW and C are powers of two: no division)
+    for (int r = warp >> lper; r < C; r += (NT / 32) >> lper)
+      walk4(cand + (uint32_t)(r * region) * 8u, min((int)lds32(count_of + r * 4), region),
+            (warp & ((1 << lper) - 1)) * 32 + lane_id(), 32 << lper, f4);
+    if (extra > 0) walk4(cand + (uint32_t)(C * region) * 8u, extra, (int)threadIdx.x, NT, f4);
   }
 };
 
 // Block-wide threshold pick over kFinishBins counts (descending bin order); result in ctrl->t
 // (-1 if the counts sum to less than need), ctrl->above, ctrl->cnt. Ends with a barrier.
 template <int NT>
-__device__ __forceinline__ void block_pick(const uint32_t* hist, uint32_t need, Ctrl* ctrl) {
+__device__ __forceinline__ void block_pick(uint32_t hist /* shared address */, uint32_t need, Ctrl* ctrl) {
   constexpr int PER = (kFinishBins + NT - 1) / NT;
   constexpr int NW = NT / 32;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   uint32_t v[PER];
   uint32_t s = 0;
+  if constexpr (PER * NT == kFinishBins && PER % 2 == 0) {
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int b = tid * PER + j;
-    v[j] = (b < kFinishBins) ? hist[b] : 0u;
-    s += v[j];
+    for (int j = 0; j < PER; j += 2) {
+      const uint2 q = lds64x2(hist + (uint32_t)(tid * PER + j) * 4u);
+      v[j] = q.x;
+      v[j + 1] = q.y;
+      s += q.x + q.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int b = tid * PER + j;
+      v[j] = (b < kFinishBins) ? lds32(hist + b * 4) : 0u;
+      s += v[j];
+    }
   }
   uint32_t incl = s;
 #pragma unroll
@@ -535,20 +578,68 @@ __device__ __forceinline__ void block_pick(const uint32_t* hist, uint32_t need, 
     const uint32_t x = __shfl_down_sync(kFull, incl, off);
     if (lane + off < 32) incl += x;
   }
-  if (lane == 0) ctrl->wtot[warp] = incl;
+  const uint32_t wtot = smem_u32(ctrl->wtot);
+  if (lane == 0) sts32(wtot + warp * 4, incl);
   if (tid == 0) ctrl->t = -1;
   __syncthreads();
-  const uint32_t hw = (lane > warp && lane < NW) ? ctrl->wtot[lane] : 0u;
-  const uint32_t higher = warp_sum(hw);
-  uint32_t run = higher + incl - s;
+  const uint32_t hw = (lane > warp && lane < NW) ? lds32(wtot + lane * 4) : 0u;
+  uint32_t run = __reduce_add_sync(kFull, hw) + incl - s;
+  if (run < need && need <= run + s) {  // (one thread)
 #pragma unroll
-  for (int j = PER - 1; j >= 0; --j) {
-    if (run < need && need <= run + v[j]) {
-      ctrl->t = tid * PER + j;
-      ctrl->above = run;
-      ctrl->cnt = v[j];
+    for (int j = PER - 1; j >= 0; --j) {
+      if (run < need && need <= run + v[j]) {
+        ctrl->t = tid * PER + j;
+        ctrl->above = run;
+        ctrl->cnt = v[j];
+      }
+      run += v[j];
     }
-    run += v[j];
+  }
+  __syncthreads();
+}
+
+// Block-wide search over a sample histogram of kSampleBins counts (descending bin order):
+// found(bin, above, count) is called by one thread for the bin of rank `need`, found_hi(bin) by one
+// for the bin of rank `need_hi` (neither if the counts do not reach that rank, or the rank is 0).
+// Ends with a barrier, which publishes what they leave in shared memory. Written for few
+// instructions: with 32 warps on an SM each of them costs a block eight issue cycles.
+template <int NT, class Found, class FoundHi>
+__device__ __forceinline__ void block_pick_sample(uint32_t hist /* shared address */, uint32_t need, uint32_t need_hi,
+                                                  uint32_t wtot /* shared address */,
+                                                  Found&& found, FoundHi&& found_hi) {
+  constexpr int PER = kSampleBins / NT;
+  constexpr int NW = NT / 32;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  uint32_t v[PER];
+  uint32_t s = 0;
+#pragma unroll
+  for (int j = 0; j < PER / 4; ++j) {
+    const uint4 q = lds128(hist + (uint32_t)(tid * PER + 4 * j) * 4u);
+    v[4 * j] = q.x;
+    v[4 * j + 1] = q.y;
+    v[4 * j + 2] = q.z;
+    v[4 * j + 3] = q.w;
+    s += (q.x + q.y) + (q.z + q.w);
+  }
+  uint32_t incl = s;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t x = __shfl_down_sync(kFull, incl, off);
+    if (lane + off < 32) incl += x;
+  }
+  if (lane == 0) sts32(wtot + warp * 4, incl);
+  __syncthreads();
+  const uint32_t w = (lane < NW && lane > warp) ? lds32(wtot + lane * 4) : 0u;
+  uint32_t run = __reduce_add_sync(kFull, w) + incl - s;
+  // (a thread whose bins lie wholly above or wholly below both ranks has nothing to look for)
+  if ((run < need && need <= run + s) || (run < need_hi && need_hi <= run + s)) {
+#pragma unroll
+    for (int j = PER - 1; j >= 0; --j) {
+      if (run < need && need <= run + v[j]) found((uint32_t)(tid * PER + j), run, v[j]);
+      if (run < need_hi && need_hi <= run + v[j]) found_hi((uint32_t)(tid * PER + j));
+      run += v[j];
+    }
   }
   __syncthreads();
 }
@@ -572,25 +663,30 @@ __device__ __forceinline__ void block_pick(const uint32_t* hist, uint32_t need, 
 // `known_total`: when not 0, the number of candidates in the source; if it equals `need` they all
 // win and no round is run. kTrackMin: the smallest key among the winners - the key of the
 // need-th largest candidate - is left in ctrl->thr_key (atomic min; the caller presets it).
+// Inlined, and the source comes by value: as a call, source and arguments went through every thread's
+// stack, and beside 200 KB of shared memory L1 has no room for the stacks of 1024 threads - each access
+// was a round trip to L2 (the passes over the candidates took 1.4 and 2 to 4 us instead of 0.4 and 0.7).
 template <int NT, class Src, bool kTrackMin = false>
-__device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t cap, uint64_t focus, bool have_hist,
+__device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_t lo, uint64_t cap, uint64_t focus, bool have_hist,
                            int idx_bits, uint32_t* hist /* >= kFinishBins words */, Ctrl* ctrl, int32_t* out_idx,
                            uint32_t* out_key, uint32_t out_base, uint32_t out_slots /* k of the row */,
                            int32_t idx_offset, uint32_t* status,
-                           const int32_t* page = nullptr /* when set: out = page[idx] */, uint32_t known_total = 0u) {
+                           const int32_t* page = nullptr /* when set: out = page[idx] */, uint32_t known_total = 0u,
+                           bool hist_clear = false /* `hist` is all zero already */) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    ctrl->fslot = 0u;  // (every path below has a block barrier before these are used)
-    ctrl->small_n = 0u;
-  }
+  const uint32_t hist_s = smem_u32(hist);
   if (lo > cap) {
     // Range unknown: the smallest and the largest key present bound it.
     uint32_t kmin = ~0u, kmax = 0u;
-    src.for_each_key([&](uint32_t k) {
-      if (k != 0u) {
-        kmin = min(kmin, k);
-        kmax = max(kmax, k);
+    src.for_each4([&](const uint64_t (&c)[4]) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t k = (uint32_t)(c[u] >> 32);
+        if (c[u] != 0ull) {
+          kmin = min(kmin, k);
+          kmax = max(kmax, k);
+        }
       }
     });
     kmin = __reduce_min_sync(kFull, kmin);
@@ -610,7 +706,7 @@ __device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t 
       return;
     }
     focus = cap;
-    have_hist = false;
+    have_hist = hist_clear = false;
     __syncthreads();  // the scratch words are about to be cleared as the histogram
     FFTOPK_MARK(31);
   }
@@ -628,7 +724,7 @@ __device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t 
     t_hi = cap;
     cnt = need2 = need;
     all_bin = found = true;
-    __syncthreads();  // (the counters cleared above are used by the pass below)
+    __syncthreads();  // (as in a round: what the caller has read through ctrl may be overwritten from here on)
   } else if (known_total != 0u && known_total <= (uint32_t)kSmall && known_total >= need && lo <= cap) {
     // so few candidates that they are ranked directly: the whole range is the "threshold bin"
     t_lo = lo;
@@ -651,24 +747,33 @@ __device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t 
     if (focus < lo || focus > cap) focus = cap;
     const FinishDigit dg = make_finish_digit(lo, focus);
     if (!(round == 0 && have_hist)) {
-      for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
-      __syncthreads();
+      if (!(round == 0 && hist_clear)) {
+        for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
+        __syncthreads();
+      }
       const uint64_t span = cap - lo;
       if (dg.key_only()) {
         // the digit depends on the key alone: work on the high words only (an empty slot has key 0)
         const uint32_t klo = (uint32_t)(lo >> 32), kspan = (uint32_t)(span >> 32);
-        src.for_each_key([&](uint32_t k) {
-          if ((!Src::kEmpties || k != 0u) && (k - klo) <= kspan) red_shared_add(&hist[dg.of_key(k)], 1u);
+        src.for_each4([&](const uint64_t (&c)[4]) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t k = (uint32_t)(c[u] >> 32);
+            red_shared_inc_if(hist_s + dg.of_key(k) * 4u, k, k - klo, kspan);
+          }
         });
       } else {
-        src.for_each_uniform([&](uint64_t c) {
-          if (c != 0ull && (c - lo) <= span) red_shared_add(&hist[dg.of(c)], 1u);
+        src.for_each4([&](const uint64_t (&c)[4]) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (c[u] != 0ull && (c[u] - lo) <= span) red_shared_inc(hist_s + dg.of(c[u]) * 4u);
+          }
         });
       }
       __syncthreads();
     }
     FFTOPK_MARK(16);
-    block_pick<NT>(hist, need, ctrl);
+    block_pick<NT>(hist_s, need, ctrl);
     FFTOPK_MARK(17);
     const int t = ctrl->t;
     if (t < 0) {
@@ -693,52 +798,57 @@ __device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t 
     if (tid == 0 && status) atomicOr(status, 2u);
     return;
   }
-  // ---- one pass writes the certain winners (a ballot and one slot-allocating atomic per warp
-  // and trip; the order of the output is unspecified) and sets the undecided candidates aside ----
+  // ---- the certain winners go out (in unspecified order), the undecided candidates are set aside ----
+  // First every thread counts both kinds in its share, a scan over the lanes and one over the warps
+  // gives it its slots, then it writes. (A slot-allocating atomic per warp serialised on the one
+  // counter - 30 cycles per warp -, and ballots per candidate cost more instructions than they saved;
+  // instructions are what bounds this pass: with all warps of an SM at it each one costs eight cycles.)
   FFTOPK_MARK(32);
   const uint64_t wthr = all_bin ? (t_lo ? t_lo - 1ull : 0ull) : t_hi;  // winners: c > wthr
-  const unsigned lt = (1u << lane) - 1u;
-  // Slots come from one shared counter; the warps' atomics on it serialise (~30 cycles each), so
-  // a warp allocates for four candidates per lane with one of them.
+  const uint64_t uthr = all_bin ? wthr : (t_lo ? t_lo - 1ull : 0ull);  // undecided: uthr < c <= wthr
+  uint32_t mine = 0u;  // winners << 16 | winners and undecided
+  src.for_each4([&](const uint64_t (&c)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      count_if_above(mine, c[u], wthr, 0x10000u);
+      count_if_above(mine, c[u], uthr, 1u);
+    }
+  });
+  uint32_t incl = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFull, incl, off);
+    if (lane >= off) incl += x;
+  }
+  const uint32_t wsum = smem_u32(ctrl->wmax);
+  if (lane == 31) sts32(wsum + warp * 4, incl);
+  __syncthreads();
+  const uint32_t before = __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u) + incl - mine;
+  uint32_t wpos = out_base + (before >> 16), upos = (before & 0xffffu) - (before >> 16);
   uint32_t win_min = 0xffffffffu;  // (kTrackMin) smallest key among the winners this thread wrote
+  const uint32_t small_s = smem_u32(ctrl->small);
   auto pass = [&](auto paged) {
-    src.for_each_uniform4([&](uint64_t c0, uint64_t c1, uint64_t c2, uint64_t c3) {
-      const uint64_t c[4] = {c0, c1, c2, c3};
-      unsigned b[4];
-      uint32_t nwin = 0;
+    src.for_each4([&](const uint64_t (&c)[4]) {
+      int32_t v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        b[u] = __ballot_sync(kFull, c[u] > wthr);
-        nwin += (uint32_t)__popc(b[u]);
-      }
-      if (nwin) {
-        uint32_t base = 0;
-        if (lane == 0) base = atom_shared_add(&ctrl->fslot, nwin);
-        base = out_base + __shfl_sync(kFull, base, 0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t pos = base + (uint32_t)__popc(b[u] & lt);
-          if (c[u] > wthr && FFTOPK_CHECK(3, pos, out_slots, status) && pos < out_slots) {
-            const int32_t idx = (int32_t)(~(uint32_t)c[u]);
-            if constexpr (decltype(paged)::value) {
-              out_idx[pos] = __ldg(page + idx);
-            } else {
-              out_idx[pos] = idx + idx_offset;
-            }
-            if (out_key) out_key[pos] = (uint32_t)(c[u] >> 32);
-            if constexpr (kTrackMin) win_min = min(win_min, (uint32_t)(c[u] >> 32));
-          }
-          base += (uint32_t)__popc(b[u]);
+        const int32_t idx = (int32_t)(~(uint32_t)c[u]);
+        v[u] = idx + idx_offset;
+        if constexpr (decltype(paged)::value) {  // (the four table reads in flight together)
+          if (c[u] > wthr) v[u] = __ldg(page + idx);
         }
       }
-      if (!all_bin) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (c[u] <= wthr && c[u] >= t_lo && c[u] != 0ull) {
-            const uint32_t s = warp_alloc(&ctrl->small_n);
-            if (FFTOPK_CHECK(4, s, kSmall, status) && s < (uint32_t)kSmall) ctrl->small[s] = c[u];
-          }
-        }
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t w = c[u] > wthr ? 1u : 0u, g = c[u] > uthr ? 1u : 0u;
+        const bool put = w != 0u && FFTOPK_CHECK(3, wpos, out_slots, status) && wpos < out_slots;
+        st_global_if(put, out_idx + wpos, (uint32_t)v[u]);
+        if (out_key) st_global_if(put, out_key + wpos, (uint32_t)(c[u] >> 32));
+        if constexpr (kTrackMin) win_min = min(win_min, w != 0u ? (uint32_t)(c[u] >> 32) : 0xffffffffu);
+        wpos += w;
+        const bool set = g != w && FFTOPK_CHECK(4, upos, kSmall, status) && upos < (uint32_t)kSmall;
+        sts64_if(set, small_s + upos * 8u, c[u]);
+        upos += g - w;
       }
     });
   };
@@ -755,11 +865,11 @@ __device__ void cta_finish(const Src& src, uint32_t need, uint64_t lo, uint64_t 
 #ifdef FFTOPK_CHECKED
   {
     // every certain winner took exactly one slot, every undecided candidate was set aside
-    __syncthreads();
+    const uint32_t sum = __reduce_add_sync(kFull, lane < NT / 32 ? ctrl->wmax[lane] : 0u);
     const uint32_t want_w = all_bin ? need_total : need_total - need2;
     if (tid == 0) {
-      if (ctrl->fslot != want_w) check_fail(10, ctrl->fslot, want_w, status);
-      if (!all_bin && ctrl->small_n != cnt) check_fail(11, ctrl->small_n, cnt, status);
+      if ((sum >> 16) != want_w) check_fail(10, sum >> 16, want_w, status);
+      if (!all_bin && (sum & 0xffffu) - (sum >> 16) != cnt) check_fail(11, (sum & 0xffffu) - (sum >> 16), cnt, status);
     }
   }
 #endif

@@ -17,13 +17,14 @@
 #endif
 
 FFTOPK_HD uint32_t fftopk_key_from_bits(uint32_t bits) {
-  // NaN (exponent all ones, mantissa non-zero) -> the largest key.
-  if ((bits & 0x7fffffffu) > 0x7f800000u) return 0xffffffffu;
-  // -0.0 -> +0.0
-  if (bits == 0x80000000u) bits = 0u;
-  // negative: flip all bits; non-negative: set the sign bit.
+  // negative: flip all bits; non-negative: set the sign bit. (Selects, no branches: lanes of a warp
+  // that part here would go through the rest of the caller's loop one after the other.)
   const uint32_t mask = (uint32_t)((int32_t)bits >> 31) | 0x80000000u;
-  return bits ^ mask;
+  uint32_t key = bits ^ mask;
+  // -0.0 -> +0.0
+  key = bits == 0x80000000u ? 0x80000000u : key;
+  // NaN (exponent all ones, mantissa non-zero) -> the largest key.
+  return (bits & 0x7fffffffu) > 0x7f800000u ? 0xffffffffu : key;
 }
 
 // Inverse on canonical keys (NaN comes back as one quiet NaN pattern).

@@ -6,36 +6,37 @@
 //
 // Shape of the computation for one row of `len` > 2048 valid fp32 logits, C CTAs in the cluster,
 // each owning a contiguous shard of the row:
-//   1. SAMPLE. Every warp reads one to four 512-byte slabs; the slabs are spread evenly over the
-//      shards, so the cluster samples the row uniformly in position. The top 12 bits of the
-//      order-preserving key are histogrammed per CTA (4096 bins); a cluster also histograms key
-//      bits [27:16], which give a 16-bit guess when the whole sample shares its top four key bits.
-//      When the whole shard fits in registers (<= 3 granules per thread) the "sample" is the
-//      shard and step 2 is exact.
-//   2. PICK. After ONE cluster barrier every CTA reads its peers' 64 super-bin sums, then the 64
-//      fine bins of the threshold super-bin, over distributed shared memory, and finds the bin
-//      with a warp-shuffle suffix scan (no L2 atomics, no reduce-then-broadcast). From a sample it
-//      takes the bin whose sample rank is the expected rank of the k-th element plus five standard
-//      deviations: a lower bound of the true threshold with overwhelming probability. A lone CTA
-//      does all of this in one warp and also finds the mirror-image upper bound.
-//   3. FILTER. One streaming pass over the shard (128-bit loads, four or eight in flight per
-//      thread) with ONE float compare per element against the bin's lower edge; the few thousand
-//      elements that pass are appended, by ballot, to dense per-warp segments of a list in shared
-//      memory and become (key << 32 | ~index) composites. This is the only full read of the row.
-//   4. GATHER + FINISH. The segments are copied into rank 0's shared memory (one remote atomic per
-//      CTA reserves the range), and after the second cluster barrier rank 0 finishes: radix rounds
-//      over the composites' range, one fused output pass, and the last <= 256 undecided
-//      candidates ranked by votes. A lone CTA finishes over its segments where they lie. The
-//      inverted index in the composite makes equal values resolve to the lower index.
+//   1. SAMPLE. Every CTA reads the same 8K elements (16K of rows beyond 256K), in slabs of 512 bytes
+//      spread evenly over the row, and histograms them on a digit of 64 bins per octave. A CTA whose
+//      whole shard fits in registers has those loads in flight at the same time.
+//   2. PICK. One block-wide suffix scan finds the bin whose sample rank is the expected rank of the k-th
+//      element plus five standard deviations - a lower bound of the true threshold with overwhelming
+//      probability - and the mirror-image upper bound. All CTAs of a cluster find the same bin by
+//      themselves: no histogram is exchanged and no cluster barrier is waited for here (exchanging
+//      them took 0.8 us for the barrier and 1.8 us for two rounds of remote reads).
+//   3. FILTER. ONE float compare per element against the bin's lower edge, on the shard in registers
+//      (counted, scanned over the warp, stored: no second read) or in one streaming pass (128-bit
+//      loads, four or eight in flight per thread); the few thousand elements that pass go to dense
+//      per-warp segments of a list in shared memory.
+//   4. GATHER + FINISH. They become (key << 32 | ~index) composites on their way into rank 0's shared
+//      memory, where every CTA owns a region; every CTA also tells every other its count, so that
+//      after the one cluster barrier each knows whether the guess held and all but rank 0 leave. Rank 0
+//      finishes: radix rounds over the composites' range, a counting and a writing pass, and the last
+//      <= 256 undecided candidates ranked by votes. A lone CTA finishes over its segments where they
+//      lie. The inverted index in the composite makes equal values resolve to the lower index.
+//      Measured (us per call in a chain of calls on B200, before -> with steps 1 to 4 as they are now):
+//      B=1, L=96K 12.9 -> 10.3, 1M 15.4 -> 14.4; B=4, L=200K 13.6 -> 11.1; B=64 ragged rows of up to 128K
+//      17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5); B=2048, one CTA per row, L=32K 132 -> 101, 8K
+//      106 -> 70. What bounds it is no bandwidth but the chain of short phases and the instructions in it.
 //   5. If the guess admitted fewer than k elements, a list overflowed or the threshold bin is
 //      larger than rank 0's buffer (heavy ties, rows of equal values), the cluster falls back to
 //      full histograms over the data: 12 + 12 + 8 key bits, re-reading the shard from L2 each
 //      round, and exact ties left after 32 bits are taken in index order, shard by shard.
 //
 // Build-time knobs (all optional, for experiments; the defaults are what was measured best):
-//   FFTOPK_SAMPLE_GRANULES  granules the cluster samples per row and thread column (2048)
-//   FFTOPK_EXACT_SLABS      granules per thread up to which the shard stays in registers (3)
-//   FFTOPK_1B_FACTOR        second sample round when the guessed bin holds more than factor*k (2)
+//   FFTOPK_LONG_SAMPLE      row length from which the sample is 16K elements instead of 8K (262144)
+//   FFTOPK_REG_SLABS        granules per thread up to which the shard stays in registers (4; see reg_slabs)
+//   FFTOPK_1B_FACTOR        second look at the sample when the guessed bin holds more than factor*k (2)
 //   FFTOPK_U512             128-bit loads in flight per thread of the 512-thread filter (8; 16 allowed)
 //   FFTOPK_CTAS_512         512-thread CTAs per SM the register budget allows (2)
 //   FFTOPK_KSMALL           undecided candidates ranked by votes (256)
@@ -57,6 +58,13 @@
 
 namespace fftopk {
 
+
+#ifndef FFTOPK_REG_SLABS
+#define FFTOPK_REG_SLABS 4
+#endif
+#ifndef FFTOPK_LONG_SAMPLE
+#define FFTOPK_LONG_SAMPLE 262144
+#endif
 
 struct SelectParams {
   const void* score;  // fp32, or fp16 / bf16 for the kernels instantiated on those types
@@ -102,7 +110,15 @@ struct SelectParams {
 };
 
 
-constexpr int kRegSlabs = 4;  // granules a thread keeps in registers when the whole shard fits
+constexpr uint32_t kOverflowed = 1u << 31;   // in a CTA's candidate count: one of its lists has overflowed
+#ifndef FFTOPK_1B_FACTOR
+#define FFTOPK_1B_FACTOR 2.0f
+#endif
+constexpr float kCoarseFactor = FFTOPK_1B_FACTOR;
+#ifndef FFTOPK_U512
+#define FFTOPK_U512 8
+#endif
+
 
 // digit schedule of the full-histogram rounds: 12 + 12 + 8 bits
 __device__ __forceinline__ int round_width(int r) { return r < 2 ? 12 : 8; }
@@ -176,24 +192,20 @@ __device__ __forceinline__ float4 load_granule(const Shard<T>& sh, int g, float 
   return load_granule_partial(sh.gbase, sh.a, sh.len, g, fill);
 }
 
-// A kept element on its way into the list: the raw float bits and the row index. It becomes a
-// (key << 32 | ~idx) composite later, in a dense pass - the hit loop is the divergent part of
-// the filter and every instruction in it is paid by a whole warp for one or two lanes.
-__device__ __forceinline__ uint64_t raw_to_composite(uint64_t raw, uint32_t& kmax) {
-  const uint32_t key = fftopk_key_from_bits((uint32_t)(raw >> 32));
-  kmax = max(kmax, key);
-  return ((uint64_t)key << 32) | (uint64_t)(~(uint32_t)raw);
+// A kept element on its way into the list: the raw float bits (high word) and the row index. It becomes
+// a (key << 32 | ~idx) composite later, in a dense pass - the loop that finds the hits is the divergent
+// part of the filter and every instruction in it is paid by a whole warp for one or two lanes.
+__device__ __forceinline__ uint64_t raw_to_composite(uint64_t raw) {
+  return ((uint64_t)fftopk_key_from_bits((uint32_t)(raw >> 32)) << 32) | (uint64_t)(~(uint32_t)raw);
 }
 
-// Overflow of a thread's private candidate slots: a shared spill area, slots from one counter
+// Overflow of a warp's segment: a shared spill area, slots from one counter
 // (rare, so the serialising atomic does not matter). Converts on the spot. Out of line to keep
 // the filter loop small.
 __device__ __noinline__ void spill_push(Ctrl* ctrl, uint64_t* spill, uint32_t spill_cap, uint64_t raw) {
   const uint32_t slot = warp_alloc(&ctrl->lcount);
   if (slot < spill_cap) {
-    uint32_t k = 0;
-    spill[slot] = raw_to_composite(raw, k);
-    atomicMax(&ctrl->spill_kmax, k);
+    spill[slot] = raw_to_composite(raw);
   } else {
     ctrl->pub_flag = 1u;
   }
@@ -213,11 +225,10 @@ __device__ __noinline__ void spill_push(Ctrl* ctrl, uint64_t* spill, uint32_t sp
 // values in the dense pass that builds the composites afterwards, several loads in flight per
 // lane (best when most trips have hits: a dependent load per trip of the hit loop would stall
 // the warp each time). Candidates beyond the segment's capacity go to the shared spill area.
-// Returns the number of candidates the warp found (those beyond seg_cap went to the spill area);
-// kmax is the largest key among the entries this lane converted; post(key) is called for each of them.
-template <int NT, int U, bool kStage, class T, class Post>
+// Returns the number of candidates the warp found (those beyond seg_cap went to the spill area).
+template <int NT, int U, bool kStage, class T>
 __device__ __forceinline__ uint32_t filter_shard(const Shard<T>& sh, float edge, uint64_t* seg, uint32_t seg_cap, Ctrl* ctrl,
-                                                 uint64_t* spill, uint32_t spill_cap, uint32_t& kmax, Post&& post) {
+                                                 uint64_t* spill, uint32_t spill_cap) {
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -225,19 +236,19 @@ __device__ __forceinline__ uint32_t filter_shard(const Shard<T>& sh, float edge,
   const T* gbase = sh.gbase;
   const int fa = sh.a, fi1 = sh.i1, len = sh.len;
   uint32_t wcnt = 0;  // candidates of this warp so far (warp-uniform)
-  uint32_t* seg32 = reinterpret_cast<uint32_t*>(seg);  // staging: candidate j's row index in word j
+  const uint32_t seg_s = smem_u32(seg);  // staging: candidate j's row index in word j
   auto keep = [&](bool has, int idx) {  // called by the whole warp
     const unsigned b = __ballot_sync(kFull, has);
     if (has) {
       const uint32_t pos = wcnt + (uint32_t)__popc(b & lt);
       if (kStage && pos < seg_cap) {
-        seg32[pos] = (uint32_t)idx;
+        sts32(seg_s + pos * 4u, (uint32_t)idx);
       } else {
-        const uint64_t raw = ((uint64_t)__float_as_uint(Elem<T>::ld1(gbase + idx + fa)) << 32) | (uint64_t)(uint32_t)idx;
+        const uint32_t bits = __float_as_uint(Elem<T>::ld1(gbase + idx + fa));
         if (pos < seg_cap) {
-          seg[pos] = raw;
+          sts64(seg_s + pos * 8u, (uint32_t)idx, bits);
         } else {
-          spill_push(ctrl, spill, spill_cap, raw);
+          spill_push(ctrl, spill, spill_cap, ((uint64_t)bits << 32) | (uint64_t)(uint32_t)idx);
         }
       }
     }
@@ -266,10 +277,10 @@ __device__ __forceinline__ uint32_t filter_shard(const Shard<T>& sh, float edge,
     Mask mask = 0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (!(x[u].x < edge)) mask |= (Mask)1u << (4 * u);
-      if (!(x[u].y < edge)) mask |= (Mask)2u << (4 * u);
-      if (!(x[u].z < edge)) mask |= (Mask)4u << (4 * u);
-      if (!(x[u].w < edge)) mask |= (Mask)8u << (4 * u);
+      mask |= !(x[u].x < edge) ? (Mask)1u << (4 * u) : (Mask)0;
+      mask |= !(x[u].y < edge) ? (Mask)2u << (4 * u) : (Mask)0;
+      mask |= !(x[u].z < edge) ? (Mask)4u << (4 * u) : (Mask)0;
+      mask |= !(x[u].w < edge) ? (Mask)8u << (4 * u) : (Mask)0;
     }
     if constexpr (!decltype(full)::value) mask &= vmask;
     const int el0 = 4 * (gb + tid);
@@ -298,46 +309,43 @@ __device__ __forceinline__ uint32_t filter_shard(const Shard<T>& sh, float edge,
         keep(mine && (unsigned)(e0 + e) < (unsigned)len && !(xv[e] < edge), e0 + e);
     }
   }
-  // Dense conversion of the warp's segment.
-  kmax = 0u;
-  const uint32_t own = min(wcnt, seg_cap);
+  return wcnt;
+}
+
+// The dense pass over a warp's segment of `own` entries that follows the filter: sink(j, composite) for
+// each of them. Staged segments hold row indices only: the values are fetched again (L1/L2 hits, four
+// loads in flight per lane). From the top down, so that a sink may put composite j back into the
+// segment as its j-th 64-bit word: the composites of entries [j0, j0 + 128) cover words
+// [2*j0, 2*j0 + 256), which hold no index not yet read.
+template <class T, class Sink>
+__device__ __forceinline__ void drain_segment(bool staged, const Shard<T>& sh, const uint64_t* seg, uint32_t own, Ctrl* ctrl, Sink&& sink) {
+  const int lane = lane_id();
+  const uint32_t seg_s = smem_u32(seg);
   __syncwarp();
-  if constexpr (kStage) {
-    // Fetch the values again (L1/L2 hits, four loads in flight per lane) and expand the staged
-    // indices into composites in place, from the top down: the composites of entries
-    // [j0, j0 + 128) cover words [2*j0, 2*j0 + 256), which holds no index not yet read.
+  if (staged) {
     for (int j0 = (int)((own + 127u) & ~127u) - 128; j0 >= 0; j0 -= 128) {
       uint32_t idx[4], bits[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t j = (uint32_t)j0 + 32u * u + lane;
-        idx[u] = j < own ? seg32[j] : 0u;
+        idx[u] = j < own ? lds32(seg_s + j * 4u) : 0u;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        if (!FFTOPK_CHECK(7, idx[u], len, ctrl_status(ctrl))) idx[u] = 0u;
-        bits[u] = __float_as_uint(Elem<T>::ld1(gbase + idx[u] + fa));  // (index 0 is always readable)
+        if (!FFTOPK_CHECK(7, idx[u], sh.len, ctrl_status(ctrl))) idx[u] = 0u;
+        bits[u] = __float_as_uint(Elem<T>::ld1(sh.gbase + idx[u] + sh.a));  // (index 0 is always readable)
       }
       __syncwarp();
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const uint32_t j = (uint32_t)j0 + 32u * u + lane;
-        if (j < own) {
-          const uint64_t c = raw_to_composite(((uint64_t)bits[u] << 32) | idx[u], kmax);
-          seg[j] = c;
-          post((uint32_t)(c >> 32));
-        }
+        if (j < own) sink(j, raw_to_composite(((uint64_t)bits[u] << 32) | idx[u]));
       }
       __syncwarp();
     }
   } else {
-    for (uint32_t j = lane; j < own; j += 32) {
-      const uint64_t c = raw_to_composite(seg[j], kmax);
-      seg[j] = c;
-      post((uint32_t)(c >> 32));
-    }
+    for (uint32_t j = lane; j < own; j += 32) sink(j, raw_to_composite(lds64(seg_s + j * 8u)));
   }
-  return wcnt;
 }
 
 // Visit every valid element of the shard: op(key, idx). Interior granules are read with
@@ -383,158 +391,116 @@ __device__ __forceinline__ void scan_shard(const Shard<T>& sh, Op&& op) {
   }
 }
 
-// First search of the sampled path, over TWO sample histograms built in the same pass:
-//   A: key bits [31:20]   (4096 bins, valid for any data, 8 bins per octave of magnitude)
-//   B: key bits [27:16]   (4096 bins, 128 per octave) - meaningful only among keys that share the
-//      top four bits (sign and the three high exponent bits)
-// If every sampled key shares those four bits - one super-bin group of A holds the whole sample,
-// which is the normal case for indexer logits (one sign, magnitudes within a factor of 2^32) - the
-// pick is made on B and yields a 16-bit key prefix, fine enough that no second sample round is
-// needed; otherwise on A (12 bits). Same two barriers and two rounds of remote reads as one search.
-struct DualPick {
-  bool ok;
-  uint32_t prefix;  // the guessed key prefix ...
-  int pbits;        // ... and its length in bits (12 or 16)
-  uint32_t need2;   // sample rank still to go inside the guessed bin
-  uint32_t cnt;     // sample elements in the guessed bin
-  uint32_t total;   // sample size (cluster-wide)
-  int focus_bin;    // lone CTA only: bin (same width as the guess) the threshold will not lie above; -1: unknown
-};
-
-template <int NT, class NeedFn, class NeedHiFn>
-__device__ __forceinline__ DualPick cluster_pick_dual(cg::cluster_group& cluster, int C, const uint32_t* ha,
-                                                      const uint32_t* sa, const uint32_t* hb, const uint32_t* sb,
-                                                      bool dual, Ctrl* ctrl, int& pick_no, NeedFn&& need_of,
-                                                      NeedHiFn&& need_hi_of) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  constexpr int fine = kMaxBins / kSup;
-  if (C == 1) {
-    // A lone CTA has nothing to exchange: one warp reads the super-bin sums, picks, reads the fine
-    // bins of the super-bins it needs and picks again; one block barrier publishes the result.
-    // (The totals buffers stay untouched, so the search counter does not advance.)
-    // It also brackets the threshold from above: the bin of the mirror-image sample rank, which
-    // the true threshold lies below with the same confidence. The finish then spends its first
-    // digit between the two bins instead of on the whole range up to the row's maximum.
-    if (warp == 0) {
-      const uint32_t lo = sa[2 * lane], hi = sa[2 * lane + 1];
-      const uint32_t total = warp_sum(lo + hi);
-      const uint32_t need = need_of(total);
-      const uint32_t need_hi = need_hi_of(total);
-      int ts = -1, ts_hi = -1, tf = -1, focus_bin = -1;
-      uint32_t above = 0, cnt = 0, above_hi = 0, cnt_hi = 0, above_f = 0, cnt_t = 0;
-      bool ok = need > 0 && warp_pick64(lo, hi, need, ts, above, cnt);
-      if (ok) {
-        const uint32_t flo = ha[ts * fine + 2 * lane], fhi = ha[ts * fine + 2 * lane + 1];
-        ok = warp_pick64(flo, fhi, need - above, tf, above_f, cnt_t);
-        if (ok && need_hi > 0 && warp_pick64(lo, hi, need_hi, ts_hi, above_hi, cnt_hi)) {
-          int tf_hi = -1;
-          uint32_t a2 = 0, c2 = 0;
-          const uint32_t glo = ha[ts_hi * fine + 2 * lane], ghi = ha[ts_hi * fine + 2 * lane + 1];
-          if (warp_pick64(glo, ghi, need_hi - above_hi, tf_hi, a2, c2)) focus_bin = ts_hi * fine + tf_hi;
-        }
+// The filter of a shard that sits in registers (x[j]: granule j*NT + thread of the shard, -inf where an
+// element is not the row's; `edge` > -inf). Every lane counts its hits, a scan over the warp gives it
+// its slots, and a predicated store per element writes what passes: no second read of the value, no
+// loop over hits. Same result as filter_shard.
+template <int R>
+__device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, int el_step, float edge, uint64_t* seg,
+                                                uint32_t seg_cap, Ctrl* ctrl, uint64_t* spill, uint32_t spill_cap) {
+  const int lane = lane_id();
+  uint32_t n = 0u;
+  auto count = [&](float v) {
+    asm("{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p add.u32 %0, %0, 1;\n\t}" : "+r"(n) : "f"(v), "f"(edge));
+  };
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    count(x[j].x);
+    count(x[j].y);
+    count(x[j].z);
+    count(x[j].w);
+  }
+  uint32_t incl = n;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFull, incl, off);
+    if (lane >= off) incl += v;
+  }
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  uint32_t pos = incl - n;
+  uint32_t at = smem_u32(seg) + pos * 8u;
+  auto put = [&](float v, int idx) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p st.shared.v2.u32 [%0], {%3, %4};\n\t@p add.u32 %0, %0, 8;\n\t}"
+        : "+r"(at)
+        : "f"(v), "f"(edge), "r"(idx), "r"(__float_as_uint(v))
+        : "memory");
+  };
+  auto put_checked = [&](float v, int idx) {
+    if (!(v < edge)) {
+      const uint64_t raw = ((uint64_t)__float_as_uint(v) << 32) | (uint32_t)idx;
+      if (pos < seg_cap) {
+        seg[pos] = raw;
+      } else {
+        spill_push(ctrl, spill, spill_cap, raw);
       }
-      if (lane == 0) {
-        ctrl->t = ok ? ts * fine + tf : -1;
-        ctrl->above = ok ? need - above - above_f : 0u;
-        ctrl->cnt = cnt_t;
-        ctrl->run_total = total;
-        ctrl->focus_bin = focus_bin;
-      }
+      ++pos;
     }
-    __syncthreads();
-    FFTOPK_MARK(43);
-    DualPick d;
-    d.focus_bin = ctrl->focus_bin;
-    d.ok = ctrl->t >= 0;
-    d.pbits = 12;
-    d.prefix = (uint32_t)ctrl->t;
-    d.need2 = ctrl->above;
-    d.cnt = ctrl->cnt;
-    d.total = ctrl->run_total;
-    return d;
-  }
-  uint32_t* tot = ctrl->tot[pick_no & 1];
-  uint32_t* tot2 = ctrl->tot2[pick_no & 1];
-  for (int i = tid; i < C * kSup; i += NT) {
-    const int q = i / kSup, b = i % kSup;
-    const uint32_t* ra = C == 1 ? sa : cluster.map_shared_rank(sa, q);
-    red_shared_add(&tot[b], ra[b]);
-    if (dual) {
-      const uint32_t* rb = C == 1 ? sb : cluster.map_shared_rank(sb, q);
-      red_shared_add(&ctrl->totb[b], rb[b]);
+  };
+  if (total <= seg_cap) {  // (uniform over the warp)
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      put(x[j].x, el0 + j * el_step);
+      put(x[j].y, el0 + j * el_step + 1);
+      put(x[j].z, el0 + j * el_step + 2);
+      put(x[j].w, el0 + j * el_step + 3);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      put_checked(x[j].x, el0 + j * el_step);
+      put_checked(x[j].y, el0 + j * el_step + 1);
+      put_checked(x[j].z, el0 + j * el_step + 2);
+      put_checked(x[j].w, el0 + j * el_step + 3);
     }
   }
-  __syncthreads();
-  FFTOPK_MARK(40);
-  if (warp == 0) {
-    const uint32_t lo = tot[2 * lane], hi = tot[2 * lane + 1];
-    const uint32_t total = warp_sum(lo + hi);
-    const uint32_t need = need_of(total);
-    // four super-bins = 256 bins of A = one value of the top four key bits
-    const uint32_t pair = lo + hi;
-    const uint32_t grp = pair + __shfl_xor_sync(kFull, pair, 1);
-    const unsigned one = __ballot_sync(kFull, fine_histogram_usable(dual, total, grp));
-    const bool use_b = one != 0u;
-    const uint32_t lob = ctrl->totb[2 * lane], hib = ctrl->totb[2 * lane + 1];
-    uint32_t above = 0, cnt = 0;
-    int ts = -1;
-    const uint32_t plo = use_b ? lob : lo, phi = use_b ? hib : hi;
-    const bool ok = need > 0 && warp_pick64(plo, phi, need, ts, above, cnt);
-    if (lane == 0) {
-      ctrl->sup_sel = ok ? ts : -1;
-      ctrl->sup_above = above;
-      ctrl->need = need;
-      ctrl->run_total = total;
-      ctrl->dual_b = use_b ? 1u : 0u;
-      ctrl->dual_g = use_b ? (uint32_t)((__ffs(one) - 1) >> 1) : 0u;
-    }
-  }
-  __syncthreads();
-  FFTOPK_MARK(41);
-  const int ssel = ctrl->sup_sel;
-  const bool use_b = ctrl->dual_b != 0u;
-  if (ssel >= 0) {
-    const uint32_t* h = use_b ? hb : ha;
-    for (int i = tid; i < C * kSup; i += NT) {
-      const int q = i / kSup, f = i % kSup;
-      const uint32_t* rh = C == 1 ? h : cluster.map_shared_rank(h, q);
-      red_shared_add(&tot2[f], rh[ssel * fine + f]);
-    }
-  }
-  __syncthreads();
-  FFTOPK_MARK(42);
-  if (tid < kSup) {
-    ctrl->tot[(pick_no + 1) & 1][tid] = 0u;
-    ctrl->tot2[(pick_no + 1) & 1][tid] = 0u;
-  }
-  ++pick_no;
-  if (warp == 0) {
-    int tf = -1;
-    uint32_t above_f = 0, cnt_t = 0;
-    bool ok = false;
-    if (ssel >= 0) {
-      const uint32_t lo = tot2[2 * lane], hi = tot2[2 * lane + 1];
-      ok = warp_pick64(lo, hi, ctrl->need - ctrl->sup_above, tf, above_f, cnt_t);
-    }
-    if (lane == 0) {
-      ctrl->t = ok ? ssel * fine + tf : -1;
-      ctrl->above = ok ? ctrl->need - ctrl->sup_above - above_f : 0u;
-      ctrl->cnt = cnt_t;
-    }
-  }
-  __syncthreads();
-  FFTOPK_MARK(43);
-  DualPick d;
-  d.focus_bin = -1;
-  d.ok = ctrl->t >= 0;
-  d.pbits = use_b ? 16 : 12;
-  d.prefix = guess_prefix(use_b, ctrl->dual_g, (uint32_t)ctrl->t);
-  d.need2 = ctrl->above;
-  d.cnt = ctrl->cnt;
-  d.total = ctrl->run_total;
-  return d;
+  return total;
 }
+
+// The sample of a row: `nb` batches of G slabs of 32 granules per warp, spread evenly over the whole row
+// (uniform in position, so recency-correlated logits are sampled fairly). Every CTA of a cluster takes
+// the SAME sample, so each finds the same guess by itself: no exchange of histograms and no cluster
+// barrier in front of the search. A row that is no larger than the sample is read completely.
+// Granules that straddle the row's ends are left out.
+template <int NT, int G>
+struct RowSample {
+  int i0, gi;  // first granule completely inside the row, and how many there are
+  int nb;      // a power of two
+  bool whole;
+  __device__ __forceinline__ int granule(int b, int u) const {
+    constexpr int kLogSlabs = (NT == 1024 ? 5 : (NT == 512 ? 4 : 3)) + (G == 4 ? 2 : 1);
+    static_assert(G == 2 || G == 4, "");
+    const int warp = threadIdx.x >> 5;
+    const int sl = (b * G + u) * (NT / 32) + warp;
+    const int first = whole ? sl * 32 : ((int)(((uint64_t)(uint32_t)gi * (uint32_t)sl) >> (kLogSlabs + (31 - __clz(nb)))) & ~7);
+    return first + lane_id();
+  }
+  __device__ __forceinline__ bool valid(int g) const { return !whole || g < gi; }
+  __device__ __forceinline__ uint32_t size() const { return 4u * (uint32_t)(whole ? gi : NT * G * nb); }
+  template <class T>
+  __device__ __forceinline__ void load(const T* gbase, int b, float4 (&x)[G]) const {
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const int g = granule(b, u);
+      if (valid(g)) x[u] = Elem<T>::ld4(gbase, i0 + g);
+    }
+  }
+  template <class Op>
+  __device__ __forceinline__ void use(int b, const float4 (&x)[G], Op&& op) const {
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      if (!whole || valid(granule(b, u))) {
+        op(__float_as_uint(x[u].x));
+        op(__float_as_uint(x[u].y));
+        op(__float_as_uint(x[u].z));
+        op(__float_as_uint(x[u].w));
+      }
+    }
+  }
+};
+// what the sample search tells the CTA to do (Ctrl::guess_flags)
+constexpr uint32_t kGuessCoarse = 1u;  // the guessed bin is crowded: look at the sample again, inside that bin
+constexpr uint32_t kGuessGiveUp = 2u;  // the guess admits far more than there is room for: full histograms at once
 
 // Everything one CTA needs to know about its row and its shared memory.
 template <int NT, class T>
@@ -579,7 +545,7 @@ __device__ __forceinline__ void emit_winner(const Cx& cx, uint32_t base_w, uint3
 // Returns the final mode; `need`, `P` and `r` describe where it stopped.
 // -----------------------------------------------------------------------------------------
 template <int NT, class T>
-__device__ __forceinline__ int refine_from_data(RowCtx<NT, T>& cx, uint32_t& need, uint32_t& P, int& r, int& pick_no) {
+__device__ __forceinline__ int refine_from_data(const RowCtx<NT, T>& cx, uint32_t& need_out, uint32_t& P_out, int& r_out) {
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -597,15 +563,13 @@ __device__ __forceinline__ int refine_from_data(RowCtx<NT, T>& cx, uint32_t& nee
       ctrl->pub_flag = 0u;
       ctrl->win_count = 0u;   // rank 0's copies are the cluster-wide counters; nobody touches
       ctrl->cand_count = 0u;  // them again before the cluster barrier of the first histogram pass
-      ctrl->over_flag = 0u;
-      ctrl->max_key = 0u;
     }
     if (tid < kSup) {
       ctrl->tot[0][tid] = ctrl->tot[1][tid] = 0u;
       ctrl->tot2[0][tid] = ctrl->tot2[1][tid] = 0u;
     }
-    pick_no = 0;
   }
+  int pick_no = 0;  // number of cluster-wide searches so far (selects their total buffers)
   __syncthreads();
   {
     uint32_t* h0 = cx.hist(0);
@@ -613,10 +577,10 @@ __device__ __forceinline__ int refine_from_data(RowCtx<NT, T>& cx, uint32_t& nee
   }
   __syncthreads();
 
-  need = cx.k;
-  P = 0;
+  uint32_t need = cx.k, P = 0;
   int mode = kModeAbort;
-  for (r = 0;; ++r) {
+  int r = 0;
+  for (;; ++r) {
     const int w = round_width(r);
     const int shift = round_shift(r);
     const int nb = 1 << w;
@@ -740,20 +704,74 @@ __device__ __forceinline__ int refine_from_data(RowCtx<NT, T>& cx, uint32_t& nee
     }
     break;
   }
+  need_out = need;
+  P_out = P;
+  r_out = r;
   return mode;
+}
+
+// The full-histogram path from start to finish, out of line (the common path neither pays its registers
+// nor its instructions). Returns the row's threshold as the next call's guess (rank 0; 0: none).
+template <int NT, bool kTrack, class T>
+__device__ __noinline__ uint32_t select_by_full_histograms(const RowCtx<NT, T> passed) {
+  const RowCtx<NT, T> cx = passed;  // (out of the stack, into registers)
+  cg::cluster_group cluster = cg::this_cluster();
+  uint32_t need = 0u, P = 0u;
+  int r = 0;
+  const int mode = refine_from_data<NT, T>(cx, need, P, r);
+  cluster_sync(cluster, cx.C);  // candidates that peers pushed into rank 0 are complete
+  if (cx.rank != 0) return 0u;
+  uint32_t thr = 0u;
+  if (mode == kModeGather) {
+    // every candidate shares the key prefix P above bit `shift` of the key
+    const int shift = round_shift(r);
+    const uint64_t lo = (uint64_t)P << (32 + shift);
+    const uint64_t cap = lo | ((1ull << (32 + shift)) - 1ull);
+    const DenseCands<NT> src{cx.cand, (int)min(cx.ctrl->cand_count, (uint32_t)cx.cand_cap)};
+    cta_finish<NT, DenseCands<NT>, kTrack>(src, need, lo, cap, cap, false, 32 - __clz(cx.sh.len - 1), cx.hist(1), cx.ctrl,
+                                           cx.out_idx, cx.out_key, cx.k - need, cx.k, cx.idx_offset, cx.status, cx.page,
+                                           (uint32_t)src.n);
+    if constexpr (kTrack) {
+      __syncthreads();
+      thr = cx.ctrl->thr_key != 0xffffffffu ? cx.ctrl->thr_key : 0u;
+    }
+  } else if (mode == kModeTakeAll || mode == kModeTies) {
+    // no finish ran: the lower edge of the bin the threshold was found in (a lower bound: the next
+    // call then admits a few more candidates and tightens it again)
+    thr = P << round_shift(r);
+  } else if (threadIdx.x == 0 && cx.status) {
+    atomicOr(cx.status, (uint32_t)FFTOPK_ST_INTERNAL);
+  }
+  return thr;
 }
 
 #ifndef FFTOPK_CTAS_512
 #define FFTOPK_CTAS_512 2
 #endif
+// Form of the kernel: a row has one CTA (a grid of clusters of one), or a cluster of 2 to 16 with one CTA
+// per SM, or one of which two CTAs - of different calls - share an SM (512 threads; the others have the
+// registers for one form only).
+enum Form : int { kLoneForm = 0, kRoomyForm = 1, kTightForm = 2 };
+template <int NT>
+__host__ __device__ constexpr int min_ctas(int form) {
+  return NT == 512 ? (form == kRoomyForm ? 1 : FFTOPK_CTAS_512) : 1024 / NT;
+}
+// Granules a thread keeps in registers when its CTA's whole shard fits: with 512 threads and one CTA
+// per SM (128 registers a thread) rows of up to 256K elements over 16 CTAs.
+template <int NT>
+__host__ __device__ constexpr int reg_slabs(int form) {
+  return NT == 512 && form == kRoomyForm ? 2 * FFTOPK_REG_SLABS : FFTOPK_REG_SLABS;
+}
 // kAnyK = false: k is the constant 2048 of the reference's op (the compiler folds it: one register
 // less in a kernel that sits at its register limit); true: k comes from the parameters.
-template <int NT, bool kAnyK, bool kWarm = false, class T = float>
+template <int NT, bool kAnyK, bool kWarm, class T, int kForm>
 __device__ __forceinline__ void select_row(const SelectParams& p) {
+  constexpr bool kLone = kForm == kLoneForm;
+  constexpr int kRegSlabs = reg_slabs<NT>(kForm);
   RowCtx<NT, T> cx;
   cg::cluster_group cluster = cg::this_cluster();
-  const int C = cx.C = (int)cluster.num_blocks();
-  const int rank = cx.rank = (int)cluster.block_rank();
+  const int C = cx.C = kLone ? 1 : (int)cluster.num_blocks();
+  const int rank = cx.rank = kLone ? 0 : (int)cluster.block_rank();
   const int row = (int)(blockIdx.x / (unsigned)C);
   // Back-to-back kernels on one stream (every launch of this kernel is a programmatic dependent
   // launch): once every CTA of this grid has passed this point - or exited - the next kernel on
@@ -842,28 +860,21 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   sh.g1 = min(sh.g0 + per, gn);
   sh.i0 = max(sh.g0, sh.a > 0 ? 1 : 0);
   sh.i1 = max(sh.i0, min(sh.g1, ((sh.a + len) & 3) ? gn - 1 : gn));
-  const int n_g = sh.g1 - sh.g0;
   // Whole shard in registers (same answer in every CTA of the cluster: `per` is rank-independent).
-#ifndef FFTOPK_EXACT_SLABS
-#define FFTOPK_EXACT_SLABS 3  // (with 4 the 256K row of the decode sweep took 16.4 us instead of 13.9 us)
-#endif
-  const bool exact = per <= NT * FFTOPK_EXACT_SLABS;
-  // A second, finer sample histogram (see cluster_pick_dual) saves a cluster-wide sample round on
-  // crowded data. A lone CTA does that round without any cluster traffic, and only when it is
-  // needed, which costs it less than building the second histogram for every row.
-  const bool dual = !exact && C > 1;
-  // sampled mode: slabs read per warp
-  #ifndef FFTOPK_SAMPLE_GRANULES
-#define FFTOPK_SAMPLE_GRANULES 2048
-#endif
-  const int ns = min(kRegSlabs, max(1, FFTOPK_SAMPLE_GRANULES / (C * NT)));
+  const bool in_regs = per <= NT * kRegSlabs;
+  constexpr int G = NT >= 1024 ? 2 : 4;  // sample granules per thread and batch
+  RowSample<NT, G> smp;
+  smp.i0 = sh.a > 0 ? 1 : 0;
+  smp.gi = ((sh.a + len) & 3 ? gn - 1 : gn) - smp.i0;
+  // 8K elements; 16K for rows so long that 8K would need a margin of several thousand candidates
+  smp.nb = (NT >= 512 ? 1 : 2) << (len > FFTOPK_LONG_SAMPLE ? 1 : 0);
+  smp.whole = smp.gi <= NT * G * smp.nb;
 
   // ---- warm start: a key guess of the row's k-th largest element from an earlier call ----------
-  // With a guess the row skips the sample, its histograms and the cluster-wide search: it is
-  // filtered at once against the guess (minus the caller's margin). The checks after the filter
-  // are the same as for a sampled guess - at least k admitted, no list overflowed - and a guess
-  // that fails them sends the row to the full-histogram path, so the result is exact whatever the
-  // guess was.
+  // With a guess the row skips the sample, its histogram and the search: it is filtered at once
+  // against the guess (minus the caller's margin). The checks after the filter are the same as for
+  // a sampled guess - at least k admitted, no list overflowed - and a guess that fails them sends
+  // the row to the full-histogram path, so the result is exact whatever the guess was.
   uint32_t warm_key = 0u;
   if constexpr (kWarm) {
     if (p.prev_threshold != nullptr && !p.force_slow) {
@@ -872,412 +883,301 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     }
   }
   const bool warm = kWarm && warm_key != 0u;  // (uniform over the cluster)
+  const bool sampled = !warm && !p.force_slow;
 
-  // ---- prologue: clear the search totals, both histograms and the control block --------------
-  if (tid < kSup) {
-    ctrl->tot[0][tid] = 0u;  // (the buffers with index 1 are cleared by the first search)
-    ctrl->tot2[0][tid] = 0u;
-    ctrl->totb[tid] = 0u;
-  }
-  {
-    uint4* h4 = reinterpret_cast<uint4*>(cx.hist(0));
-    if (!warm) {
-      for (int i = tid; i < 2 * kMaxBins / 4; i += NT) h4[i] = make_uint4(0u, 0u, 0u, 0u);
+  // ---- loads: the shard, if it fits in registers, and the sample ----------------------------------
+  float4 xr[kRegSlabs];
+  const float ninf = __uint_as_float(0xff800000u);
+  if (in_regs) {
+#pragma unroll
+    for (int j = 0; j < kRegSlabs; ++j) {
+      const int g = sh.g0 + j * NT + tid;
+      xr[j] = make_float4(ninf, ninf, ninf, ninf);
+      if (g >= sh.i0 && g < sh.i1) xr[j] = Elem<T>::ld4(sh.gbase, g);
     }
+  }
+  float4 xs[G];
+  if (sampled) smp.load(sh.gbase, 0, xs);
+  // ---- clear both histograms and the control block --------------------------------------------------
+  uint32_t* const fin_hist = cx.hist(1);  // round 0 of the finish
+  const uint32_t h0 = smem_u32(cx.hist(0)), fh = smem_u32(fin_hist);  // shared addresses
+  {
+    for (int i = tid + (warm ? kMaxBins / 4 : 0); i < (kMaxBins + kFinishBins) / 4; i += NT) sts_zero16(h0 + i * 16);
     if (tid == 0) {
       if constexpr (kWarm) ctrl->thr_key = 0xffffffffu;
-      ctrl->win_count = 0u;
-      ctrl->cand_count = 0u;
+      ctrl->extra_count = 0u;
       ctrl->pub_flag = 0u;
-      ctrl->over_flag = 0u;
-      ctrl->max_key = 0u;
-      ctrl->wslot = 0u;
-      ctrl->cslot = 0u;
       ctrl->lcount = 0u;
-      ctrl->spill_kmax = 0u;
+      ctrl->guess_flags = 0u;
+      ctrl->guess = 0u;
+      ctrl->focus = 0u;
 #ifdef FFTOPK_CHECKED
       ctrl->status_ptr = p.status;
 #endif
     }
-  }
-  // ---- sample (or, for a shard that fits in registers, the whole shard) ------------------------
-  // exact:   thread keeps granules g0 + j*NT + tid, j < kRegSlabs
-  // sampled: warp w reads one 512-byte slab at g0 + w*stride; the slabs are spread evenly over the
-  //          shard, so together the cluster samples the row uniformly in position
-  float4 xr[kRegSlabs];
-  int gr[kRegSlabs];
-#pragma unroll
-  for (int j = 0; j < kRegSlabs; ++j) {
-    gr[j] = sh.g1;  // "none"
-    xr[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  if (warm) {
-    // Rank 0's counters are cleared: tell the cluster now, check just before the first remote
-    // access - the barrier's latency hides behind the filter pass.
-    __syncthreads();
-    if (C > 1) cluster.barrier_arrive();
-  } else {
-  {
-    if (exact) {
-#pragma unroll
-      for (int j = 0; j < kRegSlabs; ++j) {
-        const int g = sh.g0 + j * NT + tid;
-        if (g < sh.g1) gr[j] = g;
-        if (g >= sh.i0 && g < sh.i1) xr[j] = Elem<T>::ld4(sh.gbase, g);
+    if (sampled && warp == NW - 1) {
+      // The sample rank whose true rank is >= k with overwhelming probability (m expected sample
+      // elements among the true top k, plus five standard deviations), and the mirror image: a
+      // sample element the threshold will not lie above (or the sample's largest). Of a row that
+      // was read completely: rank k itself, or none if the granules left out bring it below k. One
+      // warp works this out while the loads travel (a division and a square root in every warp
+      // would cost the CTA as much as the search itself).
+      const uint32_t n_s = smp.size();
+      uint32_t need_s = K <= n_s ? K : 0u, hi_s = need_s;
+      if (!smp.whole) {
+        need_s = sample_lower_rank(K, n_s, (float)len);
+        hi_s = max(sample_upper_rank(K, n_s, (float)len), 1u);
       }
-    } else {
-      // ns slabs per warp: small clusters of small CTAs sample more per thread, so that a row
-      // is always sampled at about 8K positions or more (a thin sample needs a wide safety margin,
-      // which means more candidates to carry)
-#pragma unroll
-      for (int j = 0; j < kRegSlabs; ++j) {
-        if (j < ns) {
-          int g;
-          if (n_g >= NT * ns) {
-            const int stride = (n_g / (NW * ns)) & ~7;
-            g = sh.g0 + (warp * ns + j) * stride + lane;
-          } else {
-            g = sh.g0 + j * NT + tid;
-          }
-          if (g < sh.g1) gr[j] = g;
-          if (g >= sh.i0 && g < sh.i1) xr[j] = Elem<T>::ld4(sh.gbase, g);
-        }
+      if (lane == 0) {
+        ctrl->need = need_s;
+        ctrl->need_hi = hi_s;
       }
     }
-    // granules straddling the row's ends (at most two per row), after every bulk load is in flight
+  }
+  if (in_regs) {  // granules straddling the row's ends (at most two per row)
 #pragma unroll
     for (int j = 0; j < kRegSlabs; ++j) {
-      if (gr[j] < sh.g1 && (gr[j] < sh.i0 || gr[j] >= sh.i1))
-        xr[j] = load_granule_partial(sh.gbase, sh.a, sh.len, gr[j], 0.f);
+      const int g = sh.g0 + j * NT + tid;
+      if (g < sh.g1 && (g < sh.i0 || g >= sh.i1)) xr[j] = load_granule_partial(sh.gbase, sh.a, sh.len, g, ninf);
     }
   }
-  __syncthreads();  // histograms are cleared
+  __syncthreads();  // histograms and counters are clear
+  // Every CTA tells the cluster so, and checks just before its first remote access: the barrier's
+  // latency hides behind the sample and the filter.
+  if (C > 1) cluster.barrier_arrive();
   FFTOPK_MARK(1);
-  {
-    uint32_t* h0 = cx.hist(0);
-#pragma unroll
-    for (int j = 0; j < kRegSlabs; ++j) {
-      if (j < ns || exact) {  // uniform over the CTA
-        const bool in = gr[j] < sh.g1;
-        const int i0 = 4 * gr[j] - sh.a;
-        const float xv[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t key = fftopk_key_from_bits(__float_as_uint(xv[e]));
-          const bool ok = in && (unsigned)(i0 + e) < (unsigned)len;
-          hist_add(h0, key >> 20, ok);
-          if (dual) hist_add(h0 + kMaxBins, (key >> 16) & 0xfffu, ok);  // histogram B (see cluster_pick_dual)
-        }
-      }
-    }
+
+  uint32_t gkey = warm_key;  // what the shard is filtered with: a lower bound of the k-th largest key
+  // A bound the threshold will not lie above (the finish's first digit spreads [guess, focus] over
+  // its bins): from the sample; of a warm guess, twice the margin and 1/16 octave.
+  uint32_t focus_key = 0u;
+  bool guessed = warm;
+  if constexpr (kWarm) {
+    const uint32_t reach = 2u * min(p.warm_margin, 0x3fffffffu) + (1u << 19);
+    focus_key = warm_key > 0xffffffffu - reach ? 0xffffffffu : warm_key + reach;
   }
-  // (Asking L2 for the shard here with prefetch.global.L2, to hide HBM latency behind the
-  // cluster-wide search, was measured: issuing the requests cost about as much as it saved.)
-  __syncthreads();
-  compute_sup<NT>(cx.hist(0), cx.sup(0), kMaxBins);
-  if (dual) compute_sup<NT>(cx.hist(1), cx.sup(1), kMaxBins);
-  FFTOPK_MARK(2);
-  cluster_sync(cluster, C);  // #1: sample histograms complete
-  }  // (!warm)
-  FFTOPK_MARK(3);
-
-  uint32_t need = K;
-  uint32_t P = 0;
-  int r = 0;
-  int mode = kModeAbort;
-  int pick_no = 0;        // number of cluster-wide searches so far (selects their total buffers)
-  // what the finish starts from when the sampled path gathered (r < 0): the candidates' range,
-  // the bound the first digit is focused below, and whether that digit's histogram is built
-  // (as keys: the composites' bounds are (lo << 32) and (cap << 32) | 0xffffffff)
-  uint32_t fin_lo = 0u, fin_cap = 0u, fin_focus = 0u;
-  bool fin_hist = false;
-  auto low_end = [](uint32_t key) { return (uint64_t)key << 32; };
-  auto high_end = [](uint32_t key) { return ((uint64_t)key << 32) | 0xffffffffull; };
-  int fin_wn = 0, fin_sn = 0;  // ... and, for a lone CTA, this warp's segment length and the spill count
-
-  // Filter the shard against a key guess, gather what passes in rank 0 and check it: fills in what
-  // the finish starts from, or sets mode to kModeFallback. `focus_bin` (lone CTA): a bin of `pbits`
-  // bits the threshold will not lie above, or -1. `after_arrive`: the CTA has arrived at a cluster
-  // barrier that must complete before rank 0's counters are touched.
-  auto filter_gather = [&](const uint32_t gkey, const int focus_bin, const int pbits, const bool after_arrive) {
-    // Lower edge of the guess as a float: key(x) >= gkey  <=>  !(x < edge), NaN included.
-    // Keys outside the range real values map to (below -inf's key / above +inf's) admit
-    // everything instead; that only lengthens the lists.
-    const float edge = __uint_as_float(guess_edge_bits(gkey));
-    // list layout: one segment per warp, then the spill area (an eighth of the list)
-    const uint32_t spill_cap = (uint32_t)p.list_cap / 8u;
-    const uint32_t seg_cap = ((uint32_t)p.list_cap - spill_cap) / NW;
-    uint64_t* seg = list + (size_t)warp * seg_cap;
-    uint64_t* spill = list + (size_t)NW * seg_cap;
-    uint32_t kmax = 0u;
-    // A lone CTA that knows a bin the threshold will not lie above builds the histogram of the
-    // finish's first round while it converts its candidates (they pass through registers there
-    // anyway): the digit rule needs only the guess and that bound.
-    const uint32_t lowkey = guess_low_key(gkey);
-    fin_lo = lowkey;
-    if (C == 1 && focus_bin >= 0) {
-      fin_focus = (((uint32_t)focus_bin + 1u) << (32 - pbits)) - 1u;
-      fin_hist = fin_focus >= lowkey && make_finish_digit(low_end(lowkey), high_end(fin_focus)).key_only();
+  if (sampled) {
+    const uint32_t wtot_s = smem_u32(ctrl->wtot);
+    for (int b = 0;;) {
+      smp.use(b, xs, [&](uint32_t bits) { red_shared_inc(h0 + sample_digit(bits) * 4u); });
+      if (++b >= smp.nb) break;
+      smp.load(sh.gbase, b, xs);
     }
-    if (fin_hist) {  // (uniform over the CTA)
-      uint32_t* fh = cx.hist(0);
-      for (int b = tid; b < kFinishBins; b += NT) fh[b] = 0u;
-      __syncthreads();
-    }
-    uint32_t* fh = cx.hist(0);
-    auto round0 = [&](uint32_t key) {
-      if (fin_hist) red_shared_add(&fh[make_finish_digit(low_end(fin_lo), high_end(fin_focus)).of_key(key)], 1u);
+    __syncthreads();
+    FFTOPK_MARK(2);
+    const uint32_t room = (uint32_t)(C == 1 ? p.list_cap : p.cand_cap);
+    // (one thread, when it has found the bin) what the guess is and what to do about it. A bin that
+    // holds more than ~2k row elements - values crowded into a sliver of the key space - is worth a
+    // second look at the sample, inside that bin. (Below that, carrying the extra candidates is
+    // cheaper. And a bin that still holds most of the bin it was cut out of holds copies of one value:
+    // cutting it further thins nothing out.) A guess that admits far more than there is room for is not worth the pass.
+    auto judge = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
+      const bool copies = cnt >= parent - parent / 4u;
+      uint32_t flags = 0u;
+      if (width > 1u && !copies && sample_bin_too_coarse(cnt, smp.size(), (float)len, K, kCoarseFactor)) {
+        flags = kGuessCoarse;
+      } else if (sample_admits_too_much(above + cnt, smp.size(), (float)len, room)) {
+        flags = kGuessGiveUp;
+      } else if (copies) {
+        ctrl->focus = low + width - 1u;  // the threshold is that value: the finish need not search above it
+      }
+      ctrl->guess = low;
+      ctrl->guess_flags = flags;
+      if (flags & kGuessCoarse) {
+        ctrl->cnt = width;
+        ctrl->local_c = cnt;
+        ctrl->above = above;
+        ctrl->need = rest;
+      }
     };
-#ifndef FFTOPK_U512
-#define FFTOPK_U512 8
-#endif
-    constexpr int U = NT >= 1024 ? 4 : FFTOPK_U512;
-    // about 1.5 k candidates per row: up to ~192K elements most trips of the hit loop have work
-    const bool stage = len <= 196608;
-    const uint32_t wcnt = stage ? filter_shard<NT, U, true>(sh, edge, seg, seg_cap, ctrl, spill, spill_cap, kmax, round0)
-                                : filter_shard<NT, U, false>(sh, edge, seg, seg_cap, ctrl, spill, spill_cap, kmax, round0);
-    FFTOPK_MARK(8);
-    if (after_arrive && C > 1) cluster.barrier_wait();  // every CTA's counters are cleared (see the prologue)
-    const uint32_t wown = min(wcnt, seg_cap);
-    fin_wn = (int)wown;
-    kmax = __reduce_max_sync(kFull, kmax);
-    if (lane == 0) {
-      ctrl->wtot[warp] = wown;
-      ctrl->wmax[warp] = kmax;
-    }
-    __syncthreads();
-    FFTOPK_MARK(44);
-    // hand the candidates to rank 0: one remote atomic per CTA allocates the range
-    if (warp == 0) {
-      const uint32_t wmine = lane < NW ? ctrl->wtot[lane] : 0u;
-      uint32_t incl = wmine;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t v = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += v;
-      }
-      const uint32_t cmax = max(__reduce_max_sync(kFull, lane < NW ? ctrl->wmax[lane] : 0u), ctrl->spill_kmax);
-      uint32_t base = 0;
-      if (lane == 31) {
-        const uint32_t spill_n = min(ctrl->lcount, spill_cap);
-        base = atomicAdd(&cx.ctrl0->cand_count, incl + spill_n);
-        atomicMax(&cx.ctrl0->max_key, cmax);
-        if (ctrl->pub_flag) atomicOr(&cx.ctrl0->over_flag, 1u);
-        ctrl->base_c = base + incl;  // where the spill entries go
-      }
-      base = __shfl_sync(kFull, base, 31);
-      if (lane < NW) ctrl->wtot[lane] = base + incl - wmine;
-    }
-    __syncthreads();
-    FFTOPK_MARK(45);
-    fin_sn = (int)min(ctrl->lcount, spill_cap);
-    if (fin_hist) {  // the entries that went to the spill area
-      const uint32_t* sp32 = reinterpret_cast<const uint32_t*>(spill) + 1;
-      const FinishDigit dg = make_finish_digit(low_end(fin_lo), high_end(fin_focus));
-      for (int j = tid; j < fin_sn; j += NT) red_shared_add(&fh[dg.of_key(sp32[2 * j])], 1u);
-    }
-    if (C > 1) {
-      const uint32_t dst = ctrl->wtot[warp];
-      for (uint32_t j = lane; j < wown; j += 32) {
-        if (dst + j < (uint32_t)p.cand_cap) cx.cand0[dst + j] = seg[j];
-      }
-      const uint32_t sbase = ctrl->base_c;
-      for (uint32_t j = tid; j < (uint32_t)fin_sn; j += NT) {
-        if (sbase + j < (uint32_t)p.cand_cap) cx.cand0[sbase + j] = spill[j];
-      }
-    }
-    FFTOPK_MARK(46);
-    cluster_sync(cluster, C);  // #2: every candidate has landed in rank 0
-    FFTOPK_MARK(9);
     {
-      // every thread reads rank 0's totals itself (no broadcast barrier; for rank 0, whose finish
-      // is the critical path, these are local reads)
-      const Ctrl* c0 = rank == 0 ? ctrl : cx.ctrl0;
-      const uint32_t total = c0->cand_count;
-      const uint32_t over = c0->over_flag;
-      const uint32_t maxkey = c0->max_key;
-      // fewer than k admitted (the guess was too high), a list overflowed, or more than rank 0
-      // can hold: start over with full histograms
-      const uint32_t room = C == 1 ? 0xffffffffu : (uint32_t)p.cand_cap;  // (a lone CTA keeps them in the list)
-      mode = sampled_attempt_ok(over, total, K, room) ? kModeGather : kModeFallback;
-      // every candidate's key lies in [lowkey, maxkey]
-      fin_cap = maxkey;
-      if (fin_hist) {
-        if (fin_cap < fin_focus) fin_cap = fin_focus;  // (a looser bound keeps the digit rule of the histogram)
-      } else {
-        fin_focus = fin_cap;
-      }
+      const uint32_t need_s = ctrl->need, need_hi = ctrl->need_hi;
+      block_pick_sample<NT>(h0, need_s, need_hi, wtot_s,
+                            [&](uint32_t bin, uint32_t above, uint32_t cnt) {
+                              const uint32_t low = sample_digit_low(bin);
+                              judge(low, sample_digit_high(bin) - low + 1u, above, cnt, need_s - above, 0xffffffffu);
+                            },
+                            [&](uint32_t bin) { ctrl->focus = sample_digit_high(bin); });
     }
-    need = K;
-    P = 0;
-    r = -1;  // finish first, final barrier afterwards
-    FFTOPK_MARK(10);
-  };
-
-  if (p.force_slow) {
-    mode = kModeFallback;
-  } else if (warm) {
-    filter_gather(warm_key, -1, 12, true);
-    FFTOPK_MARK(4);
-    // (a miss is worth knowing about: the row is then selected by the full-histogram path)
-    if (mode == kModeFallback && rank == 0 && tid == 0 && p.status) atomicOr(p.status, (uint32_t)FFTOPK_ST_GUESS_MISSED);
-  } else if (exact) {
-    // ---- the sample is the row: its histogram gives the threshold bin directly -----------------
-    cluster_pick<NT>(
-        cluster, C, cx.hist(0), cx.sup(0), cx.xch, ctrl, pick_no, kMaxBins, [&](uint32_t) { return K; },
-        [&](Picked& pk) { decide_and_allocate(cx, pk, kModeFallback, false); });
-    mode = ctrl->mode;
-    FFTOPK_MARK(4);
-    if (mode == kModeGather || mode == kModeTakeAll) {
-      const uint32_t t = (uint32_t)ctrl->t;
-      const uint32_t base_w = ctrl->base_w, base_c = ctrl->base_c;
-      const bool take_eq = (mode == kModeTakeAll);
-      need = ctrl->above;
-      P = t;
-#pragma unroll
-      for (int j = 0; j < kRegSlabs; ++j) {
-        const int i0 = 4 * gr[j] - sh.a;
-        const float xv[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
-        if (gr[j] < sh.g1) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if ((unsigned)(i0 + e) < (unsigned)len) {
-              const uint32_t key = fftopk_key_from_bits(__float_as_uint(xv[e]));
-              const uint32_t bin = key >> 20;
-              if (bin > t || (take_eq && bin == t)) {
-                emit_winner(cx, base_w, key, i0 + e);
-              } else if (bin == t) {
-                const uint32_t slot = base_c + warp_alloc(&ctrl->cslot);
-                if (FFTOPK_CHECK(2, slot, p.cand_cap, p.status) && slot < (uint32_t)p.cand_cap)
-                  cx.cand0[slot] = ((uint64_t)key << 32) | (uint64_t)(~(uint32_t)(i0 + e));
-              }
-            }
-          }
-        }
-      }
-    }
-  } else {
-    // ---- sampled: pick a conservative lower bound from the sample, filter the shard once ------
-    // need_of: sample rank whose true rank is >= k with overwhelming probability
-    // (m expected sample elements among the true top k, plus five standard deviations).
-    const float flen = (float)len;
-    const DualPick dp = cluster_pick_dual<NT>(cluster, C, cx.hist(0), cx.sup(0), cx.hist(1), cx.sup(1), dual, ctrl, pick_no,
-                                              [&](uint32_t n_s) { return sample_lower_rank(K, n_s, flen); },
-                                              [&](uint32_t n_s) { return sample_upper_rank(K, n_s, flen); });
-    FFTOPK_MARK(4);
-    // If the sample says the guessed bin alone holds more than ~2k row elements (values crowded
-    // into a sliver of the key space), a second sample round on the next 12 key bits sharpens it.
-    // (Below that, carrying the extra candidates is cheaper than the round: measured 1.0-1.5 us
-    // per call on N(0,1) rows of 384K..2M elements.)
-#ifndef FFTOPK_1B_FACTOR
-#define FFTOPK_1B_FACTOR 2.0f
-#endif
-    int smode = !dp.ok ? kModeFallback
-                       : (sample_bin_too_coarse(dp.cnt, dp.total, flen, K, FFTOPK_1B_FACTOR) ? kModeNext : kModeGather);
-    uint32_t gkey = guess_key(dp.prefix, dp.pbits);
-    if (smode == kModeNext) {
-      const int sb = 32 - dp.pbits - 12;  // position of the next 12 bits
-      const uint32_t rem = dp.need2;
-      // Peers may still be reading, from this CTA, the histogram the guess was made on and both
-      // super-bin arrays; the other histogram buffer and the third super-bin array are free.
-      uint32_t* h1 = cx.hist(dp.pbits == 16 ? 0 : 1);
-      uint32_t* s1 = cx.sup(2);
-      {
-        uint4* h4 = reinterpret_cast<uint4*>(h1);
-        for (int i = tid; i < kMaxBins / 4; i += NT) h4[i] = make_uint4(0u, 0u, 0u, 0u);
+    FFTOPK_MARK(3);
+    uint32_t flags = ctrl->guess_flags;
+    while (flags & kGuessCoarse) {  // (uniform; every round narrows the bin by 12 bits)
+      const uint32_t low = ctrl->guess, width = ctrl->cnt, above0 = ctrl->above, rest = ctrl->need;
+      const uint32_t cnt0 = ctrl->local_c;
+      const int shift = max(0, 32 - __clz(width - 1u) - 12);
+      __syncthreads();  // everybody has read the result of the search before
+      for (int i = tid; i < kMaxBins / 4; i += NT) sts_zero16(h0 + i * 16);
+      if (tid == 0) ctrl->guess_flags = kGuessGiveUp;
+      __syncthreads();
+      for (int b = 0; b < smp.nb; ++b) {
+        smp.load(sh.gbase, b, xs);
+        smp.use(b, xs, [&](uint32_t bits) {
+          const uint32_t off = fftopk_key_from_bits(bits) - low;
+          if (off < width) red_shared_inc(h0 + ((off >> shift) & (uint32_t)(kMaxBins - 1)) * 4u);
+        });
       }
       __syncthreads();
-#pragma unroll
-      for (int j = 0; j < kRegSlabs; ++j) {
-        if (j < ns && gr[j] < sh.g1) {
-          const int e0 = 4 * gr[j] - sh.a;
-          const float xv[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t key = fftopk_key_from_bits(__float_as_uint(xv[e]));
-            hist_add(h1, (key >> sb) & 0xfffu,
-                     (unsigned)(e0 + e) < (unsigned)len && (key >> (32 - dp.pbits)) == dp.prefix);
-          }
-        }
-      }
-      __syncthreads();
-      compute_sup<NT>(h1, s1, kMaxBins);
-      cluster_sync(cluster, C);  // #1b
-      cluster_pick<NT>(
-          cluster, C, h1, s1, cx.xch, ctrl, pick_no, kMaxBins, [&](uint32_t) { return rem; },
-          [&](Picked& pk) {
-            if (lane == 0) {
-              ctrl->mode = pk.ok ? kModeGather : kModeFallback;
-              ctrl->t = pk.t;
-            }
-          });
-      smode = ctrl->mode;
-      gkey |= (uint32_t)ctrl->t << sb;
+      block_pick_sample<NT>(h0, rest, 0u, wtot_s,
+                            [&](uint32_t bin, uint32_t above, uint32_t cnt) {
+                              judge(low + (bin << shift), 1u << shift, above0 + above, cnt, rest - above, cnt0);
+                            },
+                            [&](uint32_t) {});
+      flags = ctrl->guess_flags;
       FFTOPK_MARK(11);
     }
-    if (smode == kModeGather) {
-      filter_gather(gkey, dp.focus_bin, dp.pbits, false);
-    } else {
-      mode = kModeFallback;
-    }
+    gkey = ctrl->guess;
+    focus_key = ctrl->focus;
+    guessed = flags == 0u;
   }
+  FFTOPK_MARK(4);
 
-  if (mode == kModeFallback) mode = refine_from_data<NT, T>(cx, need, P, r, pick_no);
+  uint32_t thr = 0u;  // this call's threshold key
+  int mode = kModeFallback;
+  auto low_end = [](uint32_t key) { return (uint64_t)key << 32; };
+  auto high_end = [](uint32_t key) { return ((uint64_t)key << 32) | 0xffffffffull; };
+  // list layout: one segment per warp, then the spill area (an eighth of the list)
+  const uint32_t spill_cap = (uint32_t)p.list_cap / 8u;
+  const uint32_t seg_cap = ((uint32_t)p.list_cap - spill_cap) / NW;
+  uint64_t* const seg = list + (size_t)warp * seg_cap;
+  uint64_t* const spill = list + (size_t)NW * seg_cap;
 
-  // Candidates that peers pushed into rank 0 are complete after a cluster barrier. The sampled
-  // path has had that barrier already (#2) and only needs one more so that rank 0 outlives the
-  // peers' reads of its counters: it goes after the finish, off the critical path. Every other
-  // path pushes right up to here, so the barrier comes first.
-  const bool finish_first = (r < 0);  // uniform over the cluster
-  FFTOPK_MARK(5);
-  if (!finish_first) cluster_sync(cluster, C);
-  FFTOPK_MARK(6);
-  if (mode == kModeGather && rank == 0) {
-    const int idx_bits = 32 - __clz(len - 1);
-    if (r < 0 && C == 1) {
-      // sampled path of a lone CTA: the warps' segments where the filter left them
-      const uint32_t spill_cap1 = (uint32_t)p.list_cap / 8u;
-      const uint32_t seg_cap1 = ((uint32_t)p.list_cap - spill_cap1) / NW;
-      const WarpSegCands<NT> src{list + (size_t)warp * seg_cap1, fin_wn, list + (size_t)NW * seg_cap1, fin_sn};
-      cta_finish<NT, WarpSegCands<NT>, kWarm>(src, need, low_end(fin_lo), high_end(fin_cap), high_end(fin_focus), fin_hist,
-                                              idx_bits, cx.hist(0), ctrl, out_idx, out_key, K - need, K, cx.idx_offset,
-                                              p.status, cx.page, ctrl->cand_count);
-    } else {
-      // every candidate shares the key prefix P above bit `sh` of the key (sampled path: range known)
-      const int sh = r < 0 ? 0 : round_shift(r);
-      const uint64_t lo = r < 0 ? low_end(fin_lo) : ((uint64_t)P << (32 + sh));
-      const uint64_t cap = r < 0 ? high_end(fin_cap) : (lo | ((1ull << (32 + sh)) - 1ull));
-      const DenseCands<NT> src{cx.cand, (int)min(ctrl->cand_count, (uint32_t)p.cand_cap)};
-      cta_finish<NT, DenseCands<NT>, kWarm>(src, need, lo, cap, cap, false, idx_bits, cx.hist(0), ctrl, out_idx, out_key,
-                                            K - need, K, cx.idx_offset, p.status, cx.page, (uint32_t)src.n);
+  // ---- filter the shard against the guess -------------------------------------------------------
+  // Lower edge of the guess as a float: key(x) >= gkey  <=>  !(x < edge), NaN included. Keys outside
+  // the range real values map to (below -inf's key / above +inf's) admit everything instead; that
+  // only lengthens the lists.
+  const float edge = __uint_as_float(guess_edge_bits(gkey));
+  const uint32_t lowkey = guess_low_key(gkey);  // every candidate's key lies in [lowkey, 0xffffffff]
+  if (focus_key <= lowkey) focus_key = 0xffffffffu;
+  constexpr int U = NT >= 1024 ? 4 : FFTOPK_U512;
+  uint32_t wcnt = 0u;
+  bool staged = false;
+  if (!guessed) {
+    // No guess to filter with: say so the way an overflowed list does. (Every step from here on
+    // depends on what the cluster's CTAs tell each other, not on what each has read for itself.)
+    if (tid == 0) ctrl->pub_flag = 1u;
+  } else if (in_regs && edge > ninf) {
+    wcnt = filter_regs<kRegSlabs>(xr, 4 * (sh.g0 + tid) - sh.a, 4 * NT, edge, seg, seg_cap, ctrl, spill, spill_cap);
+  } else if (len <= 196608) {  // about 1.5 k candidates per row: most trips of the hit loop have work
+    staged = true;
+    wcnt = filter_shard<NT, U, true>(sh, edge, seg, seg_cap, ctrl, spill, spill_cap);
+  } else {
+    wcnt = filter_shard<NT, U, false>(sh, edge, seg, seg_cap, ctrl, spill, spill_cap);
+  }
+  const uint32_t wown = min(wcnt, seg_cap);
+  FFTOPK_MARK(8);
+  bool have_hist = false;  // (lone CTA) round 0 of the finish has its histogram
+  const int region = C == 1 ? 0 : ((p.cand_cap - p.cand_cap / 4) / C);  // slots of each CTA in rank 0's buffer
+  int extra = 0;           // candidates beyond their CTAs' regions
+  uint32_t total = 0u;     // candidates of the row
+  uint32_t fin_sn = 0u;
+  if (C == 1) {
+    // ---- a lone CTA keeps its candidates where they are ------------------------------------------
+    // They become composites in place, and the histogram of the finish's first round is built on
+    // the way (they pass through registers here anyway).
+    const FinishDigit dg = make_finish_digit(low_end(lowkey), high_end(focus_key));
+    have_hist = dg.key_only();
+    const uint32_t seg_s = smem_u32(seg);
+    drain_segment(staged, sh, seg, wown, ctrl, [&](uint32_t j, uint64_t c) {
+      sts64(seg_s + j * 8u, (uint32_t)c, (uint32_t)(c >> 32));
+      if (have_hist) red_shared_inc(fh + dg.of_key((uint32_t)(c >> 32)) * 4u);
+    });
+    const uint32_t wn_s = smem_u32(ctrl->wmax);
+    if (lane == 0) sts32(wn_s + warp * 4, wown);  // (not wtot: the finish's search may write that before every warp has read it)
+    __syncthreads();
+    fin_sn = min(ctrl->lcount, spill_cap);
+    total = __reduce_add_sync(kFull, lane < NW ? lds32(wn_s + lane * 4) : 0u) + fin_sn;
+    if (have_hist && fin_sn > 0u) {  // (uniform) the entries that went to the spill area
+      const uint32_t sp = smem_u32(spill) + 4u;  // (the keys)
+      for (uint32_t j = tid; j < fin_sn; j += NT) red_shared_inc(fh + dg.of_key(lds32(sp + j * 8u)) * 4u);
+      __syncthreads();
     }
+    mode = sampled_attempt_ok(ctrl->pub_flag, total, K, 0xffffffffu) ? kModeGather : kModeFallback;
+  } else {
+    // ---- gather in rank 0 ----------------------------------------------------------------------
+    // Every CTA owns a region of rank 0's buffer and fills it densely, so no slot has to be asked
+    // for; only what does not fit there (a window of winners in one shard) takes a remote atomic and
+    // goes behind the last region. Every CTA tells every other its count, so that each decides by
+    // itself whether the guess held.
+    const uint32_t wn_s = smem_u32(ctrl->wtot);
+    if (lane == 0) sts32(wn_s + warp * 4, wown);
+    cluster.barrier_wait();  // every CTA's control block is clear (see the prologue)
+    __syncthreads();
+    FFTOPK_MARK(44);
+    const uint32_t w = lane < NW ? lds32(wn_s + lane * 4) : 0u;
+    const uint32_t own = __reduce_add_sync(kFull, w);
+    const uint32_t before = __reduce_add_sync(kFull, lane < warp ? w : 0u);
+    const uint32_t sn = min(ctrl->lcount, spill_cap);
+    if (warp == 0 && lane < C)
+      st_peer32(peer_smem(smem_u32(&ctrl->cnt_of[rank]), lane), (own + sn) | (ctrl->pub_flag ? kOverflowed : 0u));
+    uint32_t xbase = 0u;  // where the candidates beyond the region go: region * C + xbase + (their number - region)
+    if (own + sn > (uint32_t)region) {  // (uniform over the CTA)
+      if (tid == 0) ctrl->base_c = atomicAdd(&cx.ctrl0->extra_count, own + sn - (uint32_t)region);
+      __syncthreads();
+      xbase = ctrl->base_c;
+    }
+    const uint32_t cand0 = peer_smem(smem_u32(cx.cand), 0);
+    auto push = [&](uint32_t q, uint64_t c) {  // candidate number q of this CTA
+      uint32_t at = (uint32_t)(rank * region) + q;
+      if (q >= (uint32_t)region) at = (uint32_t)(C * region) + xbase + (q - (uint32_t)region);
+      if (at < (uint32_t)p.cand_cap) st_peer64(cand0 + at * 8u, c);
+    };
+    drain_segment(staged, sh, seg, wown, ctrl, [&](uint32_t j, uint64_t c) { push(before + j, c); });
+    for (uint32_t j = tid; j < sn; j += NT) push(own + j, spill[j]);
+    FFTOPK_MARK(46);
+    cluster.sync();  // every candidate has landed in rank 0, every CTA knows the counts
+    FFTOPK_MARK(9);
+    const uint32_t n_r = lane < C ? lds32(smem_u32(ctrl->cnt_of) + lane * 4) : 0u;
+    const uint32_t over = __any_sync(kFull, n_r >= kOverflowed) ? 1u : 0u;
+    const uint32_t cnt_r = n_r & (kOverflowed - 1u);
+    total = __reduce_add_sync(kFull, cnt_r);
+    extra = (int)__reduce_add_sync(kFull, cnt_r > (uint32_t)region ? cnt_r - (uint32_t)region : 0u);
+    // fewer than k admitted (the guess was too high), a list overflowed, or more than rank 0
+    // can hold: start over with full histograms
+    mode = sampled_attempt_ok(over | (extra > p.cand_cap - C * region ? 1u : 0u), total, K, 0xffffffffu) ? kModeGather
+                                                                                                       : kModeFallback;
   }
   if constexpr (kWarm) {
-    // This call's threshold for the next one: the smallest key the finish let win (the row's k-th
-    // largest key), or, where no finish ran, the lower edge of the bin the threshold was found in
-    // (a lower bound: the next call then admits a few more candidates and tightens it again).
-    if (rank == 0 && p.next_threshold != nullptr) {
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t thr = 0u;
-        if (mode == kModeGather) {
-          thr = ctrl->thr_key != 0xffffffffu ? ctrl->thr_key : 0u;
-        } else if ((mode == kModeTakeAll || mode == kModeTies) && r >= 0) {
-          thr = P << round_shift(r);
-        }
-        p.next_threshold[row] = thr;
-      }
-    }
+    // (a miss is worth knowing about: the row is then selected by the full-histogram path)
+    if (warm && mode == kModeFallback && rank == 0 && tid == 0 && p.status)
+      atomicOr(p.status, (uint32_t)FFTOPK_ST_GUESS_MISSED);
   }
-  FFTOPK_MARK(34);
-  if (finish_first) cluster_sync(cluster, C);
+  // The candidates are rank 0's business now. Nobody reads a peer's memory any more, so the others may
+  // leave, and rank 0 needs no barrier at the end.
+  if (mode == kModeGather && rank != 0) return;
+  FFTOPK_MARK(5);
+
+  const int idx_bits = 32 - __clz(len - 1);
+  if (mode == kModeGather) {
+    const uint64_t lo = low_end(lowkey), focus = high_end(focus_key);
+    if (C == 1) {
+      const WarpSegCands<NT> src{smem_u32(seg), (int)wown, smem_u32(spill), (int)fin_sn};
+      cta_finish<NT, WarpSegCands<NT>, kWarm>(src, K, lo, ~0ull, focus, have_hist, idx_bits, fin_hist, ctrl, out_idx, out_key,
+                                              0u, K, cx.idx_offset, p.status, cx.page, total, true);
+    } else {
+      const RegionCands<NT> src{smem_u32(cx.cand), smem_u32(ctrl->cnt_of), region, C, extra};
+      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lo, ~0ull, focus, false, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
+                                             K, cx.idx_offset, p.status, cx.page, total, true);
+    }
+    // This call's threshold for the next one: the smallest key the finish let win (the row's k-th
+    // largest key).
+    if constexpr (kWarm) {
+      __syncthreads();
+      thr = ctrl->thr_key != 0xffffffffu ? ctrl->thr_key : 0u;
+    }
+  } else {
+    const RowCtx<NT, T> ctx = cx;  // (a copy: an object that is passed on this way lives on the stack)
+    thr = select_by_full_histograms<NT, kWarm, T>(ctx);
+    if (rank != 0) return;
+  }
+  if constexpr (kWarm) {
+    if (tid == 0 && p.next_threshold != nullptr) p.next_threshold[row] = thr;
+  }
   FFTOPK_MARK(7);
-  if (tid == 0 && p.status && mode == kModeAbort) atomicOr(p.status, (uint32_t)FFTOPK_ST_INTERNAL);
 }
 
-template <int NT, bool kAnyK = false, bool kWarm = false, class T = float>
-__global__ void __launch_bounds__(NT, (NT == 512 ? FFTOPK_CTAS_512 : 1024 / NT)) select2048_kernel(const SelectParams p) {
-  select_row<NT, kAnyK, kWarm, T>(p);
+template <int NT, int kForm, bool kAnyK = false, bool kWarm = false, class T = float>
+__global__ void __launch_bounds__(NT, min_ctas<NT>(kForm)) select2048_kernel(const SelectParams p) {
+  select_row<NT, kAnyK, kWarm, T, kForm>(p);
   if (p.cp_publish) {
     // Context-parallel publication folded into the selection: the CTA's barrier orders every
     // thread's output writes before thread 0's arrival, a release at device scope (one operation
@@ -1325,8 +1225,7 @@ struct CpFused {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(NT, (NT == 512 ? FFTOPK_CTAS_512 : 1024 / NT)) select_merge2048_kernel(const SelectParams p,
-                                                                                                      const CpFused f) {
+__global__ void __launch_bounds__(NT, min_ctas<NT>(kRoomyForm)) select_merge2048_kernel(const SelectParams p, const CpFused f) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
@@ -1340,7 +1239,11 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? FFTOPK_CTAS_512 : 1024 / NT))
   // (the previous call's update of the counter is complete - stream order - and this call's comes
   // at the very end: every CTA of the cluster reads the same value)
   const uint32_t epoch = f.epoch ? f.epoch : __ldcg(my_epoch) + 1u;
-  select_row<NT, false>(p);
+  if (C == 1) {
+    select_row<NT, false, false, float, kLoneForm>(p);
+  } else {
+    select_row<NT, false, false, float, kRoomyForm>(p);
+  }
   // Every output of the row is written: by this CTA, or by its peers before a cluster barrier
   // this CTA has passed.
   FFTOPK_MARK(60);
@@ -1431,36 +1334,47 @@ constexpr int64_t kOverlapShortRow = 196608;
 constexpr int kOverlapListCap = 3072, kOverlapCandCap = 6144;   // two CTAs per SM
 
 
-template <int NT>
-int setup_kernel(int smem_optin) {
-  cudaError_t e = cudaFuncSetAttribute(select2048_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-  if (e != cudaSuccess) return cuda_fail(e);
-  e = cudaFuncSetAttribute(select2048_kernel<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return cuda_fail(e);
-  e = cudaFuncSetAttribute(select2048_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-  if (e != cudaSuccess) return cuda_fail(e);
-  e = cudaFuncSetAttribute(select2048_kernel<NT, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return cuda_fail(e);
-  if constexpr (NT >= 512) {
-    e = cudaFuncSetAttribute(select2048_kernel<NT, true, false, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select2048_kernel<NT, true, false, __half>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select2048_kernel<NT, true, false, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem_optin);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select2048_kernel<NT, true, false, __nv_bfloat16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select2048_kernel<NT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select2048_kernel<NT, false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select_merge2048_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-    if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaFuncSetAttribute(select_merge2048_kernel<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return cuda_fail(e);
+using SelectFn = void (*)(SelectParams);
+
+// The instantiations of the selection kernel.
+enum Variant : int { kVar2048 = 0, kVarAnyK, kVarF16, kVarBF16, kVarWarm, kVariants };
+template <int NT, int kForm>
+SelectFn select_fn(int variant) {
+  if constexpr (NT >= 512) {  // (256 threads: fp32 without a warm start only)
+    switch (variant) {
+      case kVarF16: return select2048_kernel<NT, kForm, true, false, __half>;
+      case kVarBF16: return select2048_kernel<NT, kForm, true, false, __nv_bfloat16>;
+      case kVarWarm: return select2048_kernel<NT, kForm, false, true>;
+      default: break;
+    }
   }
-  return 0;
+  return variant == kVarAnyK ? select2048_kernel<NT, kForm, true> : select2048_kernel<NT, kForm>;
+}
+SelectFn select_fn(int threads, int form, int variant) {
+  const bool lone = form == kLoneForm;
+  if (threads == 1024) return lone ? select_fn<1024, kLoneForm>(variant) : select_fn<1024, kRoomyForm>(variant);
+  if (threads == 256) return lone ? select_fn<256, kLoneForm>(variant) : select_fn<256, kRoomyForm>(variant);
+  return lone ? select_fn<512, kLoneForm>(variant)
+              : (form == kTightForm ? select_fn<512, kTightForm>(variant) : select_fn<512, kRoomyForm>(variant));
+}
+
+template <class Fn>
+int setup_fn(Fn fn, int smem_optin) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e == cudaSuccess ? 0 : cuda_fail(e);
+}
+int setup_kernels(int smem_optin) {
+  for (int threads = 256; threads <= 1024; threads *= 2) {
+    for (int v = 0; v < kVariants; ++v) {
+      for (int form = kLoneForm; form <= kTightForm; ++form) {
+        const int rc = setup_fn(select_fn(threads, form, v), smem_optin);
+        if (rc) return rc;
+      }
+    }
+  }
+  const int rc = setup_fn(select_merge2048_kernel<512>, smem_optin);
+  return rc ? rc : setup_fn(select_merge2048_kernel<1024>, smem_optin);
 }
 
 int init_device(DeviceInfo& d, int dev) {
@@ -1471,11 +1385,7 @@ int init_device(DeviceInfo& d, int dev) {
   d.smem_optin = (int)prop.sharedMemPerBlockOptin;
   d.cc_major = prop.major;
   if (prop.major < 10) return FFTOPK_EDEVICE;
-  int rc = setup_kernel<1024>(d.smem_optin);
-  if (rc) return rc;
-  rc = setup_kernel<512>(d.smem_optin);
-  if (rc) return rc;
-  rc = setup_kernel<256>(d.smem_optin);
+  const int rc = setup_kernels(d.smem_optin);
   if (rc) return rc;
   // can a 16-CTA cluster with the latency-mode shared-memory footprint be co-scheduled, and how
   // many clusters of 16 / of 8 CTAs does the device hold at once? (A cluster lives inside one
@@ -1497,7 +1407,7 @@ int init_device(DeviceInfo& d, int dev) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&nclusters, select2048_kernel<1024>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&nclusters, select2048_kernel<1024, kRoomyForm>, &cfg);
     if (e == cudaSuccess && nclusters >= 1) {
       if (cs == 16) {
         d.max_cluster = 16;
@@ -1550,10 +1460,12 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
   const int by_len = floor_pow2(L / 2048 > 0 ? L / 2048 : 1);
   if (c > by_len) c = by_len;
   pl.cluster = c < 1 ? 1 : c;
-  // Short rows spread over many CTAs leave a thread one or two granules: 512 threads do the same
-  // with cheaper block barriers (measured at B=1 and B=4: 10.2-11.0 us against 11.4-12.3 us for
-  // L = 16K and 32K; from 64K on 1024 threads win).
-  pl.threads = (L <= 32768 && pl.cluster >= 8) ? 512 : 1024;
+  // A cluster's CTAs are bound by the instructions their warps issue, and much of that is per warp
+  // (scans, searches, address arithmetic): 512 threads do it with half the warps and, one CTA per SM,
+  // twice the registers. Measured, us per call in a chain, 512 / 1024 threads: B=1, L=16K 9.2 / 10.9,
+  // 96K 10.0 / 11.6, 1M 14.9 / 15.9; B=64 ragged rows of up to 128K 15.5 / 15.9. A lone CTA has no
+  // other CTA to share its row with: 1024.
+  pl.threads = pl.cluster > 1 ? 512 : 1024;
   const bool one_per_sm = (int64_t)rows * pl.cluster <= d.sm_count;
   pl.list_cap = one_per_sm ? kLatencyListCap : kBatchListCap;
   pl.cand_cap = one_per_sm ? kLatencyCandCap : kBatchCandCap;
@@ -1681,27 +1593,14 @@ int launch_select(const SelectCall& c) {
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  cudaError_t e;
-  const bool any_k = c.k != kK;
+  int variant = c.k != kK ? kVarAnyK : kVar2048;
   if (half_width) {
     if (warm || c.src_page_table || c.cp_flag || c.cp_publish) return FFTOPK_EINVAL;
-    if (c.dtype == kDtypeF16) {
-      e = pl.threads == 1024 ? cudaLaunchKernelEx(&cfg, select2048_kernel<1024, true, false, __half>, p)
-                             : cudaLaunchKernelEx(&cfg, select2048_kernel<512, true, false, __half>, p);
-    } else {
-      e = pl.threads == 1024 ? cudaLaunchKernelEx(&cfg, select2048_kernel<1024, true, false, __nv_bfloat16>, p)
-                             : cudaLaunchKernelEx(&cfg, select2048_kernel<512, true, false, __nv_bfloat16>, p);
-    }
+    variant = c.dtype == kDtypeF16 ? kVarF16 : kVarBF16;
   } else if (warm) {
-    e = pl.threads == 1024 ? cudaLaunchKernelEx(&cfg, select2048_kernel<1024, false, true>, p)
-                           : cudaLaunchKernelEx(&cfg, select2048_kernel<512, false, true>, p);
-  } else if (pl.threads == 1024) {
-    e = any_k ? cudaLaunchKernelEx(&cfg, select2048_kernel<1024, true>, p) : cudaLaunchKernelEx(&cfg, select2048_kernel<1024>, p);
-  } else if (pl.threads == 512) {
-    e = any_k ? cudaLaunchKernelEx(&cfg, select2048_kernel<512, true>, p) : cudaLaunchKernelEx(&cfg, select2048_kernel<512>, p);
-  } else {
-    e = any_k ? cudaLaunchKernelEx(&cfg, select2048_kernel<256, true>, p) : cudaLaunchKernelEx(&cfg, select2048_kernel<256>, p);
+    variant = kVarWarm;
   }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, select_fn(pl.threads, pl.cluster == 1 ? kLoneForm : (overlap ? kTightForm : kRoomyForm), variant), p);
   if (e != cudaSuccess) return cuda_fail(e);
   return FFTOPK_OK;
 }

@@ -13,6 +13,12 @@ uint32_t dh_sample_upper_rank(uint32_t k, uint32_t n_s, float len) { return samp
 int dh_sample_bin_too_coarse(uint32_t cnt, uint32_t total, float len, uint32_t k, float factor) {
   return sample_bin_too_coarse(cnt, total, len, k, factor) ? 1 : 0;
 }
+uint32_t dh_sample_digit(uint32_t bits) { return sample_digit(bits); }
+uint32_t dh_sample_digit_low(uint32_t bin) { return sample_digit_low(bin); }
+uint32_t dh_sample_digit_high(uint32_t bin) { return sample_digit_high(bin); }
+int dh_sample_admits_too_much(uint32_t admitted, uint32_t total, float len, uint32_t room) {
+  return sample_admits_too_much(admitted, total, len, room) ? 1 : 0;
+}
 int dh_fine_histogram_usable(int built, uint32_t total, uint32_t group) {
   return fine_histogram_usable(built != 0, total, group) ? 1 : 0;
 }
