@@ -28,6 +28,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
     "-shared", "-Xcompiler", "-fPIC",
+    "--threads", "4",  # the sources side by side
 ]
 
 
@@ -50,10 +51,10 @@ def is_stale(path: Path = LIB_PATH) -> bool:
 
 
 @contextlib.contextmanager
-def build_lock():
-    """One builder at a time across processes (the ranks of a multi-GPU job all import the package)."""
+def build_lock(out: Path = LIB_PATH):
+    """One builder of a library at a time across processes (the ranks of a multi-GPU job all import the package)."""
     LIB_DIR.mkdir(parents=True, exist_ok=True)
-    with open(LIB_DIR / ".build.lock", "w") as f:
+    with open(LIB_DIR / (".build.lock" if out == LIB_PATH else f".{out.name}.build.lock"), "w") as f:
         fcntl.flock(f, fcntl.LOCK_EX)
         try:
             yield
@@ -75,7 +76,7 @@ def build_library(force: bool = False, verbose: bool = False, extra_flags: list[
     if nvcc is None:
         raise RuntimeError("nvcc not found: cannot build libfftopk.so (set NVCC or CUDA_HOME)")
     out.parent.mkdir(parents=True, exist_ok=True)
-    with build_lock():
+    with build_lock(out):
         if not force and not is_stale(out):
             return out  # another process built it while this one waited for the lock
         tmp = out.with_name(f".{out.name}.{os.getpid()}.tmp")
