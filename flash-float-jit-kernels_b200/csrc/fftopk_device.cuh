@@ -211,6 +211,7 @@ struct Ctrl {
   uint32_t wslot;
   uint32_t cslot;
   uint32_t fslot;
+  uint32_t small_n;  // (one-pass finish) undecided candidates set aside so far
   uint32_t lcount;  // entries pushed to this CTA's spill area (may exceed its capacity)
   // what the sample search leaves: the guess and the bound for the finish (keys), what to do about them
   uint32_t guess;
@@ -487,14 +488,23 @@ __device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked&
 
 // A dense array in shared memory walked by a group of warps (`first`: this lane's first index, `step`: lanes in
 // the group; first - lane is the same in all lanes of a warp)
-template <class F4>
+// kSelect: plain bounds tests instead of predicated loads, which hold more registers at once (the fused
+// indexer's producer, at its register limit, spilled three for them).
+template <bool kSelect = false, class F4>
 __device__ __forceinline__ void walk4(uint32_t a /* shared address */, int n, int first, int step, F4&& f4) {
   const int lane = lane_id();
   for (int i = first; i - lane < n; i += 4 * step) {
     const uint32_t at = a + (uint32_t)i * 8u;
     uint64_t c[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) c[u] = lds64_if(i + u * step < n, at + (uint32_t)(u * step) * 8u);
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t au = at + (uint32_t)(u * step) * 8u;
+      if constexpr (kSelect) {
+        c[u] = i + u * step < n ? lds64(au) : 0ull;
+      } else {
+        c[u] = lds64_if(i + u * step < n, au);
+      }
+    }
     f4(c);
   }
 }
@@ -507,7 +517,7 @@ struct DenseCands {
   __device__ __forceinline__ DenseCands(const uint64_t* c, int n_) : cand(smem_u32(c)), n(n_) {}
   template <class F4>
   __device__ __forceinline__ void for_each4(F4&& f4) const {
-    walk4(cand, n, (int)threadIdx.x, NT, f4);
+    walk4<(NT < 512)>(cand, n, (int)threadIdx.x, NT, f4);
   }
 };
 
@@ -676,6 +686,13 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const uint32_t hist_s = smem_u32(hist);
+  // How the output pass hands out slots. With 16 or 32 warps: a counting pass in front, so that no
+  // warp waits for another. With ten (the fused indexer) a second walk over the list costs each of them
+  // more than the few atomics (a call with a guess, 16K keys in fp8: 11.1 us, 10.75 in one pass).
+  constexpr bool kOnePass = NT < 512;
+  if constexpr (kOnePass) {
+    if (tid == 0) ctrl->fslot = ctrl->small_n = 0u;  // (every path has a block barrier before they are used)
+  }
   if (lo > cap) {
     // Range unknown: the smallest and the largest key present bound it.
     uint32_t kmin = ~0u, kmax = 0u;
@@ -799,63 +816,130 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_
     return;
   }
   // ---- the certain winners go out (in unspecified order), the undecided candidates are set aside ----
-  // First every thread counts both kinds in its share, a scan over the lanes and one over the warps
-  // gives it its slots, then it writes. (A slot-allocating atomic per warp serialised on the one
-  // counter - 30 cycles per warp -, and ballots per candidate cost more instructions than they saved;
-  // instructions are what bounds this pass: with all warps of an SM at it each one costs eight cycles.)
   FFTOPK_MARK(32);
   const uint64_t wthr = all_bin ? (t_lo ? t_lo - 1ull : 0ull) : t_hi;  // winners: c > wthr
   const uint64_t uthr = all_bin ? wthr : (t_lo ? t_lo - 1ull : 0ull);  // undecided: uthr < c <= wthr
-  uint32_t mine = 0u;  // winners << 16 | winners and undecided
-  src.for_each4([&](const uint64_t (&c)[4]) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      count_if_above(mine, c[u], wthr, 0x10000u);
-      count_if_above(mine, c[u], uthr, 1u);
-    }
-  });
-  uint32_t incl = mine;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const uint32_t x = __shfl_up_sync(kFull, incl, off);
-    if (lane >= off) incl += x;
-  }
-  const uint32_t wsum = smem_u32(ctrl->wmax);
-  if (lane == 31) sts32(wsum + warp * 4, incl);
-  __syncthreads();
-  const uint32_t before = __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u) + incl - mine;
-  uint32_t wpos = out_base + (before >> 16), upos = (before & 0xffffu) - (before >> 16);
   uint32_t win_min = 0xffffffffu;  // (kTrackMin) smallest key among the winners this thread wrote
   const uint32_t small_s = smem_u32(ctrl->small);
-  auto pass = [&](auto paged) {
-    src.for_each4([&](const uint64_t (&c)[4]) {
-      int32_t v[4];
+  auto put_winner = [&](bool w, uint32_t pos, uint64_t c, int32_t v) {
+    const bool put = w && FFTOPK_CHECK(3, pos, out_slots, status) && pos < out_slots;
+    st_global_if(put, out_idx + pos, (uint32_t)v);
+    if (out_key) st_global_if(put, out_key + pos, (uint32_t)(c >> 32));
+    if constexpr (kTrackMin) win_min = min(win_min, w ? (uint32_t)(c >> 32) : 0xffffffffu);
+  };
+  auto put_aside = [&](bool g, uint32_t pos, uint64_t c) {
+    sts64_if(g && FFTOPK_CHECK(4, pos, kSmall, status) && pos < (uint32_t)kSmall, small_s + pos * 8u, c);
+  };
+  auto values = [&](const uint64_t (&c)[4], int32_t (&v)[4], auto paged) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int32_t idx = (int32_t)(~(uint32_t)c[u]);
-        v[u] = idx + idx_offset;
-        if constexpr (decltype(paged)::value) {  // (the four table reads in flight together)
-          if (c[u] > wthr) v[u] = __ldg(page + idx);
-        }
+    for (int u = 0; u < 4; ++u) {
+      const int32_t idx = (int32_t)(~(uint32_t)c[u]);
+      v[u] = idx + idx_offset;
+      if constexpr (decltype(paged)::value) {  // (the four table reads in flight together)
+        if (c[u] > wthr) v[u] = __ldg(page + idx);
       }
+    }
+  };
+#ifdef FFTOPK_CHECKED
+  uint32_t set_w, set_u;  // winners and undecided candidates found
+#endif
+  if constexpr (kOnePass) {
+    // One pass: a warp takes the slots of its 128 candidates' winners with one atomic on the shared
+    // counter, and those of its undecided ones with another.
+    const unsigned lt = (1u << lane) - 1u;
+    auto pass = [&](auto paged) {
+      src.for_each4([&](const uint64_t (&c)[4]) {
+        unsigned bw[4], bu[4];
+        uint32_t nw = 0u, nu = 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          bw[u] = __ballot_sync(kFull, c[u] > wthr);
+          bu[u] = __ballot_sync(kFull, c[u] > uthr) & ~bw[u];
+          nw += (uint32_t)__popc(bw[u]);
+          nu += (uint32_t)__popc(bu[u]);
+        }
+        if (nw != 0u) {
+          uint32_t base = 0u;
+          if (lane == 0) base = atom_shared_add(&ctrl->fslot, nw);
+          base = out_base + __shfl_sync(kFull, base, 0);
+          int32_t v[4];
+          values(c, v, paged);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            put_winner((bw[u] >> lane) & 1u, base + (uint32_t)__popc(bw[u] & lt), c[u], v[u]);
+            base += (uint32_t)__popc(bw[u]);
+          }
+        }
+        if (nu != 0u) {
+          uint32_t base = 0u;
+          if (lane == 0) base = atom_shared_add(&ctrl->small_n, nu);
+          base = __shfl_sync(kFull, base, 0);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            put_aside((bu[u] >> lane) & 1u, base + (uint32_t)__popc(bu[u] & lt), c[u]);
+            base += (uint32_t)__popc(bu[u]);
+          }
+        }
+      });
+    };
+    if (page) {
+      pass(std::true_type{});
+    } else {
+      pass(std::false_type{});
+    }
+#ifdef FFTOPK_CHECKED
+    __syncthreads();
+    set_w = ctrl->fslot;
+    set_u = ctrl->small_n;
+#endif
+  } else {
+    // First every thread counts both kinds in its share, a scan over the lanes and one over the warps
+    // gives it its slots, then it writes. (A slot-allocating atomic per warp serialised on the one
+    // counter - 30 cycles per warp -, and ballots per candidate cost more instructions than they saved;
+    // instructions are what bounds this pass: with all warps of an SM at it each one costs eight cycles.)
+    uint32_t mine = 0u;  // winners << 16 | winners and undecided
+    src.for_each4([&](const uint64_t (&c)[4]) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint32_t w = c[u] > wthr ? 1u : 0u, g = c[u] > uthr ? 1u : 0u;
-        const bool put = w != 0u && FFTOPK_CHECK(3, wpos, out_slots, status) && wpos < out_slots;
-        st_global_if(put, out_idx + wpos, (uint32_t)v[u]);
-        if (out_key) st_global_if(put, out_key + wpos, (uint32_t)(c[u] >> 32));
-        if constexpr (kTrackMin) win_min = min(win_min, w != 0u ? (uint32_t)(c[u] >> 32) : 0xffffffffu);
-        wpos += w;
-        const bool set = g != w && FFTOPK_CHECK(4, upos, kSmall, status) && upos < (uint32_t)kSmall;
-        sts64_if(set, small_s + upos * 8u, c[u]);
-        upos += g - w;
+        count_if_above(mine, c[u], wthr, 0x10000u);
+        count_if_above(mine, c[u], uthr, 1u);
       }
     });
-  };
-  if (page) {
-    pass(std::true_type{});
-  } else {
-    pass(std::false_type{});
+    uint32_t incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t x = __shfl_up_sync(kFull, incl, off);
+      if (lane >= off) incl += x;
+    }
+    const uint32_t wsum = smem_u32(ctrl->wmax);
+    if (lane == 31) sts32(wsum + warp * 4, incl);
+    __syncthreads();
+    const uint32_t before = __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u) + incl - mine;
+    uint32_t wpos = out_base + (before >> 16), upos = (before & 0xffffu) - (before >> 16);
+    auto pass = [&](auto paged) {
+      src.for_each4([&](const uint64_t (&c)[4]) {
+        int32_t v[4];
+        values(c, v, paged);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t w = c[u] > wthr ? 1u : 0u, g = c[u] > uthr ? 1u : 0u;
+          put_winner(w != 0u, wpos, c[u], v[u]);
+          wpos += w;
+          put_aside(g != w, upos, c[u]);
+          upos += g - w;
+        }
+      });
+    };
+    if (page) {
+      pass(std::true_type{});
+    } else {
+      pass(std::false_type{});
+    }
+#ifdef FFTOPK_CHECKED
+    const uint32_t sum = __reduce_add_sync(kFull, lane < NT / 32 ? ctrl->wmax[lane] : 0u);
+    set_w = sum >> 16;
+    set_u = (sum & 0xffffu) - (sum >> 16);
+#endif
   }
   FFTOPK_MARK(33);
   if constexpr (kTrackMin) {
@@ -865,11 +949,10 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_
 #ifdef FFTOPK_CHECKED
   {
     // every certain winner took exactly one slot, every undecided candidate was set aside
-    const uint32_t sum = __reduce_add_sync(kFull, lane < NT / 32 ? ctrl->wmax[lane] : 0u);
     const uint32_t want_w = all_bin ? need_total : need_total - need2;
     if (tid == 0) {
-      if ((sum >> 16) != want_w) check_fail(10, sum >> 16, want_w, status);
-      if (!all_bin && (sum & 0xffffu) - (sum >> 16) != cnt) check_fail(11, (sum & 0xffffu) - (sum >> 16), cnt, status);
+      if (set_w != want_w) check_fail(10, set_w, want_w, status);
+      if (!all_bin && set_u != cnt) check_fail(11, set_u, cnt, status);
     }
   }
 #endif
