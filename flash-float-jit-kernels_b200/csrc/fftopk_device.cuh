@@ -47,11 +47,21 @@ static __device__ __noinline__ void check_fail(int site, uint32_t idx, uint32_t 
   }
   if (status) atomicOr(status, (uint32_t)FFTOPK_ST_CHECK);
 }
+// ... and it counts the rows by the way they took (see kRoute*); fftopk_checked_routes() returns the counts.
+static __device__ unsigned int g_routes[3];
+#define FFTOPK_ROUTE(route) \
+  do {                      \
+    if (threadIdx.x == 0) atomicAdd(&g_routes[route], 1u); \
+  } while (0)
 #define FFTOPK_CHECK(site, idx, limit, status) \
   (((uint32_t)(idx) < (uint32_t)(limit)) ? true : (::fftopk::check_fail((site), (uint32_t)(idx), (uint32_t)(limit), (status)), false))
 #else
 #define FFTOPK_CHECK(site, idx, limit, status) true
+#define FFTOPK_ROUTE(route)
 #endif
+// finished from the candidates of one filter pass; of these, with candidates beyond their CTAs' regions of
+// the gather buffer; selected by full histograms
+constexpr int kRouteHeld = 0, kRouteBeyond = 1, kRouteHistograms = 2;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -420,6 +420,9 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, i
   uint32_t pos = incl - n;
   uint32_t at = smem_u32(seg) + pos * 8u;
   auto put = [&](float v, int idx) {
+#ifdef FFTOPK_CHECKED
+    if (!(v < edge) && !FFTOPK_CHECK(13, (at - smem_u32(seg)) / 8u, seg_cap, ctrl_status(ctrl))) return;
+#endif
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p st.shared.v2.u32 [%0], {%3, %4};\n\t@p add.u32 %0, %0, 8;\n\t}"
         : "+r"(at)
@@ -1116,9 +1119,11 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       xbase = ctrl->base_c;
     }
     const uint32_t cand0 = peer_smem(smem_u32(cx.cand), 0);
+    bool dropped = false;
     auto push = [&](uint32_t q, uint64_t c) {  // candidate number q of this CTA
       uint32_t at = (uint32_t)(rank * region) + q;
       if (q >= (uint32_t)region) at = (uint32_t)(C * region) + xbase + (q - (uint32_t)region);
+      dropped = dropped || at >= (uint32_t)p.cand_cap;
       if (at < (uint32_t)p.cand_cap) st_peer64(cand0 + at * 8u, c);
     };
     drain_segment(staged, sh, seg, wown, ctrl, [&](uint32_t j, uint64_t c) { push(before + j, c); });
@@ -1135,6 +1140,10 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     // can hold: start over with full histograms
     mode = sampled_attempt_ok(over | (extra > p.cand_cap - C * region ? 1u : 0u), total, K, 0xffffffffu) ? kModeGather
                                                                                                        : kModeFallback;
+#ifdef FFTOPK_CHECKED
+    // (a candidate may be dropped only where the counts tell every CTA that the buffer was too small)
+    if (dropped && mode == kModeGather) check_fail(14, (uint32_t)extra, (uint32_t)p.cand_cap, p.status);
+#endif
   }
   if constexpr (kWarm) {
     // (a miss is worth knowing about: the row is then selected by the full-histogram path)
@@ -1147,6 +1156,8 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   FFTOPK_MARK(5);
 
   const int idx_bits = 32 - __clz(len - 1);
+  if (rank == 0) FFTOPK_ROUTE(mode == kModeGather ? kRouteHeld : kRouteHistograms);
+  if (rank == 0 && mode == kModeGather && extra > 0) FFTOPK_ROUTE(kRouteBeyond);
   if (mode == kModeGather) {
     const uint64_t lo = low_end(lowkey), focus = high_end(focus_key);
     if (C == 1) {
@@ -1704,6 +1715,14 @@ int fftopk_checked_read(uint32_t rec[8]) {
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(fftopk::g_check_rec, zero, sizeof(zero));
   if (e != cudaSuccess) return fftopk::cuda_fail(e);
   return fftopk::checked_read_merge(rec + 4);
+}
+
+// Checked builds only: the rows selected since the last call, by the way they took (kRoute*). Clears the counts.
+int fftopk_checked_routes(uint32_t counts[3]) {
+  const uint32_t zero[3] = {0u, 0u, 0u};
+  cudaError_t e = cudaMemcpyFromSymbol(counts, fftopk::g_routes, sizeof(zero));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(fftopk::g_routes, zero, sizeof(zero));
+  return e == cudaSuccess ? 0 : fftopk::cuda_fail(e);
 }
 #endif
 
