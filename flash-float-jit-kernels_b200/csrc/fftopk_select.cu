@@ -6,12 +6,13 @@
 //
 // Shape of the computation for one row of `len` > 2048 valid fp32 logits, C CTAs in the cluster,
 // each owning a contiguous shard of the row:
-//   1. SAMPLE. Every CTA reads the same 8K elements (16K of rows beyond 256K), in slabs of 512 bytes
+//   1. SAMPLE. Every CTA reads the same 8K elements (16K of rows beyond 256K), in pieces of 32
 //      spread evenly over the row, and histograms them on a digit of 64 bins per octave. A CTA whose
 //      whole shard fits in registers has those loads in flight at the same time.
 //   2. PICK. One block-wide suffix scan finds the bin whose sample rank is the expected rank of the k-th
 //      element plus five standard deviations - a lower bound of the true threshold with overwhelming
-//      probability - and the mirror-image upper bound. All CTAs of a cluster find the same bin by
+//      probability where the sample elements are independent (see sample_piece_start) - and the mirror-image
+//      upper bound. All CTAs of a cluster find the same bin by
 //      themselves: no histogram is exchanged and no cluster barrier is waited for here (exchanging
 //      them took 0.8 us for the barrier and 1.8 us for two rounds of remote reads).
 //   3. FILTER. ONE float compare per element against the bin's lower edge, on the shard in registers
@@ -460,39 +461,45 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, i
   return total;
 }
 
-// The sample of a row: `nb` batches of G slabs of 32 granules per warp, spread evenly over the whole row
-// (uniform in position, so recency-correlated logits are sampled fairly). Every CTA of a cluster takes
-// the SAME sample, so each finds the same guess by itself: no exchange of histograms and no cluster
-// barrier in front of the search. A row that is no larger than the sample is read completely.
-// Granules that straddle the row's ends are left out.
+// The sample of a row: `nb` batches of G loads of 32 granules per warp, spread over the whole row in pieces
+// (see sample_piece_start). Every CTA of a cluster takes the SAME sample, so each finds the same guess by
+// itself: no exchange of histograms and no cluster barrier in front of the search. A row that is no larger
+// than the sample is read completely. Granules that straddle the row's ends are left out.
 template <int NT, int G>
 struct RowSample {
   int i0, gi;  // first granule completely inside the row, and how many there are
   int nb;      // a power of two
+  uint32_t off;  // granule i0's position within a piece
   bool whole;
-  __device__ __forceinline__ int granule(int b, int u) const {
-    constexpr int kLogSlabs = (NT == 1024 ? 5 : (NT == 512 ? 4 : 3)) + (G == 4 ? 2 : 1);
-    static_assert(G == 2 || G == 4, "");
-    const int warp = threadIdx.x >> 5;
-    const int sl = (b * G + u) * (NT / 32) + warp;
-    const int first = whole ? sl * 32 : ((int)(((uint64_t)(uint32_t)gi * (uint32_t)sl) >> (kLogSlabs + (31 - __clz(nb)))) & ~7);
-    return first + lane_id();
-  }
-  __device__ __forceinline__ bool valid(int g) const { return !whole || g < gi; }
-  __device__ __forceinline__ uint32_t size() const { return 4u * (uint32_t)(whole ? gi : NT * G * nb); }
+  // load u of batch b: which of the sample's loads of 32 granules it is
+  static __device__ __forceinline__ int load_no(int b, int u) { return (b * G + u) * (NT / 32) + (int)(threadIdx.x >> 5); }
+  __device__ __forceinline__ int granules() const { return NT * G * nb; }
+  __device__ __forceinline__ uint32_t size() const { return 4u * (uint32_t)(whole ? gi : granules()); }
+  // (one branch around all loads of a batch, so that they are in flight together)
   template <class T>
   __device__ __forceinline__ void load(const T* gbase, int b, float4 (&x)[G]) const {
+    if (whole) {
 #pragma unroll
-    for (int u = 0; u < G; ++u) {
-      const int g = granule(b, u);
-      if (valid(g)) x[u] = Elem<T>::ld4(gbase, i0 + g);
+      for (int u = 0; u < G; ++u) {
+        const int g = load_no(b, u) * 32 + lane_id();
+        if (g < gi) x[u] = Elem<T>::ld4(gbase, i0 + g);
+      }
+    } else {
+      constexpr int kPer = 32 / kSamplePiece;  // pieces per load
+      const int log_pieces = 31 - __clz(granules() / kSamplePiece);
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const uint32_t piece = (uint32_t)(load_no(b, u) * kPer + lane_id() / kSamplePiece);
+        const uint32_t first = sample_piece_start((uint32_t)gi, piece, log_pieces, off);
+        x[u] = Elem<T>::ld4(gbase, i0 + (int)first + (lane_id() & (kSamplePiece - 1)));
+      }
     }
   }
   template <class Op>
   __device__ __forceinline__ void use(int b, const float4 (&x)[G], Op&& op) const {
 #pragma unroll
     for (int u = 0; u < G; ++u) {
-      if (!whole || valid(granule(b, u))) {
+      if (!whole || load_no(b, u) * 32 + lane_id() < gi) {
         op(__float_as_uint(x[u].x));
         op(__float_as_uint(x[u].y));
         op(__float_as_uint(x[u].z));
@@ -501,6 +508,7 @@ struct RowSample {
     }
   }
 };
+
 // what the sample search tells the CTA to do (Ctrl::guess_flags)
 constexpr uint32_t kGuessCoarse = 1u;  // the guessed bin is crowded: look at the sample again, inside that bin
 constexpr uint32_t kGuessGiveUp = 2u;  // the guess admits far more than there is room for: full histograms at once
@@ -871,7 +879,8 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   smp.gi = ((sh.a + len) & 3 ? gn - 1 : gn) - smp.i0;
   // 8K elements; 16K for rows so long that 8K would need a margin of several thousand candidates
   smp.nb = (NT >= 512 ? 1 : 2) << (len > FFTOPK_LONG_SAMPLE ? 1 : 0);
-  smp.whole = smp.gi <= NT * G * smp.nb;
+  smp.whole = smp.gi <= smp.granules();
+  smp.off = (uint32_t)(reinterpret_cast<uintptr_t>(sh.gbase + 4 * smp.i0) / (4 * sizeof(T))) & (uint32_t)(kSamplePiece - 1);
 
   // ---- warm start: a key guess of the row's k-th largest element from an earlier call ----------
   // With a guess the row skips the sample, its histogram and the search: it is filtered at once

@@ -19,6 +19,10 @@ uint32_t dh_sample_digit_high(uint32_t bin) { return sample_digit_high(bin); }
 int dh_sample_admits_too_much(uint32_t admitted, uint32_t total, float len, uint32_t room) {
   return sample_admits_too_much(admitted, total, len, room) ? 1 : 0;
 }
+int dh_sample_piece(void) { return kSamplePiece; }
+uint32_t dh_sample_piece_start(uint32_t gi, uint32_t piece, int log_pieces, uint32_t off) {
+  return sample_piece_start(gi, piece, log_pieces, off);
+}
 int dh_fine_histogram_usable(int built, uint32_t total, uint32_t group) {
   return fine_histogram_usable(built != 0, total, group) ? 1 : 0;
 }

@@ -80,6 +80,8 @@ CASES = {
     "plain, one row": (("normal", 1, 98305, 2048, 0, 0), 16, False, False),
     "plain, throughput plan, 2 CTAs a row": (("normal", 16, 131072, 2048, 1, 0), 2, False, False),
     "plain, throughput plan, 4 CTAs a row": (("normal", 8, 131072, 2048, 1, 0), 4, False, None),
+    "window of winners": (("window", 4, 98305, 2048, 0, 0), 16, False, True),
+    "window of winners, throughput plan": (("window", 64, 98305, 2048, 1, 0), 1, False, False),
     "all equal": (("equal", 2, 65536, 2048, 0, 0), 16, True, False),
 }
 
