@@ -6,7 +6,7 @@
 //
 // Shape of the computation for one row of `len` > 2048 valid fp32 logits, C CTAs in the cluster,
 // each owning a contiguous shard of the row:
-//   1. SAMPLE. Every CTA reads the same 8K elements (16K of rows beyond 256K), in pieces of 32
+//   1. SAMPLE. Every CTA reads the same 8K elements (more of rows beyond 256K), in pieces of 32
 //      spread evenly over the row, and histograms them on a digit of 64 bins per octave. A CTA whose
 //      whole shard fits in registers has those loads in flight at the same time.
 //   2. PICK. One block-wide suffix scan finds the bin whose sample rank is the expected rank of the k-th
@@ -35,7 +35,6 @@
 //      round, and exact ties left after 32 bits are taken in index order, shard by shard.
 //
 // Build-time knobs (all optional, for experiments; the defaults are what was measured best):
-//   FFTOPK_LONG_SAMPLE      row length from which the sample is 16K elements instead of 8K (262144)
 //   FFTOPK_REG_SLABS        granules per thread up to which the shard stays in registers (4; see reg_slabs)
 //   FFTOPK_1B_FACTOR        second look at the sample when the guessed bin holds more than factor*k (2)
 //   FFTOPK_U512             128-bit loads in flight per thread of the 512-thread filter (8; 16 allowed)
@@ -62,9 +61,6 @@ namespace fftopk {
 
 #ifndef FFTOPK_REG_SLABS
 #define FFTOPK_REG_SLABS 4
-#endif
-#ifndef FFTOPK_LONG_SAMPLE
-#define FFTOPK_LONG_SAMPLE 262144
 #endif
 
 struct SelectParams {
@@ -475,9 +471,10 @@ struct RowSample {
   static __device__ __forceinline__ int load_no(int b, int u) { return (b * G + u) * (NT / 32) + (int)(threadIdx.x >> 5); }
   __device__ __forceinline__ int granules() const { return NT * G * nb; }
   __device__ __forceinline__ uint32_t size() const { return 4u * (uint32_t)(whole ? gi : granules()); }
-  // (one branch around all loads of a batch, so that they are in flight together)
-  template <class T>
-  __device__ __forceinline__ void load(const T* gbase, int b, float4 (&x)[G]) const {
+  // (one branch around all loads of a batch, so that they are in flight together; x may be longer than G)
+  template <class T, int N>
+  __device__ __forceinline__ void load(const T* gbase, int b, float4 (&x)[N]) const {
+    static_assert(N >= G, "");
     if (whole) {
 #pragma unroll
       for (int u = 0; u < G; ++u) {
@@ -495,8 +492,8 @@ struct RowSample {
       }
     }
   }
-  template <class Op>
-  __device__ __forceinline__ void use(int b, const float4 (&x)[G], Op&& op) const {
+  template <int N, class Op>
+  __device__ __forceinline__ void use(int b, const float4 (&x)[N], Op&& op) const {
 #pragma unroll
     for (int u = 0; u < G; ++u) {
       if (!whole || load_no(b, u) * 32 + lane_id() < gi) {
@@ -877,8 +874,8 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   RowSample<NT, G> smp;
   smp.i0 = sh.a > 0 ? 1 : 0;
   smp.gi = ((sh.a + len) & 3 ? gn - 1 : gn) - smp.i0;
-  // 8K elements; 16K for rows so long that 8K would need a margin of several thousand candidates
-  smp.nb = (NT >= 512 ? 1 : 2) << (len > FFTOPK_LONG_SAMPLE ? 1 : 0);
+  // 8K elements, more for rows so long that 8K would need a margin of several thousand candidates
+  smp.nb = (NT >= 512 ? 1 : 2) << sample_log_batches(len, K);
   smp.whole = smp.gi <= smp.granules();
   smp.off = (uint32_t)(reinterpret_cast<uintptr_t>(sh.gbase + 4 * smp.i0) / (4 * sizeof(T))) & (uint32_t)(kSamplePiece - 1);
 
@@ -970,10 +967,26 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   }
   if (sampled) {
     const uint32_t wtot_s = smem_u32(ctrl->wtot);
-    for (int b = 0;;) {
-      smp.use(b, xs, [&](uint32_t bits) { red_shared_inc(h0 + sample_digit(bits) * 4u); });
-      if (++b >= smp.nb) break;
-      smp.load(sh.gbase, b, xs);
+    auto tally = [&](uint32_t bits) { red_shared_inc(h0 + sample_digit(bits) * 4u); };
+    if constexpr (NT >= 512 && kForm != kRoomyForm) {
+      // The next batch of a long row is on its way while this one is counted: its shards are far too long for
+      // the registers, and the next batch takes their place. (Not where a thread has registers to spare: a
+      // row of two batches over 16 CTAs took 15.1 us like this, and 14.85 with one batch after the other.)
+      static_assert(NT * kRegSlabs * 4 * kMaxCluster <= 262144, "rows of one batch");
+      for (int b = 0;; b += 2) {
+        if (b + 1 < smp.nb) smp.load(sh.gbase, b + 1, xr);
+        smp.use(b, xs, tally);
+        if (b + 1 >= smp.nb) break;
+        if (b + 2 < smp.nb) smp.load(sh.gbase, b + 2, xs);
+        smp.use(b + 1, xr, tally);
+        if (b + 2 >= smp.nb) break;
+      }
+    } else {
+      for (int b = 0;;) {
+        smp.use(b, xs, tally);
+        if (++b >= smp.nb) break;
+        smp.load(sh.gbase, b, xs);
+      }
     }
     __syncthreads();
     FFTOPK_MARK(2);

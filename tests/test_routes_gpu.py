@@ -82,6 +82,8 @@ CASES = {
     "plain, throughput plan, 4 CTAs a row": (("normal", 8, 131072, 2048, 1, 0), 4, False, None),
     "window of winners": (("window", 4, 98305, 2048, 0, 0), 16, False, True),
     "window of winners, throughput plan": (("window", 64, 98305, 2048, 1, 0), 1, False, False),
+    "4M elements, k = 4096": (("normal", 1, (1 << 22) + 3, 4096, 0, 0), 16, False, True),
+    "12M elements": (("normal", 1, 12 << 20, 2048, 0, 0), 16, False, None),
     "all equal": (("equal", 2, 65536, 2048, 0, 0), 16, True, False),
 }
 

@@ -19,6 +19,7 @@ def dh(tmp_path_factory):
                     "-o", str(out), str(REPO / "tests" / "decide_harness.cpp")], check=True)
     lib = ctypes.CDLL(str(out))
     lib.dh_sample_piece_start.restype, lib.dh_sample_piece_start.argtypes = u32, [u32, u32, i32, u32]
+    lib.dh_sample_log_batches.argtypes = [i32, u32]
     lib.dh_sample_lower_rank.restype, lib.dh_sample_lower_rank.argtypes = u32, [u32, u32, f32]
     return lib
 
@@ -88,3 +89,14 @@ def test_smooth_rows_are_guessed_like_others(dh, reach, share):
         guess = np.partition(sample, sample.size - rank)[sample.size - rank]
         short += int((row >= guess).sum() < K)
     assert short <= 0.1 * rows, f"{short} of {rows} rows"
+
+
+@pytest.mark.parametrize("k", [1, 512, 2048, 4096])
+def test_long_rows_leave_room_for_what_the_guess_admits(dh, k):
+    """The number of elements expected to pass stays well below what the gather buffer of a cluster holds
+    (16384) for rows of any length, and the sample a small part of the row."""
+    for length in [8193, 98304, 262144, 262145] + [n + d for n in (1 << e for e in range(19, 31)) for d in (0, 1)] + [(1 << 31) - 9]:
+        n_s = 8192 << dh.dh_sample_log_batches(length, k)
+        expected = dh.dh_sample_lower_rank(k, n_s, length) * length / n_s
+        assert expected <= (9300 if k <= 2048 else 9800), (length, n_s, expected)
+        assert n_s <= 8192 or n_s * 16 < length
