@@ -393,7 +393,7 @@ __device__ __forceinline__ void scan_shard(const Shard<T>& sh, Op&& op) {
 // its slots, and a predicated store per element writes what passes: no second read of the value, no
 // loop over hits. Same result as filter_shard.
 template <int R>
-__device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, int el_step, float edge, uint64_t* seg,
+__device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int slabs, int el0, int el_step, float edge, uint64_t* seg,
                                                 uint32_t seg_cap, Ctrl* ctrl, uint64_t* spill, uint32_t spill_cap) {
   const int lane = lane_id();
   uint32_t n = 0u;
@@ -402,10 +402,12 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, i
   };
 #pragma unroll
   for (int j = 0; j < R; ++j) {
-    count(x[j].x);
-    count(x[j].y);
-    count(x[j].z);
-    count(x[j].w);
+    if (j < slabs) {  // (uniform)
+      count(x[j].x);
+      count(x[j].y);
+      count(x[j].z);
+      count(x[j].w);
+    }
   }
   uint32_t incl = n;
 #pragma unroll
@@ -440,10 +442,12 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, i
   if (total <= seg_cap) {  // (uniform over the warp)
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      put(x[j].x, el0 + j * el_step);
-      put(x[j].y, el0 + j * el_step + 1);
-      put(x[j].z, el0 + j * el_step + 2);
-      put(x[j].w, el0 + j * el_step + 3);
+      if (j < slabs) {
+        put(x[j].x, el0 + j * el_step);
+        put(x[j].y, el0 + j * el_step + 1);
+        put(x[j].z, el0 + j * el_step + 2);
+        put(x[j].w, el0 + j * el_step + 3);
+      }
     }
   } else {
 #pragma unroll
@@ -464,12 +468,13 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int el0, i
 template <int NT, int G>
 struct RowSample {
   int i0, gi;  // first granule completely inside the row, and how many there are
-  int nb;      // a power of two
+  int nb;      // batches, a power of two
+  int gu;      // loads per thread and batch: G, or half of that
   uint32_t off;  // granule i0's position within a piece
   bool whole;
   // load u of batch b: which of the sample's loads of 32 granules it is
-  static __device__ __forceinline__ int load_no(int b, int u) { return (b * G + u) * (NT / 32) + (int)(threadIdx.x >> 5); }
-  __device__ __forceinline__ int granules() const { return NT * G * nb; }
+  __device__ __forceinline__ int load_no(int b, int u) const { return (b * gu + u) * (NT / 32) + (int)(threadIdx.x >> 5); }
+  __device__ __forceinline__ int granules() const { return NT * gu * nb; }
   __device__ __forceinline__ uint32_t size() const { return 4u * (uint32_t)(whole ? gi : granules()); }
   // (one branch around all loads of a batch, so that they are in flight together; x may be longer than G)
   template <class T, int N>
@@ -479,7 +484,7 @@ struct RowSample {
 #pragma unroll
       for (int u = 0; u < G; ++u) {
         const int g = load_no(b, u) * 32 + lane_id();
-        if (g < gi) x[u] = Elem<T>::ld4(gbase, i0 + g);
+        if (u < gu && g < gi) x[u] = Elem<T>::ld4(gbase, i0 + g);
       }
     } else {
       constexpr int kPer = 32 / kSamplePiece;  // pieces per load
@@ -488,7 +493,7 @@ struct RowSample {
       for (int u = 0; u < G; ++u) {
         const uint32_t piece = (uint32_t)(load_no(b, u) * kPer + lane_id() / kSamplePiece);
         const uint32_t first = sample_piece_start((uint32_t)gi, piece, log_pieces, off);
-        x[u] = Elem<T>::ld4(gbase, i0 + (int)first + (lane_id() & (kSamplePiece - 1)));
+        if (u < gu) x[u] = Elem<T>::ld4(gbase, i0 + (int)first + (lane_id() & (kSamplePiece - 1)));
       }
     }
   }
@@ -496,7 +501,7 @@ struct RowSample {
   __device__ __forceinline__ void use(int b, const float4 (&x)[N], Op&& op) const {
 #pragma unroll
     for (int u = 0; u < G; ++u) {
-      if (!whole || load_no(b, u) * 32 + lane_id() < gi) {
+      if (u < gu && (!whole || load_no(b, u) * 32 + lane_id() < gi)) {
         op(__float_as_uint(x[u].x));
         op(__float_as_uint(x[u].y));
         op(__float_as_uint(x[u].z));
@@ -870,12 +875,17 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   sh.i1 = max(sh.i0, min(sh.g1, ((sh.a + len) & 3) ? gn - 1 : gn));
   // Whole shard in registers (same answer in every CTA of the cluster: `per` is rank-independent).
   const bool in_regs = per <= NT * kRegSlabs;
+  const int slabs = (per + NT - 1) / NT;  // granules of the shard per thread
   constexpr int G = NT >= 1024 ? 2 : 4;  // sample granules per thread and batch
   RowSample<NT, G> smp;
   smp.i0 = sh.a > 0 ? 1 : 0;
   smp.gi = ((sh.a + len) & 3 ? gn - 1 : gn) - smp.i0;
   // 8K elements, more for rows so long that 8K would need a margin of several thousand candidates
   smp.nb = (NT >= 512 ? 1 : 2) << sample_log_batches(len, K);
+  // ... and 4K for rows of up to 32K elements over several CTAs that cannot be read completely: a CTA's
+  // shard is no more than that, and the sample would be most of its work (one row, us per call with 8K / 4K: 16K
+  // elements 9.7 / 9.4, 32K 10.1 / 9.8; one of 8K, where it would no longer be all of the row, 9.2 / 9.5)
+  smp.gu = !kLone && len <= 32768 && smp.gi > NT * G * smp.nb ? G / 2 : G;
   smp.whole = smp.gi <= smp.granules();
   smp.off = (uint32_t)(reinterpret_cast<uintptr_t>(sh.gbase + 4 * smp.i0) / (4 * sizeof(T))) & (uint32_t)(kSamplePiece - 1);
 
@@ -902,7 +912,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     for (int j = 0; j < kRegSlabs; ++j) {
       const int g = sh.g0 + j * NT + tid;
       xr[j] = make_float4(ninf, ninf, ninf, ninf);
-      if (g >= sh.i0 && g < sh.i1) xr[j] = Elem<T>::ld4(sh.gbase, g);
+      if (j < slabs && g >= sh.i0 && g < sh.i1) xr[j] = Elem<T>::ld4(sh.gbase, g);
     }
   }
   float4 xs[G];
@@ -947,7 +957,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
 #pragma unroll
     for (int j = 0; j < kRegSlabs; ++j) {
       const int g = sh.g0 + j * NT + tid;
-      if (g < sh.g1 && (g < sh.i0 || g >= sh.i1)) xr[j] = load_granule_partial(sh.gbase, sh.a, sh.len, g, ninf);
+      if (j < slabs && g < sh.g1 && (g < sh.i0 || g >= sh.i1)) xr[j] = load_granule_partial(sh.gbase, sh.a, sh.len, g, ninf);
     }
   }
   __syncthreads();  // histograms and counters are clear
@@ -1081,7 +1091,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     // depends on what the cluster's CTAs tell each other, not on what each has read for itself.)
     if (tid == 0) ctrl->pub_flag = 1u;
   } else if (in_regs && edge > ninf) {
-    wcnt = filter_regs<kRegSlabs>(xr, 4 * (sh.g0 + tid) - sh.a, 4 * NT, edge, seg, seg_cap, ctrl, spill, spill_cap);
+    wcnt = filter_regs<kRegSlabs>(xr, slabs, 4 * (sh.g0 + tid) - sh.a, 4 * NT, edge, seg, seg_cap, ctrl, spill, spill_cap);
   } else if (len <= 196608) {  // about 1.5 k candidates per row: most trips of the hit loop have work
     staged = true;
     wcnt = filter_shard<NT, U, true>(sh, edge, seg, seg_cap, ctrl, spill, spill_cap);
