@@ -161,6 +161,25 @@ FFTOPK_DECIDE_HD bool sampled_attempt_ok(uint32_t overflowed, uint32_t admitted,
   return overflowed == 0u && admitted >= k && admitted <= room;
 }
 
+// The gather buffer of a cluster: every CTA has a region of its own, which it fills without asking for
+// slots, and what does not fit there goes behind the last region, for a remote atomic per CTA. The regions
+// leave room behind them for 4/3 of a whole list of any one CTA - what a window of recent keys fills, or a sorted
+// row -, and take no more than three quarters of the buffer. (With three quarters whatever the list, one CTA
+// could hand on 4,864 candidates at 16 CTAs per row and 2,112 at 8 in the throughput plan, and such rows
+// went through full histograms. The walk over the part behind is shared by all warps of the finish, so
+// they are also faster with small regions: 2,048 consecutive winners in a row of 98,305 elements 11.1 us
+// instead of 12.0. One row of 1M elements leaves some 300 candidates per CTA, for 546 slots.)
+FFTOPK_DECIDE_HD int gather_region(int cand_cap, int list_cap, int ctas) {
+  const int most = (cand_cap - cand_cap / 4) / ctas;
+  const int room = (cand_cap - list_cap - list_cap / 3) / (ctas > 1 ? ctas - 1 : 1);
+  return room < 0 ? 0 : (most < room ? most : room) & ~15;  // (whole 128-byte lines: 3 % of a call at k = 4096, 1M)
+}
+// ... and of a CTA's list: the warps' segments, and an area behind them for what a warp's segment does not
+// hold. Where all candidates of a row may lie in one CTA's shard, a few thousand consecutive elements fall
+// on the warps unevenly: a quarter of a short list (the throughput plan's), else an eighth. (A quarter of
+// a long one as well cost 64 rows with 6,500 copies of the threshold 26.3 us instead of 24.4.)
+FFTOPK_DECIDE_HD int list_spill(int list_cap, bool lone) { return list_cap / (lone || list_cap >= 4096 ? 8 : 4); }
+
 // ---------------------------------------------------------------------------------------------
 // Digit rule of a finish round over the composite range [lo, cap]: digit(c) = min((c - lo) >>
 // shift, kFinishBins - 1). The shift is chosen so that [lo, focus] spreads over the bins below the

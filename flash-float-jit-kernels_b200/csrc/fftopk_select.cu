@@ -1070,8 +1070,8 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   int mode = kModeFallback;
   auto low_end = [](uint32_t key) { return (uint64_t)key << 32; };
   auto high_end = [](uint32_t key) { return ((uint64_t)key << 32) | 0xffffffffull; };
-  // list layout: one segment per warp, then the spill area (an eighth of the list)
-  const uint32_t spill_cap = (uint32_t)p.list_cap / 8u;
+  // list layout: one segment per warp, then the spill area
+  const uint32_t spill_cap = (uint32_t)list_spill(p.list_cap, kLone);
   const uint32_t seg_cap = ((uint32_t)p.list_cap - spill_cap) / NW;
   uint64_t* const seg = list + (size_t)warp * seg_cap;
   uint64_t* const spill = list + (size_t)NW * seg_cap;
@@ -1101,7 +1101,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   const uint32_t wown = min(wcnt, seg_cap);
   FFTOPK_MARK(8);
   bool have_hist = false;  // (lone CTA) round 0 of the finish has its histogram
-  const int region = C == 1 ? 0 : ((p.cand_cap - p.cand_cap / 4) / C);  // slots of each CTA in rank 0's buffer
+  const int region = C == 1 ? 0 : gather_region(p.cand_cap, p.list_cap, C);  // slots of each CTA in rank 0's buffer
   int extra = 0;           // candidates beyond their CTAs' regions
   uint32_t total = 0u;     // candidates of the row
   uint32_t fin_sn = 0u;

@@ -24,6 +24,7 @@ uint32_t dh_sample_piece_start(uint32_t gi, uint32_t piece, int log_pieces, uint
   return sample_piece_start(gi, piece, log_pieces, off);
 }
 int dh_sample_log_batches(int len, uint32_t k) { return sample_log_batches(len, k); }
+int dh_gather_region(int cand_cap, int list_cap, int ctas) { return gather_region(cand_cap, list_cap, ctas); }
 int dh_fine_histogram_usable(int built, uint32_t total, uint32_t group) {
   return fine_histogram_usable(built != 0, total, group) ? 1 : 0;
 }

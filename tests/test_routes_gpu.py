@@ -80,8 +80,15 @@ CASES = {
     "plain, one row": (("normal", 1, 98305, 2048, 0, 0), 16, False, False),
     "plain, throughput plan, 2 CTAs a row": (("normal", 16, 131072, 2048, 1, 0), 2, False, False),
     "plain, throughput plan, 4 CTAs a row": (("normal", 8, 131072, 2048, 1, 0), 4, False, None),
+    "k = 4096, throughput plan": (("normal", 8, 65536, 4096, 1, 0), 4, False, True),
     "window of winners": (("window", 4, 98305, 2048, 0, 0), 16, False, True),
     "window of winners, throughput plan": (("window", 64, 98305, 2048, 1, 0), 1, False, False),
+    "recent keys": (("recent", 1, 1 << 20, 2048, 0, 0), 16, False, True),
+    "recent keys, 8 CTAs a row": (("recent", 8, 200000, 2048, 0, 0), 8, False, True),
+    "recent keys, throughput plan, 2 CTAs a row": (("recent", 16, 40000, 2048, 1, 0), 2, False, True),
+    "recent keys, throughput plan, 8 CTAs a row": (("recent", 4, 65536, 2048, 1, 0), 8, False, True),
+    "recent keys, throughput plan, warm": (("recent", 4, 65536, 2048, 1, 1), 8, False, True),
+    "keys around a shard boundary": (("straddling", 4, 131072, 2048, 1, 0), 8, False, True),
     "4M elements, k = 4096": (("normal", 1, (1 << 22) + 3, 4096, 0, 0), 16, False, True),
     "12M elements": (("normal", 1, 12 << 20, 2048, 0, 0), 16, False, None),
     "all equal": (("equal", 2, 65536, 2048, 0, 0), 16, True, False),

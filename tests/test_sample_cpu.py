@@ -100,3 +100,24 @@ def test_long_rows_leave_room_for_what_the_guess_admits(dh, k):
         expected = dh.dh_sample_lower_rank(k, n_s, length) * length / n_s
         assert expected <= (9300 if k <= 2048 else 9800), (length, n_s, expected)
         assert n_s <= 8192 or n_s * 16 < length
+
+
+@pytest.mark.parametrize("ctas", [2, 4, 8, 16])
+@pytest.mark.parametrize("cand_cap,list_cap", [(16384, 6144), (6144, 3072)])  # latency plan, throughput plan
+def test_the_gather_buffer_takes_what_one_shard_or_two_hold(dh, ctas, cand_cap, list_cap):
+    """All candidates in one CTA's shard: as many as its list holds. In two: what the guess is expected to admit of
+    rows of up to 1M elements (a cluster by itself) or 256K (sharing its SMs with other calls)."""
+    region = dh.dh_gather_region(cand_cap, list_cap, ctas)
+    behind = cand_cap - ctas * region
+    assert region > 0 and behind > 0
+    assert region + behind >= list_cap
+    length, n_s = (1 << 20, 16384) if cand_cap == 16384 else (262144, 8192)
+    assert 2 * region + behind >= min(1.1 * dh.dh_sample_lower_rank(K, n_s, length) * length / n_s, 2 * list_cap)
+
+
+@pytest.mark.parametrize("ctas", [2, 4, 8, 16])
+def test_regions_fit_buffers_of_any_size(dh, ctas):
+    for cand_cap in (32, 48, 256, 2048, 6144, 16384):
+        for list_cap in (32, 512, 6144, 16384):
+            region = dh.dh_gather_region(cand_cap, list_cap, ctas)
+            assert 0 <= region and ctas * region <= cand_cap
