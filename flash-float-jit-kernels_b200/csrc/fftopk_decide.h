@@ -132,18 +132,46 @@ FFTOPK_DECIDE_HD bool sample_admits_too_much(uint32_t admitted, uint32_t sample_
   return (float)admitted * len > 1.25f * (float)room * (float)(sample_total ? sample_total : 1u);
 }
 
+// The ranks sought in a sample of n_s elements: the guess is the bin of rank `need` (0: there is none,
+// and no element is filtered out), and the finish is focused below the bin of rank `need_hi`. Of a row
+// that was read completely (but for the granules that straddle its ends) rank k itself.
+struct SampleRanks {
+  uint32_t need, need_hi;
+};
+FFTOPK_DECIDE_HD SampleRanks sample_ranks(bool whole, uint32_t k, uint32_t n_s, float len) {
+  if (whole) return SampleRanks{k <= n_s ? k : 0u, k <= n_s ? k : 0u};
+  const uint32_t hi = sample_upper_rank(k, n_s, len);
+  return SampleRanks{sample_lower_rank(k, n_s, len), hi > 1u ? hi : 1u};
+}
+
+// What to do about a guess: a bin of `width` keys that holds `cnt` sample elements, `above` of them lie
+// above it, and the bin it was cut out of holds `parent`.
+//   look again   the bin stands for more than factor * k row elements - values crowded into a sliver of
+//                the key space -, and cutting it thins it out: not if it still holds most of the bin it
+//                was cut out of, which are then copies of one value. (Below factor * k, carrying the
+//                extra candidates is cheaper than the second look.)
+//   give up      it admits far more than there is room for: not worth the pass
+//   copies       the threshold is the value the bin holds copies of: the finish need not search above it
+constexpr uint32_t kGuessCoarse = 1u, kGuessGiveUp = 2u, kGuessCopies = 4u;
+FFTOPK_DECIDE_HD uint32_t judge_guess(uint32_t width, uint32_t above, uint32_t cnt, uint32_t parent, uint32_t n_s,
+                                      float len, uint32_t k, float factor, uint32_t room) {
+  const bool copies = cnt >= parent - parent / 4u;
+  if (width > 1u && !copies && sample_bin_too_coarse(cnt, n_s, len, k, factor)) return kGuessCoarse;
+  if (sample_admits_too_much(above + cnt, n_s, len, room)) return kGuessGiveUp;
+  return copies ? kGuessCopies : 0u;
+}
+// ... and how a second look cuts a bin of `width` keys into at most kSampleBins (key offset >> shift)
+FFTOPK_DECIDE_HD int second_look_shift(uint32_t width) {
+  const int bits = 64 - clz64((uint64_t)(width - 1u));
+  return bits > 12 ? bits - 12 : 0;
+}
+
 // The finer sample histogram (key bits [27:16]) may replace the coarse one (bits [31:20]) only if
 // one group of four consecutive coarse super-bins - one value of the key's top four bits - holds
 // the whole sample.
 FFTOPK_DECIDE_HD bool fine_histogram_usable(bool built, uint32_t sample_total, uint32_t group_total) {
   return built && sample_total > 0u && group_total == sample_total;
 }
-
-// Key guess from a bin: prefix of pbits bits (12: the coarse bin; 16: top nibble, then the fine bin).
-FFTOPK_DECIDE_HD uint32_t guess_prefix(bool fine, uint32_t top_nibble, uint32_t bin) {
-  return fine ? ((top_nibble << 12) | bin) : bin;
-}
-FFTOPK_DECIDE_HD uint32_t guess_key(uint32_t prefix, int pbits) { return prefix << (32 - pbits); }
 
 // Lower edge of a key guess as float bits: key(x) >= gkey <=> !(x < edge), NaN included. Keys
 // outside the range that real values map to (below -inf's key, above +inf's) give -inf: the filter

@@ -511,10 +511,6 @@ struct RowSample {
   }
 };
 
-// what the sample search tells the CTA to do (Ctrl::guess_flags)
-constexpr uint32_t kGuessCoarse = 1u;  // the guessed bin is crowded: look at the sample again, inside that bin
-constexpr uint32_t kGuessGiveUp = 2u;  // the guess admits far more than there is room for: full histograms at once
-
 // Everything one CTA needs to know about its row and its shared memory.
 template <int NT, class T>
 struct RowCtx {
@@ -935,21 +931,12 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
 #endif
     }
     if (sampled && warp == NW - 1) {
-      // The sample rank whose true rank is >= k with overwhelming probability (m expected sample
-      // elements among the true top k, plus five standard deviations), and the mirror image: a
-      // sample element the threshold will not lie above (or the sample's largest). Of a row that
-      // was read completely: rank k itself, or none if the granules left out bring it below k. One
-      // warp works this out while the loads travel (a division and a square root in every warp
-      // would cost the CTA as much as the search itself).
-      const uint32_t n_s = smp.size();
-      uint32_t need_s = K <= n_s ? K : 0u, hi_s = need_s;
-      if (!smp.whole) {
-        need_s = sample_lower_rank(K, n_s, (float)len);
-        hi_s = max(sample_upper_rank(K, n_s, (float)len), 1u);
-      }
+      // The ranks sought in the sample (see sample_lower_rank). One warp works them out while the loads
+      // travel (a division and a square root in every warp would cost the CTA as much as the search itself).
+      const SampleRanks ranks = sample_ranks(smp.whole, K, smp.size(), (float)len);
       if (lane == 0) {
-        ctrl->need = need_s;
-        ctrl->need_hi = hi_s;
+        ctrl->need = ranks.need;
+        ctrl->need_hi = ranks.need_hi;
       }
     }
   }
@@ -1001,23 +988,12 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     __syncthreads();
     FFTOPK_MARK(2);
     const uint32_t room = (uint32_t)(C == 1 ? p.list_cap : p.cand_cap);
-    // (one thread, when it has found the bin) what the guess is and what to do about it. A bin that
-    // holds more than ~2k row elements - values crowded into a sliver of the key space - is worth a
-    // second look at the sample, inside that bin. (Below that, carrying the extra candidates is
-    // cheaper. And a bin that still holds most of the bin it was cut out of holds copies of one value:
-    // cutting it further thins nothing out.) A guess that admits far more than there is room for is not worth the pass.
+    // (one thread, when it has found the bin) what the guess is and what to do about it: see judge_guess
     auto judge = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
-      const bool copies = cnt >= parent - parent / 4u;
-      uint32_t flags = 0u;
-      if (width > 1u && !copies && sample_bin_too_coarse(cnt, smp.size(), (float)len, K, kCoarseFactor)) {
-        flags = kGuessCoarse;
-      } else if (sample_admits_too_much(above + cnt, smp.size(), (float)len, room)) {
-        flags = kGuessGiveUp;
-      } else if (copies) {
-        ctrl->focus = low + width - 1u;  // the threshold is that value: the finish need not search above it
-      }
+      const uint32_t flags = judge_guess(width, above, cnt, parent, smp.size(), (float)len, K, kCoarseFactor, room);
+      if (flags & kGuessCopies) ctrl->focus = low + width - 1u;
       ctrl->guess = low;
-      ctrl->guess_flags = flags;
+      ctrl->guess_flags = flags & ~kGuessCopies;
       if (flags & kGuessCoarse) {
         ctrl->cnt = width;
         ctrl->local_c = cnt;
@@ -1039,7 +1015,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     while (flags & kGuessCoarse) {  // (uniform; every round narrows the bin by 12 bits)
       const uint32_t low = ctrl->guess, width = ctrl->cnt, above0 = ctrl->above, rest = ctrl->need;
       const uint32_t cnt0 = ctrl->local_c;
-      const int shift = max(0, 32 - __clz(width - 1u) - 12);
+      const int shift = second_look_shift(width);
       __syncthreads();  // everybody has read the result of the search before
       for (int i = tid; i < kMaxBins / 4; i += NT) sts_zero16(h0 + i * 16);
       if (tid == 0) ctrl->guess_flags = kGuessGiveUp;

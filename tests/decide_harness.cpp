@@ -2,6 +2,8 @@
 // header the kernels include, compiled by g++ and exposed as plain C functions.
 #include "fftopk_decide.h"
 
+#include <vector>
+
 using namespace fftopk;
 
 extern "C" {
@@ -28,13 +30,57 @@ int dh_gather_region(int cand_cap, int list_cap, int ctas) { return gather_regio
 int dh_fine_histogram_usable(int built, uint32_t total, uint32_t group) {
   return fine_histogram_usable(built != 0, total, group) ? 1 : 0;
 }
-uint32_t dh_guess_key(int fine, uint32_t nibble, uint32_t bin) {
-  return guess_key(guess_prefix(fine != 0, nibble, bin), fine ? 16 : 12);
-}
 uint32_t dh_guess_edge_bits(uint32_t gkey) { return guess_edge_bits(gkey); }
 uint32_t dh_guess_low_key(uint32_t gkey) { return guess_low_key(gkey); }
 int dh_sampled_attempt_ok(uint32_t over, uint32_t admitted, uint32_t k, uint32_t room) {
   return sampled_attempt_ok(over, admitted, k, room) ? 1 : 0;
+}
+// One guess from a sample (n float bit patterns; n_s of them count, as in the kernel), made step by step
+// the way the selection kernel makes it. out: guess, focus, flags, second looks. Returns 0, or -1 when
+// the second looks do not come to an end.
+int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, uint32_t k, uint32_t room, int whole, uint32_t* out) {
+  std::vector<uint32_t> hist(kSampleBins, 0u);
+  uint32_t guess = 0u, focus = 0u, flags = 0u, width = 0u, above0 = 0u, rest = 0u, cnt0 = 0u;
+  // the bin of rank `need` from the top
+  auto pick = [&](uint32_t need, uint32_t& above, uint32_t& cnt) {
+    above = 0u;
+    for (int b = kSampleBins - 1; b >= 0; --b) {
+      cnt = hist[b];
+      if (above < need && need <= above + cnt) return b;
+      above += cnt;
+    }
+    return -1;
+  };
+  auto judge = [&](uint32_t low, uint32_t w, uint32_t above, uint32_t cnt, uint32_t r, uint32_t parent) {
+    const uint32_t f = judge_guess(w, above, cnt, parent, n_s, len, k, 2.0f, room);
+    if (f & kGuessCopies) focus = low + w - 1u;
+    guess = low;
+    flags = f & ~kGuessCopies;
+    if (f & kGuessCoarse) width = w, cnt0 = cnt, above0 = above, rest = r;
+  };
+  const SampleRanks ranks = sample_ranks(whole != 0, k, n_s, len);
+  for (uint32_t i = 0; i < n; ++i) ++hist[sample_digit(bits[i])];
+  uint32_t above, cnt;
+  int b = pick(ranks.need, above, cnt);
+  if (b >= 0) judge(sample_digit_low(b), sample_digit_high(b) - sample_digit_low(b) + 1u, above, cnt, ranks.need - above, 0xffffffffu);
+  b = pick(ranks.need_hi, above, cnt);
+  if (b >= 0) focus = sample_digit_high(b);
+  uint32_t looks = 0u;
+  for (; flags & kGuessCoarse; ++looks) {
+    if (looks == 8u) return -1;
+    const uint32_t low = guess, w = width, a0 = above0, r = rest, c0 = cnt0;
+    const int shift = second_look_shift(w);
+    hist.assign(kSampleBins, 0u);
+    flags = kGuessGiveUp;
+    for (uint32_t i = 0; i < n; ++i) {
+      const uint32_t off = fftopk_key_from_bits(bits[i]) - low;
+      if (off < w) ++hist[(off >> shift) & (uint32_t)(kSampleBins - 1)];
+    }
+    b = pick(r, above, cnt);
+    if (b >= 0) judge(low + ((uint32_t)b << shift), 1u << shift, a0 + above, cnt, r - above, c0);
+  }
+  out[0] = guess, out[1] = focus, out[2] = flags, out[3] = looks;
+  return 0;
 }
 int dh_finish_bins(void) { return kFinishBins; }
 int dh_finish_shift(uint64_t lo, uint64_t focus) { return make_finish_digit(lo, focus).shift; }

@@ -1,7 +1,8 @@
 """CPU tests of the selector's decision rules. The kernels take every guess / fall-back decision
 through csrc/fftopk_decide.h; here the same header is compiled by g++ and driven with generated
-inputs, and a numpy restatement of the sampled attempt (sample -> histogram -> rank bound -> key
-guess -> float edge -> filter -> keep-or-fall-back) is run end to end on the host:
+inputs, and one sampled attempt (sample positions -> histogram on the sample digit -> rank bound -> bin,
+cut again where it is crowded -> key guess -> float edge -> filter -> keep-or-fall-back) is run end to
+end on the host, through the functions the kernel calls and in its order (the harness's dh_sample_guess):
 
   * whatever the data and the sample, the attempt is either abandoned or admits a superset of the
     true top k; on i.i.d. rows it is practically never abandoned and admits few extras;
@@ -37,7 +38,9 @@ def dh(tmp_path_factory):
         "dh_sample_lower_rank": (u32, [u32, u32, f32]), "dh_sample_upper_rank": (u32, [u32, u32, f32]),
         "dh_sample_bin_too_coarse": (i32, [u32, u32, f32, u32, f32]),
         "dh_fine_histogram_usable": (i32, [i32, u32, u32]),
-        "dh_guess_key": (u32, [i32, u32, u32]), "dh_guess_edge_bits": (u32, [u32]), "dh_guess_low_key": (u32, [u32]),
+        "dh_sample_guess": (i32, [ctypes.c_void_p, u32, u32, f32, u32, u32, i32, ctypes.c_void_p]),
+        "dh_sample_piece": (i32, []), "dh_sample_piece_start": (u32, [u32, u32, i32, u32]),
+        "dh_guess_edge_bits": (u32, [u32]), "dh_guess_low_key": (u32, [u32]),
         "dh_sampled_attempt_ok": (i32, [u32, u32, u32, u32]),
         "dh_finish_bins": (i32, []), "dh_finish_shift": (i32, [u64, u64]), "dh_finish_key_only": (i32, [u64, u64]),
         "dh_finish_digit": (u32, [u64, u64, u64]), "dh_finish_digit_of_key": (u32, [u64, u64, u32]),
@@ -79,33 +82,34 @@ def _edge_admits(dh, row, gkey):
     return admitted
 
 
-def sampled_attempt(dh, row, positions, k=K, room=1 << 30):
-    """numpy restatement of one sampled attempt; returns (kept, admitted mask)."""
-    keys = orc.keys_of(row)
-    sample = keys[positions]
-    n_s, length = sample.size, float(row.size)
-    need = dh.dh_sample_lower_rank(k, n_s, length)
-    hist_a = np.bincount(sample >> 20, minlength=4096)
-    # the finer histogram applies when one value of the top four key bits holds the whole sample
-    nib = np.bincount(sample >> 28, minlength=16)
-    fine = bool(dh.dh_fine_histogram_usable(1, n_s, int(nib.max())))
-    hist = np.bincount((sample >> 16) & 0xFFF, minlength=4096) if fine else hist_a
-    suffix = np.cumsum(hist[::-1])[::-1]  # elements in bins >= b
-    if need == 0 or suffix[0] < need:
+def sample_positions(dh, length, n_s):
+    """Row indices of the kernel's sample of a row (aligned to a granule of four elements): all of a row that
+    is no longer than the sample, else pieces of consecutive granules."""
+    gi = length // 4
+    if 4 * gi <= n_s:
+        return np.arange(4 * gi)
+    pieces = n_s // (4 * dh.dh_sample_piece())
+    first = np.array([dh.dh_sample_piece_start(gi, i, pieces.bit_length() - 1, 0) for i in range(pieces)], np.int64)
+    return (4 * first[:, None] + np.arange(4 * dh.dh_sample_piece())[None, :]).reshape(-1)
+
+
+GIVE_UP = 2
+
+
+def sample_guess(dh, row, positions, k=K, room=1 << 30, whole=False):
+    """(guess, focus, flags, second looks) the kernel makes on this sample of the row"""
+    sample = np.ascontiguousarray(row[positions].view(np.uint32))
+    out = np.zeros(4, np.uint32)
+    assert dh.dh_sample_guess(sample.ctypes.data, sample.size, sample.size, float(row.size), k, room, int(whole), out.ctypes.data) == 0
+    return [int(v) for v in out]
+
+
+def sampled_attempt(dh, row, positions, k=K, room=1 << 30, whole=False):
+    """One sampled attempt with `room` for the candidates; returns (kept, admitted mask)."""
+    guess, _, flags, _ = sample_guess(dh, row, positions, k, room, whole)
+    if flags & GIVE_UP:
         return False, None
-    t = int(np.nonzero(suffix >= need)[0].max())
-    gkey = dh.dh_guess_key(int(fine), int(nib.argmax()), t)
-    pbits = 16 if fine else 12
-    if dh.dh_sample_bin_too_coarse(int(hist[t]), n_s, length, k, 2.0):
-        rem = need - (int(suffix[t + 1]) if t + 1 < 4096 else 0)
-        sb = 32 - pbits - 12
-        inside = sample[(sample >> (32 - pbits)) == (gkey >> (32 - pbits))]
-        h2 = np.bincount((inside >> sb) & 0xFFF, minlength=4096)
-        s2 = np.cumsum(h2[::-1])[::-1]
-        if s2[0] < rem:
-            return False, None
-        gkey |= int(np.nonzero(s2 >= rem)[0].max()) << sb
-    admitted = _edge_admits(dh, row, gkey)
+    admitted = _edge_admits(dh, row, guess)
     return bool(dh.dh_sampled_attempt_ok(0, int(admitted.sum()), k, room)), admitted
 
 
@@ -120,22 +124,25 @@ def _rows(rng, length):
     yield "all equal", np.full(length, 2.5, np.float32)
     yield "specials", np.where(rng.random(length) < 0.01, np.nan, np.where(rng.random(length) < 0.01, -np.inf,
                                rng.standard_normal(length))).astype(np.float32)
+    # the k-th largest is one of the copies of -0, a quarter of the row; few elements lie above them
+    yield "zeros at the threshold", np.where(rng.random(length) < 0.25, np.float32(-0.0), np.where(
+        rng.random(length) < 0.01, 1, -rng.random(length) - 0.1)).astype(np.float32)
     r = rng.standard_normal(length).astype(np.float32)
     r[1000:2900] += 100  # a window of winners the sample may miss entirely
     yield "window", r
 
 
-@pytest.mark.parametrize("length,n_s", [(9000, 8192), (40000, 8192), (131072, 8192), (1 << 20, 16384)])
-def test_sampled_attempt_is_a_superset_or_is_abandoned(dh, length, n_s):
+# the room candidates have: a cluster's buffer, the throughput plan's, a lone CTA's lists
+@pytest.mark.parametrize("room", [16384, 6144, 9216])
+@pytest.mark.parametrize("length,n_s", [(8000, 8192), (9000, 8192), (40000, 8192), (131072, 8192), (1 << 20, 16384)])
+def test_sampled_attempt_is_a_superset_or_is_abandoned(dh, length, n_s, room):
     rng = np.random.default_rng(length)
     for name, row in _rows(rng, length):
-        for slab_sampling in (True, False):
-            if slab_sampling:  # what the kernel does: evenly spaced runs of 128 elements
-                starts = (np.arange(n_s // 128) * (length // (n_s // 128)))[:, None]
-                pos = np.minimum(starts + np.arange(128)[None, :], length - 1).reshape(-1)
-            else:
-                pos = rng.choice(length, n_s, replace=False)
-            kept, admitted = sampled_attempt(dh, row, pos)
+        for as_the_kernel in (True, False):
+            pos = sample_positions(dh, length, n_s) if as_the_kernel else rng.choice(length, min(n_s, length), replace=False)
+            kept, admitted = sampled_attempt(dh, row, pos, room=room, whole=length <= n_s)
+            if name in ("normal", "relu heads", "all negative") and as_the_kernel and (room > 6144 or length < 1 << 20):
+                assert kept, f"{name}: abandoned"
             if not kept:
                 continue  # the kernel falls back to full histograms: always exact
             top = orc.numpy_oracle(row[None, :], np.array([length]), K)[0]
@@ -148,12 +155,28 @@ def test_sampled_attempt_is_rarely_abandoned_on_iid_rows(dh):
     abandoned, extra = 0, []
     for _ in range(300):
         row = rng.standard_normal(65536).astype(np.float32)
-        kept, admitted = sampled_attempt(dh, row, rng.choice(row.size, 8192, replace=False))
+        kept, admitted = sampled_attempt(dh, row, sample_positions(dh, row.size, 8192), room=6144)
         abandoned += 0 if kept else 1
         if kept:
             extra.append(int(admitted.sum()) - K)
     assert abandoned == 0
     assert np.median(extra) < 2 * K  # the safety margin costs a bounded number of extra candidates
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+def test_crowded_bins_are_cut_and_copies_are_recognised(dh, sign):
+    """Values crowded into a sliver of the key space are looked at again, with a finer digit, until the guess
+    admits few enough; a bin of copies is not cut any further and bounds the finish's search from above."""
+    rng = np.random.default_rng(17)
+    row = (sign * (1.0 + 1e-5 * rng.random(131072))).astype(np.float32)
+    guess, _, flags, looks = sample_guess(dh, row, sample_positions(dh, row.size, 8192))
+    assert flags == 0 and looks >= 1
+    assert K <= _edge_admits(dh, row, guess).sum() < 3 * K
+    copies = np.where(rng.random(131072) < 0.05, 2.5, rng.random(131072)).astype(np.float32)
+    guess, focus, flags, looks = sample_guess(dh, copies, sample_positions(dh, copies.size, 8192))
+    assert flags == 0 and looks >= 1 and guess <= int(orc.keys_of(np.float32([2.5]))[0]) <= focus
+    # more copies than there is room for: not worth a pass
+    assert sample_guess(dh, copies, sample_positions(dh, copies.size, 8192), room=4096)[2] == GIVE_UP
 
 
 def test_abandon_conditions(dh):
