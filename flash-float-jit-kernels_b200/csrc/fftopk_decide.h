@@ -97,7 +97,10 @@ FFTOPK_DECIDE_HD bool sample_bin_too_coarse(uint32_t bin_count, uint32_t sample_
 // two. A bin then holds about 1/64 octave of values: the guess made on it admits few elements beyond
 // the sampling margin (a plain 12-bit digit has 8 bins per octave, which on crowded rows - sums over
 // heads, all of one sign and magnitude - costs thousands of extra candidates or a second look).
-// The sample only makes a guess that is checked afterwards: where NaN and -0 fall is of no concern.
+// -0 falls into the bin just below zero, although its key is the first one above it: a second look at that
+// bin takes it in (sample_digit_width). A NaN of negative sign counts as the smallest value here and is
+// the largest key: the guess then lies lower than it need. The sample only makes a guess, which is checked
+// afterwards.
 // ---------------------------------------------------------------------------------------------
 constexpr int kSampleBins = 4096;
 constexpr int kSampleShift = 17;
@@ -124,6 +127,11 @@ FFTOPK_DECIDE_HD uint32_t sample_digit_low(uint32_t bin) {
 }
 FFTOPK_DECIDE_HD uint32_t sample_digit_high(uint32_t bin) {
   return bin == (uint32_t)kSampleBins - 1 ? 0xffffffffu : sample_digit_low(bin + 1u) - 1u;
+}
+
+// the number of keys, from the smallest on, that the elements of a bin may have
+FFTOPK_DECIDE_HD uint32_t sample_digit_width(uint32_t bin) {
+  return sample_digit_high(bin) - sample_digit_low(bin) + (bin == (uint32_t)kSampleBins / 2 - 1 ? 2u : 1u);
 }
 
 // A guess whose share of the sample stands for a quarter more row elements than there is room for is

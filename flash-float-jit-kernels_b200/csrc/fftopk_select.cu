@@ -1005,8 +1005,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       const uint32_t need_s = ctrl->need, need_hi = ctrl->need_hi;
       block_pick_sample<NT>(h0, need_s, need_hi, wtot_s,
                             [&](uint32_t bin, uint32_t above, uint32_t cnt) {
-                              const uint32_t low = sample_digit_low(bin);
-                              judge(low, sample_digit_high(bin) - low + 1u, above, cnt, need_s - above, 0xffffffffu);
+                              judge(sample_digit_low(bin), sample_digit_width(bin), above, cnt, need_s - above, 0xffffffffu);
                             },
                             [&](uint32_t bin) { ctrl->focus = sample_digit_high(bin); });
     }

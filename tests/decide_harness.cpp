@@ -62,7 +62,7 @@ int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, u
   for (uint32_t i = 0; i < n; ++i) ++hist[sample_digit(bits[i])];
   uint32_t above, cnt;
   int b = pick(ranks.need, above, cnt);
-  if (b >= 0) judge(sample_digit_low(b), sample_digit_high(b) - sample_digit_low(b) + 1u, above, cnt, ranks.need - above, 0xffffffffu);
+  if (b >= 0) judge(sample_digit_low(b), sample_digit_width(b), above, cnt, ranks.need - above, 0xffffffffu);
   b = pick(ranks.need_hi, above, cnt);
   if (b >= 0) focus = sample_digit_high(b);
   uint32_t looks = 0u;

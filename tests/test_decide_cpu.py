@@ -179,6 +179,14 @@ def test_crowded_bins_are_cut_and_copies_are_recognised(dh, sign):
     assert sample_guess(dh, copies, sample_positions(dh, copies.size, 8192), room=4096)[2] == GIVE_UP
 
 
+def test_negative_zeros_at_the_threshold_are_found_by_both_looks(dh):
+    rng = np.random.default_rng(23)
+    row = np.where(rng.random(131072) < 0.1, np.float32(-0.0), -rng.random(131072) - 0.1).astype(np.float32)
+    row[rng.random(row.size) < 0.005] = 1.0
+    guess, _, flags, _ = sample_guess(dh, row, sample_positions(dh, row.size, 8192), room=16384)
+    assert flags == 0 and K <= _edge_admits(dh, row, guess).sum() <= 16384
+
+
 def test_abandon_conditions(dh):
     assert dh.dh_sampled_attempt_ok(0, K, K, 4096) == 1
     assert dh.dh_sampled_attempt_ok(0, K - 1, K, 4096) == 0  # guess too high

@@ -91,6 +91,7 @@ CASES = {
     "keys around a shard boundary": (("straddling", 4, 131072, 2048, 1, 0), 8, False, True),
     "4M elements, k = 4096": (("normal", 1, (1 << 22) + 3, 4096, 0, 0), 16, False, True),
     "12M elements": (("normal", 1, 12 << 20, 2048, 0, 0), 16, False, None),
+    "copies of -0 at the threshold": (("negative zeros", 2, 131072, 2048, 0, 0), 16, False, True),
     "all equal": (("equal", 2, 65536, 2048, 0, 0), 16, True, False),
 }
 
