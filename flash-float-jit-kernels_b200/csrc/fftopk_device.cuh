@@ -235,7 +235,6 @@ struct Ctrl {
   int32_t sup_sel;
   uint32_t sup_above;
   uint32_t need;
-  uint32_t any_flag;
   int32_t mode;
   uint32_t base_w;
   uint32_t base_c;
@@ -311,7 +310,6 @@ struct Picked {
   uint32_t local_w;   // this CTA's elements in bins above t
   uint32_t local_c;   // this CTA's elements in bin t
   uint32_t total;     // cluster-wide number of histogrammed elements
-  uint32_t any_flag;  // OR of the peers' published flags
   int tf;             // t's position inside its super-bin (index into xch rows)
   bool fine;          // the search ran on the second, finer histogram (see cluster_pick)
   uint32_t group;     // ... whose bins all lie under this value of the key's top four bits
@@ -419,7 +417,6 @@ __device__ __forceinline__ void cluster_pick(cg::cluster_group& cluster, int C, 
     pk.t = -1;
     pk.need2 = pk.cnt = pk.local_w = pk.local_c = 0;
     pk.total = ctrl->run_total;
-    pk.any_flag = 0u;
     pk.tf = 0;
     pk.fine = dual && ctrl->dual_b != 0u;
     pk.group = ctrl->dual_g;
@@ -455,14 +452,11 @@ __device__ __forceinline__ void cluster_pick(cg::cluster_group& cluster, int C, 
 // each on rank 0's counters.
 // `cx` is anything with the members ctrl, ctrl0 (rank 0's control block) and cand_cap.
 template <class Ctx>
-__device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked& pk, int otherwise,
-                                                    bool force_otherwise) {
+__device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked& pk, int otherwise) {
   int md = kModeAbort;
   uint32_t base_w = 0, base_c = 0, lw = pk.local_w;
   if (pk.ok) {
-    if (force_otherwise) {
-      md = otherwise;
-    } else if (pk.cnt == pk.need2) {
+    if (pk.cnt == pk.need2) {
       md = kModeTakeAll;
       lw += pk.local_c;
     } else if (pk.cnt <= (uint32_t)cx.cand_cap) {
@@ -470,7 +464,7 @@ __device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked&
     } else {
       md = otherwise;
     }
-    if (lane_id() == 0 && md != kModeFallback) {
+    if (lane_id() == 0) {
       base_w = atomicAdd(&cx.ctrl0->win_count, lw);
       if (md == kModeGather) base_c = atomicAdd(&cx.ctrl0->cand_count, pk.local_c);
     }

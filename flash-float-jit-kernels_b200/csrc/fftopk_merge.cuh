@@ -283,7 +283,7 @@ __device__ __forceinline__ void merge_row(cg::cluster_group& cluster, int C, int
   int pick_no = 0;
   cluster_pick<NT>(
       cluster, G, hist, sm.sup, sm.xch, ctrl, pick_no, kMaxBins, [&](uint32_t) { return (uint32_t)kK; },
-      [&](Picked& pk) { decide_and_allocate(cx, pk, kModeAbort, false); }, hist + kMaxBins, sm.sup + kSup);
+      [&](Picked& pk) { decide_and_allocate(cx, pk, kModeAbort); }, hist + kMaxBins, sm.sup + kSup);
   FFTOPK_MARK(65);
   const int mode = ctrl->mode;
   // the threshold bin as a key prefix: 12 bits, or 16 when the finer histogram was searched

@@ -517,7 +517,7 @@ struct RowCtx {
   int C, rank;
   Shard<T> sh;
   uint32_t* hist0;  // two histograms of kMaxBins words, back to back
-  uint32_t* sup0;   // three super-bin arrays of kSup words, back to back
+  uint32_t* sup0;   // two super-bin arrays of kSup words, back to back
   // (computed addresses instead of pointer arrays: indexing an array member with the round number
   // would force the whole struct into local memory)
   __device__ __forceinline__ uint32_t* hist(int i) const { return hist0 + i * kMaxBins; }
@@ -533,7 +533,6 @@ struct RowCtx {
   int32_t idx_offset;
   const int32_t* page;  // fused page-table transform: out = page[idx] (NULL: out = idx + idx_offset)
   int32_t cand_cap;
-  int32_t list_cap;
   uint32_t* status;
   uint32_t k;  // elements to select per row (2048 for the reference's op)
 };
@@ -602,7 +601,7 @@ __device__ __forceinline__ int refine_from_data(const RowCtx<NT, T>& cx, uint32_
         cluster, C, h, s, xch, ctrl, pick_no, nb, [&](uint32_t) { return need_now; },
         [&](Picked& pk) {
           const bool last = (shift == 0);
-          decide_and_allocate(cx, pk, last ? kModeTies : kModeNext, false);
+          decide_and_allocate(cx, pk, last ? kModeTies : kModeNext);
           if (pk.ok && last && pk.cnt > (uint32_t)cx.cand_cap && pk.cnt != pk.need2) {
             // exact duplicates of the threshold key: ties before this shard, in rank order
             const uint32_t tp = (lane < rank) ? xch[lane * kSup + pk.tf] : 0u;
@@ -827,7 +826,6 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     cx.page = p.src_page_table + req * p.src_stride;
   }
   cx.cand_cap = p.cand_cap;
-  cx.list_cap = p.list_cap;
   cx.status = p.status;
 
   // Short rows: 0..len-1 then -1 (reference: naive_topk_cuda, topk_indexer_radix.cu:152-163).
@@ -849,7 +847,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   cx.hist0 = reinterpret_cast<uint32_t*>(smem_raw);
   cx.sup0 = cx.hist0 + 2 * kMaxBins;
-  cx.xch = cx.sup0 + 3 * kSup;                                             // kMaxCluster * 64 words
+  cx.xch = cx.sup0 + 2 * kSup;                                             // kMaxCluster * 64 words
   Ctrl* ctrl = cx.ctrl = reinterpret_cast<Ctrl*>(cx.xch + kMaxCluster * kSup);  // 8-byte aligned
   cx.list = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(ctrl) + ((sizeof(Ctrl) + 127) & ~127u));
   // a cluster of one CTA has nobody to gather from: its candidate buffer IS the list
@@ -1292,7 +1290,7 @@ __global__ void __launch_bounds__(NT, min_ctas<NT>(kRoomyForm)) select_merge2048
   MergeSmem sm;
   sm.hist = reinterpret_cast<uint32_t*>(smem_raw);
   sm.sup = sm.hist + 2 * kMaxBins;
-  sm.xch = sm.sup + 3 * kSup;
+  sm.xch = sm.sup + 2 * kSup;
   sm.ctrl = reinterpret_cast<Ctrl*>(sm.xch + kMaxCluster * kSup);
   sm.cand = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(sm.ctrl) + ((sizeof(Ctrl) + 127) & ~127u));
   sm.cand_cap = C == 1 ? p.list_cap : p.list_cap + p.cand_cap;
@@ -1338,11 +1336,10 @@ struct DeviceInfo {
 DeviceInfo g_dev[kMaxDevices];
 
 constexpr size_t fixed_smem_bytes() {
-  return (size_t)(2 * kMaxBins + 3 * kSup + kMaxCluster * kSup) * 4 + ((sizeof(Ctrl) + 127) & ~(size_t)127);
+  return (size_t)(2 * kMaxBins + 2 * kSup + kMaxCluster * kSup) * 4 + ((sizeof(Ctrl) + 127) & ~(size_t)127);
 }
 
 constexpr int kLatencyListCap = 6144, kLatencyCandCap = 16384;  // one CTA per SM: use the shared memory
-constexpr int kBatchListCap = 4096, kBatchCandCap = 4096;       // several CTAs per SM
 // One CTA per row (list = candidates), two CTAs per SM. Rows of up to ~192K elements leave about
 // 3600 candidates; with the small list two CTAs take 2 x 90 KB of the SM's 256 KB and the rest
 // stays L1, which the value re-reads of the filter hit (measured on B=64 ragged rows <= 128K:
@@ -1415,7 +1412,7 @@ int init_device(DeviceInfo& d, int dev) {
   for (int cs = 16; cs >= 8; cs /= 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs * 32, 1, 1);
-    cfg.blockDim = dim3(1024, 1, 1);
+    cfg.blockDim = dim3(512, 1, 1);  // (the form that such a plan launches)
     cfg.dynamicSmemBytes = fixed_smem_bytes() + (size_t)(kLatencyListCap + kLatencyCandCap) * 8;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1425,7 +1422,7 @@ int init_device(DeviceInfo& d, int dev) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&nclusters, select2048_kernel<1024, kRoomyForm>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&nclusters, select2048_kernel<512, kRoomyForm>, &cfg);
     if (e == cudaSuccess && nclusters >= 1) {
       if (cs == 16) {
         d.max_cluster = 16;
@@ -1484,18 +1481,19 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
   // 96K 10.0 / 11.6, 1M 14.9 / 15.9; B=64 ragged rows of up to 128K 15.5 / 15.9. A lone CTA has no
   // other CTA to share its row with: 1024.
   pl.threads = pl.cluster > 1 ? 512 : 1024;
-  const bool one_per_sm = (int64_t)rows * pl.cluster <= d.sm_count;
-  pl.list_cap = one_per_sm ? kLatencyListCap : kBatchListCap;
-  pl.cand_cap = one_per_sm ? kLatencyCandCap : kBatchCandCap;
+  pl.list_cap = kLatencyListCap;
+  pl.cand_cap = kLatencyCandCap;
   if (rows > d.sm_count) {
     // More rows than SMs: the batch fills the device by itself. One 512-thread CTA per row with
     // the list of the throughput plan, two CTAs per SM (measured on ragged rows of up to 128K
     // elements: 29.7 us per call at B=256 and 52.6 us at B=512, against 38.5 / 68.1 us with 1024
     // threads; a list of 4096 entries split over 32 warps overflowed its segments and sent rows
-    // to the full-histogram path: 78 / 113 us).
+    // to the full-histogram path: 78 / 113 us). (The gather buffer is for tunings that ask for more
+    // CTAs per row.)
     pl.cluster = 1;
     pl.threads = 512;
     pl.list_cap = L <= kOverlapShortRow ? kOverlapListCap1 : kOverlapListCap1Long;
+    pl.cand_cap = kOverlapCandCap;
   }
   if (overlap) {
     // Back-to-back calls may overlap: what counts is work per row, not the latency of one call.
