@@ -77,6 +77,7 @@ struct SelectParams {
   int32_t idx_offset;
   int32_t list_cap;  // per-CTA candidate list capacity (entries), multiple of 16
   int32_t cand_cap;  // rank 0's gathered-candidate capacity (entries), multiple of 16
+  int32_t region;    // slots of each CTA in it (gather_region; two divisions that no thread has to wait for)
   int32_t force_slow;  // tests: skip the filter path and run the full-histogram path
   int32_t overlap;     // let the next launch on the stream start before this one has finished
   // fused output transforms (all optional; reference: topk_transform_decode_kernel,
@@ -1074,7 +1075,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   const uint32_t wown = min(wcnt, seg_cap);
   FFTOPK_MARK(8);
   bool have_hist = false;  // (lone CTA) round 0 of the finish has its histogram
-  const int region = C == 1 ? 0 : gather_region(p.cand_cap, p.list_cap, C);  // slots of each CTA in rank 0's buffer
+  const int region = kLone ? 0 : p.region;  // slots of each CTA in rank 0's buffer
   int extra = 0;           // candidates beyond their CTAs' regions
   uint32_t total = 0u;     // candidates of the row
   uint32_t fin_sn = 0u;
@@ -1574,6 +1575,7 @@ int launch_select(const SelectCall& c) {
   p.idx_offset = c.idx_offset;
   p.list_cap = pl.list_cap;
   p.cand_cap = pl.cand_cap;
+  p.region = pl.cluster > 1 ? gather_region(pl.cand_cap, pl.list_cap, pl.cluster) : 0;
   p.force_slow = tn.force_slow;
   p.overlap = overlap ? 1 : 0;
   p.src_page_table = c.src_page_table;
@@ -1670,6 +1672,7 @@ int launch_select_merge(const SelectCall& c, void* const* comms, int32_t G, int3
   p.idx_offset = c.idx_offset;
   p.list_cap = pl.list_cap;
   p.cand_cap = pl.cand_cap;
+  p.region = pl.cluster > 1 ? gather_region(pl.cand_cap, pl.list_cap, pl.cluster) : 0;
   p.force_slow = tn.force_slow;
 
   cudaLaunchConfig_t cfg = {};
