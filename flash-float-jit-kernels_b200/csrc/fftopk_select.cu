@@ -25,10 +25,10 @@
 //      finishes: radix rounds over the composites' range, a counting and a writing pass, and the last
 //      <= 256 undecided candidates ranked by votes. A lone CTA finishes over its segments where they
 //      lie. The inverted index in the composite makes equal values resolve to the lower index.
-//      Measured (us per call in a chain of calls on B200, before -> with steps 1 to 4 as they are now):
-//      B=1, L=96K 12.9 -> 10.3, 1M 15.4 -> 14.4; B=4, L=200K 13.6 -> 11.1; B=64 ragged rows of up to 128K
-//      17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5); B=2048, one CTA per row, L=32K 132 -> 101, 8K
-//      106 -> 70. What bounds it is no bandwidth but the chain of short phases and the instructions in it.
+//      Measured (us per call in a chain of calls on B200, when histograms were exchanged -> with steps 1 to 4
+//      as they are now): B=1, L=96K 12.9 -> 10.0, 1M 15.4 -> 14.1; B=4, L=200K 13.6 -> 10.7; B=64 ragged rows
+//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5); B=2048, one CTA per row, L=32K
+//      132 -> 102, 8K 106 -> 67. What bounds it is no bandwidth but the chain of short phases and the instructions in it.
 //   5. If the guess admitted fewer than k elements, a list overflowed or the threshold bin is
 //      larger than rank 0's buffer (heavy ties, rows of equal values), the cluster falls back to
 //      full histograms over the data: 12 + 12 + 8 key bits, re-reading the shard from L2 each
