@@ -161,7 +161,7 @@ FFTOPK_DECIDE_HD SampleRanks sample_ranks(bool whole, uint32_t k, uint32_t n_s, 
 //   give up      it admits far more than there is room for: not worth the pass
 //   copies       the threshold is the value the bin holds copies of: the finish need not search above it
 constexpr uint32_t kGuessCoarse = 1u, kGuessGiveUp = 2u, kGuessCopies = 4u;
-FFTOPK_DECIDE_HD uint32_t judge_guess(uint32_t width, uint32_t above, uint32_t cnt, uint32_t parent, uint32_t n_s,
+FFTOPK_DECIDE_HD uint32_t weigh_guess(uint32_t width, uint32_t above, uint32_t cnt, uint32_t parent, uint32_t n_s,
                                       float len, uint32_t k, float factor, uint32_t room) {
   const bool copies = cnt >= parent - parent / 4u;
   if (width > 1u && !copies && sample_bin_too_coarse(cnt, n_s, len, k, factor)) return kGuessCoarse;

@@ -987,9 +987,9 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     __syncthreads();
     FFTOPK_MARK(2);
     const uint32_t room = (uint32_t)(C == 1 ? p.list_cap : p.cand_cap);
-    // (one thread, when it has found the bin) what the guess is and what to do about it: see judge_guess
-    auto judge = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
-      const uint32_t flags = judge_guess(width, above, cnt, parent, smp.size(), (float)len, K, kCoarseFactor, room);
+    // (one thread, when it has found the bin) what the guess is and what to do about it: see weigh_guess
+    auto weigh = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
+      const uint32_t flags = weigh_guess(width, above, cnt, parent, smp.size(), (float)len, K, kCoarseFactor, room);
       if (flags & kGuessCopies) ctrl->focus = low + width - 1u;
       ctrl->guess = low;
       ctrl->guess_flags = flags & ~kGuessCopies;
@@ -1004,7 +1004,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       const uint32_t need_s = ctrl->need, need_hi = ctrl->need_hi;
       block_pick_sample<NT>(h0, need_s, need_hi, wtot_s,
                             [&](uint32_t bin, uint32_t above, uint32_t cnt) {
-                              judge(sample_digit_low(bin), sample_digit_width(bin), above, cnt, need_s - above, 0xffffffffu);
+                              weigh(sample_digit_low(bin), sample_digit_width(bin), above, cnt, need_s - above, 0xffffffffu);
                             },
                             [&](uint32_t bin) { ctrl->focus = sample_digit_high(bin); });
     }
@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       __syncthreads();
       block_pick_sample<NT>(h0, rest, 0u, wtot_s,
                             [&](uint32_t bin, uint32_t above, uint32_t cnt) {
-                              judge(low + (bin << shift), 1u << shift, above0 + above, cnt, rest - above, cnt0);
+                              weigh(low + (bin << shift), 1u << shift, above0 + above, cnt, rest - above, cnt0);
                             },
                             [&](uint32_t) {});
       flags = ctrl->guess_flags;

@@ -51,8 +51,8 @@ int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, u
     }
     return -1;
   };
-  auto judge = [&](uint32_t low, uint32_t w, uint32_t above, uint32_t cnt, uint32_t r, uint32_t parent) {
-    const uint32_t f = judge_guess(w, above, cnt, parent, n_s, len, k, 2.0f, room);
+  auto weigh = [&](uint32_t low, uint32_t w, uint32_t above, uint32_t cnt, uint32_t r, uint32_t parent) {
+    const uint32_t f = weigh_guess(w, above, cnt, parent, n_s, len, k, 2.0f, room);
     if (f & kGuessCopies) focus = low + w - 1u;
     guess = low;
     flags = f & ~kGuessCopies;
@@ -62,7 +62,7 @@ int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, u
   for (uint32_t i = 0; i < n; ++i) ++hist[sample_digit(bits[i])];
   uint32_t above, cnt;
   int b = pick(ranks.need, above, cnt);
-  if (b >= 0) judge(sample_digit_low(b), sample_digit_width(b), above, cnt, ranks.need - above, 0xffffffffu);
+  if (b >= 0) weigh(sample_digit_low(b), sample_digit_width(b), above, cnt, ranks.need - above, 0xffffffffu);
   b = pick(ranks.need_hi, above, cnt);
   if (b >= 0) focus = sample_digit_high(b);
   uint32_t looks = 0u;
@@ -77,7 +77,7 @@ int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, u
       if (off < w) ++hist[(off >> shift) & (uint32_t)(kSampleBins - 1)];
     }
     b = pick(r, above, cnt);
-    if (b >= 0) judge(low + ((uint32_t)b << shift), 1u << shift, a0 + above, cnt, r - above, c0);
+    if (b >= 0) weigh(low + ((uint32_t)b << shift), 1u << shift, a0 + above, cnt, r - above, c0);
   }
   out[0] = guess, out[1] = focus, out[2] = flags, out[3] = looks;
   return 0;
