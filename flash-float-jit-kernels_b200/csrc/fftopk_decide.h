@@ -106,16 +106,19 @@ constexpr int kSampleBins = 4096;
 constexpr int kSampleShift = 17;
 constexpr int32_t kSampleBase = 111 << 23;              // 2^-16
 constexpr int32_t kSampleSpan = (32 << 23) - 1;         // 32 octaves
-FFTOPK_DECIDE_HD uint32_t sample_digit(uint32_t bits) {
+// ... as the byte offset of the bin's counter from that of the bin above zero: what a histogram update wants
+FFTOPK_DECIDE_HD int32_t sample_digit_offset(uint32_t bits) {
   const int32_t sign = (int32_t)bits >> 31;
-  int32_t d = (int32_t)(bits & 0x7fffffffu) - kSampleBase;
+  const int32_t mag = (int32_t)(bits & 0x7fffffffu);
 #if defined(__CUDA_ARCH__)
-  d = __vimin_s32_relu(d, kSampleSpan);
+  const int32_t d = __viaddmin_s32_relu(mag, -kSampleBase, kSampleSpan);
 #else
-  d = d < 0 ? 0 : (d < kSampleSpan ? d : kSampleSpan);
+  const int32_t a = mag - kSampleBase;
+  const int32_t d = a < 0 ? 0 : (a < kSampleSpan ? a : kSampleSpan);
 #endif
-  return (uint32_t)(((d >> kSampleShift) ^ sign) + kSampleBins / 2);
+  return ((d >> (kSampleShift - 2)) ^ sign) & ~3;
 }
+FFTOPK_DECIDE_HD uint32_t sample_digit(uint32_t bits) { return (uint32_t)((sample_digit_offset(bits) >> 2) + kSampleBins / 2); }
 // the smallest key of a bin (a bin ends where the next one starts; the last one holds every key above)
 FFTOPK_DECIDE_HD uint32_t sample_digit_low(uint32_t bin) {
   if (bin >= (uint32_t)kSampleBins / 2) {
@@ -216,49 +219,57 @@ FFTOPK_DECIDE_HD int gather_region(int cand_cap, int list_cap, int ctas) {
 // a long one as well cost 64 rows with 6,500 copies of the threshold 26.3 us instead of 24.4.)
 FFTOPK_DECIDE_HD int list_spill(int list_cap, bool lone) { return list_cap / (lone || list_cap >= 4096 ? 8 : 4); }
 
+// A lone CTA's segments hold row indices (words, in the memory of list_cap composites less the spill area), and the finish
+// has their keys in registers: so many per thread, and no more candidates per warp than that.
+FFTOPK_DECIDE_HD constexpr int lone_regs(int threads) { return threads >= 1024 ? 8 : 16; }
+FFTOPK_DECIDE_HD int lone_segment(int list_cap, int threads) {
+  const int own = 2 * (list_cap - list_spill(list_cap, true)) / (threads / 32);
+  return own < 32 * lone_regs(threads) ? own : 32 * lone_regs(threads);
+}
+// ... the whole list in bytes (composites of the spill area behind the segments), and in candidates
+FFTOPK_DECIDE_HD int lone_list_bytes(int list_cap, int threads) {
+  return ((threads / 32 * lone_segment(list_cap, threads) + 1) / 2 + list_spill(list_cap, true)) * 8;
+}
+FFTOPK_DECIDE_HD int lone_room(int list_cap, int threads) {
+  return threads / 32 * lone_segment(list_cap, threads) + list_spill(list_cap, true);
+}
+
 // ---------------------------------------------------------------------------------------------
-// Digit rule of a finish round over the composite range [lo, cap]: digit(c) = min((c - lo) >>
+// Digit rule of a finish round over a field's range [lo, cap]: digit(v) = min((v - lo) >>
 // shift, kFinishBins - 1). The shift is chosen so that [lo, focus] spreads over the bins below the
 // last one; everything above `focus` (cap >= focus >= lo) lands in the last bin. With focus == cap
 // this is a plain radix digit of the range; a caller that knows where in the range the threshold
-// will fall passes a tighter focus and gets finer bins there.
+// will fall passes a tighter focus and gets finer bins there. The rounds work on 32-bit fields: the keys, and
+// the inverted indices under one key.
 // ---------------------------------------------------------------------------------------------
-struct FinishDigit {
-  uint64_t lo;
+template <class V>
+struct FieldDigit {
+  V lo;
   int shift;
-  FFTOPK_DECIDE_HD uint32_t of(uint64_t c) const {
-    const uint64_t d = (c - lo) >> shift;
-    return d < (uint64_t)(kFinishBins - 1) ? (uint32_t)d : (uint32_t)(kFinishBins - 1);
+  FFTOPK_DECIDE_HD uint32_t of(V v) const {
+    const V d = (V)(v - lo) >> shift;
+    return d < (V)(kFinishBins - 1) ? (uint32_t)d : (uint32_t)(kFinishBins - 1);
   }
-  // the same for a digit that depends on the key alone (shift >= 32 and the low word of lo is 0)
-  FFTOPK_DECIDE_HD uint32_t of_key(uint32_t k) const {
-    const uint32_t d = (k - (uint32_t)(lo >> 32)) >> (shift - 32);
-    return d < (uint32_t)(kFinishBins - 1) ? d : (uint32_t)(kFinishBins - 1);
+  // the values of bin t (one that holds a value of [lo, cap])
+  FFTOPK_DECIDE_HD V bin_low(uint32_t t) const { return lo + ((V)t << shift); }
+  FFTOPK_DECIDE_HD V bin_high(uint32_t t, V cap) const {
+    const V low = bin_low(t), high = low + (((V)1 << shift) - 1u);
+    return t == (uint32_t)kFinishBins - 1u || high > cap || high < low ? cap : high;
   }
-  FFTOPK_DECIDE_HD bool key_only() const { return shift >= 32 && (uint32_t)lo == 0u; }
 };
-
-FFTOPK_DECIDE_HD FinishDigit make_finish_digit(uint64_t lo, uint64_t focus) {
-  const uint64_t width = focus - lo;
-  const int bits = width ? 64 - clz64(width) : 0;
+template <class V>
+FFTOPK_DECIDE_HD FieldDigit<V> make_field_digit(V lo, V focus) {
+  const V width = focus - lo;
+  const int bits = 64 - clz64((uint64_t)width);
   int shift = bits > kFinishBits ? bits - kFinishBits : 0;
-  if ((width >> shift) >= (uint64_t)(kFinishBins - 1)) ++shift;  // keep the last bin for what lies above
-  return FinishDigit{lo, shift};
+  if ((width >> shift) >= (V)(kFinishBins - 1)) ++shift;  // keep the last bin for what lies above
+  return FieldDigit<V>{lo, shift};
 }
+using KeyDigit = FieldDigit<uint32_t>;
+FFTOPK_DECIDE_HD KeyDigit make_key_digit(uint32_t lo, uint32_t focus) { return make_field_digit<uint32_t>(lo, focus); }
 
-// Composite range of finish bin t under digit rule dg over [lo, cap].
-FFTOPK_DECIDE_HD void finish_bin_range(const FinishDigit& dg, uint64_t lo, uint64_t cap, int t, uint64_t& t_lo,
-                                       uint64_t& t_hi) {
-  t_lo = lo + ((uint64_t)t << dg.shift);
-  t_hi = (t == kFinishBins - 1) ? cap : t_lo + ((1ull << dg.shift) - 1ull);
-  if (t_hi > cap || t_hi < t_lo) t_hi = cap;
-}
-
-// When a round has narrowed the range to one key, every composite there starts its low word with
-// the same run of ones (indices are < 2^idx_bits and stored inverted): the smallest possible one.
-FFTOPK_DECIDE_HD uint64_t single_key_floor(uint64_t lo, int idx_bits) {
-  return (lo & 0xffffffff00000000ull) | (uint64_t)(~((idx_bits >= 32 ? 0u : (1u << idx_bits)) - 1u));
-}
+// (indices are < 2^idx_bits and stored inverted: the smallest inverted index)
+FFTOPK_DECIDE_HD uint32_t inverted_index_floor(int idx_bits) { return ~((idx_bits >= 32 ? 0u : (1u << idx_bits)) - 1u); }
 
 // ---------------------------------------------------------------------------------------------
 // Work split of the fused indexer's producer. The tiles of all rows, row after row, form one

@@ -108,6 +108,9 @@ __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t lo, uint32_t hi) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(lo), "r"(hi) : "memory");
 }
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 __device__ __forceinline__ void sts_zero16(uint32_t a) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(a), "r"(0) : "memory");
 }
@@ -125,8 +128,11 @@ __device__ __forceinline__ void red_shared_inc(uint32_t a) { asm volatile("red.s
 // if ...` over four candidates became a tree of branches whose lanes came together only behind the
 // last of them: up to 81 paths, one after the other (2,300 cycles for counting four candidates per
 // lane; 300 like this).
-__device__ __forceinline__ void count_if_above(uint32_t& n, uint64_t c, uint64_t thr, uint32_t add) {
-  asm("{\n\t.reg .pred p;\n\tsetp.gt.u64 p, %1, %2;\n\t@p add.u32 %0, %0, %3;\n\t}" : "+r"(n) : "l"(c), "l"(thr), "r"(add));
+__device__ __forceinline__ void count_if_above(uint32_t& n, uint32_t k, uint32_t thr) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.u32 p, %1, %2;\n\t@p add.u32 %0, %0, 1;\n\t}" : "+r"(n) : "r"(k), "r"(thr));
+}
+__device__ __forceinline__ void count_if_above(uint32_t& n, uint64_t c, uint64_t thr) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.u64 p, %1, %2;\n\t@p add.u32 %0, %0, 1;\n\t}" : "+r"(n) : "l"(c), "l"(thr));
 }
 __device__ __forceinline__ void red_shared_inc_if(uint32_t a, uint32_t nonzero, uint32_t off, uint32_t span) {
   asm volatile(
@@ -138,15 +144,39 @@ __device__ __forceinline__ void st_global_if(bool on, void* a, uint32_t v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(a), "r"(v), "r"((uint32_t)on)
                : "memory");
 }
+// (on: a slot from the counter at `counter`, and v into slot of the array at `a`, if the array has it)
+__device__ __forceinline__ uint32_t append64_if(bool on, uint32_t counter, uint32_t a, uint32_t cap, uint64_t v) {
+  uint32_t slot;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 at;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\t@p atom.shared.add.u32 %0, [%1], 1;\n\t"
+      "setp.lt.and.u32 q, %0, %3, p;\n\tmad.lo.u32 at, %0, 8, %2;\n\t@q st.shared.u64 [at], %4;\n\t}"
+      : "=&r"(slot)
+      : "r"(counter), "r"(a), "r"(cap), "l"(v), "r"((uint32_t)on)
+      : "memory");
+  return slot;
+}
+__device__ __forceinline__ void st_global_if_above(uint32_t k, uint32_t thr, void* a, uint32_t v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.u32 p, %2, %3;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(a), "r"(v), "r"(k), "r"(thr)
+               : "memory");
+}
 __device__ __forceinline__ void sts64_if(bool on, uint32_t a, uint64_t v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u64 [%0], %1;\n\t}" ::"r"(a), "l"(v), "r"((uint32_t)on)
                : "memory");
 }
-__device__ __forceinline__ uint64_t lds64_if(bool on, uint32_t a) {
+// (i < n: the word at `a`, else 0)
+__device__ __forceinline__ uint32_t lds32_below(int i, int n, uint32_t a) {
+  uint32_t v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\tmov.u32 %0, 0;\n\t@p ld.shared.u32 %0, [%1];\n\t}"
+               : "=&r"(v)
+               : "r"(a), "r"(i), "r"(n)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint64_t lds64_below(int i, int n, uint32_t a) {
   uint64_t v;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u64 %0, 0;\n\t@p ld.shared.u64 %0, [%1];\n\t}"
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\tmov.u64 %0, 0;\n\t@p ld.shared.u64 %0, [%1];\n\t}"
                : "=&l"(v)
-               : "r"(a), "r"((uint32_t)on)
+               : "r"(a), "r"(i), "r"(n)
                : "memory");
   return v;
 }
@@ -211,6 +241,7 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
 // Shared-memory control block (one per CTA; rank 0's counters are the cluster-wide ones).
 // ---------------------------------------------------------------------------------------------
 struct Ctrl {
+  uint4 fin;  // (finish) the threshold bin: smallest and largest value of the digit's field, elements above, in it
   // cluster-wide allocation counters, meaningful in rank 0 only (targets of remote atomics)
   uint32_t win_count;
   uint32_t cand_count;
@@ -221,7 +252,7 @@ struct Ctrl {
   uint32_t wslot;
   uint32_t cslot;
   uint32_t fslot;
-  uint32_t small_n;  // (one-pass finish) undecided candidates set aside so far
+  uint32_t small_n;  // (finish) undecided candidates set aside so far
   uint32_t lcount;  // entries pushed to this CTA's spill area (may exceed its capacity)
   // what the sample search leaves: the guess and the bound for the finish (keys), what to do about them
   uint32_t guess;
@@ -255,6 +286,8 @@ struct Ctrl {
   uint32_t thr_key;      // warm start: smallest key among the winners of the finish
   uint32_t merge_count;  // valid candidates
   uint32_t merge_fail;   // the bounded wait for the shard's flag ran out
+  const int32_t* row_page;  // the row's page table (or NULL) and the offset of its indices
+  int32_t row_idx_offset;
   uint64_t small[kSmall];
 #ifdef FFTOPK_CHECKED
   uint32_t* status_ptr;  // the call's status word, for checks in code that has no other way to it
@@ -485,31 +518,36 @@ __device__ __forceinline__ void decide_and_allocate(const Ctx& cx, const Picked&
 
 // ---------------------------------------------------------------------------------------------
 // Candidate sources of the finish. A source tells a thread which candidates are its share:
-// for_each4(f4) calls f4 with an array of four composites at a time - loads in flight together, same trip count in
+// for_each(f) calls f with an array of kWalk composites at a time - loads in flight together, same trip count in
 // all lanes of a warp - and 0 where there is none. Which candidates a thread sees, and in which order,
 // is the same in every call.
 // ---------------------------------------------------------------------------------------------
 
 // A dense array in shared memory walked by a group of warps (`first`: this lane's first index, `step`: lanes in
 // the group; first - lane is the same in all lanes of a warp)
-// kSelect: plain bounds tests instead of predicated loads, which hold more registers at once (the fused
-// indexer's producer, at its register limit, spilled three for them).
-template <bool kSelect = false, class F4>
-__device__ __forceinline__ void walk4(uint32_t a /* shared address */, int n, int first, int step, F4&& f4) {
+constexpr int kWalk = 4;
+template <class F>
+__device__ __forceinline__ void walk(uint32_t a /* shared address */, int n, int first, int step, F&& f) {
   const int lane = lane_id();
-  for (int i = first; i - lane < n; i += 4 * step) {
+  for (int i = first; i - lane < n; i += kWalk * step) {
     const uint32_t at = a + (uint32_t)i * 8u;
-    uint64_t c[4];
+    uint64_t c[kWalk];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t au = at + (uint32_t)(u * step) * 8u;
-      if constexpr (kSelect) {
-        c[u] = i + u * step < n ? lds64(au) : 0ull;
-      } else {
-        c[u] = lds64_if(i + u * step < n, au);
-      }
-    }
-    f4(c);
+    for (int u = 0; u < kWalk; ++u) c[u] = lds64_below(i + u * step, n, at + (uint32_t)(u * step) * 8u);
+    f(c);
+  }
+}
+
+// ... and over their keys alone
+template <class F>
+__device__ __forceinline__ void walk_keys(uint32_t a, int n, int first, int step, F&& f) {
+  const int lane = lane_id();
+  for (int i = first; i - lane < n; i += kWalk * step) {
+    const uint32_t at = a + (uint32_t)i * 8u + 4u;
+    uint32_t k[kWalk];
+#pragma unroll
+    for (int u = 0; u < kWalk; ++u) k[u] = lds32_below(i + u * step, n, at + (uint32_t)(u * step) * 8u);
+    f(k);
   }
 }
 
@@ -519,24 +557,55 @@ struct DenseCands {
   uint32_t cand;  // shared address
   int n;
   __device__ __forceinline__ DenseCands(const uint64_t* c, int n_) : cand(smem_u32(c)), n(n_) {}
-  template <class F4>
-  __device__ __forceinline__ void for_each4(F4&& f4) const {
-    walk4<(NT < 512)>(cand, n, (int)threadIdx.x, NT, f4);
+  template <class F>
+  __device__ __forceinline__ void for_each(F&& f) const {
+    walk(cand, n, (int)threadIdx.x, NT, f);
+  }
+  template <class F>
+  __device__ __forceinline__ void for_each_key(F&& f) const {
+    walk_keys(cand, n, (int)threadIdx.x, NT, f);
   }
 };
 
-// What the filter of a lone CTA leaves behind: one dense segment per warp (each warp walks its own;
-// `wn`, its length, is the same in all lanes) plus the shared spill area of `sn` entries.
-template <int NT>
-struct WarpSegCands {
-  uint32_t seg;  // shared address of this warp's segment
+// What the filter of a lone CTA leaves behind: per warp up to 32 * R candidates, their keys in registers (candidate j
+// of the warp in key[j / 32] of lane j % 32; 0 where there is none) and their indices in a dense segment in shared
+// memory (`wn` of them, the same in all lanes), plus the shared spill area of `sn` composites.
+template <int NT, int R>
+struct RegSegCands {
+  uint32_t key[R];
+  uint32_t seg;  // shared address of this warp's indices
   int wn;
   uint32_t spill;
   int sn;
-  template <class F4>
-  __device__ __forceinline__ void for_each4(F4&& f4) const {
-    walk4(seg, wn, lane_id(), 32, f4);
-    if (sn > 0) walk4(spill, sn, (int)threadIdx.x, NT, f4);
+  template <class F>
+  __device__ __forceinline__ void for_each(F&& f) const {
+    static_assert(R % kWalk == 0, "");
+#pragma unroll
+    for (int i = 0; i < R; i += kWalk) {
+      if (i * 32 < wn) {
+        uint64_t c[kWalk];
+#pragma unroll
+        for (int u = 0; u < kWalk; ++u) {
+          const int j = (i + u) * 32 + lane_id();
+          c[u] = ((uint64_t)key[i + u] << 32) | (uint64_t)(~lds32_below(j, wn, seg + (uint32_t)j * 4u));
+        }
+        f(c);
+      }
+    }
+    if (sn > 0) walk(spill, sn, (int)threadIdx.x, NT, f);
+  }
+  template <class F>
+  __device__ __forceinline__ void for_each_key(F&& f) const {
+#pragma unroll
+    for (int i = 0; i < R; i += kWalk) {
+      if (i * 32 < wn) {
+        uint32_t k[kWalk];
+#pragma unroll
+        for (int u = 0; u < kWalk; ++u) k[u] = key[i + u];
+        f(k);
+      }
+    }
+    if (sn > 0) walk_keys(spill, sn, (int)threadIdx.x, NT, f);
   }
 };
 
@@ -548,22 +617,32 @@ struct RegionCands {
   uint32_t cand;      // shared addresses
   uint32_t count_of;
   int region, C, extra;
-  template <class F4>
-  __device__ __forceinline__ void for_each4(F4&& f4) const {
+  template <class W>
+  __device__ __forceinline__ void each_part(W&& w) const {
     constexpr int kLogNW = NT == 1024 ? 5 : (NT == 512 ? 4 : 3);
     const int warp = threadIdx.x >> 5;
     const int lper = max(kLogNW - (31 - __clz(C)), 0);  // (NW and C are powers of two: no division)
     for (int r = warp >> lper; r < C; r += (NT / 32) >> lper)
-      walk4(cand + (uint32_t)(r * region) * 8u, min((int)lds32(count_of + r * 4), region),
-            (warp & ((1 << lper) - 1)) * 32 + lane_id(), 32 << lper, f4);
-    if (extra > 0) walk4(cand + (uint32_t)(C * region) * 8u, extra, (int)threadIdx.x, NT, f4);
+      w(cand + (uint32_t)(r * region) * 8u, min((int)lds32(count_of + r * 4), region), (warp & ((1 << lper) - 1)) * 32 + lane_id(),
+        32 << lper);
+    if (extra > 0) w(cand + (uint32_t)(C * region) * 8u, extra, (int)threadIdx.x, NT);
+  }
+  template <class F>
+  __device__ __forceinline__ void for_each(F&& f) const {
+    each_part([&](uint32_t a, int n, int first, int step) { walk(a, n, first, step, f); });
+  }
+  template <class F>
+  __device__ __forceinline__ void for_each_key(F&& f) const {
+    each_part([&](uint32_t a, int n, int first, int step) { walk_keys(a, n, first, step, f); });
   }
 };
 
-// Block-wide threshold pick over kFinishBins counts (descending bin order); result in ctrl->t
-// (-1 if the counts sum to less than need), ctrl->above, ctrl->cnt. Ends with a barrier.
-template <int NT>
-__device__ __forceinline__ void block_pick(uint32_t hist /* shared address */, uint32_t need, Ctrl* ctrl) {
+// Block-wide threshold pick over kFinishBins counts (descending bin order): one thread calls
+// found(bin, above, count) for the bin that holds rank `need`; nobody does if the counts sum to less. Ends
+// with a barrier, which publishes what it leaves in shared memory; before() runs in thread 0 before that.
+template <int NT, class Before, class Found>
+__device__ __forceinline__ void block_pick(uint32_t hist /* shared address */, uint32_t need, uint32_t wtot /* shared address */,
+                                           Before&& before, Found&& found) {
   constexpr int PER = (kFinishBins + NT - 1) / NT;
   constexpr int NW = NT / 32;
   const int tid = threadIdx.x;
@@ -592,20 +671,15 @@ __device__ __forceinline__ void block_pick(uint32_t hist /* shared address */, u
     const uint32_t x = __shfl_down_sync(kFull, incl, off);
     if (lane + off < 32) incl += x;
   }
-  const uint32_t wtot = smem_u32(ctrl->wtot);
   if (lane == 0) sts32(wtot + warp * 4, incl);
-  if (tid == 0) ctrl->t = -1;
+  if (tid == 0) before();
   __syncthreads();
   const uint32_t hw = (lane > warp && lane < NW) ? lds32(wtot + lane * 4) : 0u;
   uint32_t run = __reduce_add_sync(kFull, hw) + incl - s;
   if (run < need && need <= run + s) {  // (one thread)
 #pragma unroll
     for (int j = PER - 1; j >= 0; --j) {
-      if (run < need && need <= run + v[j]) {
-        ctrl->t = tid * PER + j;
-        ctrl->above = run;
-        ctrl->cnt = v[j];
-      }
+      if (run < need && need <= run + v[j]) found((uint32_t)(tid * PER + j), run, v[j]);
       run += v[j];
     }
   }
@@ -658,9 +732,194 @@ __device__ __forceinline__ void block_pick_sample(uint32_t hist /* shared addres
   __syncthreads();
 }
 
+// The bin of rank `need` in the histogram of a finish round: (bin, or kNoBin if there is none; elements above it; elements in it).
+constexpr uint32_t kNoBin = 0xffffffffu;
+template <int NT>
+__device__ __forceinline__ uint4 finish_pick(uint32_t hist /* shared address */, uint32_t need, Ctrl* ctrl) {
+  const uint32_t fin = smem_u32(&ctrl->fin);
+  block_pick<NT>(hist, need, smem_u32(ctrl->wtot), [&] { sts32(fin, kNoBin); },
+                 [&](uint32_t bin, uint32_t above, uint32_t n) { sts128(fin, bin, above, n, 0u); });
+  return lds128(fin);
+}
+
+// The output pass of a finish: candidates of which field() is above `wthr` win, those above `uthr` are undecided
+// (up to kSmall, of which the `need2` best win; with all_bin there are none).
+// Every warp counts its winners and gets its output slots by a sum over the warps in front of it; then it writes
+// them, 32 candidates at a time, slots by ballot. (A slot-allocating atomic per warp serialised on the one
+// counter - 30 cycles per warp -, and slots by thread, from a scan over the lanes, scattered every store over 32
+// lines.) A threshold bin that is not taken whole holds a handful of candidates: those take an atomic.
+struct FinishOut {
+  Ctrl* ctrl;
+  int32_t* out_idx;
+  uint32_t* out_key;
+  uint32_t* status;
+  const int32_t* page;
+  uint32_t out_base, out_slots;
+  int32_t idx_offset;
+};
+// Rank by vote the `cnt` candidates set aside: warp i takes candidate i, the lanes compare it with the candidates j (32
+// per step); the number of larger ones is candidate i's rank, and the best need2 go behind the
+// `certain` winners. Up to 256 undecided candidates are cheaper to rank like this (at most 64
+// votes per warp) than to split by another round - rows of low-precision logits have
+// hundreds of exact duplicates at the threshold. (A bitonic compare-exchange network over 32
+// values is a chain of 60 dependent shuffles; this is one ballot per 32 comparisons.)
+template <int NT, bool kTrackMin>
+__device__ __forceinline__ void rank_undecided(const FinishOut& o, uint32_t certain, uint32_t need2, uint32_t cnt) {
+  const int lane = lane_id();
+  __syncthreads();
+  const int nchunk = ((int)cnt + 31) >> 5;
+  for (int i = (int)(threadIdx.x >> 5); i < (int)cnt; i += NT / 32) {
+    const uint64_t me = o.ctrl->small[i];
+    uint32_t rank = 0;
+    for (int ch = 0; ch < nchunk; ++ch) {
+      const int j = ch * 32 + lane;
+      const uint64_t other = (j < (int)cnt) ? o.ctrl->small[j] : 0ull;
+      rank += (uint32_t)__popc(__ballot_sync(kFull, other > me));
+    }
+    if (lane == 0 && rank < need2) {
+      const uint32_t pos = o.out_base + certain + rank;
+      if (FFTOPK_CHECK(5, pos, o.out_slots, o.status) && pos < o.out_slots) {
+        const int32_t idx = (int32_t)(~(uint32_t)me);
+        o.out_idx[pos] = o.page ? __ldg(o.page + idx) : idx + o.idx_offset;
+        if (o.out_key) o.out_key[pos] = (uint32_t)(me >> 32);
+      }
+      if constexpr (kTrackMin) atomicMin(&o.ctrl->thr_key, (uint32_t)(me >> 32));
+    }
+  }
+}
+
+template <int NT, bool kTrackMin, class Src, class V, class Field>
+__device__ __forceinline__ void finish_output(const Src src, const FinishOut o, uint32_t need_total, uint32_t need2, uint32_t cnt,
+                                              bool all_bin, V wthr, V uthr, Field&& field) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  Ctrl* ctrl = o.ctrl;
+  const uint32_t small_s = smem_u32(ctrl->small), small_n = smem_u32(&ctrl->small_n);
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t n = 0u;
+  if constexpr (sizeof(V) == 4) {
+    src.for_each_key([&](const uint32_t (&k)[kWalk]) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) count_if_above(n, k[u], wthr);
+    });
+  } else {
+    src.for_each([&](const uint64_t (&c)[kWalk]) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) count_if_above(n, field(c[u]), wthr);
+    });
+  }
+  n = __reduce_add_sync(kFull, n);
+  const uint32_t wsum = smem_u32(ctrl->wmax);
+  if (lane == 0) sts32(wsum + warp * 4, n);
+  __syncthreads();
+  uint32_t wpos = o.out_base + __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u);
+#ifdef FFTOPK_CHECKED
+  const uint32_t set_w = __reduce_add_sync(kFull, lane < NT / 32 ? lds32(wsum + lane * 4) : 0u);  // winners found
+#endif
+  uint32_t win_min = 0xffffffffu;  // (kTrackMin) smallest key among the certain winners, if they are all there are
+  src.for_each([&](const uint64_t (&c)[kWalk]) {
+    int32_t v[kWalk];
+#pragma unroll
+    for (int u = 0; u < kWalk; ++u) v[u] = (int32_t)(~(uint32_t)c[u]) + o.idx_offset;
+    if (o.page) {  // (the table reads in flight together)
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u)
+        if (field(c[u]) > wthr) v[u] = __ldg(o.page + (int32_t)(~(uint32_t)c[u]));
+    }
+    bool undecided = false;
+#pragma unroll
+    for (int u = 0; u < kWalk; ++u) {
+      const bool w = field(c[u]) > wthr;
+      const unsigned bw = __ballot_sync(kFull, w);
+      const uint32_t pos = wpos + (uint32_t)__popc(bw & lt);
+      const bool put = w && FFTOPK_CHECK(3, pos, o.out_slots, o.status) && pos < o.out_slots;
+      st_global_if(put, o.out_idx + pos, (uint32_t)v[u]);
+      if (o.out_key) st_global_if(put, o.out_key + pos, (uint32_t)(c[u] >> 32));
+      wpos += (uint32_t)__popc(bw);
+      undecided = undecided || (!w && field(c[u]) > uthr);
+      if constexpr (kTrackMin) {
+        if (all_bin) win_min = min(win_min, w ? (uint32_t)(c[u] >> 32) : 0xffffffffu);
+      }
+    }
+    if (__any_sync(kFull, undecided)) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) {
+        const uint32_t slot = append64_if(field(c[u]) > uthr && !(field(c[u]) > wthr), small_n, small_s, kSmall, c[u]);
+        (void)FFTOPK_CHECK(4, slot, kSmall, o.status);
+      }
+    }
+  });
+  FFTOPK_MARK(33);
+  if constexpr (kTrackMin) {
+    if (all_bin) {  // (else the smallest winner is one of those that are ranked)
+      win_min = __reduce_min_sync(kFull, win_min);
+      if (lane == 0 && win_min != 0xffffffffu) atomicMin(&ctrl->thr_key, win_min);
+    }
+  }
+#ifdef FFTOPK_CHECKED
+  {
+    // every certain winner took exactly one slot, every undecided candidate was set aside
+    __syncthreads();
+    const uint32_t want_w = all_bin ? need_total : need_total - need2;
+    if (tid == 0) {
+      if (set_w != want_w) check_fail(10, set_w, want_w, o.status);
+      if (!all_bin && ctrl->small_n != cnt) check_fail(11, ctrl->small_n, cnt, o.status);
+    }
+  }
+#endif
+  if (!all_bin) rank_undecided<NT, kTrackMin>(o, need_total - need2, need2, cnt);
+}
+
+// More copies of one key than can be ranked, the threshold among them: `need` candidates are still to be taken from
+// those with key `key` and - `more` of them - larger ones. Rounds over the inverted indices under the key, then the
+// output. Out of line: rows with thousands of copies of one value come here, and the others
+// do not carry its registers and instructions. Returns false if the threshold is a key above `key` after all.
+template <int NT, bool kTrackMin, class Src>
+__device__ __noinline__ bool finish_copies(const Src passed, const FinishOut passed_out, uint32_t need_total, uint32_t need, uint32_t key,
+                                           bool more, int idx_bits, uint32_t* hist) {
+  const Src src = passed;  // (out of the stack, into registers)
+  const FinishOut o = passed_out;
+  const int tid = threadIdx.x;
+  const uint32_t hist_s = smem_u32(hist);
+  uint32_t lo = inverted_index_floor(idx_bits), cap = 0xffffffffu;
+  for (int round = 0; round < 8; ++round) {
+    const KeyDigit dg = make_key_digit(lo, cap);
+    __syncthreads();  // every thread is through with the histogram and the result of the round before
+    for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
+    __syncthreads();
+    const uint32_t span = cap - lo;
+    src.for_each([&](const uint64_t (&c)[kWalk]) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) {
+        const uint32_t k = (uint32_t)(c[u] >> 32), v = (uint32_t)c[u];
+        if (k == key && v - lo <= span) red_shared_inc(hist_s + dg.of(v) * 4u);
+        if (more && k > key) red_shared_inc(hist_s + (uint32_t)(kFinishBins - 1) * 4u);
+      }
+    });
+    __syncthreads();
+    const uint4 f = finish_pick<NT>(hist_s, need, o.ctrl);
+    if (f.x == kNoBin) break;
+    const uint32_t cnt = f.z, need2 = need - f.y;
+    if (more && f.x == (uint32_t)kFinishBins - 1u) return false;
+    const uint32_t t_lo = dg.bin_low(f.x), t_hi = dg.bin_high(f.x, cap);
+    if (cnt == need2 || cnt <= (uint32_t)kSmall) {
+      const uint64_t k = (uint64_t)key << 32, below = (k | t_lo) - 1ull;
+      finish_output<NT, kTrackMin>(src, o, need_total, need2, cnt, cnt == need2, cnt == need2 ? below : k | t_hi, below,
+                                   [](uint64_t c) { return c; });
+      return true;
+    }
+    more = false;
+    lo = t_lo;
+    cap = t_hi;
+    need = need2;
+  }
+  if (tid == 0 && o.status) atomicOr(o.status, 2u);
+  return true;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Single-CTA finish. The source holds composites c = (key << 32) | ~idx in shared memory (0 =
-// empty slot), all of them inside [lo, cap]; lo > cap means "range unknown" and costs a pass
+// empty slot), all of them with keys inside [klo, kcap]; klo > kcap means "range unknown" and costs a pass
 // that finds it. Writes the `need` largest composites' indices (and keys) to
 // out_idx[out_base ...], in unspecified order.
 //
@@ -668,8 +927,14 @@ __device__ __forceinline__ void block_pick_sample(uint32_t hist /* shared addres
 // tail (topk_indexer_radix.cu:686-781, 109-141, 788-850). Because the index is part of the
 // composite, equal values are resolved towards the lower index by the same rounds, and the last
 // <= 256 undecided candidates are ranked by votes.
-// `focus`: see FinishDigit (fftopk_decide.h). `have_hist`: the caller has already built round 0's histogram in
-// `hist`, with make_finish_digit(lo, focus).
+//
+// What bounds it is the instructions its warps issue (rank 0's 16 warps work alone on their SM, and a batch of rows
+// fills every issue slot), so the rounds work on 32-bit fields: on the keys, and only when one key is left - more
+// copies of the threshold than can be ranked - on the inverted indices below it. (With 64-bit
+// composites as the digits' field a round cost 280 instructions per warp besides the candidates', and the output 450:
+// 11,700 of the 26,200 warp instructions of a row of 8K elements.)
+// `kfocus`: see KeyDigit (fftopk_decide.h). `have_hist`: the caller has already built round 0's histogram in
+// `hist`, with make_key_digit(klo, kfocus), klo < kfocus.
 // `idx_bits`: all indices are < 2^idx_bits, so the inverted-index bits above that are all ones.
 // `page`: optional per-row table; the value written is then page[idx] instead of idx + idx_offset
 // (the fused page-table transform of the reference's topk_transform_* kernels, :871-958).
@@ -681,7 +946,7 @@ __device__ __forceinline__ void block_pick_sample(uint32_t hist /* shared addres
 // stack, and beside 200 KB of shared memory L1 has no room for the stacks of 1024 threads - each access
 // was a round trip to L2 (the passes over the candidates took 1.4 and 2 to 4 us instead of 0.4 and 0.7).
 template <int NT, class Src, bool kTrackMin = false>
-__device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_t lo, uint64_t cap, uint64_t focus, bool have_hist,
+__device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_t klo, uint32_t kcap, uint32_t kfocus, bool have_hist,
                            int idx_bits, uint32_t* hist /* >= kFinishBins words */, Ctrl* ctrl, int32_t* out_idx,
                            uint32_t* out_key, uint32_t out_base, uint32_t out_slots /* k of the row */,
                            int32_t idx_offset, uint32_t* status,
@@ -690,23 +955,16 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const uint32_t hist_s = smem_u32(hist);
-  // How the output pass hands out slots. With 16 or 32 warps: a counting pass in front, so that no
-  // warp waits for another. With ten (the fused indexer) a second walk over the list costs each of them
-  // more than the few atomics (a call with a guess, 16K keys in fp8: 11.1 us, 10.75 in one pass).
-  constexpr bool kOnePass = NT < 512;
-  if constexpr (kOnePass) {
-    if (tid == 0) ctrl->fslot = ctrl->small_n = 0u;  // (every path has a block barrier before they are used)
-  }
-  if (lo > cap) {
+  if (tid == 0) ctrl->small_n = 0u;  // (every path has a block barrier before it is used)
+  if (klo > kcap) {
     // Range unknown: the smallest and the largest key present bound it.
     uint32_t kmin = ~0u, kmax = 0u;
-    src.for_each4([&](const uint64_t (&c)[4]) {
+    src.for_each_key([&](const uint32_t (&k)[kWalk]) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k = (uint32_t)(c[u] >> 32);
-        if (c[u] != 0ull) {
-          kmin = min(kmin, k);
-          kmax = max(kmax, k);
+      for (int u = 0; u < kWalk; ++u) {
+        if (k[u] != 0u) {
+          kmin = min(kmin, k[u]);
+          kmax = max(kmax, k[u]);
         }
       }
     });
@@ -718,277 +976,259 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint64_
     }
     __syncthreads();
     const bool in = lane < NT / 32;
-    kmin = __reduce_min_sync(kFull, in ? hist[2 * lane + 0] : ~0u);
-    kmax = __reduce_max_sync(kFull, in ? hist[2 * lane + 1] : 0u);
-    lo = (uint64_t)kmin << 32;
-    cap = ((uint64_t)kmax << 32) | 0xffffffffull;
-    if (lo > cap) {  // no candidate at all
+    klo = __reduce_min_sync(kFull, in ? hist[2 * lane + 0] : ~0u);
+    kcap = __reduce_max_sync(kFull, in ? hist[2 * lane + 1] : 0u);
+    if (klo > kcap) {  // no candidate at all
       if (tid == 0 && status) atomicOr(status, 2u);
       return;
     }
-    focus = cap;
+    kfocus = kcap;
     have_hist = hist_clear = false;
     __syncthreads();  // the scratch words are about to be cleared as the histogram
     FFTOPK_MARK(31);
   }
   // ---- rounds: only the threshold is determined here; nothing is written yet ---------------------
-  // Outcome: the threshold bin [t_lo, t_hi] of composites. Everything above t_hi wins; of the
+  // Outcome: the threshold bin, keys [t_lo, t_hi]. Everything above it wins; of the
   // bin itself either everything wins (all_bin) or, when it holds <= kSmall candidates, the best
   // `need2` of them, found by ranking.
+  const FinishOut o{ctrl, out_idx, out_key, status, page, out_base, out_slots, idx_offset};
   const uint32_t need_total = need;
-  uint64_t t_lo = 0ull, t_hi = 0ull;
-  uint32_t need2 = 0, cnt = 0;
+  uint32_t t_lo = klo, t_hi = kcap;
+  uint32_t need2 = need, cnt = known_total;
   bool all_bin = false, found = false;
-  if (known_total != 0u && known_total == need && lo <= cap) {
-    // exactly as many candidates as are wanted: all of them win
-    t_lo = lo;
-    t_hi = cap;
-    cnt = need2 = need;
-    all_bin = found = true;
-    __syncthreads();  // (as in a round: what the caller has read through ctrl may be overwritten from here on)
-  } else if (known_total != 0u && known_total <= (uint32_t)kSmall && known_total >= need && lo <= cap) {
-    // so few candidates that they are ranked directly: the whole range is the "threshold bin"
-    t_lo = lo;
-    t_hi = cap;
-    cnt = known_total;
-    need2 = need;
+  if (known_total != 0u && known_total >= need && (known_total == need || known_total <= (uint32_t)kSmall)) {
+    // exactly as many candidates as are wanted, or so few that they are ranked directly
+    all_bin = known_total == need;
     found = true;
-    __syncthreads();
+    __syncthreads();  // (as in a round: what the caller has read through ctrl may be overwritten from here on)
   }
-  for (int round = 0; round < 24 && !found; ++round) {
-    if ((uint32_t)(lo >> 32) == (uint32_t)(cap >> 32)) {
-      // one key left: the inverted indices all start with the same run of ones
-      const uint64_t floor_lo = single_key_floor(lo, idx_bits);
-      if (lo < floor_lo && floor_lo <= cap) {
-        if (focus < floor_lo) focus = cap;
-        lo = floor_lo;
-        have_hist = false;
-      }
+  uint32_t lo = klo, cap = kcap;
+  uint32_t focus = kfocus < klo || kfocus > kcap ? kcap : kfocus;
+  for (int round = 0; round < 8 && !found; ++round) {
+    if (lo == focus) {  // one key left, or bounded by
+      if (finish_copies<NT, kTrackMin>(src, o, need_total, need, lo, cap > lo, idx_bits, hist)) return;
+      ++lo;
+      focus = cap;
+      have_hist = hist_clear = false;
     }
-    if (focus < lo || focus > cap) focus = cap;
-    const FinishDigit dg = make_finish_digit(lo, focus);
-    if (!(round == 0 && have_hist)) {
-      if (!(round == 0 && hist_clear)) {
+    const KeyDigit dg = make_key_digit(lo, focus);
+    if (!have_hist) {
+      if (!hist_clear) {
+        __syncthreads();
         for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
         __syncthreads();
       }
-      const uint64_t span = cap - lo;
-      if (dg.key_only()) {
-        // the digit depends on the key alone: work on the high words only (an empty slot has key 0)
-        const uint32_t klo = (uint32_t)(lo >> 32), kspan = (uint32_t)(span >> 32);
-        src.for_each4([&](const uint64_t (&c)[4]) {
+      const uint32_t span = cap - lo;
+      src.for_each_key([&](const uint32_t (&k)[kWalk]) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const uint32_t k = (uint32_t)(c[u] >> 32);
-            red_shared_inc_if(hist_s + dg.of_key(k) * 4u, k, k - klo, kspan);
-          }
-        });
-      } else {
-        src.for_each4([&](const uint64_t (&c)[4]) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (c[u] != 0ull && (c[u] - lo) <= span) red_shared_inc(hist_s + dg.of(c[u]) * 4u);
-          }
-        });
-      }
+        for (int u = 0; u < kWalk; ++u) red_shared_inc_if(hist_s + dg.of(k[u]) * 4u, k[u], k[u] - lo, span);
+      });
       __syncthreads();
     }
     FFTOPK_MARK(16);
-    block_pick<NT>(hist_s, need, ctrl);
+    const uint4 f = finish_pick<NT>(hist_s, need, ctrl);
     FFTOPK_MARK(17);
-    const int t = ctrl->t;
-    if (t < 0) {
-      if (tid == 0 && status) atomicOr(status, 2u);
-      return;
+    if (f.x == kNoBin) break;
+    cnt = f.z;
+    need2 = need - f.y;
+    t_lo = dg.bin_low(f.x);
+    t_hi = dg.bin_high(f.x, cap);
+    all_bin = cnt == need2;
+    found = all_bin || cnt <= (uint32_t)kSmall;
+    if (!found) {
+      lo = t_lo;
+      cap = focus = t_hi;
+      need = need2;
+      have_hist = hist_clear = false;
     }
-    cnt = ctrl->cnt;
-    need2 = need - ctrl->above;
-    finish_bin_range(dg, lo, cap, t, t_lo, t_hi);
-    if (cnt == need2 || cnt <= (uint32_t)kSmall) {
-      all_bin = (cnt == need2);
-      found = true;
-      break;
-    }
-    lo = t_lo;
-    cap = focus = t_hi;
-    need = need2;
-    __syncthreads();  // every thread has read ctrl->t/cnt/above before the next round rewrites them
   }
   FFTOPK_MARK(30);
   if (!found) {
     if (tid == 0 && status) atomicOr(status, 2u);
     return;
   }
-  // ---- the certain winners go out (in unspecified order), the undecided candidates are set aside ----
-  FFTOPK_MARK(32);
-  const uint64_t wthr = all_bin ? (t_lo ? t_lo - 1ull : 0ull) : t_hi;  // winners: c > wthr
-  const uint64_t uthr = all_bin ? wthr : (t_lo ? t_lo - 1ull : 0ull);  // undecided: uthr < c <= wthr
-  uint32_t win_min = 0xffffffffu;  // (kTrackMin) smallest key among the winners this thread wrote
-  const uint32_t small_s = smem_u32(ctrl->small);
-  auto put_winner = [&](bool w, uint32_t pos, uint64_t c, int32_t v) {
-    const bool put = w && FFTOPK_CHECK(3, pos, out_slots, status) && pos < out_slots;
-    st_global_if(put, out_idx + pos, (uint32_t)v);
-    if (out_key) st_global_if(put, out_key + pos, (uint32_t)(c >> 32));
-    if constexpr (kTrackMin) win_min = min(win_min, w ? (uint32_t)(c >> 32) : 0xffffffffu);
+  const uint32_t below = t_lo ? t_lo - 1u : 0u;  // (an empty slot has key 0)
+  finish_output<NT, kTrackMin>(src, o, need_total, need2, cnt, all_bin, all_bin ? below : t_hi, below,
+                               [](uint64_t c) { return (uint32_t)(c >> 32); });
+}
+
+// The same for what the filter of a lone CTA leaves behind (out of line: lone_finish is for the common case).
+template <int NT, int R, bool kTrackMin>
+__device__ __noinline__ void lone_finish_general(const RegSegCands<NT, R> passed, const FinishOut o, uint32_t need, uint32_t klo,
+                                                 uint32_t kfocus, int idx_bits, uint32_t* hist, uint32_t total) {
+  const RegSegCands<NT, R> src = passed;  // (out of the stack, into registers)
+  __syncthreads();
+  cta_finish<NT, RegSegCands<NT, R>, kTrackMin>(src, need, klo, 0xffffffffu, kfocus, false, idx_bits, hist, o.ctrl, o.out_idx, o.out_key,
+                                                o.out_base, o.out_slots, o.idx_offset, o.status, o.page, total, false);
+}
+
+// The finish of a lone CTA: the candidates' keys are in registers, round 0's histogram (`hist`, with
+// make_key_digit(klo, kfocus)) is built. A batch of rows fills the issue slots, so this is written for few
+// instructions: the thread that finds the bin works out the bounds, keys are compared where they are, and
+// nothing but the indices is read again. Where the threshold bin holds more than can be ranked, further rounds narrow
+// it to one key, and copies of that are resolved down to the last index to be taken: the keys of those behind it are
+// cleared and everything that is left wins. With spilled candidates: lone_finish_general.
+template <int NT, int R, bool kTrackMin>
+__device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const FinishOut& o, uint32_t need, uint32_t klo,
+                                            uint32_t kfocus, int idx_bits, uint32_t* hist, uint32_t total) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  Ctrl* ctrl = o.ctrl;
+  if (held.sn > 0) {  // (uniform)
+    lone_finish_general<NT, R, kTrackMin>(held, o, need, klo, kfocus, idx_bits, hist, total);
+    return;
+  }
+  const uint32_t fin = smem_u32(&ctrl->fin), hist_s = smem_u32(hist), wtot = smem_u32(ctrl->wtot);
+  constexpr uint32_t kMany = 0xfffffffeu;
+  // fin: largest key that does not win for certain, x; undecided candidates: their keys are in (y, x]; their number (kMany:
+  // too many), z; how many of them win, w
+  auto pick = [&](const KeyDigit dg, uint32_t want, uint32_t cap, uint32_t most) {
+    block_pick<NT>(hist_s, want, wtot, [&] { sts128(fin, 0u, 0u, kNoBin, 0u); ctrl->small_n = 0u; },
+                   [&](uint32_t bin, uint32_t above, uint32_t n) {
+                     const uint32_t low = dg.bin_low(bin), below = low ? low - 1u : 0u;
+                     const bool all = n == want - above;
+                     sts128(fin, all ? below : dg.bin_high(bin, cap), below, all ? 0u : (n <= most ? n : kMany), want - above);
+                   });
+    return lds128(fin);
   };
-  auto put_aside = [&](bool g, uint32_t pos, uint64_t c) {
-    sts64_if(g && FFTOPK_CHECK(4, pos, kSmall, status) && pos < (uint32_t)kSmall, small_s + pos * 8u, c);
+  auto clear = [&] {
+    for (int b = tid; b < kFinishBins / 4; b += NT) sts_zero16(hist_s + b * 16);
+    __syncthreads();
   };
-  auto values = [&](const uint64_t (&c)[4], int32_t (&v)[4], auto paged) {
+  uint4 f = pick(make_key_digit(klo, kfocus), need, 0xffffffffu, (uint32_t)kSmall);
+  FFTOPK_MARK(17);
+  if (f.z == kMany) {  // (uniform)
+    uint32_t lo = f.y + 1u, cap = f.x;
+    while (lo < cap && f.z == kMany) {  // other values than one: by key again
+      __syncthreads();  // (everybody has read the result)
+      clear();
+      const KeyDigit dg = make_key_digit(lo, cap);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int32_t idx = (int32_t)(~(uint32_t)c[u]);
-      v[u] = idx + idx_offset;
-      if constexpr (decltype(paged)::value) {  // (the four table reads in flight together)
-        if (c[u] > wthr) v[u] = __ldg(page + idx);
-      }
+      for (int i = 0; i < R; ++i)
+        if (i * 32 < held.wn) red_shared_inc_if(hist_s + dg.of(held.key[i]) * 4u, held.key[i], held.key[i] - lo, cap - lo);
+      __syncthreads();
+      f = pick(dg, f.w, cap, (uint32_t)kSmall);
+      lo = f.y + 1u;
+      cap = f.x;
     }
-  };
-#ifdef FFTOPK_CHECKED
-  uint32_t set_w, set_u;  // winners and undecided candidates found
-#endif
-  if constexpr (kOnePass) {
-    // One pass: a warp takes the slots of its 128 candidates' winners with one atomic on the shared
-    // counter, and those of its undecided ones with another.
-    const unsigned lt = (1u << lane) - 1u;
-    auto pass = [&](auto paged) {
-      src.for_each4([&](const uint64_t (&c)[4]) {
-        unsigned bw[4], bu[4];
-        uint32_t nw = 0u, nu = 0u;
+    if (f.z == kMany) {  // copies of `lo`
+      const uint32_t key = lo;
+      uint32_t ilo = inverted_index_floor(idx_bits), icap = 0xffffffffu;
+      do {  // (indices differ: the last round ends with one candidate, or takes its bin whole)
+        __syncthreads();
+        clear();
+        const KeyDigit dg = make_key_digit(ilo, icap);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          bw[u] = __ballot_sync(kFull, c[u] > wthr);
-          bu[u] = __ballot_sync(kFull, c[u] > uthr) & ~bw[u];
-          nw += (uint32_t)__popc(bw[u]);
-          nu += (uint32_t)__popc(bu[u]);
-        }
-        if (nw != 0u) {
-          uint32_t base = 0u;
-          if (lane == 0) base = atom_shared_add(&ctrl->fslot, nw);
-          base = out_base + __shfl_sync(kFull, base, 0);
-          int32_t v[4];
-          values(c, v, paged);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            put_winner((bw[u] >> lane) & 1u, base + (uint32_t)__popc(bw[u] & lt), c[u], v[u]);
-            base += (uint32_t)__popc(bw[u]);
+        for (int i = 0; i < R; ++i) {
+          if (i * 32 < held.wn && held.key[i] == key) {
+            const uint32_t v = ~lds32(held.seg + (uint32_t)(i * 32 + lane) * 4u);
+            if (v - ilo <= icap - ilo) red_shared_inc(hist_s + dg.of(v) * 4u);
           }
         }
-        if (nu != 0u) {
-          uint32_t base = 0u;
-          if (lane == 0) base = atom_shared_add(&ctrl->small_n, nu);
-          base = __shfl_sync(kFull, base, 0);
+        __syncthreads();
+        f = pick(dg, f.w, icap, 0u);
+        ilo = f.y + 1u;
+        icap = f.x;
+      } while (f.z == kMany);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            put_aside((bu[u] >> lane) & 1u, base + (uint32_t)__popc(bu[u] & lt), c[u]);
-            base += (uint32_t)__popc(bu[u]);
-          }
+      for (int i = 0; i < R; ++i) {
+        if (i * 32 < held.wn && held.key[i] == key) {
+          if (~lds32(held.seg + (uint32_t)(i * 32 + lane) * 4u) < ilo) held.key[i] = 0u;
         }
-      });
-    };
-    if (page) {
-      pass(std::true_type{});
-    } else {
-      pass(std::false_type{});
-    }
-#ifdef FFTOPK_CHECKED
-    __syncthreads();
-    set_w = ctrl->fslot;
-    set_u = ctrl->small_n;
-#endif
-  } else {
-    // First every thread counts both kinds in its share, a scan over the lanes and one over the warps
-    // gives it its slots, then it writes. (A slot-allocating atomic per warp serialised on the one
-    // counter - 30 cycles per warp -, and ballots per candidate cost more instructions than they saved;
-    // instructions are what bounds this pass: with all warps of an SM at it each one costs eight cycles.)
-    uint32_t mine = 0u;  // winners << 16 | winners and undecided
-    src.for_each4([&](const uint64_t (&c)[4]) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        count_if_above(mine, c[u], wthr, 0x10000u);
-        count_if_above(mine, c[u], uthr, 1u);
       }
-    });
-    uint32_t incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t x = __shfl_up_sync(kFull, incl, off);
-      if (lane >= off) incl += x;
+      if (f.z != kNoBin) f = make_uint4(key - 1u, key - 1u, 0u, 0u);
     }
-    const uint32_t wsum = smem_u32(ctrl->wmax);
-    if (lane == 31) sts32(wsum + warp * 4, incl);
-    __syncthreads();
-    const uint32_t before = __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u) + incl - mine;
-    uint32_t wpos = out_base + (before >> 16), upos = (before & 0xffffu) - (before >> 16);
-    auto pass = [&](auto paged) {
-      src.for_each4([&](const uint64_t (&c)[4]) {
+  }
+  if (f.z == kNoBin) {  // (uniform)
+    if (tid == 0 && o.status) atomicOr(o.status, 2u);
+    return;
+  }
+  uint32_t n = 0u;
+#pragma unroll
+  for (int i = 0; i < R; i += 4) {
+    if (i * 32 < held.wn) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) count_if_above(n, held.key[i + u], f.x);
+    }
+  }
+  n = __reduce_add_sync(kFull, n);
+  const uint32_t wsum = smem_u32(ctrl->wmax);
+  if (lane == 0) sts32(wsum + warp * 4, n);
+  __syncthreads();
+  uint32_t wpos = o.out_base + __reduce_add_sync(kFull, lane < warp ? lds32(wsum + lane * 4) : 0u);
+  FFTOPK_MARK(70);
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t small_s = smem_u32(ctrl->small), small_n = smem_u32(&ctrl->small_n);
+  uint32_t win_min = 0xffffffffu;
+  auto pass = [&](auto plain) {  // (plain: indices alone, as they are)
+#pragma unroll
+    for (int i = 0; i < R; i += 4) {
+      if (i * 32 < held.wn) {
+        uint32_t idx[4];
         int32_t v[4];
-        values(c, v, paged);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const uint32_t w = c[u] > wthr ? 1u : 0u, g = c[u] > uthr ? 1u : 0u;
-          put_winner(w != 0u, wpos, c[u], v[u]);
-          wpos += w;
-          put_aside(g != w, upos, c[u]);
-          upos += g - w;
+          const int j = (i + u) * 32 + lane;
+          idx[u] = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
+          v[u] = (int32_t)idx[u];
+          if constexpr (!decltype(plain)::value) {
+            if (!o.page) {
+              v[u] += o.idx_offset;
+            } else if (held.key[i + u] > f.x) {
+              v[u] = __ldg(o.page + idx[u]);
+            }
+          }
         }
-      });
-    };
-    if (page) {
-      pass(std::true_type{});
-    } else {
-      pass(std::false_type{});
+        uint32_t nearest = 0xffffffffu;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t k = held.key[i + u];
+          const unsigned bw = __ballot_sync(kFull, k > f.x);
+          const uint32_t pos = wpos + (uint32_t)__popc(bw & lt);
+          if (!(k > f.x) || FFTOPK_CHECK(3, pos, o.out_slots, o.status)) {
+            st_global_if_above(k, f.x, o.out_idx + pos, (uint32_t)v[u]);
+            if constexpr (!decltype(plain)::value) {
+              if (o.out_key) st_global_if_above(k, f.x, o.out_key + pos, k);
+            }
+          }
+          wpos += (uint32_t)__popc(bw);
+          if constexpr (kTrackMin) win_min = min(win_min, k > f.x ? k : 0xffffffffu);
+          nearest = min(nearest, k - f.y - 1u);
+        }
+        if (__any_sync(kFull, nearest < f.x - f.y)) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t k = held.key[i + u];
+            const uint32_t slot =
+                append64_if(k - f.y - 1u < f.x - f.y, small_n, small_s, kSmall, ((uint64_t)k << 32) | (uint64_t)(~idx[u]));
+            (void)FFTOPK_CHECK(4, slot, kSmall, o.status);
+          }
+        }
+      }
     }
-#ifdef FFTOPK_CHECKED
-    const uint32_t sum = __reduce_add_sync(kFull, lane < NT / 32 ? ctrl->wmax[lane] : 0u);
-    set_w = sum >> 16;
-    set_u = (sum & 0xffffu) - (sum >> 16);
-#endif
+  };
+  if (o.page == nullptr && o.out_key == nullptr && o.idx_offset == 0) {
+    pass(std::true_type{});
+  } else {
+    pass(std::false_type{});
   }
   FFTOPK_MARK(33);
   if constexpr (kTrackMin) {
-    win_min = __reduce_min_sync(kFull, win_min);
-    if (lane == 0 && win_min != 0xffffffffu) atomicMin(&ctrl->thr_key, win_min);
+    if (f.z == 0u) {  // (else the smallest winner is one of those that are ranked)
+      win_min = __reduce_min_sync(kFull, win_min);
+      if (lane == 0 && win_min != 0xffffffffu) atomicMin(&ctrl->thr_key, win_min);
+    }
   }
 #ifdef FFTOPK_CHECKED
-  {
-    // every certain winner took exactly one slot, every undecided candidate was set aside
-    const uint32_t want_w = all_bin ? need_total : need_total - need2;
-    if (tid == 0) {
-      if (set_w != want_w) check_fail(10, set_w, want_w, status);
-      if (!all_bin && set_u != cnt) check_fail(11, set_u, cnt, status);
-    }
+  const uint32_t set_w = __reduce_add_sync(kFull, lane < NT / 32 ? lds32(wsum + lane * 4) : 0u);
+  __syncthreads();
+  if (tid == 0) {
+    const uint32_t want_w = f.z == 0u ? need : need - f.w;  // (undecided ones: need - f.w certain winners)
+    if (set_w != want_w) check_fail(10, set_w, want_w, o.status);
+    if (ctrl->small_n != f.z) check_fail(11, ctrl->small_n, f.z, o.status);
   }
 #endif
-  if (!all_bin) {
-    __syncthreads();
-    // Rank by vote: warp i takes candidate i, the lanes compare it with the candidates j (32 per
-    // step); the number of larger ones is candidate i's rank, and the best need2 go behind the
-    // certain winners. Up to 256 undecided candidates are cheaper to rank like this (at most 64
-    // votes per warp) than to split by another round - rows of low-precision logits have
-    // hundreds of exact duplicates at the threshold. (A bitonic compare-exchange network over 32
-    // values is a chain of 60 dependent shuffles; this is one ballot per 32 comparisons.)
-    const uint32_t certain = need_total - need2;
-    const int nchunk = ((int)cnt + 31) >> 5;
-    for (int i = warp; i < (int)cnt; i += NT / 32) {
-      const uint64_t me = ctrl->small[i];
-      uint32_t rank = 0;
-      for (int ch = 0; ch < nchunk; ++ch) {
-        const int j = ch * 32 + lane;
-        const uint64_t other = (j < (int)cnt) ? ctrl->small[j] : 0ull;
-        rank += (uint32_t)__popc(__ballot_sync(kFull, other > me));
-      }
-      if (lane == 0 && rank < need2) {
-        const uint32_t pos = out_base + certain + rank;
-        if (FFTOPK_CHECK(5, pos, out_slots, status) && pos < out_slots) {
-          const int32_t idx = (int32_t)(~(uint32_t)me);
-          out_idx[pos] = page ? __ldg(page + idx) : idx + idx_offset;
-          if (out_key) out_key[pos] = (uint32_t)(me >> 32);
-        }
-        if constexpr (kTrackMin) atomicMin(&ctrl->thr_key, (uint32_t)(me >> 32));
-      }
-    }
-  }
+  if (f.z != 0u) rank_undecided<NT, kTrackMin>(o, need - f.w, f.w, f.z);
 }
 
 }  // namespace fftopk

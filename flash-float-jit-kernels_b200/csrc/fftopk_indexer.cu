@@ -256,8 +256,8 @@ __device__ __noinline__ void indexer_finish_row(const IndexerParams& p, int row,
 #pragma unroll
   for (int w = 0; w < NT / 32; ++w) kmax = max(kmax, ctrl->wmax[w]);
   // every candidate's key lies in [the guess's lowest admitted key, kmax]
-  const uint64_t lo = (uint64_t)guess_low_key(gkey) << 32;
-  const uint64_t cap = ((uint64_t)kmax << 32) | 0xffffffffull;
+  const uint32_t lo = guess_low_key(gkey);
+  const uint32_t cap = kmax;
   const int idx_bits = 32 - __clz(len - 1);
   const DenseCands<NT> list{cand_smem, (int)count};
   cta_finish<NT, DenseCands<NT>, true>(list, (uint32_t)kK, lo, cap, cap, false, idx_bits, hist, ctrl,

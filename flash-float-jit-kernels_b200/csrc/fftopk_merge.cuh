@@ -318,8 +318,8 @@ __device__ __forceinline__ void merge_row(cg::cluster_group& cluster, int C, int
   if (mode == kModeGather) {
     const uint32_t need = ctrl->above;
     const DenseCands<NT> bin_cands{sm.cand, (int)ctrl->cand_count};
-    const uint64_t lo = (uint64_t)t << (32 + pshift);
-    const uint64_t cap = lo | ((1ull << (32 + pshift)) - 1ull);
+    const uint32_t lo = t << pshift;
+    const uint32_t cap = lo | ((1u << pshift) - 1u);
     cta_finish<NT, DenseCands<NT>, kTrackMin>(bin_cands, need, lo, cap, cap, false, 31, hist, ctrl, out_idx, out_key,
                                               (uint32_t)kK - need, (uint32_t)kK, 0, status, nullptr, ctrl->cand_count);
   } else if (mode != kModeTakeAll) {

@@ -23,12 +23,12 @@
 //      memory, where every CTA owns a region; every CTA also tells every other its count, so that
 //      after the one cluster barrier each knows whether the guess held and all but rank 0 leave. Rank 0
 //      finishes: radix rounds over the composites' range, a counting and a writing pass, and the last
-//      <= 256 undecided candidates ranked by votes. A lone CTA finishes over its segments where they
-//      lie. The inverted index in the composite makes equal values resolve to the lower index.
+//      <= 256 undecided candidates ranked by votes. A lone CTA keeps its candidates' indices in shared memory and
+//      their keys in registers, and finishes on those (lone_finish). The inverted index in the composite makes equal values resolve to the lower index.
 //      Measured (us per call in a chain of calls on B200, when histograms were exchanged -> with steps 1 to 4
 //      as they are now): B=1, L=96K 12.9 -> 10.0, 1M 15.4 -> 14.1; B=4, L=200K 13.6 -> 10.7; B=64 ragged rows
-//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5); B=2048, one CTA per row, L=32K
-//      132 -> 102, 8K 106 -> 67. What bounds it is no bandwidth but the chain of short phases and the instructions in it.
+//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5, then 3.8); B=2048, one CTA per row, L=32K
+//      132 -> 102 -> 84.6, 8K 106 -> 67 -> 58.6, 4K 62 -> 38.5 (the last figure of each: keys in registers, fewer instructions). What bounds it is no bandwidth but the chain of short phases and the instructions in it.
 //   5. If the guess admitted fewer than k elements, a list overflowed or the threshold bin is
 //      larger than rank 0's buffer (heavy ties, rows of equal values), the cluster falls back to
 //      full histograms over the data: 12 + 12 + 8 key bits, re-reading the shard from L2 each
@@ -47,6 +47,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
+
+#include <algorithm>
 
 #include "../../include/fftopk.h"
 #include "fftopk_trace.cuh"
@@ -462,6 +464,161 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int slabs,
   return total;
 }
 
+// The filters of a lone CTA. They leave the candidates' row indices in the warp's segment (word j: candidate j) and
+// nothing else: the values are fetched again by the pass that follows, several loads in flight per lane.
+// What bounds a batch of such rows is the instructions their warps issue, so: two per element for the pass mask, one
+// from the FMA pipe (the sign of x - edge; a NaN has none) and one that shifts the sign in; slots by a scan over the
+// warp, once per trip; and every lane walks its own hits, without the votes and the warp-wide counter of a
+// loop that the warp walks together (10,500 warp instructions for a row of 32K elements then).
+// Beyond the segment: into the spill area, with the value, as composites.
+struct LoneList {
+  uint32_t seg_s;  // shared address of the warp's segment
+  uint32_t seg_cap;
+  Ctrl* ctrl;
+  uint64_t* spill;
+  uint32_t spill_cap;
+};
+__device__ __forceinline__ uint32_t warp_excl_scan(uint32_t n, uint32_t& total) {
+  const int lane = lane_id();
+  uint32_t incl = n;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFull, incl, off);
+    if (lane >= off) incl += v;
+  }
+  total = __shfl_sync(kFull, incl, 31);
+  return incl - n;
+}
+// hits: bit 31 - e for element e (of at most 32) of the lane; index_of(e) is its place in the row
+template <class T, class IndexOf>
+__device__ __forceinline__ void keep_hits(const Shard<T>& sh, const LoneList& l, uint32_t hits, uint32_t& wcnt, IndexOf&& index_of) {
+  uint32_t total;
+  uint32_t pos = wcnt + warp_excl_scan((uint32_t)__popc(hits), total);
+  wcnt += total;
+  if (wcnt <= l.seg_cap) {  // (uniform over the warp)
+    uint32_t at = l.seg_s + pos * 4u;
+    while (hits != 0u) {
+      const int e = __clz((int)hits);
+      hits &= ~(0x80000000u >> e);
+      sts32(at, (uint32_t)index_of(e));
+      at += 4u;
+    }
+  } else {
+    while (hits != 0u) {
+      const int e = __clz((int)hits);
+      hits &= ~(0x80000000u >> e);
+      const int idx = index_of(e);
+      if (pos < l.seg_cap) {
+        sts32(l.seg_s + pos * 4u, (uint32_t)idx);
+      } else {
+        const uint32_t bits = __float_as_uint(Elem<T>::ld1(sh.gbase + idx + sh.a));
+        spill_push(l.ctrl, l.spill, l.spill_cap, ((uint64_t)bits << 32) | (uint32_t)idx);
+      }
+      ++pos;
+    }
+  }
+}
+// (x >= edge or NaN: 0) shifted into the mask from the right. An edge of zero has to be the negative one: -0 - (-0) is +0,
+// -0 - (+0) would be -0.
+__device__ __forceinline__ uint32_t shift_in_below(uint32_t mask, float x, float edge) {
+  return __funnelshift_l(__float_as_uint(x - edge), mask, 1);
+}
+__device__ __forceinline__ uint32_t shift_in_below4(uint32_t mask, const float4& x, float edge) {
+  return shift_in_below(shift_in_below(shift_in_below(shift_in_below(mask, x.x, edge), x.y, edge), x.z, edge), x.w, edge);
+}
+template <int NT, class T>
+__device__ __forceinline__ uint32_t filter_stream_lone(const Shard<T>& sh, float edge, const LoneList& l) {
+  constexpr int U = 8;
+  static_assert(4 * U <= 32, "the mask");
+  const int tid = threadIdx.x;
+  const float ninf = __uint_as_float(0xff800000u);
+  const T* gbase = sh.gbase;
+  uint32_t wcnt = 0u;
+  auto trip = [&](int gb, auto full) {
+    float4 x[U];
+    uint32_t valid = 0xffffffffu;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int g = gb + u * NT + tid;
+      if constexpr (decltype(full)::value) {
+        x[u] = Elem<T>::ld4(gbase, g);
+      } else {
+        x[u] = make_float4(ninf, ninf, ninf, ninf);
+        if (g < sh.i1) {
+          x[u] = Elem<T>::ld4(gbase, g);
+        } else {
+          valid &= ~(0xf0000000u >> (4 * u));  // (padding would pass an edge of -inf)
+        }
+      }
+    }
+    uint32_t below = 0u;
+#pragma unroll
+    for (int u = 0; u < U; ++u) below = shift_in_below4(below, x[u], edge);
+    const int el0 = 4 * (gb + tid) - sh.a;
+    const uint32_t hits = ~below << (32 - 4 * U);  // (bit 31 - e: element e; none beyond the 4 * U that were read)
+    keep_hits(sh, l, decltype(full)::value ? hits : hits & valid, wcnt,
+              [&](int e) { return el0 + e * NT - (e & 3) * (NT - 1); });  // element e & 3 of granule e >> 2
+  };
+  int gb = sh.i0;
+  for (; gb + NT * U <= sh.i1; gb += NT * U) trip(gb, std::true_type{});
+  if (gb < sh.i1) trip(gb, std::false_type{});
+  // edge granules [g0, i0) and [i1, g1): at most one each, visited by lane 0 of warps 0 and 1
+  if (tid < 64) {  // (whole warps)
+    const int ge = (tid == 0) ? sh.g0 : ((tid == 32) ? sh.i1 : -1);
+    const int ge_end = (tid == 0) ? sh.i0 : sh.g1;
+    const bool mine = ge >= 0 && ge < ge_end;
+    if (__any_sync(kFull, mine)) {
+      uint32_t hits = 0u;
+      const int e0 = 4 * ge - sh.a;
+      if (mine) {
+        const float4 x = load_granule_partial(sh.gbase, sh.a, sh.len, ge, ninf);
+        const uint32_t below = shift_in_below4(0u, x, edge);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if ((unsigned)(e0 + e) < (unsigned)sh.len && !((below >> (3 - e)) & 1u)) hits |= 0x80000000u >> e;
+      }
+      keep_hits(sh, l, hits, wcnt, [&](int e) { return e0 + e; });
+    }
+  }
+  return wcnt;
+}
+// ... of a shard that sits in registers (x[j]: granule j*NT + thread, -inf where an element is not the row's; edge > -inf):
+// a quarter of a short row passes, so a predicated store per element is cheaper than a walk over the hits.
+template <int R, class T>
+__device__ __forceinline__ uint32_t filter_regs_lone(const Shard<T>& sh, const float4 (&x)[R], int slabs, int el0, int el_step,
+                                                     float edge, const LoneList& l) {
+  static_assert(R <= 8, "");
+  uint32_t below = 0u;
+#pragma unroll
+  for (int j = 0; j < R; ++j) below = j < slabs ? shift_in_below4(below, x[j], edge) : (below << 4) | 0xfu;
+  const uint32_t hits = ~below << (32 - 4 * R);
+  uint32_t total;
+  const uint32_t pos = warp_excl_scan((uint32_t)__popc(hits), total);
+  if (total <= l.seg_cap) {  // (uniform over the warp)
+    uint32_t at = l.seg_s + pos * 4u;
+    auto put = [&](float v, int idx) {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p st.shared.u32 [%0], %3;\n\t@p add.u32 %0, %0, 4;\n\t}"
+          : "+r"(at)
+          : "f"(v), "f"(edge), "r"(idx)
+          : "memory");
+    };
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (j < slabs) {  // (uniform)
+        put(x[j].x, el0 + j * el_step);
+        put(x[j].y, el0 + j * el_step + 1);
+        put(x[j].z, el0 + j * el_step + 2);
+        put(x[j].w, el0 + j * el_step + 3);
+      }
+    }
+    return total;
+  }
+  uint32_t wcnt = 0u;
+  keep_hits(sh, l, hits, wcnt, [&](int e) { return el0 + (e >> 2) * el_step + (e & 3); });
+  return wcnt;
+}
+
 // The sample of a row: `nb` batches of G loads of 32 granules per warp, spread over the whole row in pieces
 // (see sample_piece_start). Every CTA of a cluster takes the SAME sample, so each finds the same guess by
 // itself: no exchange of histograms and no cluster barrier in front of the search. A row that is no larger
@@ -500,14 +657,20 @@ struct RowSample {
   }
   template <int N, class Op>
   __device__ __forceinline__ void use(int b, const float4 (&x)[N], Op&& op) const {
+    auto four = [&](const float4& v) {
+      op(__float_as_uint(v.x));
+      op(__float_as_uint(v.y));
+      op(__float_as_uint(v.z));
+      op(__float_as_uint(v.w));
+    };
+    if (whole) {
 #pragma unroll
-    for (int u = 0; u < G; ++u) {
-      if (u < gu && (!whole || load_no(b, u) * 32 + lane_id() < gi)) {
-        op(__float_as_uint(x[u].x));
-        op(__float_as_uint(x[u].y));
-        op(__float_as_uint(x[u].z));
-        op(__float_as_uint(x[u].w));
-      }
+      for (int u = 0; u < G; ++u)
+        if (u < gu && load_no(b, u) * 32 + lane_id() < gi) four(x[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < G; ++u)
+        if (u < gu) four(x[u]);
     }
   }
 };
@@ -517,11 +680,11 @@ template <int NT, class T>
 struct RowCtx {
   int C, rank;
   Shard<T> sh;
-  uint32_t* hist0;  // two histograms of kMaxBins words, back to back
+  uint32_t* hist0;  // two histograms of kMaxBins words, back to back; a lone CTA has one that serves as both
   uint32_t* sup0;   // two super-bin arrays of kSup words, back to back
   // (computed addresses instead of pointer arrays: indexing an array member with the round number
   // would force the whole struct into local memory)
-  __device__ __forceinline__ uint32_t* hist(int i) const { return hist0 + i * kMaxBins; }
+  __device__ __forceinline__ uint32_t* hist(int i) const { return C == 1 ? hist0 : hist0 + i * kMaxBins; }
   __device__ __forceinline__ uint32_t* sup(int i) const { return sup0 + i * kSup; }
   uint32_t* xch;
   Ctrl* ctrl;
@@ -734,8 +897,8 @@ __device__ __noinline__ uint32_t select_by_full_histograms(const RowCtx<NT, T> p
   if (mode == kModeGather) {
     // every candidate shares the key prefix P above bit `shift` of the key
     const int shift = round_shift(r);
-    const uint64_t lo = (uint64_t)P << (32 + shift);
-    const uint64_t cap = lo | ((1ull << (32 + shift)) - 1ull);
+    const uint32_t lo = P << shift;
+    const uint32_t cap = lo | ((1u << shift) - 1u);
     const DenseCands<NT> src{cx.cand, (int)min(cx.ctrl->cand_count, (uint32_t)cx.cand_cap)};
     cta_finish<NT, DenseCands<NT>, kTrack>(src, need, lo, cap, cap, false, 32 - __clz(cx.sh.len - 1), cx.hist(1), cx.ctrl,
                                            cx.out_idx, cx.out_key, cx.k - need, cx.k, cx.idx_offset, cx.status, cx.page,
@@ -769,7 +932,35 @@ __host__ __device__ constexpr int min_ctas(int form) {
 // per SM (128 registers a thread) rows of up to 256K elements over 16 CTAs.
 template <int NT>
 __host__ __device__ constexpr int reg_slabs(int form) {
-  return NT == 512 && form == kRoomyForm ? 2 * FFTOPK_REG_SLABS : FFTOPK_REG_SLABS;
+  return (NT == 512 && form == kRoomyForm) ? 2 * FFTOPK_REG_SLABS : FFTOPK_REG_SLABS;
+}
+// Where a row's output goes, its page table (NULL: none) and the offset of its indices. Worked out where they are
+// needed: kept from the start they would cost every thread the registers through sample and filter.
+struct RowOutput {
+  int32_t* idx;
+  uint32_t* key;
+};
+__device__ __forceinline__ RowOutput row_output(const SelectParams& p, int row, uint32_t K) {
+  const int64_t at = (p.cp_flag ? (int64_t)((__ldcg(p.cp_flag) + 1u) & 1u) * p.cp_half_words : 0) + (int64_t)row * K;
+  return RowOutput{p.out_idx + at, p.out_key ? p.out_key + at : nullptr};
+}
+__device__ __forceinline__ const int32_t* row_page(const SelectParams& p, int row) {
+  if (!p.src_page_table) return nullptr;
+  // which table row serves this score row: the request i with cu_seqlens_q[i] <= row < cu_seqlens_q[i+1]
+  // (radix.cu:925-939); without cu_seqlens_q, the row itself (decode, :880)
+  int64_t req = row;
+  if (p.cu_seqlens_q) {
+    int lo = 0, hi = p.prefill_bs;  // invariant: cu[lo] <= row, answer in [lo, hi)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(p.cu_seqlens_q + mid) <= row) lo = mid; else hi = mid;
+    }
+    req = lo;
+  }
+  return p.src_page_table + req * p.src_stride;
+}
+__device__ __forceinline__ int32_t row_idx_offset(const SelectParams& p, int row) {
+  return p.idx_offset + (p.row_offsets ? __ldg(p.row_offsets + row) : 0);
 }
 // kAnyK = false: k is the constant 2048 of the reference's op (the compiler folds it: one register
 // less in a kernel that sits at its register limit); true: k comes from the parameters.
@@ -806,32 +997,18 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   len64 = len64 > p.L - row_start ? p.L - row_start : len64;
   const int len = (int)len64;
   const T* rowp = static_cast<const T*>(p.score) + (int64_t)row * p.row_stride + row_start;
-  const int64_t cp_shift = p.cp_flag ? (int64_t)((__ldcg(p.cp_flag) + 1u) & 1u) * p.cp_half_words : 0;
   const uint32_t K = cx.k = kAnyK ? (uint32_t)p.k : (uint32_t)kK;
-  int32_t* out_idx = cx.out_idx = p.out_idx + cp_shift + (int64_t)row * K;
-  uint32_t* out_key = cx.out_key = p.out_key ? p.out_key + cp_shift + (int64_t)row * K : nullptr;
-  cx.idx_offset = p.idx_offset + (p.row_offsets ? __ldg(p.row_offsets + row) : 0);
-  cx.page = nullptr;
-  if (p.src_page_table) {
-    // which table row serves this score row: the request i with cu_seqlens_q[i] <= row < cu_seqlens_q[i+1]
-    // (radix.cu:925-939); without cu_seqlens_q, the row itself (decode, :880)
-    int64_t req = row;
-    if (p.cu_seqlens_q) {
-      int lo = 0, hi = p.prefill_bs;  // invariant: cu[lo] <= row, answer in [lo, hi)
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(p.cu_seqlens_q + mid) <= row) lo = mid; else hi = mid;
-      }
-      req = lo;
-    }
-    cx.page = p.src_page_table + req * p.src_stride;
-  }
   cx.cand_cap = p.cand_cap;
   cx.status = p.status;
 
   // Short rows: 0..len-1 then -1 (reference: naive_topk_cuda, topk_indexer_radix.cu:152-163).
   if (len <= (int)K) {
     if (rank == 0) {
+      const RowOutput ro = row_output(p, row, K);
+      int32_t* out_idx = ro.idx;
+      uint32_t* out_key = ro.key;
+      cx.page = row_page(p, row);
+      cx.idx_offset = row_idx_offset(p, row);
       for (int i = tid; i < (int)K; i += NT) {
         out_idx[i] = i < len ? (cx.page ? __ldg(cx.page + i) : i + cx.idx_offset) : -1;
         if (out_key) out_key[i] = i < len ? fftopk_key_from_bits(__float_as_uint(Elem<T>::ld1(rowp + i))) : 0u;
@@ -847,9 +1024,9 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   // ---- shared memory carve ---------------------------------------------------------------
   extern __shared__ __align__(128) unsigned char smem_raw[];
   cx.hist0 = reinterpret_cast<uint32_t*>(smem_raw);
-  cx.sup0 = cx.hist0 + 2 * kMaxBins;
-  cx.xch = cx.sup0 + 2 * kSup;                                             // kMaxCluster * 64 words
-  Ctrl* ctrl = cx.ctrl = reinterpret_cast<Ctrl*>(cx.xch + kMaxCluster * kSup);  // 8-byte aligned
+  cx.sup0 = cx.hist0 + (kLone ? 1 : 2) * kMaxBins;
+  cx.xch = cx.sup0 + 2 * kSup;                                             // 64 words per CTA of the cluster
+  Ctrl* ctrl = cx.ctrl = reinterpret_cast<Ctrl*>(cx.xch + (kLone ? 1 : kMaxCluster) * kSup);  // 16-byte aligned
   cx.list = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(ctrl) + ((sizeof(Ctrl) + 127) & ~127u));
   // a cluster of one CTA has nobody to gather from: its candidate buffer IS the list
   cx.cand = C == 1 ? cx.list : cx.list + p.list_cap;
@@ -911,12 +1088,20 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     }
   }
   float4 xs[G];
-  if (sampled) smp.load(sh.gbase, 0, xs);
-  // ---- clear both histograms and the control block --------------------------------------------------
-  uint32_t* const fin_hist = cx.hist(1);  // round 0 of the finish
-  const uint32_t h0 = smem_u32(cx.hist(0)), fh = smem_u32(fin_hist);  // shared addresses
+  // (a row that a lone CTA holds whole is its own sample)
+  const bool own_sample = kLone && in_regs && smp.whole;
+  if (sampled && !own_sample) smp.load(sh.gbase, 0, xs);
+  // ---- clear the histograms and the control block --------------------------------------------------
+  // (round 0 of the finish: a histogram of its own, or a lone CTA's only one, cleared for it after the search)
+  uint32_t* const fin_hist = kLone ? cx.hist0 : cx.hist0 + kMaxBins;
+  const uint32_t h0 = smem_u32(cx.hist0), fh = smem_u32(fin_hist);  // shared addresses
   {
-    for (int i = tid + (warm ? kMaxBins / 4 : 0); i < (kMaxBins + kFinishBins) / 4; i += NT) sts_zero16(h0 + i * 16);
+    constexpr int kOwnFin = kLone ? 0 : kFinishBins / 4;
+    if (!warm) {
+      for (int i = tid; i < kMaxBins / 4 + kOwnFin; i += NT) sts_zero16(h0 + i * 16);
+    } else {
+      for (int i = tid; i < kFinishBins / 4; i += NT) sts_zero16(fh + i * 16);
+    }
     if (tid == 0) {
       if constexpr (kWarm) ctrl->thr_key = 0xffffffffu;
       ctrl->extra_count = 0u;
@@ -928,6 +1113,10 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
 #ifdef FFTOPK_CHECKED
       ctrl->status_ptr = p.status;
 #endif
+    }
+    if (tid == 32) {  // (a search in a table, while the loads travel)
+      ctrl->row_page = row_page(p, row);
+      ctrl->row_idx_offset = row_idx_offset(p, row);
     }
     if (sampled && warp == NW - 1) {
       // The ranks sought in the sample (see sample_lower_rank). One warp works them out while the loads
@@ -963,8 +1152,20 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   }
   if (sampled) {
     const uint32_t wtot_s = smem_u32(ctrl->wtot);
-    auto tally = [&](uint32_t bits) { red_shared_inc(h0 + sample_digit(bits) * 4u); };
-    if constexpr (NT >= 512 && kForm != kRoomyForm) {
+    const uint32_t mid = h0 + kSampleBins / 2 * 4u;
+    auto tally = [&](uint32_t bits) { red_shared_inc(mid + (uint32_t)sample_digit_offset(bits)); };
+    if (own_sample) {
+#pragma unroll
+      for (int j = 0; j < kRegSlabs; ++j) {
+        const int g = sh.g0 + j * NT + tid;
+        if (j < slabs && g >= sh.i0 && g < sh.i1) {
+          tally(__float_as_uint(xr[j].x));
+          tally(__float_as_uint(xr[j].y));
+          tally(__float_as_uint(xr[j].z));
+          tally(__float_as_uint(xr[j].w));
+        }
+      }
+    } else if constexpr (kForm != kRoomyForm) {
       // The next batch of a long row is on its way while this one is counted: its shards are far too long for
       // the registers, and the next batch takes their place. (Not where a thread has registers to spare: a
       // row of two batches over 16 CTAs took 15.1 us like this, and 14.85 with one batch after the other.)
@@ -986,7 +1187,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     }
     __syncthreads();
     FFTOPK_MARK(2);
-    const uint32_t room = (uint32_t)(C == 1 ? p.list_cap : p.cand_cap);
+    const uint32_t room = (uint32_t)(kLone ? lone_room(p.list_cap, NT) : p.cand_cap);
     // (one thread, when it has found the bin) what the guess is and what to do about it: see weigh_guess
     auto weigh = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
       const uint32_t flags = weigh_guess(width, above, cnt, parent, smp.size(), (float)len, K, kCoarseFactor, room);
@@ -1037,18 +1238,23 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     gkey = ctrl->guess;
     focus_key = ctrl->focus;
     guessed = flags == 0u;
+    if constexpr (kLone) {
+      for (int i = tid; i < kFinishBins / 4; i += NT) sts_zero16(fh + i * 16);
+      __syncthreads();
+    }
   }
   FFTOPK_MARK(4);
 
   uint32_t thr = 0u;  // this call's threshold key
   int mode = kModeFallback;
-  auto low_end = [](uint32_t key) { return (uint64_t)key << 32; };
-  auto high_end = [](uint32_t key) { return ((uint64_t)key << 32) | 0xffffffffull; };
   // list layout: one segment per warp, then the spill area
+  // (a lone CTA's segments hold indices only, as many as its warps have registers for)
+  constexpr int kLoneRegs = lone_regs(NT);
   const uint32_t spill_cap = (uint32_t)list_spill(p.list_cap, kLone);
-  const uint32_t seg_cap = ((uint32_t)p.list_cap - spill_cap) / NW;
-  uint64_t* const seg = list + (size_t)warp * seg_cap;
-  uint64_t* const spill = list + (size_t)NW * seg_cap;
+  const uint32_t seg_cap = kLone ? (uint32_t)lone_segment(p.list_cap, NT) : ((uint32_t)p.list_cap - spill_cap) / NW;
+  uint64_t* const seg = kLone ? nullptr : list + (size_t)warp * seg_cap;
+  uint64_t* const spill = list + (kLone ? (size_t)(NW * seg_cap + 1u) / 2u : (size_t)NW * seg_cap);
+  const LoneList lone{smem_u32(list) + (uint32_t)warp * seg_cap * 4u, seg_cap, ctrl, spill, spill_cap};
 
   // ---- filter the shard against the guess -------------------------------------------------------
   // Lower edge of the guess as a float: key(x) >= gkey  <=>  !(x < edge), NaN included. Keys outside
@@ -1056,7 +1262,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   // only lengthens the lists.
   const float edge = __uint_as_float(guess_edge_bits(gkey));
   const uint32_t lowkey = guess_low_key(gkey);  // every candidate's key lies in [lowkey, 0xffffffff]
-  if (focus_key <= lowkey) focus_key = 0xffffffffu;
+  if (focus_key < lowkey) focus_key = 0xffffffffu;
   constexpr int U = NT >= 1024 ? 4 : FFTOPK_U512;
   uint32_t wcnt = 0u;
   bool staged = false;
@@ -1064,6 +1270,13 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     // No guess to filter with: say so the way an overflowed list does. (Every step from here on
     // depends on what the cluster's CTAs tell each other, not on what each has read for itself.)
     if (tid == 0) ctrl->pub_flag = 1u;
+  } else if (kLone) {
+    const float cut = edge == 0.f ? -0.f : edge;
+    if (in_regs && edge > ninf) {
+      wcnt = filter_regs_lone<kRegSlabs>(sh, xr, slabs, 4 * (sh.g0 + tid) - sh.a, 4 * NT, cut, lone);
+    } else {
+      wcnt = filter_stream_lone<NT>(sh, cut, lone);
+    }
   } else if (in_regs && edge > ninf) {
     wcnt = filter_regs<kRegSlabs>(xr, slabs, 4 * (sh.g0 + tid) - sh.a, 4 * NT, edge, seg, seg_cap, ctrl, spill, spill_cap);
   } else if (len <= 196608) {  // about 1.5 k candidates per row: most trips of the hit loop have work
@@ -1074,32 +1287,47 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   }
   const uint32_t wown = min(wcnt, seg_cap);
   FFTOPK_MARK(8);
-  bool have_hist = false;  // (lone CTA) round 0 of the finish has its histogram
   const int region = kLone ? 0 : p.region;  // slots of each CTA in rank 0's buffer
   int extra = 0;           // candidates beyond their CTAs' regions
   uint32_t total = 0u;     // candidates of the row
-  uint32_t fin_sn = 0u;
-  if (C == 1) {
+  RegSegCands<NT, kLoneRegs> held;
+  if constexpr (kLone) {
     // ---- a lone CTA keeps its candidates where they are ------------------------------------------
-    // They become composites in place, and the histogram of the finish's first round is built on
-    // the way (they pass through registers here anyway).
-    const FinishDigit dg = make_finish_digit(low_end(lowkey), high_end(focus_key));
-    have_hist = dg.key_only();
-    const uint32_t seg_s = smem_u32(seg);
-    drain_segment(staged, sh, seg, wown, ctrl, [&](uint32_t j, uint64_t c) {
-      sts64(seg_s + j * 8u, (uint32_t)c, (uint32_t)(c >> 32));
-      if (have_hist) red_shared_inc(fh + dg.of_key((uint32_t)(c >> 32)) * 4u);
-    });
+    // Their keys go into registers, and the histogram of the finish's first round is built on the way.
+    const KeyDigit dg = make_key_digit(lowkey, focus_key);
+    held.seg = lone.seg_s;
+    held.wn = (int)wown;
+    held.spill = smem_u32(spill);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kLoneRegs; i += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) held.key[i + u] = 0u;
+      if (i * 32 < held.wn) {  // (uniform over the warp)
+        uint32_t bits[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = (i + u) * 32 + lane;
+          uint32_t idx = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
+          if (!FFTOPK_CHECK(7, idx, sh.len, p.status)) idx = 0u;
+          bits[u] = __float_as_uint(Elem<T>::ld1(sh.gbase + idx + sh.a));  // (index 0 is always readable)
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if ((i + u) * 32 < held.wn) {  // (uniform)
+            if ((i + u) * 32 + lane < held.wn) {
+              held.key[i + u] = fftopk_key_from_bits(bits[u]);
+              red_shared_inc(fh + dg.of(held.key[i + u]) * 4u);
+            }
+          }
+        }
+      }
+    }
     const uint32_t wn_s = smem_u32(ctrl->wmax);
     if (lane == 0) sts32(wn_s + warp * 4, wown);  // (not wtot: the finish's search may write that before every warp has read it)
     __syncthreads();
-    fin_sn = min(ctrl->lcount, spill_cap);
-    total = __reduce_add_sync(kFull, lane < NW ? lds32(wn_s + lane * 4) : 0u) + fin_sn;
-    if (have_hist && fin_sn > 0u) {  // (uniform) the entries that went to the spill area
-      const uint32_t sp = smem_u32(spill) + 4u;  // (the keys)
-      for (uint32_t j = tid; j < fin_sn; j += NT) red_shared_inc(fh + dg.of_key(lds32(sp + j * 8u)) * 4u);
-      __syncthreads();
-    }
+    held.sn = (int)min(ctrl->lcount, spill_cap);
+    total = __reduce_add_sync(kFull, lane < NW ? lds32(wn_s + lane * 4) : 0u) + (uint32_t)held.sn;
     mode = sampled_attempt_ok(ctrl->pub_flag, total, K, 0xffffffffu) ? kModeGather : kModeFallback;
   } else {
     // ---- gather in rank 0 ----------------------------------------------------------------------
@@ -1160,19 +1388,22 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   // leave, and rank 0 needs no barrier at the end.
   if (mode == kModeGather && rank != 0) return;
   FFTOPK_MARK(5);
+  const RowOutput ro = row_output(p, row, K);
+  int32_t* const out_idx = cx.out_idx = ro.idx;
+  uint32_t* const out_key = cx.out_key = ro.key;
+  cx.page = ctrl->row_page;
+  cx.idx_offset = ctrl->row_idx_offset;
 
   const int idx_bits = 32 - __clz(len - 1);
   if (rank == 0) FFTOPK_ROUTE(mode == kModeGather ? kRouteHeld : kRouteHistograms);
   if (rank == 0 && mode == kModeGather && extra > 0) FFTOPK_ROUTE(kRouteBeyond);
   if (mode == kModeGather) {
-    const uint64_t lo = low_end(lowkey), focus = high_end(focus_key);
-    if (C == 1) {
-      const WarpSegCands<NT> src{smem_u32(seg), (int)wown, smem_u32(spill), (int)fin_sn};
-      cta_finish<NT, WarpSegCands<NT>, kWarm>(src, K, lo, ~0ull, focus, have_hist, idx_bits, fin_hist, ctrl, out_idx, out_key,
-                                              0u, K, cx.idx_offset, p.status, cx.page, total, true);
+    if constexpr (kLone) {
+      const FinishOut o{ctrl, out_idx, out_key, p.status, cx.page, 0u, K, cx.idx_offset};
+      lone_finish<NT, kLoneRegs, kWarm>(held, o, K, lowkey, focus_key, idx_bits, fin_hist, total);
     } else {
       const RegionCands<NT> src{smem_u32(cx.cand), smem_u32(ctrl->cnt_of), region, C, extra};
-      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lo, ~0ull, focus, false, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
+      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lowkey, 0xffffffffu, focus_key, false, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
                                              K, cx.idx_offset, p.status, cx.page, total, true);
     }
     // This call's threshold for the next one: the smallest key the finish let win (the row's k-th
@@ -1336,8 +1567,9 @@ struct DeviceInfo {
 };
 DeviceInfo g_dev[kMaxDevices];
 
-constexpr size_t fixed_smem_bytes() {
-  return (size_t)(2 * kMaxBins + 2 * kSup + kMaxCluster * kSup) * 4 + ((sizeof(Ctrl) + 127) & ~(size_t)127);
+// (everything but the lists; a lone CTA has one histogram and nobody to exchange super-bins with)
+constexpr size_t fixed_smem_bytes(bool lone) {
+  return (size_t)((lone ? 1 : 2) * kMaxBins + 2 * kSup + (lone ? 1 : kMaxCluster) * kSup) * 4 + ((sizeof(Ctrl) + 127) & ~(size_t)127);
 }
 
 constexpr int kLatencyListCap = 6144, kLatencyCandCap = 16384;  // one CTA per SM: use the shared memory
@@ -1348,6 +1580,9 @@ constexpr int kLatencyListCap = 6144, kLatencyCandCap = 16384;  // one CTA per S
 constexpr int kOverlapListCap1 = 6144, kOverlapListCap1Long = 9216;
 constexpr int64_t kOverlapShortRow = 196608;
 constexpr int kOverlapListCap = 3072, kOverlapCandCap = 6144;   // two CTAs per SM
+// Rows so short that the list of a CTA of 256 threads holds all of them, whatever they are (make_plan)
+constexpr int kLoneListCap256 = 4096, kLoneCandCap256 = 2560;
+constexpr int64_t kLoneRow256 = 4352;
 
 
 using SelectFn = void (*)(SelectParams);
@@ -1414,7 +1649,7 @@ int init_device(DeviceInfo& d, int dev) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs * 32, 1, 1);
     cfg.blockDim = dim3(512, 1, 1);  // (the form that such a plan launches)
-    cfg.dynamicSmemBytes = fixed_smem_bytes() + (size_t)(kLatencyListCap + kLatencyCandCap) * 8;
+    cfg.dynamicSmemBytes = fixed_smem_bytes(false) + (size_t)(kLatencyListCap + kLatencyCandCap) * 8;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cs;
@@ -1461,10 +1696,18 @@ int floor_pow2(int64_t v) {
   return r;
 }
 
+// The lists of a lone CTA: one for the filter, and in the same memory the one the full-histogram path gathers in.
+// What they leave of the SM's 256 KB is L1, through which every load of the stream passes.
+void lone_lists(Plan& pl, int list_cap) {
+  pl.list_cap = list_cap;
+  pl.cand_cap = pl.threads == 256 ? std::min(list_cap, kLoneCandCap256) : list_cap;
+  pl.smem_bytes = (int)(fixed_smem_bytes(true) + std::max((size_t)lone_list_bytes(list_cap, pl.threads), (size_t)pl.cand_cap * 8));
+}
+
 // Replaces the reference's split heuristic (topk_indexer_radix.cu:1081-1111: at most 8 CTAs per
 // row, a hard-coded SM count of 132). `overlap`: the launch may overlap its neighbours on the
-// stream (throughput plan).
-Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64_t L) {
+// stream (throughput plan). `narrow`: the call's kernel exists for 256 threads.
+Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64_t L, bool narrow) {
   Plan pl;
   const int rows = B > 0 ? B : 1;
   // CTAs per row: as many as keep the whole grid resident at once with one CTA per SM, but never
@@ -1510,12 +1753,22 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
       pl.cand_cap = kOverlapCandCap;
     }
   }
+  if (narrow && pl.cluster == 1 && pl.threads == 512 && L <= kLoneRow256) {
+    // Short rows: four CTAs of 256 threads share an SM, each with 41 KB, and the phases in which one of them has
+    // little to do are the others' time. Measured with 2,048 rows of N(0,1)-like sums, 256 / 512 threads: 4K elements 37 / 49 us,
+    // 8K 48 / 57, 32K 105 / 82; with 70 % zeros 4K 91 / 105, 6K 191 / 131 - rows that may overflow their list stay with 512.
+    pl.threads = 256;
+    pl.list_cap = kLoneListCap256;
+  }
   if (tn.cluster > 0) pl.cluster = tn.cluster;
   if (tn.threads > 0) pl.threads = tn.threads;
   if (tn.list_cap > 0) pl.list_cap = (tn.list_cap + 15) & ~15;
   if (tn.cand_cap > 0) pl.cand_cap = (tn.cand_cap + 15) & ~15;
-  if (pl.cluster == 1) pl.cand_cap = pl.list_cap;  // one CTA per row: the two buffers are the same memory
-  pl.smem_bytes = (int)(fixed_smem_bytes() + (size_t)(pl.cluster == 1 ? pl.list_cap : pl.list_cap + pl.cand_cap) * 8);
+  if (pl.cluster == 1) {
+    lone_lists(pl, pl.list_cap);
+  } else {
+    pl.smem_bytes = (int)(fixed_smem_bytes(false) + (size_t)(pl.list_cap + pl.cand_cap) * 8);
+  }
   return pl;
 }
 
@@ -1553,12 +1806,15 @@ int launch_select(const SelectCall& c) {
   if (rc) return rc;
   const Tuning tn = tuning_snapshot();
   const bool overlap = tn.overlap != 0 && c.may_overlap;
-  Plan pl = make_plan(*d, tn, overlap, c.B, c.L);
-  if (half_width && pl.threads < 512) pl.threads = 512;  // (the 16-bit kernels exist for 512 and 1024 threads)
+  const bool warm = c.prev_threshold != nullptr || c.next_threshold != nullptr;
+  Plan pl = make_plan(*d, tn, overlap, c.B, c.L, !half_width && !warm);
+  if (half_width && pl.threads < 512) {  // (the 16-bit kernels exist for 512 and 1024 threads)
+    pl.threads = 512;
+    if (pl.cluster == 1) lone_lists(pl, pl.list_cap);
+  }
   if (c.k > kK && pl.cluster == 1 && tn.list_cap <= 0) {
     // more winners than the lone-CTA list was sized for: the long-row list
-    pl.list_cap = pl.cand_cap = kOverlapListCap1Long;
-    pl.smem_bytes = (int)(fixed_smem_bytes() + (size_t)pl.list_cap * 8);
+    lone_lists(pl, kOverlapListCap1Long);
   }
 
   SelectParams p;
@@ -1591,7 +1847,6 @@ int launch_select(const SelectCall& c) {
   p.next_threshold = c.next_threshold;
   p.warm_margin = c.warm_margin;
   p.only_rows = c.only_rows;
-  const bool warm = c.prev_threshold != nullptr || c.next_threshold != nullptr;
   if (warm && (c.k != kK || pl.threads < 512)) return FFTOPK_EINVAL;
   if ((size_t)pl.smem_bytes > (size_t)d->smem_optin) return FFTOPK_ERANGE;
 
@@ -1639,7 +1894,8 @@ int launch_select_merge(const SelectCall& c, void* const* comms, int32_t G, int3
   int rc = device_info(&d);
   if (rc) return rc;
   const Tuning tn = tuning_snapshot();
-  const Plan pl = make_plan(*d, tn, false, c.B, c.L);
+  Plan pl = make_plan(*d, tn, false, c.B, c.L, false);
+  if (pl.cluster == 1) pl.smem_bytes = (int)(fixed_smem_bytes(false) + (size_t)pl.list_cap * 8);  // (the merge's two histograms and candidates)
   const int room = pl.cluster == 1 ? pl.list_cap : pl.list_cap + pl.cand_cap;
   if (pl.cluster < G || room < G * kK || pl.threads < 512 || (size_t)pl.smem_bytes > (size_t)d->smem_optin) return FFTOPK_ERANGE;
 
@@ -1780,7 +2036,7 @@ int fftopk_plan(int32_t B, int64_t L, int32_t plan[6]) {
   int rc = device_info(&d);
   if (rc) return rc;
   const Tuning tn = tuning_snapshot();
-  const Plan pl = make_plan(*d, tn, tn.overlap != 0, B, L);
+  const Plan pl = make_plan(*d, tn, tn.overlap != 0, B, L, true);
   plan[0] = pl.cluster;
   plan[1] = pl.threads;
   plan[2] = pl.smem_bytes;

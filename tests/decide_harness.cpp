@@ -83,17 +83,31 @@ int dh_sample_guess(const uint32_t* bits, uint32_t n, uint32_t n_s, float len, u
   return 0;
 }
 int dh_finish_bins(void) { return kFinishBins; }
-int dh_finish_shift(uint64_t lo, uint64_t focus) { return make_finish_digit(lo, focus).shift; }
-int dh_finish_key_only(uint64_t lo, uint64_t focus) { return make_finish_digit(lo, focus).key_only() ? 1 : 0; }
-uint32_t dh_finish_digit(uint64_t lo, uint64_t focus, uint64_t c) { return make_finish_digit(lo, focus).of(c); }
-uint32_t dh_finish_digit_of_key(uint64_t lo, uint64_t focus, uint32_t key) {
-  return make_finish_digit(lo, focus).of_key(key);
-}
+// the digit rule on 64-bit composites (key << 32 | inverted index) ...
+int dh_finish_shift(uint64_t lo, uint64_t focus) { return make_field_digit<uint64_t>(lo, focus).shift; }
+int dh_finish_key_only(uint64_t lo, uint64_t focus) { return dh_finish_shift(lo, focus) >= 32 && (uint32_t)lo == 0u ? 1 : 0; }
+uint32_t dh_finish_digit(uint64_t lo, uint64_t focus, uint64_t c) { return make_field_digit<uint64_t>(lo, focus).of(c); }
 void dh_finish_bin_range(uint64_t lo, uint64_t focus, uint64_t cap, int t, uint64_t* t_lo, uint64_t* t_hi) {
-  finish_bin_range(make_finish_digit(lo, focus), lo, cap, t, *t_lo, *t_hi);
+  const FieldDigit<uint64_t> dg = make_field_digit<uint64_t>(lo, focus);
+  *t_lo = dg.bin_low((uint32_t)t);
+  *t_hi = dg.bin_high((uint32_t)t, cap);
 }
-uint64_t dh_single_key_floor(uint64_t lo, int idx_bits) { return single_key_floor(lo, idx_bits); }
-
+// ... and on their keys
+uint32_t dh_finish_digit_of_key(uint64_t lo, uint64_t focus, uint32_t key) {
+  return make_key_digit((uint32_t)(lo >> 32), (uint32_t)(focus >> 32)).of(key);
+}
+void dh_key_bin_range(uint32_t lo, uint32_t focus, uint32_t cap, uint32_t t, uint32_t* t_lo, uint32_t* t_hi) {
+  const KeyDigit dg = make_key_digit(lo, focus);
+  *t_lo = dg.bin_low(t);
+  *t_hi = dg.bin_high(t, cap);
+}
+uint32_t dh_key_digit(uint32_t lo, uint32_t focus, uint32_t v) { return make_key_digit(lo, focus).of(v); }
+uint64_t dh_single_key_floor(uint64_t lo, int idx_bits) { return (lo & 0xffffffff00000000ull) | inverted_index_floor(idx_bits); }
+int dh_lone_segment(int list_cap, int threads) { return lone_segment(list_cap, threads); }
+int dh_lone_list_bytes(int list_cap, int threads) { return lone_list_bytes(list_cap, threads); }
+int dh_lone_room(int list_cap, int threads) { return lone_room(list_cap, threads); }
+int dh_lone_regs(int threads) { return lone_regs(threads); }
+int dh_list_spill(int list_cap, int lone) { return list_spill(list_cap, lone != 0); }
 
 // Walks every CTA's run of tiles the way the fused indexer's producer does (tile_run, tile_row_at,
 // then tile_segment row after row) and adds, for every (row, row-local tile) the CTAs visit, one to
