@@ -19,21 +19,25 @@
 //               tile): tcgen05.ld hands every thread the 64 head values of ONE key; relu,
 //               weights and the sum are in-thread - one logit per thread and tile. With a threshold
 //               guess for the row (the previous decode step's, see fftopk_select2048_warm) the
-//               logit is compared with the guess's edge and the few that pass are appended, by
-//               ballot and one atomic per warp, to the row's candidate list. The logit is also
+//               logit is compared with the guess's edge and the few that pass go, 32 at a time per
+//               warp, to the row's candidate list. The logit is also
 //               written (4 bytes per key beside the 256 or 132 read), but read again only by a row
 //               whose guess fails.
 // Every wait on an mbarrier has a time limit; when one runs out the CTA raises
 // FFTOPK_ST_STAGE_TIMEOUT, lets its copies in flight land, frees its TMEM and returns.
 //
-// Finish, inside the producer: the CTAs of a row count themselves off as they run out of tiles, and
-// the last one decides. If the row's guess held - at least 2048 candidates, no more than the list
-// holds - it pulls the list into the shared memory its stages no longer need and selects the exact
-// top 2048 (cta_finish: ties to the lower index) and the new threshold; otherwise it marks the row
-// and the selector of fftopk_select.cu runs on the row's logits. That launch follows as a
-// programmatic dependent: it is resident, waiting, by the time the producer ends, and rows that are
-// not marked cost it an empty CTA. The last CTA also zeroes the row's counters, so a call leaves the
-// workspace ready for the next one and a call is two launches, none of them a memset.
+// The selector of fftopk_select.cu follows as a programmatic dependent. A row whose guess held - at
+// least 2048 candidates, no more than the list has room for - it finishes on the list (exact top 2048, ties to
+// the lower index, and the new threshold; finish_given_candidates), every other row it selects on the logits;
+// and it zeroes the row's candidate count, so a call leaves the workspace ready for the next one and is
+// two launches, none of them a memset.
+//
+// What bounds the producer is reading the keys, as long as nothing interrupts the stream. Until the list was
+// finished by the selector, a CTA drained its pipeline at the end of every row's segment, counted its tiles off with a fence
+// and an atomic, and the row's last CTA put its own tiles off for the finish; and every warp waited for an atomic
+// per 32 keys with a hit. us per call, then -> now: 64 ragged rows of up to 128K, bf16 218-222 -> 171 (1.07 GB of keys: 6.3 TB/s), fp8
+// 133-151 -> 98; 42 of 150K, fp8 113 -> 78; one row of 128K, fp8 12.2 -> 10.3; one of 1M, bf16 50.4 -> 49.5; without guesses, 8 rows of 64K
+// 23.6 -> 23.1.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -92,7 +96,6 @@ struct IdxScaleRing {
   static constexpr int kSlots = kFp8 ? IdxFmt<true>::kStages + kIdxBufs : 0;
 };
 constexpr uint32_t kIdxScaleBytes = kIdxTile * 4;
-constexpr int kIdxCandCap = 8192;  // slots of a row's candidate list: what the freed stages of a CTA hold (64 KiB of composites)
 constexpr unsigned long long kIdxWaitNs = 200ull * 1000 * 1000;
 
 struct IndexerParams {
@@ -108,12 +111,8 @@ struct IndexerParams {
   int64_t logits_stride;
   const uint32_t* guess;     // [B] threshold key guesses (0: none) or nullptr
   uint32_t margin;
-  uint64_t* cand;            // [B, kIdxCandCap] candidates as (key << 32 | ~index) composites
-  uint32_t* cand_count;      // [B] candidates appended so far (may exceed the capacity: the row then falls back)
-  uint32_t* done_count;      // [B] CTAs of the row that have run out of tiles
-  uint32_t* select_rows;     // [B] out: 1 = the selector has to run on the row's logits
-  int32_t* out_idx;          // [B, 2048]
-  uint32_t* thr_out;         // [B] the row's new threshold key (rows finished here)
+  uint64_t* cand;            // [B] records: candidates as (key << 32 | ~index) composites, and the number appended
+                             // so far (may exceed the capacity: the row then falls back)
   uint32_t* status;
 };
 
@@ -213,62 +212,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "memory");
 }
 
-// ---- finish of one row, by the last of its CTAs to run out of tiles ----------------------------------
-// `gkey`: the key guess the row was filtered with (margin already subtracted); `count`: how many
-// candidates were appended. `cand_smem` holds kIdxCandCap composites, `hist` kFinishBins words.
-template <int NT>
-__device__ __noinline__ void indexer_finish_row(const IndexerParams& p, int row, int len, uint32_t gkey, uint32_t count,
-                                                   uint64_t* cand_smem, uint32_t* hist, Ctrl* ctrl) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const bool held = len > kK && count >= (uint32_t)kK && count <= (uint32_t)kIdxCandCap;
-  if (!held) {  // (uniform over the CTA)
-    if (tid == 0) {
-      p.select_rows[row] = 1u;
-      if (p.status) atomicOr(p.status, (uint32_t)FFTOPK_ST_GUESS_MISSED);
-    }
-    return;
-  }
-  // the list, out of L2 (other SMs wrote it), eight loads in flight per thread
-  const uint64_t* src = p.cand + (size_t)row * kIdxCandCap;
-  uint32_t kmax = 0u;
-  for (uint32_t i0 = 0; i0 < count; i0 += 8u * NT) {
-    uint64_t c[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t i = i0 + (uint32_t)u * NT + tid;
-      c[u] = i < count ? __ldcg(src + i) : 0ull;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t i = i0 + (uint32_t)u * NT + tid;
-      if (i < count) {
-        cand_smem[i] = c[u];
-        kmax = max(kmax, (uint32_t)(c[u] >> 32));
-      }
-    }
-  }
-  kmax = __reduce_max_sync(kFull, kmax);
-  if (lane == 0) ctrl->wmax[warp] = kmax;
-  if (tid == 0) ctrl->thr_key = 0xffffffffu;
-  __syncthreads();
-  kmax = 0u;
-#pragma unroll
-  for (int w = 0; w < NT / 32; ++w) kmax = max(kmax, ctrl->wmax[w]);
-  // every candidate's key lies in [the guess's lowest admitted key, kmax]
-  const uint32_t lo = guess_low_key(gkey);
-  const uint32_t cap = kmax;
-  const int idx_bits = 32 - __clz(len - 1);
-  const DenseCands<NT> list{cand_smem, (int)count};
-  cta_finish<NT, DenseCands<NT>, true>(list, (uint32_t)kK, lo, cap, cap, false, idx_bits, hist, ctrl,
-                                       p.out_idx + (int64_t)row * kK, nullptr, 0u, (uint32_t)kK, 0, p.status, nullptr, count);
-  __syncthreads();
-  if (tid == 0) {
-    p.thr_out[row] = ctrl->thr_key != 0xffffffffu ? ctrl->thr_key : 0u;
-    p.select_rows[row] = 0u;
-  }
-}
-
 __device__ __forceinline__ int indexer_row_tiles(const IndexerParams& p, int row, int& len) {
   int64_t len64 = p.lengths[row];
   len64 = len64 < 0 ? 0 : (len64 > p.L ? p.L : len64);
@@ -292,15 +235,30 @@ __device__ __forceinline__ uint32_t indexer_row_guess(const IndexerParams& p, in
   return raw == 0u ? 0u : (raw > p.margin ? raw - p.margin : 1u);
 }
 
+// A warp's candidates on their way to the row's list, in shared memory: the 32 oldest leave together, so that the warp waits
+// for one slot-allocating atomic per 32 candidates (one for every 32 keys with a hit among them made
+// 64 ragged rows of fp8 keys wait 40 % of their time).
+constexpr int kIdxStash = 64;  // composites per warp: up to 31 that wait and 32 of one tile
+__device__ __forceinline__ void idx_flush(const IndexerParams& p, int row, uint32_t stash, uint32_t n) {  // n <= 32, by the whole warp
+  const int lane = lane_id();
+  __syncwarp();
+  uint32_t slot = 0u;
+  if (lane == 0) slot = atomicAdd(idx_row_count(p.cand, row), n);
+  slot = __shfl_sync(kFull, slot, 0) + (uint32_t)lane;
+  if ((uint32_t)lane < n && slot < (uint32_t)kIdxCandCap) idx_row_cand(p.cand, row)[slot] = lds64(stash + lane * 8);
+}
+
 // ---- epilogue of one segment (warps 2-9): one key per thread; group g of four warps serves every
 // second tile. (With two accumulators and one group the loop MMA -> full barrier -> TMEM loads ->
 // empty barrier -> next MMA into the same accumulator took ~1.1 us per pair of tiles: as long as
 // the key tiles' copies take in bf16, twice as long as they take in fp8.) Out of line: the 64
 // accumulator values of a key want the registers the kernel's segment bookkeeping would hold.
+// The weights lie in one of two places in turn: a warp may still be at work on the segment before.
 template <bool kFp8>
 __device__ __noinline__ void indexer_epilogue_segment(const IndexerParams& p, int row, int t_lo, int t_step, int n, int it_base,
                                                       uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty,
-                                                      volatile uint32_t* abort_flag, float* w_smem, const float* ks_smem) {
+                                                      volatile uint32_t* abort_flag, float* w_smem, const float* ks_smem,
+                                                      uint64_t* stash_smem) {
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int group = (warp - 2) >> 2;
@@ -308,6 +266,8 @@ __device__ __noinline__ void indexer_epilogue_segment(const IndexerParams& p, in
   const int key_in_tile = quarter * 32 + lane;
   const unsigned lt = (1u << lane) - 1u;
   const float4* w4 = reinterpret_cast<const float4*>(w_smem);
+  const uint32_t stash = smem_u32(stash_smem) + (uint32_t)(warp - 2) * kIdxStash * 8u;
+  uint32_t held = 0u;  // composites in it
   // the row's weights, among the epilogue warps only
   if (tid >= 64 && tid < 64 + kIdxHeads) w_smem[tid - 64] = __ldg(p.w + (int64_t)row * kIdxHeads + (tid - 64));
   int len;
@@ -315,7 +275,6 @@ __device__ __noinline__ void indexer_epilogue_segment(const IndexerParams& p, in
   const uint32_t guess = indexer_row_guess(p, row);
   const bool filter_mode = guess != 0u;
   const float edge = __uint_as_float(guess_edge_bits(guess));
-  if (tid == kIdxThreads - 1 && t_lo == 0 && !filter_mode) p.select_rows[row] = 1u;  // no guess to test: the selector takes the row
   asm volatile("bar.sync 1, 256;" ::: "memory");
   for (int i = ((it_base & 1) == group) ? 0 : 1; i < n; i += 2) {
     const int it = it_base + i;
@@ -364,24 +323,30 @@ __device__ __noinline__ void indexer_epilogue_segment(const IndexerParams& p, in
       const bool hit = valid && !(logit < edge);
       const unsigned b = __ballot_sync(kFull, hit);
       if (b) {
-        uint32_t slot = 0;
-        if (lane == 0) slot = atomicAdd(p.cand_count + row, (uint32_t)__popc(b));
-        slot = __shfl_sync(kFull, slot, 0) + (uint32_t)__popc(b & lt);
-        if (hit && slot < (uint32_t)kIdxCandCap)
-          p.cand[(size_t)row * kIdxCandCap + slot] =
-              ((uint64_t)fftopk_key_from_bits(__float_as_uint(logit)) << 32) | (uint64_t)(~(uint32_t)key);
+        if (hit)
+          sts64(stash + (held + (uint32_t)__popc(b & lt)) * 8u, ~(uint32_t)key, fftopk_key_from_bits(__float_as_uint(logit)));
+        held += (uint32_t)__popc(b);
+        if (held >= 32u) {
+          idx_flush(p, row, stash, 32u);
+          held -= 32u;
+          const uint64_t rest = lds64(stash + (32u + (uint32_t)lane) * 8u);
+          __syncwarp();
+          if ((uint32_t)lane < held) sts64(stash + (uint32_t)lane * 8u, (uint32_t)rest, (uint32_t)(rest >> 32));
+        }
       }
     }
   }
+  if (held) idx_flush(p, row, stash, held);
+  __syncwarp();  // (the next segment's first candidates go where these were)
 }
 
 // ---- producer --------------------------------------------------------------------------------------
 // Work split. The tiles of all rows, row after row, form one sequence; CTA c takes the c-th run of
 // `quota` consecutive tiles of it (quota = tiles / CTAs, rounded up), so every CTA streams the same
 // number of bytes whatever the rows' lengths are, and a run may cover the end of one row, several
-// whole rows and the start of another. The part of a run inside one row is a segment: the CTA
-// loads that row's q and weights, runs its pipeline over the segment's tiles, lets it drain and
-// counts the tiles off at the row's arrival counter. The row -> first-tile table is computed by
+// whole rows and the start of another. The part of a run inside one row is a segment: it has that row's q (one of
+// two places in shared memory in turn) and weights, and the pipeline runs on from one segment into the
+// next: no barrier of the CTA lies between them. The row -> first-tile table is computed by
 // every CTA for itself (a block scan over the lengths) and kept in shared memory, for batches of up
 // to kIdxBalancedRows rows; larger batches give every row one CTA.
 constexpr int kIdxBalancedRows = 1024;
@@ -391,8 +356,6 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
     indexer_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                           const __grid_constant__ IndexerParams p) {
   using F = IdxFmt<kFp8>;
-  static_assert((size_t)F::kStages * F::kTileBytes >= (size_t)kIdxCandCap * 8, "the stages hold a row's candidate list");
-  static_assert(F::kQBytes >= (uint32_t)kFinishBins * 4u, "q's place holds the finish's histogram");
   constexpr uint32_t kIdxTileBytes = F::kTileBytes;
   constexpr uint32_t kIdxQBytes = F::kQBytes;
   constexpr int kIdxStages = F::kStages;
@@ -400,21 +363,21 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
   // 1024-byte alignment for the swizzled tiles
   unsigned char* base = idx_smem_raw + ((1024u - (smem_u32(idx_smem_raw) & 1023u)) & 1023u);
   unsigned char* a_smem = base;                                   // kIdxStages x 32 KiB
-  unsigned char* q_smem = a_smem + (size_t)kIdxStages * kIdxTileBytes;  // 16 / 8 KiB
-  float* w_smem = reinterpret_cast<float*>(q_smem + kIdxQBytes);  // 64 floats
-  float* ks_smem = w_smem + kIdxHeads;                            // fp8: ring of per-tile key scales
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ks_smem + IdxScaleRing<kFp8>::kSlots * kIdxTile);
+  unsigned char* q_smem = a_smem + (size_t)kIdxStages * kIdxTileBytes;  // 2 x 16 / 8 KiB
+  float* w_smem = reinterpret_cast<float*>(q_smem + 2 * kIdxQBytes);  // 2 x 64 floats
+  float* ks_smem = w_smem + 2 * kIdxHeads;                        // fp8: ring of per-tile key scales
+  uint64_t* stash_smem = reinterpret_cast<uint64_t*>(ks_smem + IdxScaleRing<kFp8>::kSlots * kIdxTile);  // 8 warps' candidates
+  uint64_t* bars = stash_smem + 8 * kIdxStash;
   uint64_t* full = bars;                     // [kIdxStages]
   uint64_t* empty = bars + kIdxStages;       // [kIdxStages]
   uint64_t* tfull = bars + 2 * kIdxStages;   // [kIdxBufs]
   uint64_t* tempty = tfull + kIdxBufs;       // [kIdxBufs]
-  uint64_t* qfull = tempty + kIdxBufs;       // [1]
+  uint64_t* qfull = tempty + kIdxBufs;       // [2]
+  uint64_t* qempty = qfull + 2;              // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  uint32_t* last_flag = tmem_slot + 2;       // [2]: this CTA finishes the row; the row's candidate count
   uint32_t* scan_part = tmem_slot + 4;       // [12]: warp totals of the block scan
-  Ctrl* fin_ctrl = reinterpret_cast<Ctrl*>(tmem_slot + 16);
-  uint32_t* first_tile = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(fin_ctrl) + ((sizeof(Ctrl) + 15) & ~15u));
+  uint32_t* first_tile = tmem_slot + 16;
   // first_tile[r], r <= B: tiles of the rows before r (balanced mode only)
 
   const int tid = threadIdx.x;
@@ -434,7 +397,10 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
       mbar_init(&tfull[b], 1);
       mbar_init(&tempty[b], 128);
     }
-    mbar_init(qfull, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&qfull[i], 1);
+      mbar_init(&qempty[i], 1);
+    }
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -463,7 +429,6 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
     if (tid == 0) {
       first_tile[0] = 0u;
       first_tile[1] = total;
-      if (total == 0u && blockIdx.x == 0) p.select_rows[0] = 1u;
     }
     __syncthreads();
     const TileRun run = tile_run(total, gridDim.x, blockIdx.x);
@@ -478,7 +443,6 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
       const int r = tid * PER + j;
       int len_r;
       mine[j] = r < p.B ? (uint32_t)indexer_row_tiles(p, r, len_r) : 0u;
-      if (r < p.B && mine[j] == 0u && blockIdx.x == 0) p.select_rows[r] = 1u;  // no key at all: the selector pads the row
       sum += mine[j];
     }
     uint32_t incl = sum;
@@ -508,7 +472,6 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
     row = (int)blockIdx.x;
     int len_r;
     g1 = (uint32_t)indexer_row_tiles(p, row, len_r);
-    if (g1 == 0u && tid == 0) p.select_rows[row] = 1u;
     __syncthreads();
   }
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -539,18 +502,20 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
       t_lo = (int)blockIdx.x;
       t_step = (int)gridDim.x;
     }
-    // (No barrier of the whole CTA here: the barriers at the end of the segment before have ordered
-    // everything this one overwrites. And nothing in front of the role branches that waits for
-    // global memory: the threads that issue the copies and the MMAs start at once; the row's
-    // length and guess are read by the epilogue warps, and by everybody at the segment's end.)
+    // (Nothing in front of the role branches waits for global memory: the threads that issue the copies and
+    // the MMAs run ahead of the epilogue, which reads the row's length and guess.)
+    const int qs = seg_no & 1;
+    const uint32_t qph = (uint32_t)(seg_no >> 1) & 1u;
+    unsigned char* const q_now = q_smem + (size_t)qs * kIdxQBytes;
 
     if (warp == 0) {
       // ---- TMA producer ---------------------------------------------------------------------------
       if (lane == 0) {
-        mbar_expect_tx(qfull, kIdxQBytes);
+        if (!mbar_wait(&qempty[qs], qph ^ 1u, abort_flag)) break;  // (the MMAs of the segment before the last one have read it)
+        mbar_expect_tx(&qfull[qs], kIdxQBytes);
 #pragma unroll
         for (int bx = 0; bx < F::kBoxes; ++bx)
-          tma_load_2d(q_smem + (size_t)bx * (kIdxQBytes / F::kBoxes), &map_q, bx * F::kChunk, row * kIdxHeads, qfull);
+          tma_load_2d(q_now + (size_t)bx * (kIdxQBytes / F::kBoxes), &map_q, bx * F::kChunk, row * kIdxHeads, &qfull[qs]);
         for (int i = 0; i < n; ++i) {
           const int it = it_base + i;
           const int s = it % kIdxStages;
@@ -574,7 +539,7 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
     } else if (warp == 1) {
       // ---- MMA issuer -----------------------------------------------------------------------------
       if (lane == 0) {
-        bool ok = mbar_wait(qfull, (uint32_t)seg_no & 1u, abort_flag);
+        bool ok = mbar_wait(&qfull[qs], qph, abort_flag);
         for (int i = 0; ok && i < n; ++i) {
           const int it = it_base + i;
           const int s = it % kIdxStages;
@@ -585,7 +550,7 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
           if (!mbar_wait(&full[s], ph, abort_flag)) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = smem_u32(a_smem + (size_t)s * kIdxTileBytes);
-          const uint32_t b_addr = smem_u32(q_smem);
+          const uint32_t b_addr = smem_u32(q_now);
           const uint32_t d_tmem = tmem_base + (uint32_t)buf * kIdxHeads;
 #pragma unroll
           for (int kc = 0; kc < F::kBoxes; ++kc) {
@@ -600,60 +565,26 @@ __global__ void __launch_bounds__(kIdxThreads, FFTOPK_IDX_CTAS_PER_SM)
           umma_commit(&empty[s]);     // the stage may be refilled once these MMAs have read it
           umma_commit(&tfull[buf]);   // ... and the accumulator is complete
         }
+        umma_commit(&qempty[qs]);  // (q may be replaced once the segment's MMAs have read it)
       }
     } else {
       // ---- epilogue ---------------------------------------------------------------------------------
-      indexer_epilogue_segment<kFp8>(p, row, t_lo, t_step, n, it_base, tmem_base, tfull, tempty, abort_flag, w_smem, ks_smem);
+      indexer_epilogue_segment<kFp8>(p, row, t_lo, t_step, n, it_base, tmem_base, tfull, tempty, abort_flag, w_smem + qs * kIdxHeads,
+                                     ks_smem, stash_smem);
     }
-    // The idle lanes of the two single-thread warps wait here for their working lane: what follows
-    // (global loads, a fence) would otherwise run ahead on them and hold the warp's issue slot while
-    // the working lane has copies or MMAs to issue (measured: the first tile's MMAs 1.7 us late).
-    if (warp < 2) __syncwarp();
     it_base += n;
     ++seg_no;
-    int len;
-    indexer_row_tiles(p, row, len);
-    const uint32_t guess = indexer_row_guess(p, row);
-    const bool filter_mode = guess != 0u;
-    // ---- end of the segment: every tile has been through the epilogue, so every copy and MMA of
-    // the segment has completed; the CTA counts its tiles off and the row's last CTA finishes it ----
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (__syncthreads_or((int)*abort_flag)) break;  // (uniform)
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!filter_mode) continue;  // (uniform)
-    if (tid == 0) {
-      // Release: the barrier has ordered every thread's candidate stores before this fence, the
-      // fence orders them before the arrival (the pattern of a grid-wide barrier: one fence by
-      // the arriving thread instead of one per thread - 320 of them took 1.4 us).
-      __threadfence();
-      const bool last = atomicAdd(p.done_count + row, (uint32_t)n) + (uint32_t)n == (uint32_t)ntiles;
-      uint32_t count = 0u;
-      if (last) {
-        // every tile of the row has been counted off: nobody appends any more (each CTA's appends
-        // were performed before its arrival). Take the count and leave both counters at zero for
-        // the next call.
-        count = atomicExch(p.cand_count + row, 0u);
-        p.done_count[row] = 0u;
-        __threadfence();  // acquire: the other CTAs' candidates, before this CTA reads them (behind the barrier below)
-      }
-      last_flag[0] = last ? 1u : 0u;
-      last_flag[1] = count;
-    }
-    __syncthreads();
-    if (last_flag[0] != 0u) {  // (uniform)
-      // the stages hold the list, q's place the histogram
-      indexer_finish_row<kIdxThreads>(p, row, len, guess, last_flag[1], reinterpret_cast<uint64_t*>(a_smem),
-                                      reinterpret_cast<uint32_t*>(q_smem), fin_ctrl);
-      // the next segment's copies overwrite what the threads wrote there
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-    }
   }
+  // The idle lanes of the two single-thread warps wait here for their working lane (they would hold the warp's issue slot
+  // while it has copies or MMAs to issue). Every tile has been through the epilogue behind the barrier
+  // below, so every copy and MMA has completed.
+  if (warp < 2) __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
   // ---- wind down ---------------------------------------------------------------------------------
   if (*abort_flag) {
     // a wait ran out: give copies that may still be in flight a moment to land before the shared
-    // memory goes away. The rows of this call are not all finished and their counters not all back
-    // at zero: the caller sees the status bit and zero-fills the workspace again.
+    // memory goes away. Rows of this call lack logits and candidates: the caller sees the status bit.
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     do {
@@ -688,8 +619,8 @@ std::mutex g_encode_mu;
 constexpr size_t indexer_smem_bytes(bool fp8) {
   return 1024 +
          (fp8 ? (size_t)IdxFmt<true>::kStages * IdxFmt<true>::kTileBytes : (size_t)IdxFmt<false>::kStages * IdxFmt<false>::kTileBytes) +
-         (fp8 ? IdxFmt<true>::kQBytes : IdxFmt<false>::kQBytes) + kIdxHeads * 4 + (fp8 ? IdxScaleRing<true>::kSlots * kIdxScaleBytes : 0) +
-         32 * 8 + 64 + ((sizeof(Ctrl) + 15) & ~(size_t)15) +
+         2 * (fp8 ? IdxFmt<true>::kQBytes : IdxFmt<false>::kQBytes) + 2 * kIdxHeads * 4 +
+         (fp8 ? IdxScaleRing<true>::kSlots * kIdxScaleBytes : 0) + 8 * kIdxStash * 8 + 32 * 8 + 64 +
          (size_t)(kIdxBalancedRows + 1) * 4 + 16;
 }
 
@@ -734,22 +665,6 @@ int make_map(CUtensorMap* map, const void* ptr, bool fp8, uint64_t rows, uint64_
   return r == CUDA_SUCCESS ? 0 : FFTOPK_EINVAL;
 }
 
-// Workspace: [candidate lists: B x kIdxCandCap composites][candidate counts: B words][arrival
-// counts: B words][rows the selector takes: B words]
-struct IndexerLayout {
-  size_t cand_off, count_off, done_off, select_off, total;
-};
-IndexerLayout indexer_layout(int32_t B) {
-  IndexerLayout l;
-  const size_t words = ((size_t)B * 4 + 255) & ~(size_t)255;
-  l.cand_off = 0;
-  l.count_off = (size_t)B * kIdxCandCap * 8;
-  l.done_off = l.count_off + words;
-  l.select_off = l.done_off + words;
-  l.total = l.select_off + words;
-  return l;
-}
-
 template <bool kFp8>
 cudaError_t launch_producer(dim3 grid, cudaStream_t stream, const CUtensorMap& map_q, const CUtensorMap& map_k,
                             const IndexerParams& p) {
@@ -774,7 +689,7 @@ extern "C" {
 
 size_t fftopk_indexer_workspace_bytes(int32_t B) {
   if (B <= 0) return 0;
-  return indexer_layout(B).total;
+  return (size_t)B * kIdxRecordWords * 8;
 }
 
 static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64_t k_rows_per_seq, const float* k_scale,
@@ -788,8 +703,7 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
   if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache)) & 15u) != 0) return FFTOPK_EINVAL;
   if ((reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0) return FFTOPK_EINVAL;
   if (L > (int64_t)0x7fffffff - 256 || B > 65535 || (int64_t)B * k_rows_per_seq > (int64_t)0x7fffffff - 256) return FFTOPK_ERANGE;
-  const IndexerLayout lay = indexer_layout(B);
-  if (workspace_bytes < lay.total) return FFTOPK_EINVAL;
+  if (workspace_bytes < fftopk_indexer_workspace_bytes(B)) return FFTOPK_EINVAL;
   int rc = indexer_setup();
   if (rc) return rc;
   int dev = 0, sms = 0;
@@ -797,7 +711,6 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e);
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  char* ws = static_cast<char*>(d_workspace);
 
   CUtensorMap map_q, map_k;
   rc = make_map(&map_q, q, fp8, (uint64_t)B * kIdxHeads, kIdxDim, kIdxHeads);
@@ -819,12 +732,7 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
   p.logits_stride = logits_stride;
   p.guess = thresholds;
   p.margin = margin;
-  p.cand = reinterpret_cast<uint64_t*>(ws + lay.cand_off);
-  p.cand_count = reinterpret_cast<uint32_t*>(ws + lay.count_off);
-  p.done_count = reinterpret_cast<uint32_t*>(ws + lay.done_off);
-  p.select_rows = reinterpret_cast<uint32_t*>(ws + lay.select_off);
-  p.out_idx = out_idx;
-  p.thr_out = thresholds;
+  p.cand = static_cast<uint64_t*>(d_workspace);
   p.status = status;
 
   // batches of up to kIdxBalancedRows rows: as many CTAs as are resident at once, each with an equal
@@ -837,11 +745,10 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
     if (ctas < 1) ctas = 1;
   }
   const dim3 grid((unsigned)ctas, 1u, 1u);
-  // the producer: logits; rows with a guess are filtered as the logits are produced and finished
-  // by their last CTA
+  // the producer: logits; rows with a guess are filtered as the logits are produced
   e = fp8 ? launch_producer<true>(grid, stream, map_q, map_k, p) : launch_producer<false>(grid, stream, map_q, map_k, p);
   if (e != cudaSuccess) return cuda_fail(e);
-  // the selector on the logits of the rows without a usable guess; it hands back their thresholds
+  // the selector: rows whose guess held are finished on their candidates, the others selected on their logits
   SelectCall c;
   c.score = logits;
   c.row_stride = logits_stride;
@@ -852,7 +759,9 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
   c.status = status;
   c.cuda_stream = cuda_stream;
   c.next_threshold = thresholds;
-  c.only_rows = p.select_rows;
+  c.cand = p.cand;
+  c.cand_guess = thresholds;
+  c.warm_margin = margin;
   c.may_overlap = false;  // (a programmatic dependent of the producer that waits for it, like every default launch)
   return launch_select(c);
 }

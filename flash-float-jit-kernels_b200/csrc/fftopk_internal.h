@@ -42,7 +42,10 @@ struct SelectCall {
   const uint32_t* prev_threshold = nullptr;
   uint32_t* next_threshold = nullptr;
   uint32_t warm_margin = 0;
-  const uint32_t* only_rows = nullptr;  // with next_threshold: select only rows whose entry is non-zero
+  // fused indexer (with next_threshold): the candidates its producer has found with the guesses `cand_guess` less warm_margin,
+  // a record per row (idx_row_cand, idx_row_count); this launch sets the counts back to zero
+  uint64_t* cand = nullptr;
+  const uint32_t* cand_guess = nullptr;
   // false: this launch consumes what a kernel enqueued just before it by the library itself has
   // produced (gathered rows, widened scores, slice lengths, indexer logits), or hands its output to
   // a kernel the library enqueues right after it. Such a launch keeps stream order whatever
@@ -75,6 +78,17 @@ struct DeviceOnce {
 };
 
 constexpr int kMaxDevices = 64;
+
+// Candidates of a row of the fused indexer: a record of kIdxCandCap composites - 16 for each of 512 threads - and their
+// number. Where a row's record lies does not depend on the batch, so calls of different batches may share a workspace.
+constexpr int kIdxCandCap = 8192;
+constexpr size_t kIdxRecordWords = kIdxCandCap + 32;  // 64-bit words; the count has lines of its own
+#ifdef __CUDACC__
+__device__ __forceinline__ uint64_t* idx_row_cand(uint64_t* cand, int row) { return cand + (size_t)row * kIdxRecordWords; }
+__device__ __forceinline__ uint32_t* idx_row_count(uint64_t* cand, int row) {
+  return reinterpret_cast<uint32_t*>(idx_row_cand(cand, row) + kIdxCandCap);
+}
+#endif
 
 // Layout of a context-parallel comm buffer for up to b_cap rows, in 32-bit words (K = 2048):
 //   two-launch protocol (fftopk_select2048_cp / fftopk_merge2048_cp)

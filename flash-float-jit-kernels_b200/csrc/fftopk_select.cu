@@ -106,7 +106,9 @@ struct SelectParams {
   const uint32_t* prev_threshold;
   uint32_t* next_threshold;
   uint32_t warm_margin;
-  const uint32_t* only_rows;  // (warm-start kernel only) when set: rows with only_rows[row] == 0 are left alone
+  // (warm-start kernel only) fused indexer: a row whose guess cand_guess[row] held is finished on its candidates
+  uint64_t* cand;
+  const uint32_t* cand_guess;
 };
 
 
@@ -962,6 +964,78 @@ __device__ __forceinline__ const int32_t* row_page(const SelectParams& p, int ro
 __device__ __forceinline__ int32_t row_idx_offset(const SelectParams& p, int row) {
   return p.idx_offset + (p.row_offsets ? __ldg(p.row_offsets + row) : 0);
 }
+// A row of the fused indexer whose producer has filtered it with a guess: if the guess held - at least k candidates, no more
+// than the list has room for - the cluster's first CTA finishes it on them, keys in registers like a lone
+// CTA's. False: the row has to be selected on its logits. All CTAs of the cluster decide the same.
+template <int NT, bool kLone, class T>
+__device__ __forceinline__ bool finish_given_candidates(const SelectParams& p, const RowCtx<NT, T>& cx, int row, int len, uint32_t raw,
+                                                        uint32_t count) {
+  constexpr int R = kIdxCandCap / NT;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  cg::cluster_group cluster = cg::this_cluster();
+  if (raw == 0u) return false;  // (not filtered, nothing to set back)
+  const uint32_t gkey = raw > p.warm_margin ? raw - p.warm_margin : 1u;
+  const bool held = count >= cx.k && count <= (uint32_t)kIdxCandCap;
+  // everybody has read the count before the first CTA sets it back
+  if (!kLone) cluster.barrier_arrive();
+  if (held && cx.rank != 0) return true;
+  if (held) {
+    const uint32_t hist_s = smem_u32(cx.hist0);
+    const uint32_t lowkey = guess_low_key(gkey);
+    const uint32_t reach = 2u * min(p.warm_margin, 0x3fffffffu) + (1u << 19);
+    const uint32_t focus = lowkey > 0xffffffffu - reach ? 0xffffffffu : lowkey + reach;
+    // candidates [own * warp, ...) are this warp's
+    const int own = (int)(((count + NT - 1u) / NT) * 32u);
+    const uint64_t* const src = idx_row_cand(p.cand, row) + warp * own;
+    RegSegCands<NT, R> cands;
+    cands.seg = smem_u32(cx.list) + (uint32_t)(warp * own) * 4u;
+    cands.wn = max(0, min(own, (int)count - warp * own));
+    cands.spill = 0u;
+    cands.sn = 0;
+    uint32_t inv[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      cands.key[i] = inv[i] = 0u;
+      if (i * 32 + lane < cands.wn) {
+        const uint2 c = __ldcg(reinterpret_cast<const uint2*>(src) + i * 32 + lane);
+        inv[i] = c.x;
+        cands.key[i] = c.y;
+      }
+    }
+    for (int i = tid; i < kFinishBins / 4; i += NT) sts_zero16(hist_s + i * 16);
+    if (tid == 0) cx.ctrl->thr_key = 0xffffffffu;
+    __syncthreads();
+    const KeyDigit dg = make_key_digit(lowkey, focus);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (i * 32 + lane < cands.wn) {
+        sts32(cands.seg + (uint32_t)(i * 32 + lane) * 4u, ~inv[i]);
+        red_shared_inc(hist_s + dg.of(cands.key[i]) * 4u);
+      }
+    }
+    __syncthreads();
+    const RowOutput ro = row_output(p, row, cx.k);
+    const FinishOut o{cx.ctrl, ro.idx, ro.key, p.status, nullptr, 0u, cx.k, p.idx_offset};
+    lone_finish<NT, R, true>(cands, o, cx.k, lowkey, focus, 32 - __clz(len - 1), cx.hist0, count);
+    __syncthreads();
+  }
+  if (!kLone) {
+    cluster.barrier_wait();
+  } else {
+    __syncthreads();
+  }
+  if (tid == 0 && cx.rank == 0) {
+    *idx_row_count(p.cand, row) = 0u;
+    if (held) {
+      p.next_threshold[row] = cx.ctrl->thr_key != 0xffffffffu ? cx.ctrl->thr_key : 0u;
+    } else if (p.status) {
+      atomicOr(p.status, (uint32_t)FFTOPK_ST_GUESS_MISSED);
+    }
+  }
+  return held;
+}
+
 // kAnyK = false: k is the constant 2048 of the reference's op (the compiler folds it: one register
 // less in a kernel that sits at its register limit); true: k comes from the parameters.
 template <int NT, bool kAnyK, bool kWarm, class T, int kForm>
@@ -983,9 +1057,6 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   // the next call then fills the SMs that short rows free early.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (!p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
-  if constexpr (kWarm) {
-    if (p.only_rows != nullptr && p.only_rows[row] == 0u) return;  // (uniform over the cluster)
-  }
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32;
@@ -996,6 +1067,13 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   len64 = len64 < 0 ? 0 : len64;
   len64 = len64 > p.L - row_start ? p.L - row_start : len64;
   const int len = (int)len64;
+  uint32_t given_guess = 0u, given_count = 0u;  // (fused indexer; on their way together with the length)
+  if constexpr (kWarm) {
+    if (p.cand != nullptr) {
+      given_guess = __ldcg(p.cand_guess + row);
+      given_count = __ldcg(idx_row_count(p.cand, row));
+    }
+  }
   const T* rowp = static_cast<const T*>(p.score) + (int64_t)row * p.row_stride + row_start;
   const uint32_t K = cx.k = kAnyK ? (uint32_t)p.k : (uint32_t)kK;
   cx.cand_cap = p.cand_cap;
@@ -1015,6 +1093,10 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       }
       if constexpr (kWarm) {
         if (tid == 0 && p.next_threshold) p.next_threshold[row] = 0u;  // nothing to guess for such a row
+        if (tid == 0 && p.cand) {
+          *idx_row_count(p.cand, row) = 0u;
+          if (given_guess != 0u && len > 0 && p.status) atomicOr(p.status, (uint32_t)FFTOPK_ST_GUESS_MISSED);
+        }
       }
     }
     return;  // uniform over the cluster; no shared memory of this CTA is ever read by a peer
@@ -1060,6 +1142,11 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   smp.gu = !kLone && len <= 32768 && smp.gi > NT * G * smp.nb ? G / 2 : G;
   smp.whole = smp.gi <= smp.granules();
   smp.off = (uint32_t)(reinterpret_cast<uintptr_t>(sh.gbase + 4 * smp.i0) / (4 * sizeof(T))) & (uint32_t)(kSamplePiece - 1);
+
+  // ---- fused indexer: the row's candidates are there already ----------------------------------------
+  if constexpr (kWarm && NT >= 512) {
+    if (finish_given_candidates<NT, kLone>(p, cx, row, len, given_guess, given_count)) return;  // (uniform over the cluster)
+  }
 
   // ---- warm start: a key guess of the row's k-th largest element from an earlier call ----------
   // With a guess the row skips the sample, its histogram and the search: it is filtered at once
@@ -1846,8 +1933,11 @@ int launch_select(const SelectCall& c) {
   p.prev_threshold = c.prev_threshold;
   p.next_threshold = c.next_threshold;
   p.warm_margin = c.warm_margin;
-  p.only_rows = c.only_rows;
+  p.cand = c.cand;
+  p.cand_guess = c.cand_guess;
   if (warm && (c.k != kK || pl.threads < 512)) return FFTOPK_EINVAL;
+  // (the indices of a row's given candidates lie where the list does)
+  if (c.cand) pl.smem_bytes = std::max(pl.smem_bytes, (int)fixed_smem_bytes(false) + (kIdxCandCap + pl.threads) * 4);
   if ((size_t)pl.smem_bytes > (size_t)d->smem_optin) return FFTOPK_ERANGE;
 
   cudaLaunchConfig_t cfg = {};

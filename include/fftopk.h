@@ -312,11 +312,10 @@ int fftopk_select2048_host(const float* h_score, int64_t h_row_stride, int32_t B
  * row; for a row with a threshold guess (thresholds[b] != 0: what an earlier call handed back) every
  * logit is compared with the guess as it leaves the tensor core and the few that pass are kept as
  * candidates - the logit matrix is written (4 bytes per key beside the 256 read) but not read again -
- * and the last CTA of the row to finish selects the exact top 2048 of the candidates. Rows without
+ * and the second launch, a programmatic dependent, selects the exact top 2048 of the candidates. Rows without
  * a guess, and rows whose guess did not hold (fewer than 2048 admitted, or more than the 8,192-entry
  * candidate list takes; status bit FFTOPK_ST_GUESS_MISSED), go through the selector of
- * fftopk_select2048 on `logits` (a second launch, enqueued as a programmatic dependent, that costs
- * rows in no need of it an empty CTA). Either way out_idx holds the exact top 2048 OF THE LOGITS THE KERNEL COMPUTED
+ * fftopk_select2048 on `logits` in that launch. Either way out_idx holds the exact top 2048 OF THE LOGITS THE KERNEL COMPUTED
  * (fp32 accumulation on the tensor cores; ties to the lower index) and thresholds[b] the key of the
  * row's 2048-th largest logit for the next call.
  *   q            device, bf16 [B, 64, 128], 16-byte aligned

@@ -272,3 +272,39 @@ def test_fp8_operands(B, L, with_scale):
         orc.check_result(logits_np, ln.numpy(), out.cpu().numpy(), what=f"fp8 warm {rep}")
     assert np.array_equal(f.thresholds.cpu().numpy().view(np.uint32)[:B], kth_keys(logits_np, ln.numpy()))
     assert kernel_status(DEV) == 0
+
+
+def test_batches_of_different_sizes_share_an_object():
+    """A row's candidates lie in the same place whatever the batch: calls with fewer rows between calls with more."""
+    B, L = 6, 9000
+    q, k, w = make(B, L, seed=77)
+    ln = torch.full((B,), L, dtype=torch.int32, device=DEV)
+    f = FusedIndexerTopk(B, L)
+    f(q, k, w, ln)
+    for n in (6, 2, 5, 1, 6, 3):
+        _status_word(DEV).zero_()
+        out = f(q[:n].contiguous(), k[:n].contiguous(), w[:n].contiguous(), ln[:n].contiguous(), margin=1 << 16)
+        torch.cuda.synchronize()
+        assert kernel_status() == 0  # (every guess held)
+        orc.check_result(f.logits[:n, :L].cpu().numpy(), ln[:n].cpu().numpy(), out.cpu().numpy(), what=f"{n} rows")
+
+
+@pytest.mark.parametrize("B,L", [(1, 30000), (80, 9000), (150, 5000)])  # clusters, a CTA of 1024 threads, one of 512
+def test_candidate_lists_of_every_length(B, L):
+    """From the 2048 winners alone to lists that overflow: the number of candidates grows with the margin."""
+    q, k, w = make(B, L, seed=B + L)
+    ln = torch.full((B,), L, dtype=torch.int32, device=DEV)
+    f = FusedIndexerTopk(B, L)
+    f(q, k, w, ln)
+    torch.cuda.synchronize()
+    exact = torch.from_numpy(kth_keys(f.logits[:B, :L].cpu().numpy(), ln.cpu().numpy()).view(np.int32)).to(DEV)
+    for margin in (0, 1 << 12, 1 << 18, 1 << 20, 1 << 21, 1 << 23, (1 << 32) - 1):
+        f.thresholds[:B] = exact  # (what a cold call hands back may be a lower bound)
+        _status_word(DEV).zero_()
+        out = f(q, k, w, ln, margin=margin)
+        torch.cuda.synchronize()
+        if margin <= 1 << 18:
+            assert kernel_status() == 0
+        orc.check_result(f.logits[:B, :L].cpu().numpy(), ln.cpu().numpy(), out.cpu().numpy(), what=f"margin {margin}")
+        if kernel_status() == 0:
+            assert torch.equal(f.thresholds[:B], exact)
