@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from . import _native
-from .topk_indexer import TOPK, _after_launch, _status_word
+from .topk_indexer import TOPK, _launch
 
 HEADS, DIM = 64, 128
 
@@ -47,10 +47,10 @@ class FusedIndexerTopk:
         fp8 = k_cache.dtype == torch.float8_e4m3fn
         if q.dtype != k_cache.dtype or k_cache.dtype not in (torch.bfloat16, torch.float8_e4m3fn) or w.dtype != torch.float32:
             raise RuntimeError("q and k_cache must both be bfloat16 or both float8_e4m3fn, w float32")
-        if k_scale is not None and (not fp8 or k_scale.dtype != torch.float32 or tuple(k_scale.shape) != (B, Lk)
+        if k_scale is not None and (not fp8 or k_scale.dtype != torch.float32 or k_scale.shape != (B, Lk)
                                     or not k_scale.is_contiguous()):
             raise RuntimeError("k_scale goes with fp8 operands: a contiguous float32 tensor of shape [B, L]")
-        if tuple(q.shape) != (B, HEADS, DIM) or k_cache.size(2) != DIM or tuple(w.shape) != (B, HEADS):
+        if q.shape != (B, HEADS, DIM) or k_cache.size(2) != DIM or w.shape != (B, HEADS):
             raise RuntimeError("expected q [B, 64, 128], k_cache [B, L, 128], w [B, 64]")
         if not (q.is_contiguous() and k_cache.is_contiguous() and w.is_contiguous() and lengths.is_contiguous()):
             raise RuntimeError("q, k_cache, w and lengths must be contiguous")
@@ -63,15 +63,13 @@ class FusedIndexerTopk:
         if B == 0:
             return out
         lib = _native.lib()
-        with torch.cuda.device(self.device):
-            tail = (B, Lk, lengths.data_ptr(), self.thresholds.data_ptr(), int(margin), self.logits.data_ptr(), self.l_cap,
-                    out.data_ptr(), self._ws_ptr, self._ws_bytes, _status_word(self.device).data_ptr(),
-                    torch.cuda.current_stream().cuda_stream)
-            if fp8:
-                rc = lib.fftopk_indexer_topk2048_fp8(q.data_ptr(), k_cache.data_ptr(), Lk,
-                                                     None if k_scale is None else k_scale.data_ptr(), Lk, w.data_ptr(), *tail)
-            else:
-                rc = lib.fftopk_indexer_topk2048(q.data_ptr(), k_cache.data_ptr(), Lk, w.data_ptr(), *tail)
-        _native.check(rc, "fftopk_indexer_topk2048")
-        _after_launch(self.device, "fftopk_indexer_topk2048")
+        tail = (B, Lk, lengths.data_ptr(), self.thresholds.data_ptr(), int(margin), self.logits.data_ptr(), self.l_cap,
+                out.data_ptr(), self._ws_ptr, self._ws_bytes)
+        idx = self.thresholds.get_device()
+        if fp8:
+            _launch(lib.fftopk_indexer_topk2048_fp8, "fftopk_indexer_topk2048", idx, q.data_ptr(), k_cache.data_ptr(), Lk,
+                    None if k_scale is None else k_scale.data_ptr(), Lk, w.data_ptr(), *tail)
+        else:
+            _launch(lib.fftopk_indexer_topk2048, "fftopk_indexer_topk2048", idx, q.data_ptr(), k_cache.data_ptr(), Lk, w.data_ptr(),
+                    *tail)
         return out

@@ -48,33 +48,68 @@ def _after_launch(device: torch.device, what: str) -> None:
             raise _native.FFTopkError(f"{what}: the kernels reported status {st:#x} (FFTOPK_ST_* bits, include/fftopk.h)")
 
 
-def _check_inputs(score, lengths, row_starts, out=None):
+# An eager call's host time is the pass's time where batches are small (the kernel of one row of 16K logits takes 9 us), and
+# most of it was Python: two rounds of checks, device objects compared with each other, a device context
+# entered and left, a stream object. Tensor.get_device() is a plain integer (-1 off the GPU), the context is entered only where
+# the current device is another one, and the stream handle is asked for by itself.
+_current_device = torch._C._cuda_getDevice
+_current_stream = torch._C._cuda_getCurrentRawStream
+_status_ptrs: dict[int, int] = {}
+
+
+def _status_ptr(idx: int) -> int:
+    ptr = _status_ptrs.get(idx)
+    if ptr is None:
+        ptr = _status_ptrs[idx] = _status_word(torch.device("cuda", idx)).data_ptr()
+    return ptr
+
+
+def _launch(fn, what: str, idx: int, *args) -> None:
+    """fn(*args, status word, current stream) of the C library on device `idx`."""
+    if _current_device() == idx:
+        rc = fn(*args, _status_ptr(idx), _current_stream(idx))
+    else:
+        with torch.cuda.device(idx):
+            rc = fn(*args, _status_ptr(idx), _current_stream(idx))
+    if rc != 0:
+        _native.check(rc, what)
+    if CHECK_STATUS:
+        _after_launch(torch.device("cuda", idx), what)
+
+
+def _row_stride(score: torch.Tensor, B: int) -> int:
+    stride = score.stride(0)
+    return stride if B > 1 else max(stride, 0)
+
+
+def _check_inputs(score, lengths, row_starts, out=None) -> int:
     # reference: CHECK_CUDA + get_params (topk_indexer_radix.cu:997-1027, 1049-1062) raise
-    # c10::Error, which Python sees as RuntimeError.
+    # c10::Error, which Python sees as RuntimeError. Returns score's device index.
     if not score.is_cuda:
         raise RuntimeError("score must be a CUDA tensor")
     if score.dtype != torch.float32:
         raise RuntimeError("score must be float32")
-    if score.stride(1) != 1 and score.size(1) > 1:
+    B, L = score.shape
+    if score.stride(1) != 1 and L > 1:
         raise RuntimeError("score must have unit inner stride")
-    B = score.size(0)
+    idx = score.get_device()
     if not lengths.is_cuda or lengths.dtype != torch.int32:
         raise RuntimeError("lengths must be a CUDA int32 tensor")
-    if lengths.dim() != 1 or lengths.size(0) != B or not lengths.is_contiguous():
+    if lengths.shape != (B,) or not lengths.is_contiguous():
         raise RuntimeError("lengths must be a contiguous 1-D tensor of size B")
     if row_starts is not None:
         if not row_starts.is_cuda or row_starts.dtype != torch.int32:
             raise RuntimeError("row_starts must be a CUDA int32 tensor")
-        if row_starts.dim() != 1 or row_starts.size(0) != B or not row_starts.is_contiguous():
+        if row_starts.shape != (B,) or not row_starts.is_contiguous():
             raise RuntimeError("row_starts must be a contiguous 1-D tensor of size B")
-        if row_starts.device != score.device:
+        if row_starts.get_device() != idx:
             raise RuntimeError("row_starts must be on score's device")
-    if lengths.device != score.device:
+    if lengths.get_device() != idx:
         raise RuntimeError("lengths must be on score's device")
     if out is not None:
-        if out.dtype != torch.int32 or out.dim() != 2 or out.size(0) != B or out.size(1) != TOPK \
-                or not out.is_contiguous() or out.device != score.device:
+        if out.dtype != torch.int32 or out.shape != (B, TOPK) or not out.is_contiguous() or out.get_device() != idx:
             raise RuntimeError("indices must be a contiguous CUDA int32 tensor of shape [B, 2048]")
+    return idx
 
 
 def fast_topk(score: torch.Tensor, indices: torch.Tensor, lengths: torch.Tensor,
@@ -88,20 +123,17 @@ def fast_topk(score: torch.Tensor, indices: torch.Tensor, lengths: torch.Tensor,
     `idx_offset` is added to every index. Both exist for the context-parallel mode.
     """
     assert score.dim() == 2
-    _check_inputs(score, lengths, row_starts, indices)
-    B, L = score.size(0), score.size(1)
+    idx = _check_inputs(score, lengths, row_starts, indices)
+    _select2048(score, indices, lengths, row_starts, keys, int(idx_offset), idx)
+
+
+def _select2048(score, indices, lengths, row_starts, keys, idx_offset: int, idx: int) -> None:
+    B, L = score.shape
     if B == 0:
         return
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.fftopk_select2048(
-            score.data_ptr(), score.stride(0) if B > 1 else max(score.stride(0), 0), B, L,
-            lengths.data_ptr(), row_starts.data_ptr() if row_starts is not None else None,
-            indices.data_ptr(), keys.data_ptr() if keys is not None else None, int(idx_offset),
-            _status_word(score.device).data_ptr(), stream)
-    _native.check(rc, "fftopk_select2048")
-    _after_launch(score.device, "fftopk_select2048")
+    _launch(_native.lib().fftopk_select2048, "fftopk_select2048", idx, score.data_ptr(), _row_stride(score, B), B, L,
+            lengths.data_ptr(), None if row_starts is None else row_starts.data_ptr(), indices.data_ptr(),
+            None if keys is None else keys.data_ptr(), idx_offset)
 
 
 def fast_topk_v3(
@@ -128,9 +160,9 @@ def fast_topk_v3(
         topk == 2048
     ), "fast_topk_v3 only supports topk=2048 (the DeepSeek v3.2 indexer configuration)"
     assert score.dim() == 2
-    _check_inputs(score, lengths, row_starts)
+    idx = _check_inputs(score, lengths, row_starts)
     topk_indices = torch.empty((score.size(0), topk), dtype=torch.int32, device=score.device)
-    fast_topk(score, topk_indices, lengths, row_starts)
+    _select2048(score, topk_indices, lengths, row_starts, None, 0, idx)
     return topk_indices
 
 
@@ -153,10 +185,10 @@ def fast_topk_v3_warm(
     """
     assert topk == 2048, "fast_topk_v3_warm only supports topk=2048"
     assert score.dim() == 2
-    _check_inputs(score, lengths, row_starts, out)
-    B = score.size(0)
+    idx = _check_inputs(score, lengths, row_starts, out)
+    B, L = score.shape
     if not thresholds.is_cuda or thresholds.dtype != torch.int32 or thresholds.dim() != 1 or thresholds.size(0) != B \
-            or not thresholds.is_contiguous() or thresholds.device != score.device:
+            or not thresholds.is_contiguous() or thresholds.get_device() != idx:
         raise RuntimeError("thresholds must be a contiguous CUDA int32 tensor of shape (B) on score's device")
     if not (0 <= int(margin) < (1 << 32)):
         raise ValueError("margin must fit 32 bits")
@@ -164,15 +196,9 @@ def fast_topk_v3_warm(
         out = torch.empty((B, topk), dtype=torch.int32, device=score.device)
     if B == 0:
         return out
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        rc = lib.fftopk_select2048_warm(
-            score.data_ptr(), score.stride(0) if B > 1 else max(score.stride(0), 0), B, score.size(1),
-            lengths.data_ptr(), row_starts.data_ptr() if row_starts is not None else None,
-            thresholds.data_ptr(), int(margin), thresholds.data_ptr(), out.data_ptr(),
-            _status_word(score.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
-    _native.check(rc, "fftopk_select2048_warm")
-    _after_launch(score.device, "fftopk_select2048_warm")
+    thr = thresholds.data_ptr()
+    _launch(_native.lib().fftopk_select2048_warm, "fftopk_select2048_warm", idx, score.data_ptr(), _row_stride(score, B), B, L,
+            lengths.data_ptr(), None if row_starts is None else row_starts.data_ptr(), thr, int(margin), thr, out.data_ptr())
     return out
 
 
@@ -189,19 +215,13 @@ def fast_topk_general(
     assert score.dim() == 2
     if score.is_cuda and score.dtype in (torch.float16, torch.bfloat16):
         return _fast_topk_16bit(score, lengths, int(topk), row_starts)
-    _check_inputs(score, lengths, row_starts)
-    out = torch.empty((score.size(0), int(topk)), dtype=torch.int32, device=score.device)
-    if score.size(0) == 0:
+    idx = _check_inputs(score, lengths, row_starts)
+    B, L = score.shape
+    out = torch.empty((B, int(topk)), dtype=torch.int32, device=score.device)
+    if B == 0:
         return out
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        stream = torch.cuda.current_stream(score.device)
-        rc = lib.fftopk_select_topk(score.data_ptr(), score.stride(0) if score.size(0) > 1 else max(score.stride(0), 0),
-                                    score.size(0), score.size(1), lengths.data_ptr(),
-                                    None if row_starts is None else row_starts.data_ptr(), int(topk), out.data_ptr(),
-                                    None, 0, _status_word(score.device).data_ptr(), stream.cuda_stream)
-    _native.check(rc, "fftopk_select_topk")
-    _after_launch(score.device, "fftopk_select_topk")
+    _launch(_native.lib().fftopk_select_topk, "fftopk_select_topk", idx, score.data_ptr(), _row_stride(score, B), B, L,
+            lengths.data_ptr(), None if row_starts is None else row_starts.data_ptr(), int(topk), out.data_ptr(), None, 0)
     return out
 
 
@@ -219,15 +239,9 @@ def _fast_topk_16bit(score, lengths, topk, row_starts):
     out = torch.empty((B, topk), dtype=torch.int32, device=score.device)
     if B == 0:
         return out
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        stream = torch.cuda.current_stream(score.device)
-        rc = lib.fftopk_select_topk_16bit(score.data_ptr(), 0 if score.dtype == torch.float16 else 1,
-                                          score.stride(0) if B > 1 else max(score.stride(0), 0), B, L, lengths.data_ptr(),
-                                          None if row_starts is None else row_starts.data_ptr(), topk, out.data_ptr(),
-                                          None, 0, _status_word(score.device).data_ptr(), stream.cuda_stream)
-    _native.check(rc, "fftopk_select_topk_16bit")
-    _after_launch(score.device, "fftopk_select_topk_16bit")
+    _launch(_native.lib().fftopk_select_topk_16bit, "fftopk_select_topk_16bit", score.get_device(), score.data_ptr(),
+            0 if score.dtype == torch.float16 else 1, _row_stride(score, B), B, L, lengths.data_ptr(),
+            None if row_starts is None else row_starts.data_ptr(), topk, out.data_ptr(), None, 0)
     return out
 
 
@@ -276,13 +290,8 @@ def fast_topk_v3_host(
         ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=dev)
         _host_workspaces[(dev, B, L)] = ws
     base = (ws.data_ptr() + 255) & ~255
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev)
-        _native.check(
-            lib.fftopk_select2048_host(score.data_ptr(), score.stride(0) if B > 1 else L, B, L, lengths.data_ptr(),
-                                       out.data_ptr(), base, nbytes, _status_word(dev).data_ptr(), stream.cuda_stream),
-            "fftopk_select2048_host")
-    _after_launch(dev, "fftopk_select2048_host")
+    _launch(lib.fftopk_select2048_host, "fftopk_select2048_host", ws.get_device(), score.data_ptr(),
+            score.stride(0) if B > 1 else L, B, L, lengths.data_ptr(), out.data_ptr(), base, nbytes)
     return out
 
 
@@ -305,7 +314,7 @@ def fast_topk_transform_fused(
     """
     assert topk == TOPK, "only topk=2048 is supported"
     assert score.dim() == 2
-    _check_inputs(score, lengths, row_starts)
+    idx = _check_inputs(score, lengths, row_starts)
     B = score.size(0)
     if not page_table_size_1.is_cuda or page_table_size_1.dtype != torch.int32 or page_table_size_1.dim() != 2 \
             or (page_table_size_1.stride(1) != 1 and page_table_size_1.size(1) > 1):
@@ -320,16 +329,9 @@ def fast_topk_transform_fused(
     if B == 0:
         return dst
     is_decode = row_starts is None and prefill_bs == B  # reference: radix.cu:1196
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        rc = lib.fftopk_select2048_page_table(
-            score.data_ptr(), score.stride(0), B, score.size(1), lengths.data_ptr(),
-            row_starts.data_ptr() if row_starts is not None else None, dst.data_ptr(),
-            page_table_size_1.data_ptr(), page_table_size_1.stride(0),
-            None if is_decode else cu_seqlens_q.data_ptr(), prefill_bs,
-            _status_word(score.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
-    _native.check(rc, "fftopk_select2048_page_table")
-    _after_launch(score.device, "fftopk_select2048_page_table")
+    _launch(_native.lib().fftopk_select2048_page_table, "fftopk_select2048_page_table", idx, score.data_ptr(), score.stride(0), B,
+            score.size(1), lengths.data_ptr(), None if row_starts is None else row_starts.data_ptr(), dst.data_ptr(),
+            page_table_size_1.data_ptr(), page_table_size_1.stride(0), None if is_decode else cu_seqlens_q.data_ptr(), prefill_bs)
     return dst
 
 
@@ -347,7 +349,7 @@ def fast_topk_transform_ragged_fused(
     """
     assert topk == TOPK, "only topk=2048 is supported"
     assert score.dim() == 2
-    _check_inputs(score, lengths, row_starts)
+    idx = _check_inputs(score, lengths, row_starts)
     B = score.size(0)
     if not topk_indices_offset.is_cuda or topk_indices_offset.dtype != torch.int32 \
             or topk_indices_offset.dim() != 1 or topk_indices_offset.size(0) != B \
@@ -356,13 +358,7 @@ def fast_topk_transform_ragged_fused(
     out = torch.empty((B, TOPK), dtype=torch.int32, device=score.device)
     if B == 0:
         return out
-    lib = _native.lib()
-    with torch.cuda.device(score.device):
-        rc = lib.fftopk_select2048_ragged(
-            score.data_ptr(), score.stride(0), B, score.size(1), lengths.data_ptr(),
-            row_starts.data_ptr() if row_starts is not None else None, out.data_ptr(),
-            topk_indices_offset.data_ptr(), _status_word(score.device).data_ptr(),
-            torch.cuda.current_stream().cuda_stream)
-    _native.check(rc, "fftopk_select2048_ragged")
-    _after_launch(score.device, "fftopk_select2048_ragged")
+    _launch(_native.lib().fftopk_select2048_ragged, "fftopk_select2048_ragged", idx, score.data_ptr(), score.stride(0), B,
+            score.size(1), lengths.data_ptr(), None if row_starts is None else row_starts.data_ptr(), out.data_ptr(),
+            topk_indices_offset.data_ptr())
     return out
