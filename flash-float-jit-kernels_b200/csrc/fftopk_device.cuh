@@ -181,6 +181,22 @@ __device__ __forceinline__ uint64_t lds64_below(int i, int n, uint32_t a) {
   return v;
 }
 
+// What a kernel may do with its inputs before the kernel in front of it on the stream has completed: ask for them to be
+// brought into L2, which is coherent, so that whatever that kernel still writes is what is read later. `hint_s32`: a
+// value that may be about to change, good for nothing but the size of such a request.
+__device__ __forceinline__ int32_t hint_s32(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// part i of n of the `bytes` bytes at p
+__device__ __forceinline__ void prefetch_part_l2(const void* p, int64_t bytes, int i, int n) {
+  const int64_t part = bytes / n;
+  const uintptr_t from = (reinterpret_cast<uintptr_t>(p) + (uintptr_t)(part * i) + 15u) & ~(uintptr_t)15u;
+  const uint32_t size = (uint32_t)(part > 16 ? part - 15 : 0) & ~15u;
+  if (size != 0u) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(size) : "memory");
+}
+
 // Histogram update: a plain shared-memory reduction (no result). Measured on B200 (64K updates
 // per CTA, 1024 threads): 6 to 12 updates per clock per SM whatever the bin distribution,
 // all-equal bins included - the hardware combines same-address updates, and ballot / match.any
