@@ -213,26 +213,22 @@ FFTOPK_DECIDE_HD int gather_region(int cand_cap, int list_cap, int ctas) {
   const int room = (cand_cap - list_cap - list_cap / 3) / (ctas > 1 ? ctas - 1 : 1);
   return room < 0 ? 0 : (most < room ? most : room) & ~15;  // (whole 128-byte lines: 3 % of a call at k = 4096, 1M)
 }
-// ... and of a CTA's list: the warps' segments, and an area behind them for what a warp's segment does not
+// ... and of the list of a cluster's CTA: the warps' segments, and an area behind them for what a warp's segment does not
 // hold. Where all candidates of a row may lie in one CTA's shard, a few thousand consecutive elements fall
 // on the warps unevenly: a quarter of a short list (the throughput plan's), else an eighth. (A quarter of
 // a long one as well cost 64 rows with 6,500 copies of the threshold 26.3 us instead of 24.4.)
-FFTOPK_DECIDE_HD int list_spill(int list_cap, bool lone) { return list_cap / (lone || list_cap >= 4096 ? 8 : 4); }
+FFTOPK_DECIDE_HD int list_spill(int list_cap) { return list_cap / (list_cap >= 4096 ? 8 : 4); }
 
-// A lone CTA's segments hold row indices (words, in the memory of list_cap composites less the spill area), and the finish
-// has their keys in registers: so many per thread, and no more candidates per warp than that.
+// A lone CTA's segments hold row indices (words, in the memory of list_cap composites), and the finish has their keys in
+// registers: so many per thread, and no more candidates per warp than that. (No spill area: with 512 slots for each of 16
+// warps a row overflows with its 8,193rd candidate or so, and then goes through full histograms.)
 FFTOPK_DECIDE_HD constexpr int lone_regs(int threads) { return threads >= 1024 ? 8 : 16; }
 FFTOPK_DECIDE_HD int lone_segment(int list_cap, int threads) {
-  const int own = 2 * (list_cap - list_spill(list_cap, true)) / (threads / 32);
+  const int own = 2 * list_cap / (threads / 32);
   return own < 32 * lone_regs(threads) ? own : 32 * lone_regs(threads);
 }
-// ... the whole list in bytes (composites of the spill area behind the segments), and in candidates
-FFTOPK_DECIDE_HD int lone_list_bytes(int list_cap, int threads) {
-  return ((threads / 32 * lone_segment(list_cap, threads) + 1) / 2 + list_spill(list_cap, true)) * 8;
-}
-FFTOPK_DECIDE_HD int lone_room(int list_cap, int threads) {
-  return threads / 32 * lone_segment(list_cap, threads) + list_spill(list_cap, true);
-}
+// ... the whole list in candidates (words)
+FFTOPK_DECIDE_HD int lone_room(int list_cap, int threads) { return threads / 32 * lone_segment(list_cap, threads); }
 
 // ---------------------------------------------------------------------------------------------
 // Digit rule of a finish round over a field's range [lo, cap]: digit(v) = min((v - lo) >>

@@ -585,44 +585,12 @@ struct DenseCands {
 
 // What the filter of a lone CTA leaves behind: per warp up to 32 * R candidates, their keys in registers (candidate j
 // of the warp in key[j / 32] of lane j % 32; 0 where there is none) and their indices in a dense segment in shared
-// memory (`wn` of them, the same in all lanes), plus the shared spill area of `sn` composites.
+// memory (`wn` of them, the same in all lanes).
 template <int NT, int R>
 struct RegSegCands {
   uint32_t key[R];
   uint32_t seg;  // shared address of this warp's indices
   int wn;
-  uint32_t spill;
-  int sn;
-  template <class F>
-  __device__ __forceinline__ void for_each(F&& f) const {
-    static_assert(R % kWalk == 0, "");
-#pragma unroll
-    for (int i = 0; i < R; i += kWalk) {
-      if (i * 32 < wn) {
-        uint64_t c[kWalk];
-#pragma unroll
-        for (int u = 0; u < kWalk; ++u) {
-          const int j = (i + u) * 32 + lane_id();
-          c[u] = ((uint64_t)key[i + u] << 32) | (uint64_t)(~lds32_below(j, wn, seg + (uint32_t)j * 4u));
-        }
-        f(c);
-      }
-    }
-    if (sn > 0) walk(spill, sn, (int)threadIdx.x, NT, f);
-  }
-  template <class F>
-  __device__ __forceinline__ void for_each_key(F&& f) const {
-#pragma unroll
-    for (int i = 0; i < R; i += kWalk) {
-      if (i * 32 < wn) {
-        uint32_t k[kWalk];
-#pragma unroll
-        for (int u = 0; u < kWalk; ++u) k[u] = key[i + u];
-        f(k);
-      }
-    }
-    if (sn > 0) walk_keys(spill, sn, (int)threadIdx.x, NT, f);
-  }
 };
 
 // What a cluster leaves in its first CTA: one region of `region` slots per CTA, filled densely with
@@ -1068,32 +1036,19 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_
                                [](uint64_t c) { return (uint32_t)(c >> 32); });
 }
 
-// The same for what the filter of a lone CTA leaves behind (out of line: lone_finish is for the common case).
-template <int NT, int R, bool kTrackMin>
-__device__ __noinline__ void lone_finish_general(const RegSegCands<NT, R> passed, const FinishOut o, uint32_t need, uint32_t klo,
-                                                 uint32_t kfocus, int idx_bits, uint32_t* hist, uint32_t total) {
-  const RegSegCands<NT, R> src = passed;  // (out of the stack, into registers)
-  __syncthreads();
-  cta_finish<NT, RegSegCands<NT, R>, kTrackMin>(src, need, klo, 0xffffffffu, kfocus, false, idx_bits, hist, o.ctrl, o.out_idx, o.out_key,
-                                                o.out_base, o.out_slots, o.idx_offset, o.status, o.page, total, false);
-}
-
 // The finish of a lone CTA: the candidates' keys are in registers, round 0's histogram (`hist`, with
 // make_key_digit(klo, kfocus)) is built. A batch of rows fills the issue slots, so this is written for few
 // instructions: the thread that finds the bin works out the bounds, keys are compared where they are, and
 // nothing but the indices is read again. Where the threshold bin holds more than can be ranked, further rounds narrow
 // it to one key, and copies of that are resolved down to the last index to be taken: the keys of those behind it are
-// cleared and everything that is left wins. With spilled candidates: lone_finish_general.
+// cleared and everything that is left wins.
 template <int NT, int R, bool kTrackMin>
 __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const FinishOut& o, uint32_t need, uint32_t klo,
-                                            uint32_t kfocus, int idx_bits, uint32_t* hist, uint32_t total) {
+                                            uint32_t kfocus, int idx_bits, uint32_t* hist) {
+  static_assert(R % 4 == 0, "");
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   Ctrl* ctrl = o.ctrl;
-  if (held.sn > 0) {  // (uniform)
-    lone_finish_general<NT, R, kTrackMin>(held, o, need, klo, kfocus, idx_bits, hist, total);
-    return;
-  }
   const uint32_t fin = smem_u32(&ctrl->fin), hist_s = smem_u32(hist), wtot = smem_u32(ctrl->wtot);
   constexpr uint32_t kMany = 0xfffffffeu;
   // fin: largest key that does not win for certain, x; undecided candidates: their keys are in (y, x]; their number (kMany:

@@ -474,13 +474,11 @@ __device__ __forceinline__ uint32_t filter_regs(const float4 (&x)[R], int slabs,
 // from the FMA pipe (the sign of x - edge; a NaN has none) and one that shifts the sign in; slots by a scan over the
 // warp, once per trip; and every lane walks its own hits, without the votes and the warp-wide counter of a
 // loop that the warp walks together (10,500 warp instructions for a row of 32K elements then).
-// Beyond the segment: into the spill area, with the value, as composites.
+// A segment that does not hold its warp's candidates says so, and the row goes through full histograms.
 struct LoneList {
   uint32_t seg_s;  // shared address of the warp's segment
   uint32_t seg_cap;
   Ctrl* ctrl;
-  uint64_t* spill;
-  uint32_t spill_cap;
 };
 __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t n, uint32_t& total) {
   const int lane = lane_id();
@@ -494,12 +492,12 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t n, uint32_t& total) 
   return incl - n;
 }
 // hits: bit 31 - e for element e (of at most 32) of the lane; index_of(e) is its place in the row
-template <class T, class IndexOf>
-__device__ __forceinline__ void keep_hits(const Shard<T>& sh, const LoneList& l, uint32_t hits, uint32_t& wcnt, IndexOf&& index_of) {
+template <class IndexOf>
+__device__ __forceinline__ void keep_hits(const LoneList& l, uint32_t hits, uint32_t& wcnt, IndexOf&& index_of) {
   uint32_t total;
-  uint32_t pos = wcnt + warp_excl_scan((uint32_t)__popc(hits), total);
-  wcnt += total;
-  if (wcnt <= l.seg_cap) {  // (uniform over the warp)
+  const uint32_t pos = wcnt + warp_excl_scan((uint32_t)__popc(hits), total);
+  if (wcnt + total <= l.seg_cap) {  // (uniform over the warp)
+    wcnt += total;
     uint32_t at = l.seg_s + pos * 4u;
     while (hits != 0u) {
       const int e = __clz((int)hits);
@@ -508,18 +506,7 @@ __device__ __forceinline__ void keep_hits(const Shard<T>& sh, const LoneList& l,
       at += 4u;
     }
   } else {
-    while (hits != 0u) {
-      const int e = __clz((int)hits);
-      hits &= ~(0x80000000u >> e);
-      const int idx = index_of(e);
-      if (pos < l.seg_cap) {
-        sts32(l.seg_s + pos * 4u, (uint32_t)idx);
-      } else {
-        const uint32_t bits = __float_as_uint(Elem<T>::ld1(sh.gbase + idx + sh.a));
-        spill_push(l.ctrl, l.spill, l.spill_cap, ((uint64_t)bits << 32) | (uint32_t)idx);
-      }
-      ++pos;
-    }
+    l.ctrl->pub_flag = 1u;  // (what is counted is what the segment holds)
   }
 }
 // (x >= edge or NaN: 0) shifted into the mask from the right. An edge of zero has to be the negative one: -0 - (-0) is +0,
@@ -560,7 +547,7 @@ __device__ __forceinline__ uint32_t filter_stream_lone(const Shard<T>& sh, float
     for (int u = 0; u < U; ++u) below = shift_in_below4(below, x[u], edge);
     const int el0 = 4 * (gb + tid) - sh.a;
     const uint32_t hits = ~below << (32 - 4 * U);  // (bit 31 - e: element e; none beyond the 4 * U that were read)
-    keep_hits(sh, l, decltype(full)::value ? hits : hits & valid, wcnt,
+    keep_hits(l, decltype(full)::value ? hits : hits & valid, wcnt,
               [&](int e) { return el0 + e * NT - (e & 3) * (NT - 1); });  // element e & 3 of granule e >> 2
   };
   int gb = sh.i0;
@@ -581,16 +568,16 @@ __device__ __forceinline__ uint32_t filter_stream_lone(const Shard<T>& sh, float
         for (int e = 0; e < 4; ++e)
           if ((unsigned)(e0 + e) < (unsigned)sh.len && !((below >> (3 - e)) & 1u)) hits |= 0x80000000u >> e;
       }
-      keep_hits(sh, l, hits, wcnt, [&](int e) { return e0 + e; });
+      keep_hits(l, hits, wcnt, [&](int e) { return e0 + e; });
     }
   }
   return wcnt;
 }
 // ... of a shard that sits in registers (x[j]: granule j*NT + thread, -inf where an element is not the row's; edge > -inf):
 // a quarter of a short row passes, so a predicated store per element is cheaper than a walk over the hits.
-template <int R, class T>
-__device__ __forceinline__ uint32_t filter_regs_lone(const Shard<T>& sh, const float4 (&x)[R], int slabs, int el0, int el_step,
-                                                     float edge, const LoneList& l) {
+template <int R>
+__device__ __forceinline__ uint32_t filter_regs_lone(const float4 (&x)[R], int slabs, int el0, int el_step, float edge,
+                                                     const LoneList& l) {
   static_assert(R <= 8, "");
   uint32_t below = 0u;
 #pragma unroll
@@ -618,9 +605,8 @@ __device__ __forceinline__ uint32_t filter_regs_lone(const Shard<T>& sh, const f
     }
     return total;
   }
-  uint32_t wcnt = 0u;
-  keep_hits(sh, l, hits, wcnt, [&](int e) { return el0 + (e >> 2) * el_step + (e & 3); });
-  return wcnt;
+  l.ctrl->pub_flag = 1u;
+  return 0u;
 }
 
 // The sample of a row: `nb` batches of G loads of 32 granules per warp, spread over the whole row in pieces
@@ -993,8 +979,6 @@ __device__ __forceinline__ bool finish_given_candidates(const SelectParams& p, c
     RegSegCands<NT, R> cands;
     cands.seg = smem_u32(cx.list) + (uint32_t)(warp * own) * 4u;
     cands.wn = max(0, min(own, (int)count - warp * own));
-    cands.spill = 0u;
-    cands.sn = 0;
     uint32_t inv[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -1019,7 +1003,7 @@ __device__ __forceinline__ bool finish_given_candidates(const SelectParams& p, c
     __syncthreads();
     const RowOutput ro = row_output(p, row, cx.k);
     const FinishOut o{cx.ctrl, ro.idx, ro.key, p.status, nullptr, 0u, cx.k, p.idx_offset};
-    lone_finish<NT, R, true>(cands, o, cx.k, lowkey, focus, 32 - __clz(len - 1), cx.hist0, count);
+    lone_finish<NT, R, true>(cands, o, cx.k, lowkey, focus, 32 - __clz(len - 1), cx.hist0);
     __syncthreads();
   }
   if (!kLone) {
@@ -1348,11 +1332,11 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   // list layout: one segment per warp, then the spill area
   // (a lone CTA's segments hold indices only, as many as its warps have registers for)
   constexpr int kLoneRegs = lone_regs(NT);
-  const uint32_t spill_cap = (uint32_t)list_spill(p.list_cap, kLone);
+  const uint32_t spill_cap = kLone ? 0u : (uint32_t)list_spill(p.list_cap);
   const uint32_t seg_cap = kLone ? (uint32_t)lone_segment(p.list_cap, NT) : ((uint32_t)p.list_cap - spill_cap) / NW;
   uint64_t* const seg = kLone ? nullptr : list + (size_t)warp * seg_cap;
-  uint64_t* const spill = list + (kLone ? (size_t)(NW * seg_cap + 1u) / 2u : (size_t)NW * seg_cap);
-  const LoneList lone{smem_u32(list) + (uint32_t)warp * seg_cap * 4u, seg_cap, ctrl, spill, spill_cap};
+  uint64_t* const spill = kLone ? nullptr : list + (size_t)NW * seg_cap;
+  const LoneList lone{smem_u32(list) + (uint32_t)warp * seg_cap * 4u, seg_cap, ctrl};
 
   // ---- filter the shard against the guess -------------------------------------------------------
   // Lower edge of the guess as a float: key(x) >= gkey  <=>  !(x < edge), NaN included. Keys outside
@@ -1371,7 +1355,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   } else if (kLone) {
     const float cut = edge == 0.f ? -0.f : edge;
     if (in_regs && edge > ninf) {
-      wcnt = filter_regs_lone<kRegSlabs>(sh, xr, slabs, 4 * (sh.g0 + tid) - sh.a, 4 * NT, cut, lone);
+      wcnt = filter_regs_lone<kRegSlabs>(xr, slabs, 4 * (sh.g0 + tid) - sh.a, 4 * NT, cut, lone);
     } else {
       wcnt = filter_stream_lone<NT>(sh, cut, lone);
     }
@@ -1395,7 +1379,6 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     const KeyDigit dg = make_key_digit(lowkey, focus_key);
     held.seg = lone.seg_s;
     held.wn = (int)wown;
-    held.spill = smem_u32(spill);
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < kLoneRegs; i += 4) {
@@ -1424,8 +1407,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     const uint32_t wn_s = smem_u32(ctrl->wmax);
     if (lane == 0) sts32(wn_s + warp * 4, wown);  // (not wtot: the finish's search may write that before every warp has read it)
     __syncthreads();
-    held.sn = (int)min(ctrl->lcount, spill_cap);
-    total = __reduce_add_sync(kFull, lane < NW ? lds32(wn_s + lane * 4) : 0u) + (uint32_t)held.sn;
+    total = __reduce_add_sync(kFull, lane < NW ? lds32(wn_s + lane * 4) : 0u);
     mode = sampled_attempt_ok(ctrl->pub_flag, total, K, 0xffffffffu) ? kModeGather : kModeFallback;
   } else {
     // ---- gather in rank 0 ----------------------------------------------------------------------
@@ -1498,7 +1480,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   if (mode == kModeGather) {
     if constexpr (kLone) {
       const FinishOut o{ctrl, out_idx, out_key, p.status, cx.page, 0u, K, cx.idx_offset};
-      lone_finish<NT, kLoneRegs, kWarm>(held, o, K, lowkey, focus_key, idx_bits, fin_hist, total);
+      lone_finish<NT, kLoneRegs, kWarm>(held, o, K, lowkey, focus_key, idx_bits, fin_hist);
     } else {
       const RegionCands<NT> src{smem_u32(cx.cand), smem_u32(ctrl->cnt_of), region, C, extra};
       cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lowkey, 0xffffffffu, focus_key, false, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
@@ -1680,8 +1662,8 @@ constexpr int kOverlapListCap1 = 6144, kOverlapListCap1Long = 9216;
 constexpr int64_t kOverlapShortRow = 196608;
 constexpr int kOverlapListCap = 3072, kOverlapCandCap = 6144;   // two CTAs per SM
 // Rows so short that the list of a CTA of 256 threads holds all of them, whatever they are (make_plan)
-constexpr int kLoneListCap256 = 4096, kLoneCandCap256 = 2560;
-constexpr int64_t kLoneRow256 = 4352;
+constexpr int kLoneListCap256 = 2560, kLoneCandCap256 = 2560;
+constexpr int64_t kLoneRow256 = 4096;
 
 
 using SelectFn = void (*)(SelectParams);
@@ -1800,7 +1782,7 @@ int floor_pow2(int64_t v) {
 void lone_lists(Plan& pl, int list_cap) {
   pl.list_cap = list_cap;
   pl.cand_cap = pl.threads == 256 ? std::min(list_cap, kLoneCandCap256) : list_cap;
-  pl.smem_bytes = (int)(fixed_smem_bytes(true) + std::max((size_t)lone_list_bytes(list_cap, pl.threads), (size_t)pl.cand_cap * 8));
+  pl.smem_bytes = (int)(fixed_smem_bytes(true) + std::max((size_t)lone_room(list_cap, pl.threads) * 4, (size_t)pl.cand_cap * 8));
 }
 
 // Replaces the reference's split heuristic (topk_indexer_radix.cu:1081-1111: at most 8 CTAs per

@@ -104,10 +104,8 @@ void dh_key_bin_range(uint32_t lo, uint32_t focus, uint32_t cap, uint32_t t, uin
 uint32_t dh_key_digit(uint32_t lo, uint32_t focus, uint32_t v) { return make_key_digit(lo, focus).of(v); }
 uint64_t dh_single_key_floor(uint64_t lo, int idx_bits) { return (lo & 0xffffffff00000000ull) | inverted_index_floor(idx_bits); }
 int dh_lone_segment(int list_cap, int threads) { return lone_segment(list_cap, threads); }
-int dh_lone_list_bytes(int list_cap, int threads) { return lone_list_bytes(list_cap, threads); }
 int dh_lone_room(int list_cap, int threads) { return lone_room(list_cap, threads); }
 int dh_lone_regs(int threads) { return lone_regs(threads); }
-int dh_list_spill(int list_cap, int lone) { return list_spill(list_cap, lone != 0); }
 
 // Walks every CTA's run of tiles the way the fused indexer's producer does (tile_run, tile_row_at,
 // then tile_segment row after row) and adds, for every (row, row-local tile) the CTAs visit, one to
