@@ -27,8 +27,8 @@
 //      their keys in registers, and finishes on those (lone_finish). The inverted index in the composite makes equal values resolve to the lower index.
 //      Measured (us per call in a chain of calls on B200, when histograms were exchanged -> with steps 1 to 4
 //      as they are now): B=1, L=96K 12.9 -> 10.0, 1M 15.4 -> 14.1; B=4, L=200K 13.6 -> 10.7; B=64 ragged rows
-//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5, then 3.8); B=2048, one CTA per row, L=32K
-//      132 -> 102 -> 84.6, 8K 106 -> 67 -> 58.6, 4K 62 -> 38.5 (the last figure of each: keys in registers, fewer instructions). What bounds it is no bandwidth but the chain of short phases and the instructions in it.
+//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5, then 3.55); B=2048, one CTA per row, L=32K
+//      132 -> 102 -> 81.0, 8K 106 -> 67 -> 55.3, 4K 62 -> 39.1 (the last figure of each: keys in registers, fewer instructions). What bounds it is no bandwidth but the chain of short phases and the instructions in it.
 //   5. If the guess admitted fewer than k elements, a list overflowed or the threshold bin is
 //      larger than rank 0's buffer (heavy ties, rows of equal values), the cluster falls back to
 //      full histograms over the data: 12 + 12 + 8 key bits, re-reading the shard from L2 each
@@ -1835,7 +1835,7 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
     }
   }
   if (narrow && pl.cluster == 1 && pl.threads == 512 && L <= kLoneRow256) {
-    // Short rows: four CTAs of 256 threads share an SM, each with 41 KB, and the phases in which one of them has
+    // Short rows: four CTAs of 256 threads share an SM, each with some 40 KB, and the phases in which one of them has
     // little to do are the others' time. Measured with 2,048 rows of N(0,1)-like sums, 256 / 512 threads: 4K elements 37 / 49 us,
     // 8K 48 / 57, 32K 105 / 82; with 70 % zeros 4K 91 / 105, 6K 191 / 131 - rows that may overflow their list stay with 512.
     pl.threads = 256;
