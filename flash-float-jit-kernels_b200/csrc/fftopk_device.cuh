@@ -159,10 +159,6 @@ __device__ __forceinline__ void st_global_if_above(uint32_t k, uint32_t thr, voi
   asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.u32 p, %2, %3;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(a), "r"(v), "r"(k), "r"(thr)
                : "memory");
 }
-__device__ __forceinline__ void sts64_if(bool on, uint32_t a, uint64_t v) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u64 [%0], %1;\n\t}" ::"r"(a), "l"(v), "r"((uint32_t)on)
-               : "memory");
-}
 // (i < n: the word at `a`, else 0)
 __device__ __forceinline__ uint32_t lds32_below(int i, int n, uint32_t a) {
   uint32_t v;
@@ -917,8 +913,7 @@ __device__ __noinline__ bool finish_copies(const Src passed, const FinishOut pas
 // copies of the threshold than can be ranked - on the inverted indices below it. (With 64-bit
 // composites as the digits' field a round cost 280 instructions per warp besides the candidates', and the output 450:
 // 11,700 of the 26,200 warp instructions of a row of 8K elements.)
-// `kfocus`: see KeyDigit (fftopk_decide.h). `have_hist`: the caller has already built round 0's histogram in
-// `hist`, with make_key_digit(klo, kfocus), klo < kfocus.
+// `kfocus`: see FieldDigit (fftopk_decide.h).
 // `idx_bits`: all indices are < 2^idx_bits, so the inverted-index bits above that are all ones.
 // `page`: optional per-row table; the value written is then page[idx] instead of idx + idx_offset
 // (the fused page-table transform of the reference's topk_transform_* kernels, :871-958).
@@ -930,7 +925,7 @@ __device__ __noinline__ bool finish_copies(const Src passed, const FinishOut pas
 // stack, and beside 200 KB of shared memory L1 has no room for the stacks of 1024 threads - each access
 // was a round trip to L2 (the passes over the candidates took 1.4 and 2 to 4 us instead of 0.4 and 0.7).
 template <int NT, class Src, bool kTrackMin = false>
-__device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_t klo, uint32_t kcap, uint32_t kfocus, bool have_hist,
+__device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_t klo, uint32_t kcap, uint32_t kfocus,
                            int idx_bits, uint32_t* hist /* >= kFinishBins words */, Ctrl* ctrl, int32_t* out_idx,
                            uint32_t* out_key, uint32_t out_base, uint32_t out_slots /* k of the row */,
                            int32_t idx_offset, uint32_t* status,
@@ -967,7 +962,7 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_
       return;
     }
     kfocus = kcap;
-    have_hist = hist_clear = false;
+    hist_clear = false;
     __syncthreads();  // the scratch words are about to be cleared as the histogram
     FFTOPK_MARK(31);
   }
@@ -993,22 +988,20 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_
       if (finish_copies<NT, kTrackMin>(src, o, need_total, need, lo, cap > lo, idx_bits, hist)) return;
       ++lo;
       focus = cap;
-      have_hist = hist_clear = false;
+      hist_clear = false;
     }
     const KeyDigit dg = make_key_digit(lo, focus);
-    if (!have_hist) {
-      if (!hist_clear) {
-        __syncthreads();
-        for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
-        __syncthreads();
-      }
-      const uint32_t span = cap - lo;
-      src.for_each_key([&](const uint32_t (&k)[kWalk]) {
-#pragma unroll
-        for (int u = 0; u < kWalk; ++u) red_shared_inc_if(hist_s + dg.of(k[u]) * 4u, k[u], k[u] - lo, span);
-      });
+    if (!hist_clear) {
+      __syncthreads();
+      for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
       __syncthreads();
     }
+    const uint32_t span = cap - lo;
+    src.for_each_key([&](const uint32_t (&k)[kWalk]) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) red_shared_inc_if(hist_s + dg.of(k[u]) * 4u, k[u], k[u] - lo, span);
+    });
+    __syncthreads();
     FFTOPK_MARK(16);
     const uint4 f = finish_pick<NT>(hist_s, need, ctrl);
     FFTOPK_MARK(17);
@@ -1023,7 +1016,7 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_
       lo = t_lo;
       cap = focus = t_hi;
       need = need2;
-      have_hist = hist_clear = false;
+      hist_clear = false;
     }
   }
   FFTOPK_MARK(30);

@@ -320,7 +320,7 @@ __device__ __forceinline__ void merge_row(cg::cluster_group& cluster, int C, int
     const DenseCands<NT> bin_cands{sm.cand, (int)ctrl->cand_count};
     const uint32_t lo = t << pshift;
     const uint32_t cap = lo | ((1u << pshift) - 1u);
-    cta_finish<NT, DenseCands<NT>, kTrackMin>(bin_cands, need, lo, cap, cap, false, 31, hist, ctrl, out_idx, out_key,
+    cta_finish<NT, DenseCands<NT>, kTrackMin>(bin_cands, need, lo, cap, cap, 31, hist, ctrl, out_idx, out_key,
                                               (uint32_t)kK - need, (uint32_t)kK, 0, status, nullptr, ctrl->cand_count);
   } else if (mode != kModeTakeAll) {
     if (tid == 0 && status) atomicOr(status, (uint32_t)FFTOPK_ST_INTERNAL);

@@ -890,7 +890,7 @@ __device__ __noinline__ uint32_t select_by_full_histograms(const RowCtx<NT, T> p
     const uint32_t lo = P << shift;
     const uint32_t cap = lo | ((1u << shift) - 1u);
     const DenseCands<NT> src{cx.cand, (int)min(cx.ctrl->cand_count, (uint32_t)cx.cand_cap)};
-    cta_finish<NT, DenseCands<NT>, kTrack>(src, need, lo, cap, cap, false, 32 - __clz(cx.sh.len - 1), cx.hist(1), cx.ctrl,
+    cta_finish<NT, DenseCands<NT>, kTrack>(src, need, lo, cap, cap, 32 - __clz(cx.sh.len - 1), cx.hist(1), cx.ctrl,
                                            cx.out_idx, cx.out_key, cx.k - need, cx.k, cx.idx_offset, cx.status, cx.page,
                                            (uint32_t)src.n);
     if constexpr (kTrack) {
@@ -1483,7 +1483,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
       lone_finish<NT, kLoneRegs, kWarm>(held, o, K, lowkey, focus_key, idx_bits, fin_hist);
     } else {
       const RegionCands<NT> src{smem_u32(cx.cand), smem_u32(ctrl->cnt_of), region, C, extra};
-      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lowkey, 0xffffffffu, focus_key, false, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
+      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lowkey, 0xffffffffu, focus_key, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
                                              K, cx.idx_offset, p.status, cx.page, total, true);
     }
     // This call's threshold for the next one: the smallest key the finish let win (the row's k-th
