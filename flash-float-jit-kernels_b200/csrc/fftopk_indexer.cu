@@ -745,9 +745,7 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
     if (ctas < 1) ctas = 1;
   }
   const dim3 grid((unsigned)ctas, 1u, 1u);
-  // the producer: logits; rows with a guess are filtered as the logits are produced
-  e = fp8 ? launch_producer<true>(grid, stream, map_q, map_k, p) : launch_producer<false>(grid, stream, map_q, map_k, p);
-  if (e != cudaSuccess) return cuda_fail(e);
+  bool produced = false;
   // the selector: rows whose guess held are finished on their candidates, the others selected on their logits
   SelectCall c;
   c.score = logits;
@@ -763,7 +761,20 @@ static int indexer_topk_impl(bool fp8, const void* q, const void* k_cache, int64
   c.cand_guess = thresholds;
   c.warm_margin = margin;
   c.may_overlap = false;  // (a programmatic dependent of the producer that waits for it, like every default launch)
-  return launch_select(c);
+  // the producer in front of it: logits; rows with a guess are filtered as the logits are produced. It is enqueued only when
+  // nothing can refuse the selector any more: the selector alone sets the rows' candidate counts back.
+  auto produce = [&] {
+    const cudaError_t err = fp8 ? launch_producer<true>(grid, stream, map_q, map_k, p) : launch_producer<false>(grid, stream, map_q, map_k, p);
+    produced = err == cudaSuccess;
+    return produced ? 0 : cuda_fail(err);
+  };
+  c.in_front = [](void* f) { return (*static_cast<decltype(produce)*>(f))(); };
+  c.in_front_arg = &produce;
+  rc = launch_select(c);
+  // (a launch that failed behind the producer: the workspace has to be as every call leaves it)
+  if (rc && produced)
+    (void)cudaMemset2DAsync(p.cand + kIdxCandCap, kIdxRecordWords * 8, 0, sizeof(uint32_t), (size_t)B, stream);
+  return rc;
 }
 
 int fftopk_indexer_topk2048(const void* q, const void* k_cache, int64_t k_rows_per_seq, const float* w, int32_t B, int64_t L,

@@ -53,6 +53,10 @@ struct SelectCall {
   // (a programmatic dependent launch that does not has no guarantee that its predecessor's writes
   // are visible).
   bool may_overlap = true;
+  // Enqueues what has to run in front of this launch and relies on it; called once every check of the call has passed and
+  // its plan is made, so that a call that is refused has enqueued nothing. A non-zero return ends the call with it.
+  int (*in_front)(void* arg) = nullptr;
+  void* in_front_arg = nullptr;
 };
 
 int launch_select(const SelectCall& c);

@@ -1965,6 +1965,10 @@ int launch_select(const SelectCall& c) {
   } else if (warm) {
     variant = kVarWarm;
   }
+  if (c.in_front) {  // (nothing below refuses the call)
+    rc = c.in_front(c.in_front_arg);
+    if (rc) return rc;
+  }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, select_fn(pl.threads, pl.cluster == 1 ? kLoneForm : (overlap ? kTightForm : kRoomyForm), variant), p);
   if (e != cudaSuccess) return cuda_fail(e);
   return FFTOPK_OK;

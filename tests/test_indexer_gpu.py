@@ -308,3 +308,31 @@ def test_candidate_lists_of_every_length(B, L):
         orc.check_result(f.logits[:B, :L].cpu().numpy(), ln.cpu().numpy(), out.cpu().numpy(), what=f"margin {margin}")
         if kernel_status() == 0:
             assert torch.equal(f.thresholds[:B], exact)
+
+
+@pytest.mark.parametrize("tuning", [dict(threads=256), dict(cluster_ctas=4, list_cap=16384, cand_cap=16384)])  # refused: threads, shared memory
+def test_a_refused_call_leaves_the_workspace_as_it_was(tuning):
+    B, L = 4, 30000
+    q, k, w = make(B, L, seed=31)
+    q2 = make(B, L, seed=32)[0]
+    ln = torch.full((B,), L, dtype=torch.int32, device=DEV)
+    f = FusedIndexerTopk(B, L)
+    f(q, k, w, ln)
+    torch.cuda.synchronize()
+    before = f._ws.clone()
+    try:
+        _native.set_tuning(**tuning)
+        with pytest.raises(Exception, match="fftopk_indexer_topk2048"):
+            f(q, k, w, ln, margin=1 << 18)
+    finally:
+        _native.set_tuning()
+    torch.cuda.synchronize()
+    assert torch.equal(f._ws, before)
+    _status_word(DEV).zero_()
+    for query in (q, q2):  # (q2: guesses of another query, which may not hold)
+        out = f(query, k, w, ln, margin=1 << 18)
+        torch.cuda.synchronize()
+        logits = f.logits[:B, :L].cpu().numpy()
+        orc.check_result(logits, ln.cpu().numpy(), out.cpu().numpy(), what="after a refused call")
+        thr, want = f.thresholds[:B].cpu().numpy().view(np.uint32), kth_keys(logits, ln.cpu().numpy())
+        assert np.all(thr <= want) and (query is not q or np.array_equal(thr, want))
