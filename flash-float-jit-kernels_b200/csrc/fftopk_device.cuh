@@ -1078,7 +1078,7 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
     if (f.z == kMany) {  // copies of `lo`
       const uint32_t key = lo;
       uint32_t ilo = inverted_index_floor(idx_bits), icap = 0xffffffffu;
-      do {  // (indices differ: the last round ends with one candidate, or takes its bin whole)
+      do {  // (indices differ: a round that is down to one of them takes its bin whole)
         __syncthreads();
         clear();
         const KeyDigit dg = make_key_digit(ilo, icap);
@@ -1093,7 +1093,8 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
         f = pick(dg, f.w, icap, 0u);
         ilo = f.y + 1u;
         icap = f.x;
-      } while (f.z == kMany);
+      } while (f.z == kMany && ilo < icap);
+      if (f.z == kMany) f.z = kNoBin;  // (one index many times over: not a list of the library's making)
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         if (i * 32 < held.wn && held.key[i] == key) {

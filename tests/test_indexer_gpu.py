@@ -336,3 +336,30 @@ def test_a_refused_call_leaves_the_workspace_as_it_was(tuning):
         orc.check_result(logits, ln.cpu().numpy(), out.cpu().numpy(), what="after a refused call")
         thr, want = f.thresholds[:B].cpu().numpy().view(np.uint32), kth_keys(logits, ln.cpu().numpy())
         assert np.all(thr <= want) and (query is not q or np.array_equal(thr, want))
+
+
+def test_a_list_that_names_one_key_many_times_is_reported():
+    """A workspace that was not zero-filled: 300 copies of one candidate, of the same index, where the threshold lies. No
+    round over the indices can tell them apart; the call ends and says so."""
+    B, L = 1, 30000
+    q, k, w = make(B, L, seed=33)
+    ln = torch.full((B,), L, dtype=torch.int32, device=DEV)
+    f = FusedIndexerTopk(B, L)
+    f(q, k, w, ln)
+    torch.cuda.synchronize()
+    keys = orc.keys_of(f.logits[0, :L].cpu().numpy())
+    key = int(np.sort(keys)[-1900])
+    copy = (key << 32) | (0xFFFFFFFF - int(np.flatnonzero(keys == key)[0]))
+    record = f._ws[f._ws_ptr - f._ws.data_ptr():].view(torch.int64)
+    record[:300] = copy - (1 << 64) if copy >> 63 else copy
+    record[8192] = 300
+    out = f(q, k, w, ln)
+    torch.cuda.synchronize()
+    assert out.shape == (B, K) and kernel_status(DEV) & _native.ST_INTERNAL
+    _status_word(DEV).zero_()
+    f.thresholds.zero_()
+    for _ in range(2):  # (and the workspace is as every call leaves it)
+        out = f(q, k, w, ln)
+        torch.cuda.synchronize()
+        orc.check_result(f.logits[:B, :L].cpu().numpy(), ln.cpu().numpy(), out.cpu().numpy(), what="afterwards")
+    assert kernel_status(DEV) == 0
