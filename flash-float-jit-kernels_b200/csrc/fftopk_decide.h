@@ -220,15 +220,27 @@ FFTOPK_DECIDE_HD int gather_region(int cand_cap, int list_cap, int ctas) {
 FFTOPK_DECIDE_HD int list_spill(int list_cap) { return list_cap / (list_cap >= 4096 ? 8 : 4); }
 
 // A lone CTA's segments hold row indices (words, in the memory of list_cap composites), and the finish has their keys in
-// registers: so many per thread, and no more candidates per warp than that. (No spill area: with 512 slots for each of 16
-// warps a row overflows with its 8,193rd candidate or so, and then goes through full histograms.)
-FFTOPK_DECIDE_HD constexpr int lone_regs(int threads) { return threads >= 1024 ? 8 : 16; }
+// registers: so many per thread, and no more candidates per warp than that. There is no spill area: one warp over its
+// segment sends the row through full histograms, and its call waits for it. So a segment has to hold what a guess may
+// admit of one warp's share - up to 9.5K expected per row, and that unevenly -, or many copies of the threshold. With 8
+// and 16 keys a thread (8,192 a row) most calls had such a row; us per call then / now: 100 rows of 160K, k = 4096, 78 / 19;
+// 80 of 512K, k = 4096, 189 / 39; 40 of 2M, overlapping, 150 / 42; 160 of 256K with 6,500 copies 253 / 57. Rows that need fewer
+// registers do not pay for the others (2,048 rows of 32K, k = 2048, 80.7 / 80.2). A row that gets 256 threads fits as it is.
+FFTOPK_DECIDE_HD constexpr int lone_regs(int threads) { return threads >= 1024 ? 12 : (threads >= 512 ? 20 : 16); }
 FFTOPK_DECIDE_HD int lone_segment(int list_cap, int threads) {
   const int own = 2 * list_cap / (threads / 32);
   return own < 32 * lone_regs(threads) ? own : 32 * lone_regs(threads);
 }
 // ... the whole list in candidates (words)
 FFTOPK_DECIDE_HD int lone_room(int list_cap, int threads) { return threads / 32 * lone_segment(list_cap, threads); }
+// ... and what a guess is weighed against (sample_admits_too_much tries a quarter more, since the sample's share is an
+// estimate): less than the larger lists hold, because the warps' shares differ. Rows with copies of the threshold, us for 160
+// rows of 128K / 256K with weights of 8,192, this and 10,240: 7,500 copies 36 / 111 (given up for nothing),
+// 36 / 59, 36 / 59; 12,000 copies 195 / 356, 194 / 359, 206 / 385 (read for nothing).
+FFTOPK_DECIDE_HD int lone_room_weighed(int list_cap, int threads) {
+  const int room = lone_room(list_cap, threads);
+  return room < 9216 ? room : 9216;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Digit rule of a finish round over a field's range [lo, cap]: digit(v) = min((v - lo) >>

@@ -1111,10 +1111,9 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
   uint32_t n = 0u;
 #pragma unroll
   for (int i = 0; i < R; i += 4) {
-    if (i * 32 < held.wn) {
+    if (i * 32 >= held.wn) break;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) count_if_above(n, held.key[i + u], f.x);
-    }
+    for (int u = 0; u < 4; ++u) count_if_above(n, held.key[i + u], f.x);
   }
   n = __reduce_add_sync(kFull, n);
   const uint32_t wsum = smem_u32(ctrl->wmax);
@@ -1128,46 +1127,45 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
   auto pass = [&](auto plain) {  // (plain: indices alone, as they are)
 #pragma unroll
     for (int i = 0; i < R; i += 4) {
-      if (i * 32 < held.wn) {
-        uint32_t idx[4];
-        int32_t v[4];
+      if (i * 32 >= held.wn) break;
+      uint32_t idx[4];
+      int32_t v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = (i + u) * 32 + lane;
-          idx[u] = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
-          v[u] = (int32_t)idx[u];
-          if constexpr (!decltype(plain)::value) {
-            if (!o.page) {
-              v[u] += o.idx_offset;
-            } else if (held.key[i + u] > f.x) {
-              v[u] = __ldg(o.page + idx[u]);
-            }
+      for (int u = 0; u < 4; ++u) {
+        const int j = (i + u) * 32 + lane;
+        idx[u] = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
+        v[u] = (int32_t)idx[u];
+        if constexpr (!decltype(plain)::value) {
+          if (!o.page) {
+            v[u] += o.idx_offset;
+          } else if (held.key[i + u] > f.x) {
+            v[u] = __ldg(o.page + idx[u]);
           }
         }
-        uint32_t nearest = 0xffffffffu;
+      }
+      uint32_t nearest = 0xffffffffu;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t k = held.key[i + u];
+        const unsigned bw = __ballot_sync(kFull, k > f.x);
+        const uint32_t pos = wpos + (uint32_t)__popc(bw & lt);
+        if (!(k > f.x) || FFTOPK_CHECK(3, pos, o.out_slots, o.status)) {
+          st_global_if_above(k, f.x, o.out_idx + pos, (uint32_t)v[u]);
+          if constexpr (!decltype(plain)::value) {
+            if (o.out_key) st_global_if_above(k, f.x, o.out_key + pos, k);
+          }
+        }
+        wpos += (uint32_t)__popc(bw);
+        if constexpr (kTrackMin) win_min = min(win_min, k > f.x ? k : 0xffffffffu);
+        nearest = min(nearest, k - f.y - 1u);
+      }
+      if (__any_sync(kFull, nearest < f.x - f.y)) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t k = held.key[i + u];
-          const unsigned bw = __ballot_sync(kFull, k > f.x);
-          const uint32_t pos = wpos + (uint32_t)__popc(bw & lt);
-          if (!(k > f.x) || FFTOPK_CHECK(3, pos, o.out_slots, o.status)) {
-            st_global_if_above(k, f.x, o.out_idx + pos, (uint32_t)v[u]);
-            if constexpr (!decltype(plain)::value) {
-              if (o.out_key) st_global_if_above(k, f.x, o.out_key + pos, k);
-            }
-          }
-          wpos += (uint32_t)__popc(bw);
-          if constexpr (kTrackMin) win_min = min(win_min, k > f.x ? k : 0xffffffffu);
-          nearest = min(nearest, k - f.y - 1u);
-        }
-        if (__any_sync(kFull, nearest < f.x - f.y)) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const uint32_t k = held.key[i + u];
-            const uint32_t slot =
-                append64_if(k - f.y - 1u < f.x - f.y, small_n, small_s, kSmall, ((uint64_t)k << 32) | (uint64_t)(~idx[u]));
-            (void)FFTOPK_CHECK(4, slot, kSmall, o.status);
-          }
+          const uint32_t slot =
+              append64_if(k - f.y - 1u < f.x - f.y, small_n, small_s, kSmall, ((uint64_t)k << 32) | (uint64_t)(~idx[u]));
+          (void)FFTOPK_CHECK(4, slot, kSmall, o.status);
         }
       }
     }

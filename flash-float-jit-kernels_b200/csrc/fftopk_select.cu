@@ -1269,7 +1269,7 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     }
     __syncthreads();
     FFTOPK_MARK(2);
-    const uint32_t room = (uint32_t)(kLone ? lone_room(p.list_cap, NT) : p.cand_cap);
+    const uint32_t room = (uint32_t)(kLone ? lone_room_weighed(p.list_cap, NT) : p.cand_cap);
     // (one thread, when it has found the bin) what the guess is and what to do about it: see weigh_guess
     auto weigh = [&](uint32_t low, uint32_t width, uint32_t above, uint32_t cnt, uint32_t rest, uint32_t parent) {
       const uint32_t flags = weigh_guess(width, above, cnt, parent, smp.size(), (float)len, K, kCoarseFactor, room);
@@ -1382,24 +1382,22 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < kLoneRegs; i += 4) {
+      if (i * 32 >= held.wn) break;  // (uniform over the warp; nobody looks at registers beyond)
+      uint32_t bits[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) held.key[i + u] = 0u;
-      if (i * 32 < held.wn) {  // (uniform over the warp)
-        uint32_t bits[4];
+      for (int u = 0; u < 4; ++u) {
+        const int j = (i + u) * 32 + lane;
+        uint32_t idx = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
+        if (!FFTOPK_CHECK(7, idx, sh.len, p.status)) idx = 0u;
+        bits[u] = __float_as_uint(Elem<T>::ld1(sh.gbase + idx + sh.a));  // (index 0 is always readable)
+      }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = (i + u) * 32 + lane;
-          uint32_t idx = lds32_below(j, held.wn, held.seg + (uint32_t)j * 4u);
-          if (!FFTOPK_CHECK(7, idx, sh.len, p.status)) idx = 0u;
-          bits[u] = __float_as_uint(Elem<T>::ld1(sh.gbase + idx + sh.a));  // (index 0 is always readable)
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if ((i + u) * 32 < held.wn) {  // (uniform)
-            if ((i + u) * 32 + lane < held.wn) {
-              held.key[i + u] = fftopk_key_from_bits(bits[u]);
-              red_shared_inc(fh + dg.of(held.key[i + u]) * 4u);
-            }
+      for (int u = 0; u < 4; ++u) {
+        held.key[i + u] = 0u;
+        if ((i + u) * 32 < held.wn) {  // (uniform)
+          if ((i + u) * 32 + lane < held.wn) {
+            held.key[i + u] = fftopk_key_from_bits(bits[u]);
+            red_shared_inc(fh + dg.of(held.key[i + u]) * 4u);
           }
         }
       }
@@ -1654,12 +1652,11 @@ constexpr size_t fixed_smem_bytes(bool lone) {
 
 constexpr int64_t kPrefetchRow = 1 << 20, kPrefetchBytes = 48 << 20;
 constexpr int kLatencyListCap = 6144, kLatencyCandCap = 16384;  // one CTA per SM: use the shared memory
-// One CTA per row (list = candidates), two CTAs per SM. Rows of up to ~192K elements leave about
-// 3600 candidates; with the small list two CTAs take 2 x 90 KB of the SM's 256 KB and the rest
-// stays L1, which the value re-reads of the filter hit (measured on B=64 ragged rows <= 128K:
-// 5.3 us per call with lists of 4608..7168 entries, 6.2 us with 8192 or more).
-constexpr int kOverlapListCap1 = 6144, kOverlapListCap1Long = 9216;
-constexpr int64_t kOverlapShortRow = 196608;
+// One CTA per row, whatever its length and k: 640 or 384 candidates a warp (lone_segment), some 70 KB per CTA with the buffer
+// that the full-histogram path gathers in. With two CTAs per SM the rest stays L1, which the second read of a candidate's value
+// hits: a larger buffer for rows beyond 192K and for k > 2048 (9,216 composites, 94 KB) cost 150 rows of 1M 137 us instead
+// of 114, 64 of 256K in overlapping calls 14.1 instead of 13.5.
+constexpr int kOverlapListCap1 = 6144;
 constexpr int kOverlapListCap = 3072, kOverlapCandCap = 6144;   // two CTAs per SM
 // Rows so short that the list of a CTA of 256 threads holds all of them, whatever they are (make_plan)
 constexpr int kLoneListCap256 = 2560, kLoneCandCap256 = 2560;
@@ -1817,7 +1814,7 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
     // CTAs per row.)
     pl.cluster = 1;
     pl.threads = 512;
-    pl.list_cap = L <= kOverlapShortRow ? kOverlapListCap1 : kOverlapListCap1Long;
+    pl.list_cap = kOverlapListCap1;
     pl.cand_cap = kOverlapCandCap;
   }
   if (overlap) {
@@ -1828,7 +1825,7 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
     if (ct < pl.cluster) pl.cluster = ct;
     pl.threads = 512;
     if (pl.cluster == 1) {
-      pl.list_cap = L <= kOverlapShortRow ? kOverlapListCap1 : kOverlapListCap1Long;
+      pl.list_cap = kOverlapListCap1;
     } else {
       pl.list_cap = kOverlapListCap;
       pl.cand_cap = kOverlapCandCap;
@@ -1892,10 +1889,6 @@ int launch_select(const SelectCall& c) {
   if (half_width && pl.threads < 512) {  // (the 16-bit kernels exist for 512 and 1024 threads)
     pl.threads = 512;
     if (pl.cluster == 1) lone_lists(pl, pl.list_cap);
-  }
-  if (c.k > kK && pl.cluster == 1 && tn.list_cap <= 0) {
-    // more winners than the lone-CTA list was sized for: the long-row list
-    lone_lists(pl, kOverlapListCap1Long);
   }
 
   SelectParams p;

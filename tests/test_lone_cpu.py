@@ -54,3 +54,17 @@ def test_a_short_row_fits_whole(dh):
     warp w sees [32 w, 32 w + 32) of every 256."""
     count = [sum(1 for g in range(1024) if g % 256 // 32 == w) * 4 for w in range(8)]
     assert max(count) <= dh.dh_lone_segment(2560, 256)
+
+
+@pytest.mark.parametrize("threads,k,length", [(1024, 4096, n) for n in (131072, 220000, 1 << 19, 1 << 20)]
+                         + [(512, 4096, n) for n in (65536, 131072, 262144)]
+                         + [(512, 2048, n) for n in (262144, 1 << 20, 2000000)] + [(1024, 2048, 2000000)])
+def test_a_warp_holds_its_share_of_what_a_guess_admits(dh, threads, k, length):
+    """Rows of independent values: a guess made on rank r of n samples admits r L / n elements, give or take its square root
+    in samples; they fall on the warps at random. Three and a half deviations more than a warp's share fit its segment."""
+    dh.dh_sample_lower_rank.restype, dh.dh_sample_lower_rank.argtypes = u32, [u32, u32, ctypes.c_float]
+    n = 8192 << dh.dh_sample_log_batches(length, u32(k))
+    rank, warps = dh.dh_sample_lower_rank(k, n, length), threads // 32
+    share, each = rank * length / n / warps, length / n / warps
+    deviation = (rank * each ** 2 + share) ** 0.5
+    assert share + 3.5 * deviation <= dh.dh_lone_segment(6144, threads)
