@@ -231,6 +231,10 @@ FFTOPK_DECIDE_HD int lone_segment(int list_cap, int threads) {
   const int own = 2 * list_cap / (threads / 32);
   return own < 32 * lone_regs(threads) ? own : 32 * lone_regs(threads);
 }
+// The warp that reads the granules a row's ends cut through (up to three elements each): the one with the fewest others. All
+// of a row of up to 4,096 elements may pass - rows of mostly zeros -, and 256 threads hold 512 a warp: with the ends in the
+// first two warps most rows that were not 16-byte aligned overflowed (2,048 rows of 4,095, 70 % zeros: 163 us, now 96.5).
+FFTOPK_DECIDE_HD constexpr int lone_edge_warp(int threads) { return threads / 32 - 1; }
 // ... the whole list in candidates (words)
 FFTOPK_DECIDE_HD int lone_room(int list_cap, int threads) { return threads / 32 * lone_segment(list_cap, threads); }
 // ... and what a guess is weighed against (sample_admits_too_much tries a quarter more, since the sample's share is an

@@ -553,10 +553,11 @@ __device__ __forceinline__ uint32_t filter_stream_lone(const Shard<T>& sh, float
   int gb = sh.i0;
   for (; gb + NT * U <= sh.i1; gb += NT * U) trip(gb, std::true_type{});
   if (gb < sh.i1) trip(gb, std::false_type{});
-  // edge granules [g0, i0) and [i1, g1): at most one each, visited by lane 0 of warps 0 and 1
-  if (tid < 64) {  // (whole warps)
-    const int ge = (tid == 0) ? sh.g0 : ((tid == 32) ? sh.i1 : -1);
-    const int ge_end = (tid == 0) ? sh.i0 : sh.g1;
+  // edge granules [g0, i0) and [i1, g1): at most one each, two lanes of the same warp
+  if (tid >> 5 == lone_edge_warp(NT)) {
+    const int lane = lane_id();
+    const int ge = lane == 0 ? sh.g0 : (lane == 1 ? sh.i1 : -1);
+    const int ge_end = lane == 0 ? sh.i0 : sh.g1;
     const bool mine = ge >= 0 && ge < ge_end;
     if (__any_sync(kFull, mine)) {
       uint32_t hits = 0u;
@@ -1658,7 +1659,8 @@ constexpr int kLatencyListCap = 6144, kLatencyCandCap = 16384;  // one CTA per S
 // of 114, 64 of 256K in overlapping calls 14.1 instead of 13.5.
 constexpr int kOverlapListCap1 = 6144;
 constexpr int kOverlapListCap = 3072, kOverlapCandCap = 6144;   // two CTAs per SM
-// Rows so short that the list of a CTA of 256 threads holds all of them, whatever they are (make_plan)
+// Rows so short that the list of a CTA of 256 threads holds all of them, whatever they are and wherever they start
+// (make_plan, lone_edge_warp)
 constexpr int kLoneListCap256 = 2560, kLoneCandCap256 = 2560;
 constexpr int64_t kLoneRow256 = 4096;
 

@@ -106,6 +106,7 @@ uint64_t dh_single_key_floor(uint64_t lo, int idx_bits) { return (lo & 0xfffffff
 int dh_lone_segment(int list_cap, int threads) { return lone_segment(list_cap, threads); }
 int dh_lone_room(int list_cap, int threads) { return lone_room(list_cap, threads); }
 int dh_lone_regs(int threads) { return lone_regs(threads); }
+int dh_lone_edge_warp(int threads) { return lone_edge_warp(threads); }
 
 // Walks every CTA's run of tiles the way the fused indexer's producer does (tile_run, tile_row_at,
 // then tile_segment row after row) and adds, for every (row, row-local tile) the CTAs visit, one to

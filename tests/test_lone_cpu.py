@@ -68,3 +68,15 @@ def test_a_warp_holds_its_share_of_what_a_guess_admits(dh, threads, k, length):
     share, each = rank * length / n / warps, length / n / warps
     deviation = (rank * each ** 2 + share) ** 0.5
     assert share + 3.5 * deviation <= dh.dh_lone_segment(6144, threads)
+
+
+@pytest.mark.parametrize("start", [0, 1, 2, 3])
+def test_a_short_row_fits_whole_wherever_it_starts(dh, start):
+    """... and rows that are not 16-byte aligned: inner granule i of a row lies with warp i % 256 // 32, the two that its ends
+    cut through with the edge warp."""
+    for length in range(4096, 4064, -1):
+        first = (4 - start) % 4
+        inner, last = divmod(length - first, 4)
+        count = [sum(4 for i in range(inner) if i % 256 // 32 == w) for w in range(8)]
+        count[dh.dh_lone_edge_warp(256)] += first + last
+        assert sum(count) == length and max(count) <= dh.dh_lone_segment(2560, 256)
