@@ -40,9 +40,10 @@ __global__ void publish_kernel(uint32_t* flag, uint32_t epoch) {
   st_release_sys(flag, epoch);
 }
 
-// One cluster per row, one CTA per shard (see merge_row).
+// One cluster per row, one CTA per shard (see merge_row). Two CTAs per SM: with 4 lists a row their shared memory allows it (200
+// rows 49.6 us with one, 30.4 with two).
 template <int NT>
-__global__ void __launch_bounds__(NT, 1) merge2048_kernel(const MergeSrc src, int G, int B,
+__global__ void __launch_bounds__(NT, 2) merge2048_kernel(const MergeSrc src, int G, int B,
                                                          int32_t* __restrict__ out_idx_all,
                                                          uint32_t* __restrict__ out_key_all, uint32_t* status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -252,6 +252,16 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
 // ---------------------------------------------------------------------------------------------
 // Shared-memory control block (one per CTA; rank 0's counters are the cluster-wide ones).
 // ---------------------------------------------------------------------------------------------
+// Where a finish writes: the row's output, its status word, page table (NULL: none) and the offset of its indices
+struct FinishTo {
+  int32_t* out_idx;
+  uint32_t* out_key;
+  uint32_t* status;
+  const int32_t* page;
+  uint32_t out_base, out_slots;
+  int32_t idx_offset;
+  uint32_t need;  // candidates that win
+};
 struct Ctrl {
   uint4 fin;  // (finish) the threshold bin: smallest and largest value of the digit's field, elements above, in it
   // cluster-wide allocation counters, meaningful in rank 0 only (targets of remote atomics)
@@ -301,6 +311,7 @@ struct Ctrl {
   const int32_t* row_page;  // the row's page table (or NULL) and the offset of its indices
   int32_t row_idx_offset;
   uint64_t small[kSmall];
+  FinishTo to;  // (finish: rows with many copies of the threshold)
 #ifdef FFTOPK_CHECKED
   uint32_t* status_ptr;  // the call's status word, for checks in code that has no other way to it
 #endif
@@ -728,14 +739,8 @@ __device__ __forceinline__ uint4 finish_pick(uint32_t hist /* shared address */,
 // them, 32 candidates at a time, slots by ballot. (A slot-allocating atomic per warp serialised on the one
 // counter - 30 cycles per warp -, and slots by thread, from a scan over the lanes, scattered every store over 32
 // lines.) A threshold bin that is not taken whole holds a handful of candidates: those take an atomic.
-struct FinishOut {
+struct FinishOut : FinishTo {
   Ctrl* ctrl;
-  int32_t* out_idx;
-  uint32_t* out_key;
-  uint32_t* status;
-  const int32_t* page;
-  uint32_t out_base, out_slots;
-  int32_t idx_offset;
 };
 // Rank by vote the `cnt` candidates set aside: warp i takes candidate i, the lanes compare it with the candidates j (32
 // per step); the number of larger ones is candidate i's rank, and the best need2 go behind the
@@ -769,11 +774,11 @@ __device__ __forceinline__ void rank_undecided(const FinishOut& o, uint32_t cert
 }
 
 template <int NT, bool kTrackMin, class Src, class V, class Field>
-__device__ __forceinline__ void finish_output(const Src src, const FinishOut o, uint32_t need_total, uint32_t need2, uint32_t cnt,
-                                              bool all_bin, V wthr, V uthr, Field&& field) {
+__device__ __forceinline__ void finish_output(const Src src, const FinishOut o, uint32_t need2, uint32_t cnt, bool all_bin, V wthr, V uthr,
+                                              Field&& field) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  Ctrl* ctrl = o.ctrl;
+  Ctrl* const ctrl = o.ctrl;
   const uint32_t small_s = smem_u32(ctrl->small), small_n = smem_u32(&ctrl->small_n);
   const unsigned lt = (1u << lane) - 1u;
   uint32_t n = 0u;
@@ -840,25 +845,22 @@ __device__ __forceinline__ void finish_output(const Src src, const FinishOut o, 
   {
     // every certain winner took exactly one slot, every undecided candidate was set aside
     __syncthreads();
-    const uint32_t want_w = all_bin ? need_total : need_total - need2;
+    const uint32_t want_w = all_bin ? o.need : o.need - need2;
     if (tid == 0) {
       if (set_w != want_w) check_fail(10, set_w, want_w, o.status);
       if (!all_bin && ctrl->small_n != cnt) check_fail(11, ctrl->small_n, cnt, o.status);
     }
   }
 #endif
-  if (!all_bin) rank_undecided<NT, kTrackMin>(o, need_total - need2, need2, cnt);
+  if (!all_bin) rank_undecided<NT, kTrackMin>(o, o.need - need2, need2, cnt);
 }
 
 // More copies of one key than can be ranked, the threshold among them: `need` candidates are still to be taken from
 // those with key `key` and - `more` of them - larger ones. Rounds over the inverted indices under the key, then the
-// output. Out of line: rows with thousands of copies of one value come here, and the others
-// do not carry its registers and instructions. Returns false if the threshold is a key above `key` after all.
+// output. Returns false if the threshold is a key above `key` after all.
 template <int NT, bool kTrackMin, class Src>
-__device__ __noinline__ bool finish_copies(const Src passed, const FinishOut passed_out, uint32_t need_total, uint32_t need, uint32_t key,
-                                           bool more, int idx_bits, uint32_t* hist) {
-  const Src src = passed;  // (out of the stack, into registers)
-  const FinishOut o = passed_out;
+__device__ __forceinline__ bool finish_copies(const Src src, const FinishOut& o, uint32_t need, uint32_t key, bool more, int idx_bits,
+                                              uint32_t* hist) {
   const int tid = threadIdx.x;
   const uint32_t hist_s = smem_u32(hist);
   uint32_t lo = inverted_index_floor(idx_bits), cap = 0xffffffffu;
@@ -884,7 +886,7 @@ __device__ __noinline__ bool finish_copies(const Src passed, const FinishOut pas
     const uint32_t t_lo = dg.bin_low(f.x), t_hi = dg.bin_high(f.x, cap);
     if (cnt == need2 || cnt <= (uint32_t)kSmall) {
       const uint64_t k = (uint64_t)key << 32, below = (k | t_lo) - 1ull;
-      finish_output<NT, kTrackMin>(src, o, need_total, need2, cnt, cnt == need2, cnt == need2 ? below : k | t_hi, below,
+      finish_output<NT, kTrackMin>(src, o, need2, cnt, cnt == need2, cnt == need2 ? below : k | t_hi, below,
                                    [](uint64_t c) { return c; });
       return true;
     }
@@ -895,6 +897,111 @@ __device__ __noinline__ bool finish_copies(const Src passed, const FinishOut pas
   }
   if (tid == 0 && o.status) atomicOr(o.status, 2u);
   return true;
+}
+
+// What the rounds over the keys (finish_rounds) do when they have come down to one key. Rows with thousands of copies of one value
+// do; the others should not carry the registers and instructions for them, so that is a call out of line:
+//   kCopiesRest   the last thing the finish does. Kernels of 64 registers a thread spilled more around a call that the rounds go
+//                 on with than for all the rest: the throughput plan's with several CTAs per row 196 bytes instead of 64, its calls
+//                 3 to 9 % slower (12 rows of 250K 4.58 / 4.32 us, bf16 16 of 128K 3.95 / 3.6); the merge needed 92 registers
+//                 instead of 64 (200 rows of 4 lists 49.6 / 30.4); short rows with 256 threads 39.6 / 35.8 (2,048 of 4K).
+//   kCopiesBack   the rounds go on if the threshold is a larger key after all. With 128 registers a thread nothing spills,
+//                 and it is the rest that costs: one row of 96K 10.54 / 10.46, 7 of 1M 18.6 / 18.4, warm 4 of 200K 9.15 / 9.02.
+//   kCopiesHere   inside the former
+enum CopiesWay : int { kCopiesRest = 0, kCopiesBack = 1, kCopiesHere = 2 };
+template <int NT, bool kTrackMin, int kCopies, class Src>
+__device__ __forceinline__ void finish_rounds(const Src src, const FinishOut o, uint32_t need, uint32_t lo, uint32_t cap, uint32_t focus,
+                                              uint32_t known_total, int idx_bits, uint32_t* hist, bool hist_clear);
+// (both find the output in ctrl->to, left there by one thread; the source comes out of the stack, into registers)
+template <int NT, bool kTrackMin, class Src>
+__device__ __noinline__ bool finish_copies_back(const Src passed, Ctrl* ctrl, uint32_t need, uint32_t lo, uint32_t cap, int idx_bits,
+                                                uint32_t* hist) {
+  const Src src = passed;
+  __syncthreads();
+  return finish_copies<NT, kTrackMin>(src, FinishOut{ctrl->to, ctrl}, need, lo, cap > lo, idx_bits, hist);
+}
+template <int NT, bool kTrackMin, class Src>
+__device__ __noinline__ void finish_copies_rest(const Src passed, Ctrl* ctrl, uint32_t need, uint32_t lo, uint32_t cap, int idx_bits,
+                                                uint32_t* hist) {
+  const Src src = passed;
+  __syncthreads();
+  finish_rounds<NT, kTrackMin, kCopiesHere>(src, FinishOut{ctrl->to, ctrl}, need, lo, cap, lo, 0u, idx_bits, hist, false);
+}
+
+// The rounds over the keys, [lo, cap] with a focus, and the output: see cta_finish. known_total: not 0 for candidates that
+// need no round.
+template <int NT, bool kTrackMin, int kCopies, class Src>
+__device__ __forceinline__ void finish_rounds(const Src src, const FinishOut o, uint32_t need, uint32_t lo, uint32_t cap, uint32_t focus,
+                                              uint32_t known_total, int idx_bits, uint32_t* hist, bool hist_clear) {
+  const int tid = threadIdx.x;
+  const uint32_t hist_s = smem_u32(hist);
+  // Only the threshold is determined by the rounds; nothing is written yet.
+  // Outcome: the threshold bin, keys [t_lo, t_hi]. Everything above it wins; of the
+  // bin itself either everything wins (all_bin) or, when it holds <= kSmall candidates, the best
+  // `need2` of them, found by ranking.
+  uint32_t t_lo = lo, t_hi = cap;
+  uint32_t need2 = need, cnt = known_total;
+  bool all_bin = false, found = false;
+  if (known_total != 0u) {
+    // exactly as many candidates as are wanted, or so few that they are ranked directly
+    all_bin = known_total == need;
+    found = true;
+    __syncthreads();  // (as in a round: what the caller has read through ctrl may be overwritten from here on)
+  }
+  for (int round = 0; round < 8 && !found; ++round) {
+    if (lo == focus) {  // one key left, or bounded by
+      if constexpr (kCopies != kCopiesHere) {
+        if (tid == 0) o.ctrl->to = o;
+      }
+      if constexpr (kCopies == kCopiesRest) {
+        finish_copies_rest<NT, kTrackMin>(src, o.ctrl, need, lo, cap, idx_bits, hist);
+        return;
+      } else if constexpr (kCopies == kCopiesBack) {
+        if (finish_copies_back<NT, kTrackMin>(src, o.ctrl, need, lo, cap, idx_bits, hist)) return;
+      } else {
+        if (finish_copies<NT, kTrackMin>(src, o, need, lo, cap > lo, idx_bits, hist)) return;
+      }
+      ++lo;
+      focus = cap;
+      hist_clear = false;
+    }
+    const KeyDigit dg = make_key_digit(lo, focus);
+    if (!hist_clear) {
+      __syncthreads();
+      for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
+      __syncthreads();
+    }
+    const uint32_t span = cap - lo;
+    src.for_each_key([&](const uint32_t (&k)[kWalk]) {
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) red_shared_inc_if(hist_s + dg.of(k[u]) * 4u, k[u], k[u] - lo, span);
+    });
+    __syncthreads();
+    FFTOPK_MARK(16);
+    const uint4 f = finish_pick<NT>(hist_s, need, o.ctrl);
+    FFTOPK_MARK(17);
+    if (f.x == kNoBin) break;
+    cnt = f.z;
+    need2 = need - f.y;
+    t_lo = dg.bin_low(f.x);
+    t_hi = dg.bin_high(f.x, cap);
+    all_bin = cnt == need2;
+    found = all_bin || cnt <= (uint32_t)kSmall;
+    if (!found) {
+      lo = t_lo;
+      cap = focus = t_hi;
+      need = need2;
+      hist_clear = false;
+    }
+  }
+  FFTOPK_MARK(30);
+  if (!found) {
+    if (tid == 0 && o.status) atomicOr(o.status, 2u);
+    return;
+  }
+  const uint32_t below = t_lo ? t_lo - 1u : 0u;  // (an empty slot has key 0)
+  finish_output<NT, kTrackMin>(src, o, need2, cnt, all_bin, all_bin ? below : t_hi, below,
+                               [](uint64_t c) { return (uint32_t)(c >> 32); });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -924,7 +1031,7 @@ __device__ __noinline__ bool finish_copies(const Src passed, const FinishOut pas
 // Inlined, and the source comes by value: as a call, source and arguments went through every thread's
 // stack, and beside 200 KB of shared memory L1 has no room for the stacks of 1024 threads - each access
 // was a round trip to L2 (the passes over the candidates took 1.4 and 2 to 4 us instead of 0.4 and 0.7).
-template <int NT, class Src, bool kTrackMin = false>
+template <int NT, class Src, bool kTrackMin = false, int kCopies = kCopiesRest>
 __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_t klo, uint32_t kcap, uint32_t kfocus,
                            int idx_bits, uint32_t* hist /* >= kFinishBins words */, Ctrl* ctrl, int32_t* out_idx,
                            uint32_t* out_key, uint32_t out_base, uint32_t out_slots /* k of the row */,
@@ -966,67 +1073,10 @@ __device__ __forceinline__ void cta_finish(const Src src, uint32_t need, uint32_
     __syncthreads();  // the scratch words are about to be cleared as the histogram
     FFTOPK_MARK(31);
   }
-  // ---- rounds: only the threshold is determined here; nothing is written yet ---------------------
-  // Outcome: the threshold bin, keys [t_lo, t_hi]. Everything above it wins; of the
-  // bin itself either everything wins (all_bin) or, when it holds <= kSmall candidates, the best
-  // `need2` of them, found by ranking.
-  const FinishOut o{ctrl, out_idx, out_key, status, page, out_base, out_slots, idx_offset};
-  const uint32_t need_total = need;
-  uint32_t t_lo = klo, t_hi = kcap;
-  uint32_t need2 = need, cnt = known_total;
-  bool all_bin = false, found = false;
-  if (known_total != 0u && known_total >= need && (known_total == need || known_total <= (uint32_t)kSmall)) {
-    // exactly as many candidates as are wanted, or so few that they are ranked directly
-    all_bin = known_total == need;
-    found = true;
-    __syncthreads();  // (as in a round: what the caller has read through ctrl may be overwritten from here on)
-  }
-  uint32_t lo = klo, cap = kcap;
-  uint32_t focus = kfocus < klo || kfocus > kcap ? kcap : kfocus;
-  for (int round = 0; round < 8 && !found; ++round) {
-    if (lo == focus) {  // one key left, or bounded by
-      if (finish_copies<NT, kTrackMin>(src, o, need_total, need, lo, cap > lo, idx_bits, hist)) return;
-      ++lo;
-      focus = cap;
-      hist_clear = false;
-    }
-    const KeyDigit dg = make_key_digit(lo, focus);
-    if (!hist_clear) {
-      __syncthreads();
-      for (int b = tid; b < kFinishBins; b += NT) hist[b] = 0u;
-      __syncthreads();
-    }
-    const uint32_t span = cap - lo;
-    src.for_each_key([&](const uint32_t (&k)[kWalk]) {
-#pragma unroll
-      for (int u = 0; u < kWalk; ++u) red_shared_inc_if(hist_s + dg.of(k[u]) * 4u, k[u], k[u] - lo, span);
-    });
-    __syncthreads();
-    FFTOPK_MARK(16);
-    const uint4 f = finish_pick<NT>(hist_s, need, ctrl);
-    FFTOPK_MARK(17);
-    if (f.x == kNoBin) break;
-    cnt = f.z;
-    need2 = need - f.y;
-    t_lo = dg.bin_low(f.x);
-    t_hi = dg.bin_high(f.x, cap);
-    all_bin = cnt == need2;
-    found = all_bin || cnt <= (uint32_t)kSmall;
-    if (!found) {
-      lo = t_lo;
-      cap = focus = t_hi;
-      need = need2;
-      hist_clear = false;
-    }
-  }
-  FFTOPK_MARK(30);
-  if (!found) {
-    if (tid == 0 && status) atomicOr(status, 2u);
-    return;
-  }
-  const uint32_t below = t_lo ? t_lo - 1u : 0u;  // (an empty slot has key 0)
-  finish_output<NT, kTrackMin>(src, o, need_total, need2, cnt, all_bin, all_bin ? below : t_hi, below,
-                               [](uint64_t c) { return (uint32_t)(c >> 32); });
+  const bool few = known_total != 0u && known_total >= need && (known_total == need || known_total <= (uint32_t)kSmall);
+  const FinishOut o{{out_idx, out_key, status, page, out_base, out_slots, idx_offset, need}, ctrl};
+  finish_rounds<NT, kTrackMin, kCopies>(src, o, need, klo, kcap, kfocus < klo || kfocus > kcap ? kcap : kfocus, few ? known_total : 0u,
+                                      idx_bits, hist, hist_clear);
 }
 
 // The finish of a lone CTA: the candidates' keys are in registers, round 0's histogram (`hist`, with

@@ -1003,7 +1003,7 @@ __device__ __forceinline__ bool finish_given_candidates(const SelectParams& p, c
     }
     __syncthreads();
     const RowOutput ro = row_output(p, row, cx.k);
-    const FinishOut o{cx.ctrl, ro.idx, ro.key, p.status, nullptr, 0u, cx.k, p.idx_offset};
+    const FinishOut o{{ro.idx, ro.key, p.status, nullptr, 0u, cx.k, p.idx_offset, cx.k}, cx.ctrl};
     lone_finish<NT, R, true>(cands, o, cx.k, lowkey, focus, 32 - __clz(len - 1), cx.hist0);
     __syncthreads();
   }
@@ -1478,11 +1478,12 @@ __device__ __forceinline__ void select_row(const SelectParams& p) {
   if (rank == 0 && mode == kModeGather && extra > 0) FFTOPK_ROUTE(kRouteBeyond);
   if (mode == kModeGather) {
     if constexpr (kLone) {
-      const FinishOut o{ctrl, out_idx, out_key, p.status, cx.page, 0u, K, cx.idx_offset};
+      const FinishOut o{{out_idx, out_key, p.status, cx.page, 0u, K, cx.idx_offset, K}, ctrl};
       lone_finish<NT, kLoneRegs, kWarm>(held, o, K, lowkey, focus_key, idx_bits, fin_hist);
     } else {
       const RegionCands<NT> src{smem_u32(cx.cand), smem_u32(ctrl->cnt_of), region, C, extra};
-      cta_finish<NT, RegionCands<NT>, kWarm>(src, K, lowkey, 0xffffffffu, focus_key, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
+      constexpr int kCopies = NT == 512 && kForm == kRoomyForm ? kCopiesBack : kCopiesRest;  // (128 registers a thread, or 64)
+      cta_finish<NT, RegionCands<NT>, kWarm, kCopies>(src, K, lowkey, 0xffffffffu, focus_key, idx_bits, fin_hist, ctrl, out_idx, out_key, 0u,
                                              K, cx.idx_offset, p.status, cx.page, total, true);
     }
     // This call's threshold for the next one: the smallest key the finish let win (the row's k-th
