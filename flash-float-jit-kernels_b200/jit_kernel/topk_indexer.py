@@ -52,8 +52,9 @@ def _after_launch(device: torch.device, what: str) -> None:
 # most of it was Python: two rounds of checks, device objects compared with each other, a device context
 # entered and left, a stream object. Tensor.get_device() is a plain integer (-1 off the GPU), the context is entered only where
 # the current device is another one, and the stream handle is asked for by itself.
-_current_device = torch._C._cuda_getDevice
-_current_stream = torch._C._cuda_getCurrentRawStream
+# (Both names are private, and a torch without CUDA has neither: the public calls do the same, and cost more.)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", lambda idx: torch.cuda.current_stream(idx).cuda_stream)
 _status_ptrs: dict[int, int] = {}
 
 
