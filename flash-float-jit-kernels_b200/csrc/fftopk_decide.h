@@ -247,6 +247,17 @@ FFTOPK_DECIDE_HD int lone_room_weighed(int list_cap, int threads) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Rows that are asked for in L2 ahead of time are asked for up to a length that may be out of date, so up to L: more than the call
+// reads, and more than a caller has to have. The request is made only where B rows of L elements lie inside the allocation
+// that the first of them lies in ([base, base + size), addresses in bytes).
+// ---------------------------------------------------------------------------------------------
+FFTOPK_DECIDE_HD bool rows_inside(uint64_t score, int64_t row_stride, int32_t B, int64_t L, int element_bytes, uint64_t base, uint64_t size) {
+  if (B < 1 || L < 0 || row_stride < 0 || score < base || score - base > size) return false;
+  const int64_t room = (int64_t)((size - (score - base)) / (uint64_t)element_bytes);
+  return L <= room && (B == 1 || row_stride <= (room - L) / (B - 1));
+}
+
+// ---------------------------------------------------------------------------------------------
 // Digit rule of a finish round over a field's range [lo, cap]: digit(v) = min((v - lo) >>
 // shift, kFinishBins - 1). The shift is chosen so that [lo, focus] spreads over the bins below the
 // last one; everything above `focus` (cap >= focus >= lo) lands in the last bin. With focus == cap

@@ -42,6 +42,7 @@
 //   FFTOPK_KSMALL           undecided candidates ranked by votes (256)
 //   FFTOPK_TRACE            phase timestamps of block 0 (changes no result)
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -1637,8 +1638,11 @@ Tuning tuning_snapshot() {
   return g_tuning;
 }
 
+using AddressRangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);  // cuMemGetAddressRange
+
 struct DeviceInfo {
   DeviceOnce once;
+  AddressRangeFn address_range = nullptr;
   int sm_count = 0;
   int smem_optin = 0;
   int cc_major = 0;
@@ -1719,6 +1723,11 @@ int init_device(DeviceInfo& d, int dev) {
   if (prop.major < 10) return FFTOPK_EDEVICE;
   const int rc = setup_kernels(d.smem_optin);
   if (rc) return rc;
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+    d.address_range = reinterpret_cast<AddressRangeFn>(fn);
+  (void)cudaGetLastError();  // (without it no row is asked for ahead of time)
   // can a 16-CTA cluster with the latency-mode shared-memory footprint be co-scheduled, and how
   // many clusters of 16 / of 8 CTAs does the device hold at once? (A cluster lives inside one
   // GPC, so fewer 16-CTA clusters fit than SM count / 16: a batch with more rows than that would
@@ -1765,6 +1774,17 @@ int device_info(DeviceInfo** out) {
   if (rc) return rc;
   *out = &d;
   return 0;
+}
+
+// Whether all rows of a call lie inside one allocation, as far as L. A query of the driver on the host (an eager call
+// takes 9.14 us of host time with it, 9.10 without), which fails for memory that it knows nothing about.
+bool rows_allocated(const DeviceInfo& d, const SelectCall& c, int element_bytes) {
+  if (d.address_range == nullptr) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const uint64_t score = reinterpret_cast<uint64_t>(c.score);
+  if (d.address_range(&base, &size, (CUdeviceptr)score) != CUDA_SUCCESS) return false;
+  return rows_inside(score, c.row_stride, c.B, c.L, element_bytes, (uint64_t)base, (uint64_t)size);
 }
 
 struct Plan {
@@ -1918,7 +1938,11 @@ int launch_select(const SelectCall& c) {
   // of 256K 10.7 / 10.7. Rows in L2 already: 1M 13.9 / 13.9. (A warm start waits for little else than the length, which
   // the request reads as well: 4 rows of 200K in L2 8.48 / 8.65, so it does not ask.)
   const int64_t row_bytes = c.L * (half_width ? 2 : 4);
-  p.prefetch = c.may_overlap && !overlap && !c.row_starts && row_bytes > kPrefetchRow && c.B * row_bytes <= kPrefetchBytes ? 1 : 0;
+  // (the rows have to be there as far as L: see rows_inside)
+  p.prefetch = c.may_overlap && !overlap && !c.row_starts && row_bytes > kPrefetchRow && c.B * row_bytes <= kPrefetchBytes &&
+                       rows_allocated(*d, c, half_width ? 2 : 4)
+                   ? 1
+                   : 0;
   p.src_page_table = c.src_page_table;
   p.src_stride = c.src_stride;
   p.cu_seqlens_q = c.cu_seqlens_q;

@@ -67,7 +67,8 @@ int fftopk_last_cuda_error(void);
  *   row_stride   elements between consecutive rows (>= 0)
  *   B, L         rows and padded row length; B == 0 is a no-op
  *   lengths      device, int32 [B]; valid elements of row b. Values are clamped to
- *                [0, L - row_start]
+ *                [0, L - row_start]. Nothing behind a row's valid elements is read; where all rows
+ *                lie in one allocation as far as L, it may be brought into L2
  *   row_starts   device, int32 [B] or NULL; first valid element of row b
  *                (reference: topk_indexer_radix.cu:858, 541-542)
  *   out_idx      device, int32 [B, 2048]. Row b receives, in unspecified order, the indices
@@ -384,9 +385,9 @@ int fftopk_plan(int32_t B, int64_t L, int32_t plan[6]);
 /*
  * Back-to-back calls. Every selection launch is a programmatic dependent launch and lets its own
  * dependents become resident at once. By default the kernel executes griddepcontrol.wait before
- * its first access to global memory: plain stream order - the kernel in front of it has completed
+ * it reads what its result depends on: plain stream order - the kernel in front of it has completed
  * and its writes are visible - and only the launch latency of a call hides behind the call in
- * front of it. Overlap (off by default; process-wide): with enable = 1 the kernel does NOT wait,
+ * front of it, and, for long rows, a request to bring them into L2. Overlap (off by default; process-wide): with enable = 1 the kernel does NOT wait,
  * so when two selection kernels follow each other on a stream the second starts filling SMs as
  * soon as CTAs of the first exit (short rows finish early), instead of waiting for the whole
  * grid. Enable it only if (1) no kernel that precedes a call on the

@@ -106,6 +106,9 @@ uint64_t dh_single_key_floor(uint64_t lo, int idx_bits) { return (lo & 0xfffffff
 int dh_lone_segment(int list_cap, int threads) { return lone_segment(list_cap, threads); }
 int dh_lone_room(int list_cap, int threads) { return lone_room(list_cap, threads); }
 int dh_lone_regs(int threads) { return lone_regs(threads); }
+int dh_rows_inside(uint64_t score, int64_t row_stride, int32_t B, int64_t L, int element_bytes, uint64_t base, uint64_t size) {
+  return rows_inside(score, row_stride, B, L, element_bytes, base, size) ? 1 : 0;
+}
 int dh_lone_edge_warp(int threads) { return lone_edge_warp(threads); }
 
 // Walks every CTA's run of tiles the way the fused indexer's producer does (tile_run, tile_row_at,
