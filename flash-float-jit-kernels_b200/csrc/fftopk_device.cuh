@@ -907,24 +907,25 @@ __device__ __forceinline__ bool finish_copies(const Src src, const FinishOut& o,
 //                 instead of 64 (200 rows of 4 lists 49.6 / 30.4); short rows with 256 threads 39.6 / 35.8 (2,048 of 4K).
 //   kCopiesBack   the rounds go on if the threshold is a larger key after all. With 128 registers a thread nothing spills,
 //                 and it is the rest that costs: one row of 96K 10.54 / 10.46, 7 of 1M 18.6 / 18.4, warm 4 of 200K 9.15 / 9.02.
+//                 (With the output passed through shared memory here too, one of 96K 10.54.)
 //   kCopiesHere   inside the former
 enum CopiesWay : int { kCopiesRest = 0, kCopiesBack = 1, kCopiesHere = 2 };
 template <int NT, bool kTrackMin, int kCopies, class Src>
 __device__ __forceinline__ void finish_rounds(const Src src, const FinishOut o, uint32_t need, uint32_t lo, uint32_t cap, uint32_t focus,
                                               uint32_t known_total, int idx_bits, uint32_t* hist, bool hist_clear);
-// (both find the output in ctrl->to, left there by one thread; the source comes out of the stack, into registers)
+// (what is passed by value comes out of the stack, into registers)
 template <int NT, bool kTrackMin, class Src>
-__device__ __noinline__ bool finish_copies_back(const Src passed, Ctrl* ctrl, uint32_t need, uint32_t lo, uint32_t cap, int idx_bits,
-                                                uint32_t* hist) {
+__device__ __noinline__ bool finish_copies_back(const Src passed, const FinishOut passed_out, uint32_t need, uint32_t lo, uint32_t cap,
+                                                int idx_bits, uint32_t* hist) {
   const Src src = passed;
-  __syncthreads();
-  return finish_copies<NT, kTrackMin>(src, FinishOut{ctrl->to, ctrl}, need, lo, cap > lo, idx_bits, hist);
+  const FinishOut o = passed_out;
+  return finish_copies<NT, kTrackMin>(src, o, need, lo, cap > lo, idx_bits, hist);
 }
 template <int NT, bool kTrackMin, class Src>
 __device__ __noinline__ void finish_copies_rest(const Src passed, Ctrl* ctrl, uint32_t need, uint32_t lo, uint32_t cap, int idx_bits,
                                                 uint32_t* hist) {
   const Src src = passed;
-  __syncthreads();
+  __syncthreads();  // (ctrl->to, left there by one thread)
   finish_rounds<NT, kTrackMin, kCopiesHere>(src, FinishOut{ctrl->to, ctrl}, need, lo, cap, lo, 0u, idx_bits, hist, false);
 }
 
@@ -950,14 +951,12 @@ __device__ __forceinline__ void finish_rounds(const Src src, const FinishOut o, 
   }
   for (int round = 0; round < 8 && !found; ++round) {
     if (lo == focus) {  // one key left, or bounded by
-      if constexpr (kCopies != kCopiesHere) {
-        if (tid == 0) o.ctrl->to = o;
-      }
       if constexpr (kCopies == kCopiesRest) {
+        if (tid == 0) o.ctrl->to = o;
         finish_copies_rest<NT, kTrackMin>(src, o.ctrl, need, lo, cap, idx_bits, hist);
         return;
       } else if constexpr (kCopies == kCopiesBack) {
-        if (finish_copies_back<NT, kTrackMin>(src, o.ctrl, need, lo, cap, idx_bits, hist)) return;
+        if (finish_copies_back<NT, kTrackMin>(src, o, need, lo, cap, idx_bits, hist)) return;
       } else {
         if (finish_copies<NT, kTrackMin>(src, o, need, lo, cap > lo, idx_bits, hist)) return;
       }
