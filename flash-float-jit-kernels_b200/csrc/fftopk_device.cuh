@@ -1117,8 +1117,10 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
       clear();
       const KeyDigit dg = make_key_digit(lo, cap);
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        if (i * 32 < held.wn) red_shared_inc_if(hist_s + dg.of(held.key[i]) * 4u, held.key[i], held.key[i] - lo, cap - lo);
+      for (int i = 0; i < R; ++i) {
+        if (i * 32 >= held.wn) break;
+        red_shared_inc_if(hist_s + dg.of(held.key[i]) * 4u, held.key[i], held.key[i] - lo, cap - lo);
+      }
       __syncthreads();
       f = pick(dg, f.w, cap, (uint32_t)kSmall);
       lo = f.y + 1u;
@@ -1133,7 +1135,8 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
         const KeyDigit dg = make_key_digit(ilo, icap);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-          if (i * 32 < held.wn && held.key[i] == key) {
+          if (i * 32 >= held.wn) break;
+          if (held.key[i] == key) {
             const uint32_t v = ~lds32(held.seg + (uint32_t)(i * 32 + lane) * 4u);
             if (v - ilo <= icap - ilo) red_shared_inc(hist_s + dg.of(v) * 4u);
           }
@@ -1146,7 +1149,8 @@ __device__ __forceinline__ void lone_finish(RegSegCands<NT, R>& held, const Fini
       if (f.z == kMany) f.z = kNoBin;  // (one index many times over: not a list of the library's making)
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        if (i * 32 < held.wn && held.key[i] == key) {
+        if (i * 32 >= held.wn) break;
+        if (held.key[i] == key) {
           if (~lds32(held.seg + (uint32_t)(i * 32 + lane) * 4u) < ilo) held.key[i] = 0u;
         }
       }
