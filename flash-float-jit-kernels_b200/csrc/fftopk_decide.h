@@ -75,7 +75,8 @@ FFTOPK_DECIDE_HD uint32_t sample_piece_start(uint32_t gi, uint32_t piece, int lo
 // How much of a row is sampled: 2^log batches of 8K elements. With m of them expected among the k largest,
 // the rank bound admits about k (1 + 5 / sqrt(m) + 14 / m) elements, so the sample grows with the row:
 // 16K elements beyond 256K, and twice as many each time a row beyond 4M (2M for k beyond 2048) doubles. For
-// k = 2048 m stays above 8, and no more than 9.3K elements are expected to pass. (With 16K elements for rows of any length, a row beyond
+// k = 2048 m stays above 8, and no more than 9.3K elements are expected to pass (a cluster's buffer holds 16K, a lone CTA's list
+// 10K or 12K). (With 16K elements for rows of any length, a row beyond
 // 10M passed more than a cluster's buffer holds and went through three full-histogram rounds: one row of
 // 12M 273 us instead of 43, of 32M 760 instead of 193. With twice the sample, from 2M on, 12M took 48 us.)
 FFTOPK_DECIDE_HD int sample_log_batches(int len, uint32_t k) {

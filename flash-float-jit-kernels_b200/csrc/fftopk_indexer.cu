@@ -6,9 +6,9 @@
 // the step (README.md:24) - so there is no reference counterpart; this is the step in front of the
 // hot path, fused with it.
 //
-// Producer kernel, one CTA per (row, slice of key tiles), two CTAs per SM, 320 threads in three roles:
+// Producer kernel, two CTAs per SM, each with an equal run of the tiles of all rows, 320 threads in three roles:
 //   warp 0      one thread issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle, no multicast):
-//               the row's q once (64 heads x 128), then key tiles of 128 keys x 128 through a ring
+//               a row's q (64 heads x 128), then its key tiles of 128 keys x 128 through a ring
 //               of shared-memory stages guarded by full / empty mbarriers;
 //   warp 1      allocates 256 TMEM columns; one thread issues, per tile, eight tcgen05.mma of
 //               K=16 (bf16; four of K=32 for fp8), M=128 keys, N=64 heads, that accumulate
@@ -35,9 +35,9 @@
 // What bounds the producer is reading the keys, as long as nothing interrupts the stream. Until the list was
 // finished by the selector, a CTA drained its pipeline at the end of every row's segment, counted its tiles off with a fence
 // and an atomic, and the row's last CTA put its own tiles off for the finish; and every warp waited for an atomic
-// per 32 keys with a hit. us per call, then -> now: 64 ragged rows of up to 128K, bf16 218-222 -> 171 (1.07 GB of keys: 6.3 TB/s), fp8
-// 133-151 -> 98; 42 of 150K, fp8 113 -> 78; one row of 128K, fp8 12.2 -> 10.3; one of 1M, bf16 50.4 -> 49.5; without guesses, 8 rows of 64K
-// 23.6 -> 23.1.
+// per 32 keys with a hit. us per call, then -> now: 64 ragged rows of up to 128K, bf16 218-222 -> 168 (1.07 GB of keys: 6.3 TB/s), fp8
+// 133-151 -> 97; one row of 128K, fp8 12.2 -> 10.4; one of 1M, bf16 50.4 -> 49.1; without guesses, 8 rows of 64K
+// 26.3 -> 25.0. (It spills 24 bytes per row segment, none per tile.)
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -341,8 +341,8 @@ __device__ __noinline__ void indexer_epilogue_segment(const IndexerParams& p, in
 }
 
 // ---- producer --------------------------------------------------------------------------------------
-// Work split. The tiles of all rows, row after row, form one sequence; CTA c takes the c-th run of
-// `quota` consecutive tiles of it (quota = tiles / CTAs, rounded up), so every CTA streams the same
+// Work split. The tiles of all rows, row after row, form one sequence; CTA c takes the c-th run of it,
+// tiles / CTAs of them or one more (tile_run), so every CTA streams the same
 // number of bytes whatever the rows' lengths are, and a run may cover the end of one row, several
 // whole rows and the start of another. The part of a run inside one row is a segment: it has that row's q (one of
 // two places in shared memory in turn) and weights, and the pipeline runs on from one segment into the

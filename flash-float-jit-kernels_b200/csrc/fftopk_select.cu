@@ -22,13 +22,15 @@
 //   4. GATHER + FINISH. They become (key << 32 | ~index) composites on their way into rank 0's shared
 //      memory, where every CTA owns a region; every CTA also tells every other its count, so that
 //      after the one cluster barrier each knows whether the guess held and all but rank 0 leave. Rank 0
-//      finishes: radix rounds over the composites' range, a counting and a writing pass, and the last
-//      <= 256 undecided candidates ranked by votes. A lone CTA keeps its candidates' indices in shared memory and
-//      their keys in registers, and finishes on those (lone_finish). The inverted index in the composite makes equal values resolve to the lower index.
-//      Measured (us per call in a chain of calls on B200, when histograms were exchanged -> with steps 1 to 4
-//      as they are now): B=1, L=96K 12.9 -> 10.0, 1M 15.4 -> 14.1; B=4, L=200K 13.6 -> 10.7; B=64 ragged rows
-//      of up to 128K 17.3 -> 15.4 (calls that may overlap 5.4 -> 4.5, then 3.55); B=2048, one CTA per row, L=32K
-//      132 -> 102 -> 81.0, 8K 106 -> 67 -> 55.3, 4K 62 -> 39.1 (the last figure of each: keys in registers, fewer instructions). What bounds it is no bandwidth but the chain of short phases and the instructions in it.
+//      finishes (cta_finish): radix rounds over the keys in the composites, a counting and a writing pass, and the
+//      last <= 256 undecided candidates ranked by votes. A lone CTA gathers nothing: it keeps its candidates'
+//      indices in shared memory and their keys in registers, and finishes on those (lone_finish). Equal values resolve
+//      to the lower index: votes compare whole composites, and more copies than are ranked go through
+//      rounds over the inverted indices.
+//      Measured (us per call in a chain of calls on B200, when histograms were exchanged -> as it is now):
+//      B=1, L=96K 12.9 -> 10.5, 1M 15.4 -> 14.2 from L2; B=64 ragged rows of up to 128K 20.0 -> 18.0, calls that may
+//      overlap 5.4 -> 3.2; B=2048, one CTA per row, L=32K 132 -> 80.2, 8K 106 -> 54.0, 4K 62 -> 35.8. What bounds it is no
+//      bandwidth but the chain of short phases and the instructions in it.
 //   5. If the guess admitted fewer than k elements, a list overflowed or the threshold bin is
 //      larger than rank 0's buffer (heavy ties, rows of equal values), the cluster falls back to
 //      full histograms over the data: 12 + 12 + 8 key bits, re-reading the shard from L2 each
@@ -1822,19 +1824,17 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
   pl.cluster = c < 1 ? 1 : c;
   // A cluster's CTAs are bound by the instructions their warps issue, and much of that is per warp
   // (scans, searches, address arithmetic): 512 threads do it with half the warps and, one CTA per SM,
-  // twice the registers. Measured, us per call in a chain, 512 / 1024 threads: B=1, L=16K 9.2 / 10.9,
-  // 96K 10.0 / 11.6, 1M 14.9 / 15.9; B=64 ragged rows of up to 128K 15.5 / 15.9. A lone CTA has no
+  // twice the registers. Measured, us per call in a chain, 512 / 1024 threads: B=1, L=16K 9.5 / 10.1,
+  // 96K 10.5 / 11.35, 1M 14.6 / 14.9; B=64 ragged rows of up to 128K 18.5 / 18.5. A lone CTA has no
   // other CTA to share its row with: 1024.
   pl.threads = pl.cluster > 1 ? 512 : 1024;
   pl.list_cap = kLatencyListCap;
   pl.cand_cap = kLatencyCandCap;
   if (rows > d.sm_count) {
     // More rows than SMs: the batch fills the device by itself. One 512-thread CTA per row with
-    // the list of the throughput plan, two CTAs per SM (measured on ragged rows of up to 128K
-    // elements: 29.7 us per call at B=256 and 52.6 us at B=512, against 38.5 / 68.1 us with 1024
-    // threads; a list of 4096 entries split over 32 warps overflowed its segments and sent rows
-    // to the full-histogram path: 78 / 113 us). (The gather buffer is for tunings that ask for more
-    // CTAs per row.)
+    // the list of the throughput plan, two CTAs per SM (ragged rows of up to 128K elements, 512 / 1024 threads:
+    // 22.0 / 25.9 us per call at B=256, 37.2 / 42.5 at B=512; 2,048 rows of 32K 81 / 115). (The gather buffer is for
+    // tunings that ask for more CTAs per row.)
     pl.cluster = 1;
     pl.threads = 512;
     pl.list_cap = kOverlapListCap1;
@@ -1842,7 +1842,7 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
   }
   if (overlap) {
     // Back-to-back calls may overlap: what counts is work per row, not the latency of one call.
-    // Few CTAs per row (less cluster traffic per row), 512 threads and about 110 KB of shared
+    // Few CTAs per row (less cluster traffic per row), 512 threads and 70 KB (one CTA per row) or 115 KB of shared
     // memory so that two CTAs - of different calls - share an SM, and about four calls in flight.
     int ct = floor_pow2(d.sm_count / (4 * rows) > 0 ? d.sm_count / (4 * rows) : 1);
     if (ct < pl.cluster) pl.cluster = ct;
@@ -1856,8 +1856,8 @@ Plan make_plan(const DeviceInfo& d, const Tuning& tn, bool overlap, int B, int64
   }
   if (narrow && pl.cluster == 1 && pl.threads == 512 && L <= kLoneRow256) {
     // Short rows: four CTAs of 256 threads share an SM, each with some 40 KB, and the phases in which one of them has
-    // little to do are the others' time. Measured with 2,048 rows of N(0,1)-like sums, 256 / 512 threads: 4K elements 37 / 49 us,
-    // 8K 48 / 57, 32K 105 / 82; with 70 % zeros 4K 91 / 105, 6K 191 / 131 - rows that may overflow their list stay with 512.
+    // little to do are the others' time. 2,048 rows, 256 / 512 threads: 4K elements 35.9 / 46.9 us, with 70 % zeros
+    // 87 / 90, 6K with zeros 176 / 119 - rows that may overflow their list stay with 512 (8K of N(0,1) 45.9 / 53.8).
     pl.threads = 256;
     pl.list_cap = kLoneListCap256;
   }
